@@ -58,9 +58,11 @@ YeeArgs yee_args(emlab_grid* g) {
     a.pml_cls = g->pml_cls.p;
     a.pml_coef = g->pml_coef.p;
     a.pml_z = g->pml_z.p;
+    a.pml_zi = g->pml_zi.p;
     a.pml_K = g->pml_K;
     a.L = g->cfg.pml_thickness;
     a.dt = g->cfg.courant;
+    a.minus_zero = -0.0f;
     // tile height and z chunks: enough CTAs for ~4 per SM, but at least 8 planes each (the first
     // plane of a chunk is recomputed)
     const int mode = g->tile_rows == 0 ? 64 : g->tile_rows;  // automatic: 64 x 8 pair tiles
@@ -74,7 +76,6 @@ YeeArgs yee_args(emlab_grid* g) {
     zc = std::max(zc, std::min(8, a.nz));
     a.zchunk = zc;
     a.work = g->d_work.p;
-    a.work_base = g->work_base;
     a.wait_polls = wait_limit();
     a.pml_cls_xy = g->pml_cls.p, a.pml_xy = g->pml.p, a.pml_xy_stride = g->pml_stride, a.pml_xy_scene = 0;
     a.items = nullptr, a.n_items = 0, a.scene_xy = nullptr;
@@ -232,7 +233,7 @@ int emlab::upload_pml(emlab_grid* g) {
         int dev = 0, sms = 0;
         EMLAB_CUDA(cudaGetDevice(&dev));
         EMLAB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        const int tys[3] = {4, 8, 16}, per_sm[3] = {4, 2, 1};
+        const int tys[3] = {4, 8, 16}, per_sm[3] = {3, 2, 1};
         for (int t = 0; t < 3; ++t) {
             const std::vector<int4> items = ragged_items(st.z0, st.nx, st.ny, st.nz, tys[t], per_sm[t] * sms);
             EMLAB_REQUIRE(!items.empty(), "stack: no work items");
@@ -253,6 +254,11 @@ int emlab::upload_pml(emlab_grid* g) {
     EMLAB_CUDA(cudaMemcpyAsync(g->pml_coef.p, coef.data(), coef.size() * 4, cudaMemcpyHostToDevice, g->stream));
     EMLAB_CUDA(g->pml_z.alloc(pz.size()));
     EMLAB_CUDA(cudaMemcpyAsync(g->pml_z.p, pz.data(), pz.size(), cudaMemcpyHostToDevice, g->stream));
+    std::vector<unsigned> zi((size_t)c.nz);
+    for (size_t z = 0; z < zi.size(); ++z)
+        zi[z] = (unsigned)pz[z] | (unsigned)pcls[2 * (size_t)S + z] << 8 | (unsigned)pcls[5 * (size_t)S + z] << 16;
+    EMLAB_CUDA(g->pml_zi.alloc(zi.size()));
+    EMLAB_CUDA(cudaMemcpyAsync(g->pml_zi.p, zi.data(), zi.size() * 4, cudaMemcpyHostToDevice, g->stream));
     return EMLAB_OK;
 }
 
@@ -384,9 +390,8 @@ int emlab::reset_monitors(emlab_grid* g) {
 }
 
 // The launches of one sub-step k of a staged chunk: the Yee pass (advancing the field generation),
-// the sources on the new generation, then the per-step monitors. In a graph capture (graph = true)
-// the persistent kernel's ticket counter is reset before the launch and its base is 0. Returns the
-// number of kernel launches.
+// the sources on the new generation, then the per-step monitors. graph: captured, not run. Returns
+// the number of kernel launches.
 namespace {
 uint64_t enqueue_step(emlab_grid* g, int k, bool graph, const float* d_sig, const float4* d_prot,
                       const float4* d_nrot, const float4* d_lrot, const float* d_bl, long long rec, cudaEvent_t ev0,
@@ -401,17 +406,8 @@ uint64_t enqueue_step(emlab_grid* g, int k, bool graph, const float* d_sig, cons
         launch_yee_split(a, g->wide, g->stream);
         launched += 2;
     } else {
-        unsigned long long tickets = 0;
-        bool tma = false;
-        if (g->kernel == EMLAB_KERNEL_FUSED) {
-            if (graph) {
-                cudaMemsetAsync(g->d_work.p, 0, 8, g->stream);
-                a.work_base = 0;
-            }
-            tma = launch_yee_tma(a, g->tma, g->cur, g->wide, g->d_err.p, g->stream, &tickets);
-        }
-        if (graph) g->graph_tickets = tickets;
-        else g->work_base += tickets;
+        const bool tma = g->kernel == EMLAB_KERNEL_FUSED &&
+                         launch_yee_tma(a, g->tma, g->cur, g->wide, g->d_err.p, g->stream);
         if (!tma && g->stack.ragged) g->launch_failed = true;  // no kernel here knows the scenes' cross-sections
         else if (!tma) launch_yee_fused(a, g->wide, g->stream);
         launched += 1;
@@ -485,8 +481,8 @@ int emlab_grid_create(emlab_grid** out) {
         cudaEventCreateWithFlags(&g->stage_done[0], cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&g->stage_done[1], cudaEventDisableTiming) != cudaSuccess ||
         g->d_flag.alloc(1) != cudaSuccess || g->d_err.alloc(1) != cudaSuccess ||
-        cudaMemsetAsync(g->d_err.p, 0, 4, g->stream) != cudaSuccess || g->d_work.alloc(1) != cudaSuccess ||
-        cudaMemsetAsync(g->d_work.p, 0, 8, g->stream) != cudaSuccess) {
+        cudaMemsetAsync(g->d_err.p, 0, 4, g->stream) != cudaSuccess || g->d_work.alloc(2) != cudaSuccess ||
+        cudaMemsetAsync(g->d_work.p, 0, 16, g->stream) != cudaSuccess) {
         delete g;
         return fail(EMLAB_ERR_CUDA, "stream or event creation failed");
     }
@@ -692,7 +688,6 @@ int emlab_grid_step(emlab_grid* g, int count) {
             cudaGraphExec_t& ex = g->graph_exec[slot][g->cur];
             if (!ex) {
                 const int cur0 = g->cur;
-                const unsigned long long base0 = g->work_base;
                 uint64_t launched = 0;
                 EMLAB_CUDA(cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal));
                 cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, g->stream);
@@ -701,7 +696,7 @@ int emlab_grid_step(emlab_grid* g, int count) {
                                              g->nports && g->recording ? k : -1, nullptr, nullptr);
                 cudaGraph_t graph_def = nullptr;
                 const cudaError_t ce = cudaStreamEndCapture(g->stream, &graph_def);
-                g->cur = cur0, g->work_base = base0;
+                g->cur = cur0;
                 cudaError_t ie = ce;
                 if (ce == cudaSuccess) ie = cudaGraphInstantiate(&ex, graph_def, 0);
                 if (graph_def) cudaGraphDestroy(graph_def);
@@ -723,7 +718,6 @@ int emlab_grid_step(emlab_grid* g, int count) {
             EMLAB_CUDA(cudaEventRecord(g->stage_done[slot], g->stream));
             g->step += (uint64_t)m;
             if (g->nports && g->recording) g->recorded = (size_t)m;
-            if (g->kernel != EMLAB_KERNEL_SPLIT && g->graph_tickets) g->work_base = g->graph_tickets;
             g_launches += g->graph_launches;
             if (int rc = check_launch()) return rc;
             continue;

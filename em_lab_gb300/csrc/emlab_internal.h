@@ -46,13 +46,15 @@ struct YeeArgs {
     const float2* pml_coef;        // [K][K][K]: (e^{-x}, dt phi(x)), x = dt ((V_i + V_j) + V_k)
     const unsigned char* pml_z;    // [nz]: 1 where the plane lies in the absorber along z (common.glsl:40-43;
                                    // per scene in a stack of scenes)
+    const unsigned* pml_zi;        // [nz]: the plane's bit of pml_z, its integer (bits 8-15) and half-integer
+                                   // (bits 16-23) depth classes along z
     int pml_K;
     int L;
     float dt;
+    float minus_zero;  // -0, for the packed products of the pair kernel (mul2)
     int zchunk;
     int tile_rows;   // tiling mode of the fused kernels (8, 16: single-cell tiles; 64, 128: pair tiles)
-    unsigned long long* work;      // work-item ticket counter of the persistent kernel (monotonic)
-    unsigned long long work_base;  // tickets consumed by all earlier launches on this counter
+    unsigned long long* work;      // work-item tickets and leaver count of the persistent kernel (zero between launches)
     int wait_polls;                // polls of a plane's copy barrier before the CTA gives up (wait_limit())
     // x / y absorber lookups of the pair kernel: rows 0 (I_x), 1 (I_y), 3 (H_x), 4 (H_y) of a
     // [6][pml_xy_stride] table pair, one pair per scene of a stack whose scenes have their own
@@ -109,9 +111,7 @@ std::vector<int4> ragged_items(const std::vector<int>& z0, const std::vector<int
 // the uniform grid's pair-kernel schedule for g CTAs: planes per z chunk and work items
 void pair_schedule_shape(int nx, int ny, int nz, int ty, int g, int* zc, int* items);
 // Launches the TMA kernel reading generation `gen`; err receives a nonzero word if a wait timed out.
-// *tickets receives the work-counter tickets the launch consumes (0 for the non-persistent kernels)
-bool launch_yee_tma(const YeeArgs& a, const TmaMaps* m, int gen, bool wide, unsigned* err, cudaStream_t s,
-                    unsigned long long* tickets);
+bool launch_yee_tma(const YeeArgs& a, const TmaMaps* m, int gen, bool wide, unsigned* err, cudaStream_t s);
 void launch_yee_split(const YeeArgs& a, bool wide, cudaStream_t s);
 void launch_sources(const YeeArgs& a, const SourceArgs& sa, int k, bool wide, cudaStream_t s);
 

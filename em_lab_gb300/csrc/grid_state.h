@@ -109,11 +109,11 @@ struct emlab_grid {
     DevBuf<uint8_t> pml_cls;
     DevBuf<float2> pml_coef;
     DevBuf<uint8_t> pml_z;  // per plane: inside the absorber along z
+    DevBuf<unsigned> pml_zi;  // per plane: that bit and the z depth classes, packed (YeeArgs::pml_zi)
     int pml_K = 0;
     emlab::TmaMaps* tma = nullptr;
     DevBuf<unsigned> d_err;  // set by a solver kernel whose bounded on-device wait ran out
-    DevBuf<unsigned long long> d_work;  // ticket counter of the persistent Yee kernel (never reset)
-    unsigned long long work_base = 0;   // tickets consumed by the launches issued so far
+    DevBuf<unsigned long long> d_work;  // persistent Yee kernel: tickets drawn, CTAs that have left
     std::vector<float> cell_sigma, cell_eps;  // alpha channels of the textures (read-back only)
     // sources
     std::vector<emlab_source> desc;
@@ -206,7 +206,6 @@ struct emlab_grid {
     int graph_chunk = 0;  // 0: launches are issued one by one
     bool graph_warm = false;
     cudaGraphExec_t graph_exec[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
-    unsigned long long graph_tickets = 0;  // work tickets the last solver launch of a chunk consumes
     uint64_t graph_launches = 0;           // kernel launches in one chunk graph
     // solver-pass timing: event pairs recorded around each Yee launch, read back lazily
     bool timing = false;

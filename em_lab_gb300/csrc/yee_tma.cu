@@ -338,8 +338,20 @@ __global__ void __launch_bounds__(32 * (TY + 1), TY <= 8 ? 3 : 1)
 
 // ------------------------------------------------------------------------------------------------
 // Two cells per thread along x: a CTA owns a 64 x TY tile (warp w = row y0+w, lane l = cells
-// x0+2l and x0+2l+1) and moves pairs with 64-bit shared and global accesses, so the per-plane
-// bookkeeping and most address arithmetic are paid once per two cells. Same arithmetic per cell.
+// x0+2l and x0+2l+1) and marches it along z. Same arithmetic per cell as above, bit for bit.
+//
+// What bounds it: HBM on large grids (48.6 bytes of traffic per cell-step), and before that the
+// instructions issued per cell, so the own warps' inner loop is written for few of them:
+//  * every field is a pair of FP32 in one 64-bit register and the curls and updates are packed
+//    .f32x2 operations (each half rounds as the scalar operation does, no contraction);
+//  * the branches are uniform over the warp: a row of 64 cells outside the absorber takes one of two
+//    straight paths (all vacuum, or the class table for every lane: the vacuum entry (1, dt) gives
+//    the same bits), a row that touches the absorber reads the (e^-x, dt phi) table in every lane
+//    (class 0 outside the layer is (1, dt) again); only rows with non-vacuum cells inside the
+//    absorber, and rows with a thin-wire cell, branch per lane;
+//  * E(z+1).x and .y, read for B at plane z, stay in registers as plane z+1's own E;
+//  * the -y halo row, the -x halo column and the copies have warps of their own (TY, TY+1), so no
+//    own warp waits for two halo updates in a row.
 template <int TY, typename Idx>
 struct Layout2 {
     static constexpr int STAGES = TY == 8 ? 4 : 5;
@@ -361,13 +373,51 @@ struct Layout2 {
     static constexpr int SB_OFF = STAGES * STAGE;
     static constexpr int SB_BYTES = 2 * 3 * (TY + 1) * W * 4;
     static constexpr int BAR_OFF = (SB_OFF + SB_BYTES + 127) / 128 * 128;
-    static constexpr int PROD_OFF = BAR_OFF + 8 * STAGES;           // producer cursor (leader only)
-    static constexpr int QUEUE_OFF = PROD_OFF + 8 * 4;               // item numbers [8], -1 = done
-    static constexpr int COL_OFF = (QUEUE_OFF + 8 * 4 + 15) / 16 * 16;  // column-halo rows, int4 [TY]
-    static constexpr int SMEM = COL_OFF + TY * 16;
-    static_assert(COL_OFF % 16 == 0 && BAR_OFF % 8 == 0 && SB_OFF % 16 == 0, "shared-memory alignment");
+    static constexpr int QUEUE_OFF = BAR_OFF + 8 * STAGES;  // item numbers [8], -1 = done
+    static constexpr int STOP_OFF = QUEUE_OFF + 8 * 4;       // barrier after which every warp leaves, -1 = none
+    static constexpr int SMEM = STOP_OFF + 16;
+    static constexpr int CTAS = TY == 4 ? 3 : (TY == 8 ? 2 : 1);  // per SM
+    static_assert(BAR_OFF % 8 == 0 && SB_OFF % 16 == 0, "shared-memory alignment");
     static_assert(SMEM <= 227 * 1024, "shared memory per CTA");
 };
+
+// A pair of FP32 (cells xa and xa+1) in one 64-bit register; packed IEEE operations (sm_100+).
+using pair_t = unsigned long long;
+__device__ __forceinline__ pair_t pk(float lo, float hi) {
+    pair_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float lo_of(pair_t v) {
+    float a, b;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+    return a;
+}
+__device__ __forceinline__ float hi_of(pair_t v) {
+    float a, b;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+    return b;
+}
+__device__ __forceinline__ pair_t add2(pair_t a, pair_t b) {
+    pair_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ pair_t sub2(pair_t a, pair_t b) {
+    pair_t r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// a * b, rounded once: a * b + (-0). The compiler merges a packed multiply with the packed addition
+// that uses it into one multiply-add with one rounding, whatever -fmad says, and folds a constant -0
+// away; mz (YeeArgs::minus_zero) is a -0 it cannot see.
+__device__ __forceinline__ pair_t mul2(pair_t a, pair_t b, pair_t mz) {
+    pair_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(mz));
+    return r;
+}
+__device__ __forceinline__ pair_t lds2(const float* p) { return *reinterpret_cast<const pair_t*>(p); }
+__device__ __forceinline__ void sts2(float* p, pair_t v) { *reinterpret_cast<pair_t*>(p) = v; }
 
 // The next field generation is not read again in the launch: its stores leave L2 first, so the
 // current generation's planes stay for the neighbouring tiles' halo reads. The policy is made at
@@ -377,12 +427,16 @@ __device__ __forceinline__ uint64_t evict_first_policy() {
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
     return p;
 }
-__device__ __forceinline__ void st_pair(float* p, float2 v, uint64_t policy) {
-    asm volatile("st.global.L2::cache_hint.v2.f32 [%0], {%1, %2}, %3;" ::"l"(p), "f"(v.x), "f"(v.y), "l"(policy)
-                 : "memory");
+__device__ __forceinline__ void st_pair(float* p, pair_t v, uint64_t policy) {
+    asm volatile("st.global.L2::cache_hint.b64 [%0], %1, %2;" ::"l"(p), "l"(v), "l"(policy) : "memory");
 }
 __device__ __forceinline__ void st_one(float* p, float v, uint64_t policy) {
     asm volatile("st.global.L2::cache_hint.f32 [%0], %1, %2;" ::"l"(p), "f"(v), "l"(policy) : "memory");
+}
+// The pair's cells inside the scene: both (o1), the first (o0), or none.
+__device__ __forceinline__ void st_cells(float* p, pair_t v, bool o0, bool o1, uint64_t policy) {
+    if (o1) st_pair(p, v, policy);
+    else if (o0) st_one(p, lo_of(v), policy);
 }
 
 template <typename Idx>
@@ -396,6 +450,15 @@ template <>
 __device__ __forceinline__ void load_class_pair<uint32_t>(const uint32_t* p, unsigned& a, unsigned& b) {
     const uint2 v = *reinterpret_cast<const uint2*>(p);
     a = v.x, b = v.y;
+}
+
+// Absorber coefficients (e^-x, dt phi) of a pair from the table entries ia, ib (ia alone where both
+// cells of every lane of the warp share their x depth class).
+__device__ __forceinline__ void coef_pair(const YeeArgs& a, int ia, int ib, bool same, pair_t& decay, pair_t& gain) {
+    const float2 ka = __ldg(a.pml_coef + ia);
+    float2 kb = ka;
+    if (!same) kb = __ldg(a.pml_coef + ib);
+    decay = pk(ka.x, kb.x), gain = pk(ka.y, kb.y);
 }
 
 // B^{n+1/2} of one cell outside/inside the absorber from its curl terms (update_B.comp:47-67).
@@ -427,17 +490,10 @@ __device__ __forceinline__ void e_update(const YeeArgs& a, float& ex, float& ey,
                                          float cz, unsigned c, bool inp, int R1, int R2, int R4, int iz, int hz, int x,
                                          int y, int z, int scene) {
     if (!inp) {
-        if (c == 0) {  // vacuum: ca = 1 and cb = dt exactly, so 1 * e + dt * curl == e + dt * curl
-            const float dt = a.dt;
-            ex = ex + dt * cx;
-            ey = ey + dt * cy;
-            ez = ez + dt * cz;
-        } else {
-            const float4 t0 = __ldg(a.tabE + 2 * c), t1 = __ldg(a.tabE + 2 * c + 1);
-            ex = t0.x * ex + t0.w * cx;
-            ey = t0.y * ey + t1.x * cy;
-            ez = t0.z * ez + t1.y * cz;
-        }
+        const float4 t0 = __ldg(a.tabE + 2 * c), t1 = __ldg(a.tabE + 2 * c + 1);
+        ex = t0.x * ex + t0.w * cx;
+        ey = t0.y * ey + t1.x * cy;
+        ez = t0.z * ez + t1.y * cz;
     } else if (c == 0) {
         const float2 kx = __ldg(a.pml_coef + R2 + iz), ky = __ldg(a.pml_coef + R1 + iz),
                      kz = __ldg(a.pml_coef + R4 + hz);
@@ -458,20 +514,18 @@ __device__ __forceinline__ void e_update(const YeeArgs& a, float& ex, float& ey,
     }
 }
 
-// Dynamic schedule of the persistent pair kernel: work items are (z chunk, tile) pairs, chunk-major,
-// handed out in order by a ticket counter. Items in progress at any moment are a window of
-// consecutive tiles at nearly the same z, so the halos that neighbouring tiles share are L2 hits;
-// a static assignment lets slow CTAs (absorber columns) drift planes apart from their neighbours.
-// The counter is never reset: launch n consumes exactly items + G tickets (every CTA's last grab
-// fails), and the host passes the sum over earlier launches as `base`. After a launch that stopped
-// early the counter lags; tickets below the base are skipped.
+// Schedule of the persistent pair kernel: work items are (z chunk, tile) pairs, chunk-major. CTA b
+// starts with item b; the later ones are handed out in order by a ticket counter. Items in progress
+// at any moment are a window of consecutive tiles at nearly the same z, so the halos that
+// neighbouring tiles share are L2 hits; a static assignment lets slow CTAs (absorber columns) drift
+// planes apart from their neighbours. work[0] counts tickets, work[1] the CTAs that have left: the
+// last to leave, also after a wait that ran out, clears both, so every launch starts at zero.
 struct PairSched {
     int tiles_x;  // 64-cell tiles along x
     int tiles;    // tiles per z chunk
     int items;    // tiles * z chunks
     int zc;       // planes per z chunk
     unsigned long long* work;
-    unsigned long long base;
     const int4* tab;  // a stack of scenes with their own cross-sections: the items themselves
 };
 
@@ -497,293 +551,385 @@ __device__ __forceinline__ PairItem pair_item(const PairSched& ps, int nz, int i
     return it;
 }
 
+// Table rows of the depth classes of column (px, py): entry R1 + hz is (ix, hy, hz), R2 + hz is
+// (hx, iy, hz), R3 + iz is (hx, hy, iz), R4 + hz is (ix, iy, hz).
+struct PmlRows {
+    int r1, r2, r3, r4;
+};
+__device__ __forceinline__ PmlRows pml_rows(const unsigned char* pcx, int SX, int K, int px, int py) {
+    const int ix = __ldg(pcx + px), iy = __ldg(pcx + SX + py), hx = __ldg(pcx + 3 * SX + px),
+              hy = __ldg(pcx + 4 * SX + py);
+    return {(ix * K + hy) * K, (hx * K + iy) * K, (hx * K + hy) * K, (ix * K + iy) * K};
+}
+
+// Plane classes along z, packed on the host: bit 0 in the absorber, bits 8-15 the integer depth
+// class, bits 16-23 the half-integer one.
+__device__ __forceinline__ int z_iz(unsigned v) { return (v >> 8) & 0xff; }
+__device__ __forceinline__ int z_hz(unsigned v) { return (v >> 16) & 0xff; }
+
+template <int TY>
+__device__ __forceinline__ void plane_sync() {  // every warp of the CTA, once per plane
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * (TY + 2)) : "memory");
+}
+
 // The CTA's loads form one sequence over its items: for each item, planes zstart .. ze (plane ze
 // is read as the "z+1" neighbour of the last plane; ze = nz reads TMA zeros). Load j goes to ring
 // stage j % STAGES and completes phase (j / STAGES) & 1 of that stage's mbarrier. The ring runs
-// on across item boundaries, so the pipeline never drains inside a launch. The leader takes the
-// next item when its loads reach it and posts the item number in a small shared ring that the
-// other warps read at their item boundary (always at least one barrier later).
-// 64 x 4 tiles: four 160-thread CTAs per SM; 64 x 8: two 288-thread CTAs; 64 x 16: one 544-thread
-// CTA. Registers are allocated per SM quadrant and 17-20 warps put 5 warps on one quadrant: 96
+// on across item boundaries, so the pipeline never drains inside a launch. The leader (lane 0 of
+// warp TY+1) takes the next item when its loads near it and posts the item number in a small
+// shared ring that the other warps read at their item boundary (always at least one barrier later).
+// 64 x 4 tiles: three 192-thread CTAs per SM; 64 x 8: two 320-thread CTAs; 64 x 16: one 576-thread
+// CTA. Registers are allocated per SM quadrant and 18-20 warps put 5 warps on one quadrant: 96
 // registers at most.
 template <int TY, typename Idx>
-__global__ void __launch_bounds__(32 * (TY + 1), TY == 4 ? 4 : (TY == 8 ? 2 : 1))
+__global__ void __launch_bounds__(32 * (TY + 2), Layout2<TY, Idx>::CTAS)
     yee_tma2(const __grid_constant__ CUtensorMap tex, const __grid_constant__ CUtensorMap tey,
              const __grid_constant__ CUtensorMap tez, const __grid_constant__ CUtensorMap tbx,
              const __grid_constant__ CUtensorMap tby, const __grid_constant__ CUtensorMap tbz,
              const __grid_constant__ CUtensorMap tcls, YeeArgs a, PairSched ps, unsigned* err) {
-    static_assert(TY == 4 || TY == 8 || TY == 16, "register budget assumes 5, 9 or 17 warps per CTA");
+    static_assert(TY == 4 || TY == 8 || TY == 16, "register budget assumes 6, 10 or 18 warps per CTA");
     using Lay = Layout2<TY, Idx>;
     constexpr int S_ = Lay::STAGES;
+    constexpr int EPF = Lay::EP / 4, BPF = Lay::BP / 4, W = Lay::W, SBC = (TY + 1) * W;
     extern __shared__ __align__(128) unsigned char smem[];
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Lay::BAR_OFF);
     float* sB = reinterpret_cast<float*>(smem + Lay::SB_OFF);
-    // producer cursor: item, x0, y0, z, zend, issued, waited, item ordinal
-    int* prod = reinterpret_cast<int*>(smem + Lay::PROD_OFF);
-    int* queue = reinterpret_cast<int*>(smem + Lay::QUEUE_OFF);  // item of ordinal n at [n & 7]
-    int4* colrow = reinterpret_cast<int4*>(smem + Lay::COL_OFF);
+    volatile int* queue = reinterpret_cast<volatile int*>(smem + Lay::QUEUE_OFF);  // item of ordinal n at [n & 7]
+    volatile int* stop = reinterpret_cast<volatile int*>(smem + Lay::STOP_OFF);
 
     const int lane = threadIdx.x, warp = threadIdx.y;
-    const bool ctl = warp == TY;
-    const bool leader = ctl && lane == 0;
-
-    // ---- producer (leader thread): cursor over the load sequence, kept in shared memory ----
-    auto grab = [&]() -> int {  // next work item, or -1 when all are taken
-        for (;;) {
-            const unsigned long long t = atomicAdd(ps.work, 1ull);
-            if (t < ps.base) continue;  // left over from a launch that stopped early
-            return t - ps.base < (unsigned long long)ps.items ? (int)(t - ps.base) : -1;
-        }
-    };
-    auto p_seek = [&]() {
-        if (prod[0] >= 0) {
-            const PairItem it = pair_item<TY>(ps, a.nz, prod[0]);
-            prod[1] = it.x0, prod[2] = it.y0, prod[3] = it.zstart, prod[4] = it.ze;
-        }
-    };
-    auto issue_upto = [&](int last) {  // issue loads up to index `last` while the sequence lasts
-        int issued = prod[5];
-        while (issued <= last && prod[0] >= 0) {
-            unsigned char* st = smem + (issued % S_) * Lay::STAGE;
-            uint64_t* bar = bars + issued % S_;
-            const int px = prod[1] - 4, py = prod[2] - 1, pz = prod[3];
-            mbar_expect_tx(bar, Lay::TX_BYTES);
-            tma_load_3d(st + Lay::E_OFF + 0 * Lay::EP, &tex, px, py, pz, bar);
-            tma_load_3d(st + Lay::E_OFF + 1 * Lay::EP, &tey, px, py, pz, bar);
-            tma_load_3d(st + Lay::E_OFF + 2 * Lay::EP, &tez, px, py, pz, bar);
-            tma_load_3d(st + Lay::B_OFF + 0 * Lay::BP, &tbx, px, py, pz, bar);
-            tma_load_3d(st + Lay::B_OFF + 1 * Lay::BP, &tby, px, py, pz, bar);
-            tma_load_3d(st + Lay::B_OFF + 2 * Lay::BP, &tbz, px, py, pz, bar);
-            tma_load_3d(st + Lay::C_OFF, &tcls, px - Lay::DC, py, pz, bar);
-            ++issued;
-            if (++prod[3] > prod[4]) {  // item complete: take the next one and post it
-                prod[0] = grab();
-                queue[++prod[7] & 7] = prod[0];
-                p_seek();
-            }
-        }
-        prod[5] = issued;
-    };
-    auto wait_upto = [&](int last) {  // false if a load did not complete within the bound
-        int waited = prod[6];
-        bool ok = true;
-        while (ok && waited < last) {
-            ++waited;
-            ok = mbar_wait(bars + waited % S_, (waited / S_) & 1, a.wait_polls);
-        }
-        prod[6] = waited;
-        return ok;
-    };
-    // on an expired wait: record the error, then give every copy still in flight a bounded time to
-    // land before the CTA leaves and its shared memory goes. prod[6] is the load whose wait ran out
-    // (not complete), prod[5] - 1 the last load issued.
-    auto bail = [&]() {
-        if (leader) {
-            atomicOr(err, 1u);
-            for (int w = prod[6] < 0 ? 0 : prod[6]; w < prod[5]; ++w) mbar_wait(bars + w % S_, (w / S_) & 1);
-        }
-    };
-
-    if (leader) {
+    const int L = a.L, K = a.pml_K, SX = a.pml_xy_stride;
+    if (warp == TY + 1 && lane == 0) {
         for (int s = 0; s < S_; ++s) mbar_init(bars + s, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        prod[0] = grab(), prod[5] = 0, prod[6] = -1, prod[7] = 0;
-        queue[0] = prod[0];
+        queue[0] = blockIdx.x;
+        *stop = -1;
     }
     __syncthreads();
-    if (queue[0] < 0) return;  // uniform: no work for this CTA
-    bool failed = false;
-    if (leader) {
-        p_seek();
-        issue_upto(S_ - 1);
-        failed = !wait_upto(1);  // the first iteration reads loads 0 and 1
-    }
-    if (__syncthreads_or(failed)) {
-        bail();
-        return;
-    }
 
-    constexpr int EPF = Lay::EP / 4, BPF = Lay::BP / 4, W = Lay::W, SBC = (TY + 1) * W;
-    const int L = a.L, K = a.pml_K, PS = a.pml_stride;
-    const unsigned char* pcls = a.pml_cls;
-    // box element of the own / halo-row pair (E, B and 32-bit class boxes share it; the 16-bit class
-    // box is DC elements further) and of the column cell (x0-1, y0+lane); B tile slot = element - 2
-    const int me = (ctl ? 0 : warp + 1) * W + 2 * lane + 4;
-    const int ce = (lane + 1) * W + 3;
-    const int SX = a.pml_xy_stride;
-    // x / y depth classes from the item's scene's table (pcx), z from the grid's
-    auto pml_rows = [&](const unsigned char* pcx, int px, int py, int& R1, int& R2, int& R3, int& R4) {
-        const int ix = __ldg(pcx + px), iy = __ldg(pcx + SX + py), hx = __ldg(pcx + 3 * SX + px),
-                  hy = __ldg(pcx + 4 * SX + py);
-        R1 = (ix * K + hy) * K, R2 = (hx * K + iy) * K, R3 = (hx * K + hy) * K, R4 = (ix * K + iy) * K;
-    };
-
-    int k = 0;     // load index of the current iteration's plane z
-    int iter = 0;  // iteration counter: parity selects the B tile buffer
-    for (int ord = 0, item = queue[0]; item >= 0; item = queue[++ord & 7]) {
-        const PairItem itm = pair_item<TY>(ps, a.nz, item);
-        const int x0 = itm.x0, y0 = itm.y0, zs = itm.zs, ze = itm.ze, scene = itm.scene;
-        // the absorber of the item's scene (common.glsl:40-43 with the scene's own nx, ny)
-        const unsigned char* pcx = a.pml_cls_xy + (long long)scene * a.pml_xy_scene;
-        int snx = a.nx, sny = a.ny;
+    // the absorber of an item's scene (common.glsl:40-43 with the scene's own nx, ny)
+    auto scene_size = [&](int scene, int& snx, int& sny) {
+        snx = a.nx, sny = a.ny;
         if (a.scene_xy) {
             const int2 d = __ldg(a.scene_xy + scene);
             snx = d.x, sny = d.y;
         }
-        auto pml_xy_of = [&](int px, int py) { return px < L || py < L || px >= snx - (L + 1) || py >= sny - (L + 1); };
+    };
 
-        // per-item invariants: own warps hold cells (xa, y), (xa+1, y); the halo warp holds the row
-        // cells (xa, y0-1), (xa+1, y0-1) and the column cell (x0-1, y0+lane)
-        // cells outside the item's scene (a ragged stack's frozen cells) are neither updated nor
-        // written: they keep their initial 0 in both field generations
-        const int xa = x0 + 2 * lane;
-        const int y = ctl ? y0 - 1 : y0 + warp;
-        const bool rowok = ctl ? y0 > 0 : y < sny;
-        const bool o0 = rowok && xa < snx, o1 = rowok && xa + 1 < snx;
-        int A1 = 0, A2 = 0, A3 = 0, A4 = 0, B1 = 0, B2 = 0, B3 = 0, B4 = 0;
-        if (o0) pml_rows(pcx, xa, y, A1, A2, A3, A4);
-        if (o1) pml_rows(pcx, xa + 1, y, B1, B2, B3, B4);
-        const bool pxy0 = o0 && pml_xy_of(xa, y), pxy1 = o1 && pml_xy_of(xa + 1, y);
-        if (ctl && lane < TY) {  // column cell: live flag | absorber flag, then its table rows
-            const int cy = y0 + lane;
-            int4 cr = make_int4(0, 0, 0, 0);
-            if (x0 > 0 && cy < sny) {
-                int r4;
-                pml_rows(pcx, x0 - 1, cy, cr.y, cr.z, cr.w, r4);
-                cr.x = 1 | (pml_xy_of(x0 - 1, cy) ? 2 : 0);
+    if (warp == TY + 1) {
+        // ---- copies (lane 0) and the -x halo column: By, Bz of (x0-1, y0+lane), lanes 0 .. TY-1 ----
+        const bool leader = lane == 0;
+        int p_x = 0, p_y = 0, p_z = 0, p_end = -1;  // the next load: its tile and plane, the item's last plane
+        int issued = 0, waited = -1, p_ord = 0;
+        bool more = true;
+        unsigned long long ticket = 0;
+        auto seek = [&](int item) {
+            const PairItem it = pair_item<TY>(ps, a.nz, item);
+            p_x = it.x0 - 4, p_y = it.y0 - 1, p_z = it.zstart, p_end = it.ze;
+        };
+        auto issue_upto = [&](int last) {  // issue loads up to index `last` while the sequence lasts
+            while (issued <= last && more) {
+                unsigned char* st = smem + (issued % S_) * Lay::STAGE;
+                uint64_t* bar = bars + issued % S_;
+                mbar_expect_tx(bar, Lay::TX_BYTES);
+                tma_load_3d(st + Lay::E_OFF + 0 * Lay::EP, &tex, p_x, p_y, p_z, bar);
+                tma_load_3d(st + Lay::E_OFF + 1 * Lay::EP, &tey, p_x, p_y, p_z, bar);
+                tma_load_3d(st + Lay::E_OFF + 2 * Lay::EP, &tez, p_x, p_y, p_z, bar);
+                tma_load_3d(st + Lay::B_OFF + 0 * Lay::BP, &tbx, p_x, p_y, p_z, bar);
+                tma_load_3d(st + Lay::B_OFF + 1 * Lay::BP, &tby, p_x, p_y, p_z, bar);
+                tma_load_3d(st + Lay::B_OFF + 2 * Lay::BP, &tbz, p_x, p_y, p_z, bar);
+                tma_load_3d(st + Lay::C_OFF, &tcls, p_x - Lay::DC, p_y, p_z, bar);
+                ++issued;
+                // the ticket of the next item is drawn one load ahead (every item has at least two
+                // loads), so its round trip to L2 hides behind that load's plane
+                if (p_z == p_end - 1) ticket = atomicAdd(ps.work, 1ull);
+                if (++p_z > p_end) {
+                    const int left = ps.items - (int)gridDim.x;  // items handed out by ticket
+                    const int next = ticket < (unsigned long long)left ? (int)gridDim.x + (int)ticket : -1;
+                    queue[++p_ord & 7] = next;
+                    more = next >= 0;
+                    if (more) seek(next);
+                }
             }
-            colrow[lane] = cr;  // read by the same thread only
+        };
+        auto wait_upto = [&](int last) {  // false if a load did not complete within the bound
+            bool ok = true;
+            while (ok && waited < last) {
+                ++waited;
+                ok = mbar_wait(bars + waited % S_, (waited / S_) & 1, a.wait_polls);
+            }
+            return ok;
+        };
+        // the CTA leaves: on an expired wait record the error and give every copy still in flight
+        // (from the load whose wait ran out on) a bounded time to land before the CTA's shared
+        // memory goes; then count the CTA out
+        auto leave = [&](bool failed) {
+            if (!leader) return;
+            if (failed) {
+                atomicOr(err, 1u);
+                for (int w = waited < 0 ? 0 : waited; w < issued; ++w) mbar_wait(bars + w % S_, (w / S_) & 1);
+            }
+            __threadfence();  // this CTA's tickets before its count
+            if (atomicAdd(ps.work + 1, 1ull) == (unsigned long long)gridDim.x - 1) ps.work[0] = 0, ps.work[1] = 0;
+        };
+        if (leader) {
+            seek(blockIdx.x);
+            issue_upto(S_ - 1);
+            if (!wait_upto(1)) *stop = 0;  // the first iteration reads loads 0 and 1
         }
-        const long long row_off = (long long)y * a.pitch + xa;
-
-        float2 bp_x = make_float2(0.0f, 0.0f), bp_y = bp_x;  // B^{n+1/2}(z-1).x, .y of the pair
-        int iz = __ldg(pcls + 2 * PS + itm.zstart), hz = __ldg(pcls + 5 * PS + itm.zstart);
-        for (int z = itm.zstart; z < ze; ++z, ++k, ++iter) {
-            const unsigned char* st = smem + (k % S_) * Lay::STAGE;
-            const unsigned char* st1 = smem + ((k + 1) % S_) * Lay::STAGE;
-            const bool emit = z >= zs;
-            float* sb = sB + (iter & 1) * 3 * SBC - 2;  // indexed by box element
-            const bool pz = __ldg(a.pml_z + z) != 0;
-            const int zn = min(z + 1, a.nz - 1);
-            const int iz_n = __ldg(pcls + 2 * PS + zn), hz_n = __ldg(pcls + 5 * PS + zn);
-            const float* Es = reinterpret_cast<const float*>(st + Lay::E_OFF);
-            const float* E1 = reinterpret_cast<const float*>(st1 + Lay::E_OFF);
-            const float* Bs = reinterpret_cast<const float*>(st + Lay::B_OFF);
-            const Idx* Cs = reinterpret_cast<const Idx*>(st + Lay::C_OFF) + Lay::DC;
-            const long long off = (long long)z * a.plane + row_off;
-            float2 e0x = make_float2(0.0f, 0.0f), e0y = e0x, e0z = e0x, bx = e0x, by = e0x, bz = e0x;
-            unsigned ca = 0, cb = 0;
-            if (!ctl) {
-                // update_B.comp:35-67 for both cells (halo values beyond the grid are TMA zeros)
-                e0x = *reinterpret_cast<const float2*>(Es + me);
-                e0y = *reinterpret_cast<const float2*>(Es + EPF + me);
-                e0z = *reinterpret_cast<const float2*>(Es + 2 * EPF + me);
-                bx = *reinterpret_cast<const float2*>(Bs + me);
-                by = *reinterpret_cast<const float2*>(Bs + BPF + me);
-                bz = *reinterpret_cast<const float2*>(Bs + 2 * BPF + me);
-                load_class_pair<Idx>(Cs + me, ca, cb);
-                const float e2y = Es[EPF + me + 2], e2z = Es[2 * EPF + me + 2];          // E(xa+2)
-                const float2 eyx = *reinterpret_cast<const float2*>(Es + me + W);         // E(y+1)
-                const float2 eyz = *reinterpret_cast<const float2*>(Es + 2 * EPF + me + W);
-                const float2 ezx = *reinterpret_cast<const float2*>(E1 + me);            // E(z+1)
-                const float2 ezy = *reinterpret_cast<const float2*>(E1 + EPF + me);
-                b_update(a, bx.x, by.x, bz.x, eyz.x - e0z.x, ezx.x - e0x.x, e0y.y - e0y.x, ezy.x - e0y.x,
-                         e0z.y - e0z.x, eyx.x - e0x.x, ca, pxy0 || pz, A1, A2, A3, iz, hz);
-                b_update(a, bx.y, by.y, bz.y, eyz.y - e0z.y, ezx.y - e0x.y, e2y - e0y.y, ezy.y - e0y.y, e2z - e0z.y,
-                         eyx.y - e0x.y, cb, pxy1 || pz, B1, B2, B3, iz, hz);
-                *reinterpret_cast<float2*>(sb + me) = bx;
-                *reinterpret_cast<float2*>(sb + SBC + me) = by;
-                *reinterpret_cast<float2*>(sb + 2 * SBC + me) = bz;
-                if (emit) {
-                    const uint64_t evict_first = evict_first_policy();
-                    if (o1) {
-                        st_pair(a.nbx + off, bx, evict_first);
-                        st_pair(a.nby + off, by, evict_first);
-                        st_pair(a.nbz + off, bz, evict_first);
-                    } else if (o0) {
-                        st_one(a.nbx + off, bx.x, evict_first);
-                        st_one(a.nby + off, by.x, evict_first);
-                        st_one(a.nbz + off, bz.x, evict_first);
-                    }
-                }
-            } else if (emit) {
-                // -y row: Bx, Bz of (xa, y0-1) and (xa+1, y0-1); B below the lower faces is 0
-                float2 hx2 = make_float2(0.0f, 0.0f), hz2 = hx2;
-                if (o0) {
-                    const float2 f0x = *reinterpret_cast<const float2*>(Es + me);
-                    const float2 f0y = *reinterpret_cast<const float2*>(Es + EPF + me);
-                    const float2 f0z = *reinterpret_cast<const float2*>(Es + 2 * EPF + me);
-                    const float e2y = Es[EPF + me + 2];
-                    const float2 eyx = *reinterpret_cast<const float2*>(Es + me + W);
-                    const float2 eyz = *reinterpret_cast<const float2*>(Es + 2 * EPF + me + W);
-                    const float2 ezy = *reinterpret_cast<const float2*>(E1 + EPF + me);
-                    unsigned ha, hb;
-                    load_class_pair<Idx>(Cs + me, ha, hb);
-                    hx2 = *reinterpret_cast<const float2*>(Bs + me);
-                    hz2 = *reinterpret_cast<const float2*>(Bs + 2 * BPF + me);
-                    float unused0 = 0.0f, unused1 = 0.0f;
-                    b_update(a, hx2.x, unused0, hz2.x, eyz.x - f0z.x, 0.0f, f0y.y - f0y.x, ezy.x - f0y.x, 0.0f,
-                             eyx.x - f0x.x, ha, pxy0 || pz, A1, A2, A3, iz, hz);
-                    if (o1)
-                        b_update(a, hx2.y, unused1, hz2.y, eyz.y - f0z.y, 0.0f, e2y - f0y.y, ezy.y - f0y.y, 0.0f,
-                                 eyx.y - f0x.y, hb, pxy1 || pz, B1, B2, B3, iz, hz);
-                    else
-                        hx2.y = 0.0f, hz2.y = 0.0f;
-                }
-                *reinterpret_cast<float2*>(sb + me) = hx2;
-                *reinterpret_cast<float2*>(sb + 2 * SBC + me) = hz2;
-                // -x column: By, Bz of (x0-1, y0+lane)
-                if (lane < TY) {
-                    float hby = 0.0f, hbz = 0.0f, hbx = 0.0f;
-                    const int4 cr = colrow[lane];
-                    if (cr.x & 1) {
+        plane_sync<TY>();
+        if (*stop == 0) return leave(true);
+        const int ce = (lane + 1) * W + 3;
+        int k = 0, iter = 0;
+        for (int ord = 0, item = queue[0]; item >= 0; item = queue[++ord & 7]) {
+            const PairItem it = pair_item<TY>(ps, a.nz, item);
+            int snx, sny;
+            scene_size(it.scene, snx, sny);
+            const int cy = it.y0 + lane;
+            const bool live = lane < TY && it.x0 > 0 && cy < sny;
+            PmlRows r{};
+            bool inxy = false;
+            if (live) {
+                r = pml_rows(a.pml_cls_xy + (long long)it.scene * a.pml_xy_scene, SX, K, it.x0 - 1, cy);
+                inxy = it.x0 - 1 < L || cy < L || it.x0 - 1 >= snx - (L + 1) || cy >= sny - (L + 1);
+            }
+            unsigned zi = __ldg(a.pml_zi + it.zstart);
+            for (int z = it.zstart; z < it.ze; ++z, ++k, ++iter) {
+                const unsigned char* st = smem + (k % S_) * Lay::STAGE;
+                const unsigned zn = __ldg(a.pml_zi + min(z + 1, a.nz - 1));
+                if (z >= it.zs && lane < TY) {
+                    float* sb = sB + (iter & 1) * 3 * SBC - 2;  // indexed by box element
+                    float hby = 0.0f, hbz = 0.0f, hbx = 0.0f;   // B below the lower face is 0
+                    if (live) {
+                        const float* Es = reinterpret_cast<const float*>(st + Lay::E_OFF);
+                        const float* E1 = reinterpret_cast<const float*>(smem + ((k + 1) % S_) * Lay::STAGE + Lay::E_OFF);
+                        const float* Bs = reinterpret_cast<const float*>(st + Lay::B_OFF);
+                        const Idx* Cs = reinterpret_cast<const Idx*>(st + Lay::C_OFF) + Lay::DC;
                         const float f0x = Es[ce], f0y = Es[EPF + ce], f0z = Es[2 * EPF + ce];
                         hby = Bs[BPF + ce], hbz = Bs[2 * BPF + ce];
                         b_update(a, hbx, hby, hbz, 0.0f, E1[ce] - f0x, Es[EPF + ce + 1] - f0y, 0.0f,
-                                 Es[2 * EPF + ce + 1] - f0z, Es[ce + W] - f0x, (unsigned)Cs[ce], (cr.x & 2) || pz,
-                                 cr.y, cr.z, cr.w, iz, hz);
+                                 Es[2 * EPF + ce + 1] - f0z, Es[ce + W] - f0x, (unsigned)Cs[ce], inxy || (zi & 1),
+                                 r.r1, r.r2, r.r3, z_iz(zi), z_hz(zi));
                     }
                     sb[SBC + ce] = hby;
                     sb[2 * SBC + ce] = hbz;
                 }
+                // the next iteration reads loads k+1, k+2 (or k+2, k+3 at the start of the next item,
+                // which was taken when the last load of this one was issued)
+                if (leader) {
+                    const int need = z + 1 < it.ze ? k + 2 : (queue[(ord + 1) & 7] < 0 ? -1 : k + 3);
+                    if (!wait_upto(need)) *stop = iter + 1;
+                }
+                plane_sync<TY>();
+                if (*stop == iter + 1) return leave(true);
+                // every warp is past its reads of loads <= k: refill up to k + STAGES
+                if (leader) {
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    issue_upto(k + S_);
+                }
+                zi = zn;
             }
-            // the next iteration reads loads k+1, k+2 (or k+2, k+3 at the start of the next item)
-            if (leader) {  // at the last plane the next item was taken when its first load was issued
-                const int need = z + 1 < ze ? k + 2 : (queue[(ord + 1) & 7] < 0 ? -1 : k + 3);
-                if (need >= 0) failed = !wait_upto(need);
+            ++k;  // the item's last load (plane ze) was only read as the z+1 neighbour
+        }
+        return leave(false);
+    }
+
+    // The word names the barrier (0: this one, iter + 1: iteration iter's) after which all leave: a
+    // warp that is late to read it after one barrier may already see what the leader found before the
+    // next, and has to arrive there with the others.
+    plane_sync<TY>();
+    if (*stop == 0) return;
+    // box element of the own / halo-row pair (E, B and 32-bit class boxes share it; the 16-bit class
+    // box is DC elements further); B tile slot = element - 2
+    const bool row = warp == TY;  // the -y halo row: Bx, Bz of (xa, y0-1), (xa+1, y0-1)
+    const int me = (row ? 0 : warp + 1) * W + 2 * lane + 4;
+    const pair_t dt2 = pk(a.dt, a.dt), mz = pk(a.minus_zero, a.minus_zero);
+    int k = 0;     // load index of the current iteration's plane z
+    int iter = 0;  // iteration counter: parity selects the B tile buffer
+    for (int ord = 0, item = queue[0]; item >= 0; item = queue[++ord & 7]) {
+        const PairItem it = pair_item<TY>(ps, a.nz, item);
+        int snx, sny;
+        scene_size(it.scene, snx, sny);
+        // cells outside the item's scene (a ragged stack's frozen cells) are neither updated nor
+        // written: they keep their initial 0 in both field generations
+        const int xa = it.x0 + 2 * lane;
+        const int y = row ? it.y0 - 1 : it.y0 + warp;
+        const bool rowok = row ? it.y0 > 0 : y < sny;
+        const bool o0 = rowok && xa < snx, o1 = rowok && xa + 1 < snx;
+        const unsigned char* pcx = a.pml_cls_xy + (long long)it.scene * a.pml_xy_scene;
+        PmlRows A{}, B{};
+        if (o0) A = pml_rows(pcx, SX, K, xa, y);
+        if (o1) B = pml_rows(pcx, SX, K, xa + 1, y);
+        auto inxy = [&](int px) { return px < L || y < L || px >= snx - (L + 1) || y >= sny - (L + 1); };
+        const bool pxy0 = o0 && inxy(xa), pxy1 = o1 && inxy(xa + 1);
+        const bool pmlrow = __any_sync(0xffffffffu, pxy0 || pxy1);  // uniform: the warp's row touches the layer
+        const bool same = __all_sync(0xffffffffu, A.r1 == B.r1 && A.r2 == B.r2 && A.r3 == B.r3 && A.r4 == B.r4);
+        unsigned zi = __ldg(a.pml_zi + it.zstart);
+
+        if (row) {
+            for (int z = it.zstart; z < it.ze; ++z, ++k, ++iter) {
+                const unsigned char* st = smem + (k % S_) * Lay::STAGE;
+                const unsigned zn = __ldg(a.pml_zi + min(z + 1, a.nz - 1));
+                if (z >= it.zs) {
+                    float* sb = sB + (iter & 1) * 3 * SBC - 2;
+                    pair_t hx2 = 0, hz2 = 0;  // B below the lower face is 0
+                    if (rowok) {
+                        const float* Es = reinterpret_cast<const float*>(st + Lay::E_OFF);
+                        const float* E1 = reinterpret_cast<const float*>(smem + ((k + 1) % S_) * Lay::STAGE + Lay::E_OFF);
+                        const float* Bs = reinterpret_cast<const float*>(st + Lay::B_OFF);
+                        unsigned ha, hb;
+                        load_class_pair<Idx>(reinterpret_cast<const Idx*>(st + Lay::C_OFF) + Lay::DC + me, ha, hb);
+                        const pair_t f0x = lds2(Es + me), f0y = lds2(Es + EPF + me), f0z = lds2(Es + 2 * EPF + me);
+                        pair_t t0x = sub2(lds2(Es + 2 * EPF + me + W), f0z), t1x = sub2(lds2(E1 + EPF + me), f0y);
+                        pair_t t0z = sub2(pk(hi_of(f0y), Es[EPF + me + 2]), f0y), t1z = sub2(lds2(Es + me + W), f0x);
+                        if (__any_sync(0xffffffffu, max(ha, hb) >= a.wire_start)) {
+                            const float4 w0 = __ldg(a.tabW + 2 * ha), w1 = __ldg(a.tabW + 2 * ha + 1);
+                            const float4 v0 = __ldg(a.tabW + 2 * hb), v1 = __ldg(a.tabW + 2 * hb + 1);
+                            t0x = mul2(t0x, pk(w0.x, v0.x), mz), t0z = mul2(t0z, pk(w0.z, v0.z), mz);
+                            t1x = mul2(t1x, pk(w0.w, v0.w), mz), t1z = mul2(t1z, pk(w1.y, v1.y), mz);
+                        }
+                        const pair_t cx = sub2(t0x, t1x), cz = sub2(t0z, t1z);
+                        hx2 = lds2(Bs + me), hz2 = lds2(Bs + 2 * BPF + me);
+                        if (pmlrow || (zi & 1)) {
+                            pair_t d, g;
+                            coef_pair(a, A.r1 + z_hz(zi), B.r1 + z_hz(zi), same, d, g);
+                            hx2 = sub2(mul2(d, hx2, mz), mul2(g, cx, mz));
+                            coef_pair(a, A.r3 + z_iz(zi), B.r3 + z_iz(zi), same, d, g);
+                            hz2 = sub2(mul2(d, hz2, mz), mul2(g, cz, mz));
+                        } else {
+                            hx2 = sub2(hx2, mul2(dt2, cx, mz));
+                            hz2 = sub2(hz2, mul2(dt2, cz, mz));
+                        }
+                    }
+                    sts2(sb + me, hx2);
+                    sts2(sb + 2 * SBC + me, hz2);
+                }
+                plane_sync<TY>();
+                if (*stop == iter + 1) return;
+                zi = zn;
             }
-            if (__syncthreads_or(failed)) {
-                bail();
-                return;
+            ++k;
+            continue;
+        }
+
+        const bool full = __all_sync(0xffffffffu, o1);
+        long long off = (long long)it.zstart * a.plane + (long long)y * a.pitch + xa;
+        pair_t bpx = 0, bpy = 0;  // B^{n+1/2}(z-1).x, .y of the pair
+        const float* E0 = reinterpret_cast<const float*>(smem + (k % S_) * Lay::STAGE + Lay::E_OFF) + me;
+        pair_t e0x = lds2(E0), e0y = lds2(E0 + EPF);
+        for (int z = it.zstart; z < it.ze; ++z, ++k, ++iter, off += a.plane) {
+            const unsigned char* st = smem + (k % S_) * Lay::STAGE;
+            const bool emit = z >= it.zs;
+            float* sb = sB + (iter & 1) * 3 * SBC - 2 + me;  // the pair's slot; indexed by box element
+            const unsigned zn = __ldg(a.pml_zi + min(z + 1, a.nz - 1));
+            const float* Es = reinterpret_cast<const float*>(st + Lay::E_OFF) + me;
+            const float* E1 = reinterpret_cast<const float*>(smem + ((k + 1) % S_) * Lay::STAGE + Lay::E_OFF) + me;
+            const float* Bs = reinterpret_cast<const float*>(st + Lay::B_OFF) + me;
+            // update_B.comp:35-67 for both cells (halo values beyond the grid are TMA zeros)
+            unsigned ca, cb;
+            load_class_pair<Idx>(reinterpret_cast<const Idx*>(st + Lay::C_OFF) + Lay::DC + me, ca, cb);
+            const pair_t e0z = lds2(Es + 2 * EPF);
+            const pair_t ezx = lds2(E1), ezy = lds2(E1 + EPF);  // E(z+1)
+            pair_t bx = lds2(Bs), by = lds2(Bs + BPF), bz = lds2(Bs + 2 * BPF);
+            pair_t t0x = sub2(lds2(Es + 2 * EPF + W), e0z), t1x = sub2(ezy, e0y);
+            pair_t t0y = sub2(ezx, e0x), t1y = sub2(pk(hi_of(e0z), Es[2 * EPF + 2]), e0z);
+            pair_t t0z = sub2(pk(hi_of(e0y), Es[EPF + 2]), e0y), t1z = sub2(lds2(Es + W), e0x);
+            const bool mat = __any_sync(0xffffffffu, (ca | cb) != 0);  // uniform: a non-vacuum cell in the row
+            if (mat && __any_sync(0xffffffffu, max(ca, cb) >= a.wire_start)) {
+                // thin-wire factors; the entries of other classes are 1
+                const float4 w0 = __ldg(a.tabW + 2 * ca), w1 = __ldg(a.tabW + 2 * ca + 1);
+                const float4 v0 = __ldg(a.tabW + 2 * cb), v1 = __ldg(a.tabW + 2 * cb + 1);
+                t0x = mul2(t0x, pk(w0.x, v0.x), mz), t0y = mul2(t0y, pk(w0.y, v0.y), mz), t0z = mul2(t0z, pk(w0.z, v0.z), mz);
+                t1x = mul2(t1x, pk(w0.w, v0.w), mz), t1y = mul2(t1y, pk(w1.x, v1.x), mz), t1z = mul2(t1z, pk(w1.y, v1.y), mz);
             }
-            // every warp is past its reads of loads <= k: refill up to k + STAGES
-            if (leader) {
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                issue_upto(k + S_);
+            const bool pml = pmlrow || (zi & 1);
+            {
+                const pair_t cx = sub2(t0x, t1x), cy = sub2(t0y, t1y), cz = sub2(t0z, t1z);
+                if (pml) {
+                    pair_t d, g;
+                    coef_pair(a, A.r1 + z_hz(zi), B.r1 + z_hz(zi), same, d, g);
+                    bx = sub2(mul2(d, bx, mz), mul2(g, cx, mz));
+                    coef_pair(a, A.r2 + z_hz(zi), B.r2 + z_hz(zi), same, d, g);
+                    by = sub2(mul2(d, by, mz), mul2(g, cy, mz));
+                    coef_pair(a, A.r3 + z_iz(zi), B.r3 + z_iz(zi), same, d, g);
+                    bz = sub2(mul2(d, bz, mz), mul2(g, cz, mz));
+                } else {
+                    bx = sub2(bx, mul2(dt2, cx, mz));
+                    by = sub2(by, mul2(dt2, cy, mz));
+                    bz = sub2(bz, mul2(dt2, cz, mz));
+                }
             }
-            if (emit && !ctl && o0) {
-                // update_E.comp:41-64 for both cells
-                const float bxm_y = sb[SBC + me - 1], bxm_z = sb[2 * SBC + me - 1];             // B(xa-1).y, .z
-                const float2 bym_x = *reinterpret_cast<const float2*>(sb + me - W);            // B(y-1).x
-                const float2 bym_z = *reinterpret_cast<const float2*>(sb + 2 * SBC + me - W);  // B(y-1).z
-                float2 ex = e0x, ey = e0y, ez = e0z;
-                e_update(a, ex.x, ey.x, ez.x, (bz.x - bym_z.x) - (by.x - bp_y.x), (bx.x - bp_x.x) - (bz.x - bxm_z),
-                         (by.x - bxm_y) - (bx.x - bym_x.x), ca, pxy0 || pz, A1, A2, A4, iz, hz, xa, y, z, scene);
-                e_update(a, ex.y, ey.y, ez.y, (bz.y - bym_z.y) - (by.y - bp_y.y), (bx.y - bp_x.y) - (bz.y - bz.x),
-                         (by.y - by.x) - (bx.y - bym_x.y), cb, pxy1 || pz, B1, B2, B4, iz, hz, xa + 1, y, z, scene);
+            sts2(sb, bx);
+            sts2(sb + SBC, by);
+            sts2(sb + 2 * SBC, bz);
+            if (emit) {
                 const uint64_t evict_first = evict_first_policy();
-                if (o1) {
+                if (full) {
+                    st_pair(a.nbx + off, bx, evict_first);
+                    st_pair(a.nby + off, by, evict_first);
+                    st_pair(a.nbz + off, bz, evict_first);
+                } else {
+                    st_cells(a.nbx + off, bx, o0, o1, evict_first);
+                    st_cells(a.nby + off, by, o0, o1, evict_first);
+                    st_cells(a.nbz + off, bz, o0, o1, evict_first);
+                }
+            }
+            plane_sync<TY>();
+            const bool quit = *stop == iter + 1;
+            if (emit) {
+                // update_E.comp:41-64 for both cells
+                const float bxm_y = sb[SBC - 1], bxm_z = sb[2 * SBC - 1];                 // B(xa-1).y, .z
+                const pair_t bym_x = lds2(sb - W), bym_z = lds2(sb + 2 * SBC - W);          // B(y-1).x, .z
+                const pair_t cx = sub2(sub2(bz, bym_z), sub2(by, bpy));
+                const pair_t cy = sub2(sub2(bx, bpx), sub2(bz, pk(bxm_z, lo_of(bz))));
+                const pair_t cz = sub2(sub2(by, pk(bxm_y, lo_of(by))), sub2(bx, bym_x));
+                pair_t ex, ey, ez;
+                if (!pml) {
+                    if (!mat) {  // vacuum: ca = 1 and cb = dt exactly, so 1 * e + dt * curl == e + dt * curl
+                        ex = add2(e0x, mul2(dt2, cx, mz));
+                        ey = add2(e0y, mul2(dt2, cy, mz));
+                        ez = add2(e0z, mul2(dt2, cz, mz));
+                    } else {
+                        const float4 p0 = __ldg(a.tabE + 2 * ca), p1 = __ldg(a.tabE + 2 * ca + 1);
+                        const float4 q0 = __ldg(a.tabE + 2 * cb), q1 = __ldg(a.tabE + 2 * cb + 1);
+                        ex = add2(mul2(pk(p0.x, q0.x), e0x, mz), mul2(pk(p0.w, q0.w), cx, mz));
+                        ey = add2(mul2(pk(p0.y, q0.y), e0y, mz), mul2(pk(p1.x, q1.x), cy, mz));
+                        ez = add2(mul2(pk(p0.z, q0.z), e0z, mz), mul2(pk(p1.y, q1.y), cz, mz));
+                    }
+                } else if (!mat) {
+                    pair_t d, g;
+                    coef_pair(a, A.r2 + z_iz(zi), B.r2 + z_iz(zi), same, d, g);
+                    ex = add2(mul2(d, e0x, mz), mul2(g, cx, mz));
+                    coef_pair(a, A.r1 + z_iz(zi), B.r1 + z_iz(zi), same, d, g);
+                    ey = add2(mul2(d, e0y, mz), mul2(g, cy, mz));
+                    coef_pair(a, A.r4 + z_hz(zi), B.r4 + z_hz(zi), same, d, g);
+                    ez = add2(mul2(d, e0z, mz), mul2(g, cz, mz));
+                } else {
+                    float x0 = lo_of(e0x), y0 = lo_of(e0y), z0 = lo_of(e0z), x1 = hi_of(e0x), y1 = hi_of(e0y),
+                          z1 = hi_of(e0z);
+                    if (o0)
+                        e_update(a, x0, y0, z0, lo_of(cx), lo_of(cy), lo_of(cz), ca, pxy0 || (zi & 1), A.r1, A.r2, A.r4,
+                                 z_iz(zi), z_hz(zi), xa, y, z, it.scene);
+                    if (o1)
+                        e_update(a, x1, y1, z1, hi_of(cx), hi_of(cy), hi_of(cz), cb, pxy1 || (zi & 1), B.r1, B.r2, B.r4,
+                                 z_iz(zi), z_hz(zi), xa + 1, y, z, it.scene);
+                    ex = pk(x0, x1), ey = pk(y0, y1), ez = pk(z0, z1);
+                }
+                const uint64_t evict_first = evict_first_policy();
+                if (full) {
                     st_pair(a.nex + off, ex, evict_first);
                     st_pair(a.ney + off, ey, evict_first);
                     st_pair(a.nez + off, ez, evict_first);
                 } else {
-                    st_one(a.nex + off, ex.x, evict_first);
-                    st_one(a.ney + off, ey.x, evict_first);
-                    st_one(a.nez + off, ez.x, evict_first);
+                    st_cells(a.nex + off, ex, o0, o1, evict_first);
+                    st_cells(a.ney + off, ey, o0, o1, evict_first);
+                    st_cells(a.nez + off, ez, o0, o1, evict_first);
                 }
             }
-            bp_x = bx, bp_y = by;
-            iz = iz_n, hz = hz_n;
+            if (quit) return;
+            bpx = bx, bpy = by;
+            e0x = ezx, e0y = ezy;
+            zi = zn;
         }
         ++k;  // the item's last load (plane ze) was only read as the z+1 neighbour
     }
@@ -878,8 +1024,7 @@ PairSched pair_schedule(const YeeArgs& a, int TY, int G) {
 }
 
 template <int TY, typename Idx>
-bool launch_p(const YeeArgs& a, const TmaMaps* m, int gen, unsigned* err, cudaStream_t s,
-              unsigned long long* tickets) {
+bool launch_p(const YeeArgs& a, const TmaMaps* m, int gen, unsigned* err, cudaStream_t s) {
     using Lay = Layout2<TY, Idx>;
     static int resident = 0, sms = 0;  // per process: one device model
     std::unique_lock<std::mutex> lk(g_launch_setup);
@@ -894,9 +1039,9 @@ bool launch_p(const YeeArgs& a, const TmaMaps* m, int gen, unsigned* err, cudaSt
             cudaFuncSetAttribute(yee_tma2<TY, Idx>, cudaFuncAttributeMaxDynamicSharedMemorySize, Lay::SMEM) !=
                 cudaSuccess ||
             cudaFuncSetAttribute(yee_tma2<TY, Idx>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 std::min(100, (100 * (TY == 4 ? 4 : (TY == 8 ? 2 : 1)) * (Lay::SMEM + 1024) +
+                                 std::min(100, (100 * Lay::CTAS * (Lay::SMEM + 1024) +
                                                 smem_sm - 1) / smem_sm)) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, yee_tma2<TY, Idx>, 32 * (TY + 1), Lay::SMEM) !=
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, yee_tma2<TY, Idx>, 32 * (TY + 2), Lay::SMEM) !=
                 cudaSuccess ||
             resident < 1) {
             resident = 0;
@@ -914,11 +1059,10 @@ bool launch_p(const YeeArgs& a, const TmaMaps* m, int gen, unsigned* err, cudaSt
     }
     if (ps.items <= 0) return false;
     const int grid = std::min(ps.items, resident * sms);
-    ps.work = a.work, ps.base = a.work_base;
-    yee_tma2<TY, Idx><<<grid, dim3(32, TY + 1), Lay::SMEM, s>>>(m->e[gen][0], m->e[gen][1], m->e[gen][2],
+    ps.work = a.work;
+    yee_tma2<TY, Idx><<<grid, dim3(32, TY + 2), Lay::SMEM, s>>>(m->e[gen][0], m->e[gen][1], m->e[gen][2],
                                                                m->b[gen][0], m->b[gen][1], m->b[gen][2], m->cls, a,
                                                                ps, err);
-    *tickets = (unsigned long long)ps.items + (unsigned long long)grid;
     return true;
 }
 
@@ -994,19 +1138,17 @@ std::vector<int4> ragged_items(const std::vector<int>& z0, const std::vector<int
     return out;
 }
 
-bool launch_yee_tma(const YeeArgs& a, const TmaMaps* m, int gen, bool wide, unsigned* err, cudaStream_t s,
-                    unsigned long long* tickets) {
-    *tickets = 0;
+bool launch_yee_tma(const YeeArgs& a, const TmaMaps* m, int gen, bool wide, unsigned* err, cudaStream_t s) {
     if (!m || !m->ok[gen] || !m->cls_ok) return false;
     if (pair_tiles(a) && tile_rows(a) == 16)
-        return wide ? launch_p<16, uint32_t>(a, m, gen, err, s, tickets)
-                    : launch_p<16, uint16_t>(a, m, gen, err, s, tickets);
+        return wide ? launch_p<16, uint32_t>(a, m, gen, err, s)
+                    : launch_p<16, uint16_t>(a, m, gen, err, s);
     if (pair_tiles(a) && tile_rows(a) == 4)
-        return wide ? launch_p<4, uint32_t>(a, m, gen, err, s, tickets)
-                    : launch_p<4, uint16_t>(a, m, gen, err, s, tickets);
+        return wide ? launch_p<4, uint32_t>(a, m, gen, err, s)
+                    : launch_p<4, uint16_t>(a, m, gen, err, s);
     if (pair_tiles(a))
-        return wide ? launch_p<8, uint32_t>(a, m, gen, err, s, tickets)
-                    : launch_p<8, uint16_t>(a, m, gen, err, s, tickets);
+        return wide ? launch_p<8, uint32_t>(a, m, gen, err, s)
+                    : launch_p<8, uint16_t>(a, m, gen, err, s);
     if (tile_rows(a) == 16) return wide ? launch_t<16, uint32_t>(a, m, gen, err, s) : launch_t<16, uint16_t>(a, m, gen, err, s);
     return wide ? launch_t<8, uint32_t>(a, m, gen, err, s) : launch_t<8, uint16_t>(a, m, gen, err, s);
 }
