@@ -43,7 +43,7 @@ struct YeeArgs {
     const float* pml;   // [6][pml_stride]: I_x, I_y, I_z (integer positions), H_x, H_y, H_z (half)
     int pml_stride;
     const unsigned char* pml_cls;  // [6][pml_stride]: depth class of each position (same order)
-    const float2* pml_coef;        // [K][K][K]: (e^{-x}, dt phi(x)), x = dt ((V_i + V_j) + V_k)
+    const float2* pml_coef;        // [K][K][K] (z, y, x class): (e^{-x}, dt phi(x)), x = dt ((V_i + V_j) + V_k)
     const unsigned char* pml_z;    // [nz]: 1 where the plane lies in the absorber along z (common.glsl:40-43;
                                    // per scene in a stack of scenes)
     const unsigned* pml_zi;        // [nz]: the plane's bit of pml_z, its integer (bits 8-15) and half-integer

@@ -231,7 +231,7 @@ void pml_class_tables(const emlab_grid_config& c, int stride, std::vector<uint8_
             for (int k = 0; k < K; ++k) {
                 const float sigma = (V[(size_t)i] + V[(size_t)j]) + V[(size_t)k];
                 const float x = sigma * dt;
-                float* e = &coef[(((size_t)i * K + j) * K + k) * 2];
+                float* e = &coef[(((size_t)k * K + j) * K + i) * 2];  // x class fastest: a row's lanes share lines
                 e[0] = emlab_expf(-x);
                 e[1] = dt * emlab_phi(x);
             }

@@ -36,7 +36,7 @@ __device__ __forceinline__ PmlIdx pml_idx(const YeeArgs& a, int x, int y, int z)
 }
 
 __device__ __forceinline__ float2 pml_coef(const YeeArgs& a, int i, int j, int k) {
-    return __ldg(a.pml_coef + (i * a.pml_K + j) * a.pml_K + k);
+    return __ldg(a.pml_coef + (k * a.pml_K + j) * a.pml_K + i);
 }
 
 // E update inside the absorber for a non-vacuum edge material (update_E.comp:51-64).

@@ -24,8 +24,9 @@
 namespace emlab {
 
 struct TmaMaps {
-    CUtensorMap e[2][3];
+    CUtensorMap e[2][3];   // single-cell tiles: one map per component
     CUtensorMap b[2][3];
+    CUtensorMap e3[2], b3[2];  // pair tiles: the three components of E, of B, as the fourth dimension
     CUtensorMap cls;
     bool ok[2] = {false, false};
     bool cls_ok = false;
@@ -66,6 +67,15 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
         "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
         "[%5];" ::"r"(smem_u32(dst)),
         "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+        : "memory");
+}
+
+// One copy of a tile's plane of all three components (component index 0 of the map's last dimension).
+__device__ __forceinline__ void tma_load_3comp(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
+        "[%6];" ::"r"(smem_u32(dst)),
+        "l"(map), "r"(x), "r"(y), "r"(z), "r"(0), "r"(smem_u32(bar))
         : "memory");
 }
 
@@ -179,7 +189,7 @@ __global__ void __launch_bounds__(32 * (TY + 1), TY <= 8 ? 3 : 1)
     auto pml_rows = [&](int px, int py, int& R1, int& R2, int& R3, int& R4) {
         const int ix = __ldg(pcls + px), iy = __ldg(pcls + PS + py), hx = __ldg(pcls + 3 * PS + px),
                   hy = __ldg(pcls + 4 * PS + py);
-        R1 = (ix * K + hy) * K, R2 = (hx * K + iy) * K, R3 = (hx * K + hy) * K, R4 = (ix * K + iy) * K;
+        R1 = hy * K + ix, R2 = iy * K + hx, R3 = hy * K + hx, R4 = iy * K + ix;
     };
     auto pml_xy_of = [&](int px, int py) { return px < L || py < L || px >= a.nx - (L + 1) || py >= a.ny - (L + 1); };
     int R1 = 0, R2 = 0, R3 = 0, R4 = 0, C1 = 0, C2 = 0, C3 = 0, C4 = 0;
@@ -202,7 +212,7 @@ __global__ void __launch_bounds__(32 * (TY + 1), TY <= 8 ? 3 : 1)
         const bool emit = z >= zs;
         const int buf = rel & 1;
         const bool pz = __ldg(a.pml_z + z) != 0;
-        const int iz = __ldg(pcls + 2 * PS + z), hz = __ldg(pcls + 5 * PS + z);
+        const int iz = __ldg(pcls + 2 * PS + z) * K * K, hz = __ldg(pcls + 5 * PS + z) * K * K;  // table planes
         const float* Es = reinterpret_cast<const float*>(st + Lay::E_OFF);
         const float* E1 = reinterpret_cast<const float*>(st1 + Lay::E_OFF);
         const float* Bs = reinterpret_cast<const float*>(st + Lay::B_OFF);
@@ -349,30 +359,34 @@ __global__ void __launch_bounds__(32 * (TY + 1), TY <= 8 ? 3 : 1)
 //    the same bits), a row that touches the absorber reads the (e^-x, dt phi) table in every lane
 //    (class 0 outside the layer is (1, dt) again); only rows with non-vacuum cells inside the
 //    absorber, and rows with a thin-wire cell, branch per lane;
+//  * outside the z layers the coefficients of a cell of the x / y layers do not change along z: they
+//    are read once per item and kept in shared memory as the packed operands (one 16-byte load each);
 //  * E(z+1).x and .y, read for B at plane z, stay in registers as plane z+1's own E;
-//  * the -y halo row, the -x halo column and the copies have warps of their own (TY, TY+1), so no
-//    own warp waits for two halo updates in a row.
+//  * the halo (row y0-1 and column x0-1) and the copies have warps of their own (TY, TY+1). Issuing a
+//    copy takes its thread about a hundred cycles, so a plane's E and B are one copy each (the three
+//    components are the fourth dimension of the tensor map): three copies a plane instead of seven,
+//    and nothing else in that warp's way; it was the longest chain of the plane.
 template <int TY, typename Idx>
 struct Layout2 {
-    static constexpr int STAGES = TY == 8 ? 4 : 5;
+    static constexpr int STAGES = 4;
     static constexpr int W = 72;                        // box row width of E, B and the class index
     static constexpr int CX = sizeof(Idx) == 2 ? 8 : 4;  // boxes start at x0 - 4 (16-bit class: x0 - 8)
     static constexpr int DC = CX - 4;                   // class element offset from the E/B element
-    static constexpr int E_BYTES = W * (TY + 2) * 4;    // rows y0-1 .. y0+TY
-    static constexpr int B_BYTES = W * (TY + 1) * 4;    // rows y0-1 .. y0+TY-1
+    static constexpr int EP = W * (TY + 2) * 4;         // one component: rows y0-1 .. y0+TY
+    static constexpr int BP = W * (TY + 1) * 4;         // rows y0-1 .. y0+TY-1
     static constexpr int C_BYTES = W * (TY + 1) * (int)sizeof(Idx);
-    static constexpr int EP = (E_BYTES + 127) / 128 * 128;
-    static constexpr int BP = (B_BYTES + 127) / 128 * 128;
-    static constexpr int CP = (C_BYTES + 127) / 128 * 128;
-    static constexpr int E_OFF = 0;
-    static constexpr int B_OFF = 3 * EP;
-    static constexpr int C_OFF = B_OFF + 3 * BP;
-    static constexpr int STAGE = C_OFF + CP;
-    static constexpr uint32_t TX_BYTES = 3 * E_BYTES + 3 * B_BYTES + C_BYTES;
+    static constexpr int E_OFF = 0;                     // the three components of a copy lie back to back
+    static constexpr int B_OFF = (3 * EP + 127) / 128 * 128;
+    static constexpr int C_OFF = B_OFF + (3 * BP + 127) / 128 * 128;
+    static constexpr int STAGE = C_OFF + (C_BYTES + 127) / 128 * 128;
+    static constexpr uint32_t TX_BYTES = 3 * EP + 3 * BP + C_BYTES;
     // B tile row: element e of a box row maps to slot e - 2 (col 1 = x0-1, col 2+i = x0+i)
     static constexpr int SB_OFF = STAGES * STAGE;
     static constexpr int SB_BYTES = 2 * 3 * (TY + 1) * W * 4;
-    static constexpr int BAR_OFF = (SB_OFF + SB_BYTES + 127) / 128 * 128;
+    // absorber coefficients of every own pair outside the z layers: [entry r1..r4][thread]{decay, gain}
+    static constexpr int COEF_OFF = (SB_OFF + SB_BYTES + 127) / 128 * 128;
+    static constexpr int COEF_BYTES = 4 * 32 * TY * 16;
+    static constexpr int BAR_OFF = COEF_OFF + COEF_BYTES;
     static constexpr int QUEUE_OFF = BAR_OFF + 8 * STAGES;  // item numbers [8], -1 = done
     static constexpr int STOP_OFF = QUEUE_OFF + 8 * 4;       // barrier after which every warp leaves, -1 = none
     static constexpr int SMEM = STOP_OFF + 16;
@@ -461,30 +475,6 @@ __device__ __forceinline__ void coef_pair(const YeeArgs& a, int ia, int ib, bool
     decay = pk(ka.x, kb.x), gain = pk(ka.y, kb.y);
 }
 
-// B^{n+1/2} of one cell outside/inside the absorber from its curl terms (update_B.comp:47-67).
-__device__ __forceinline__ void b_update(const YeeArgs& a, float& bx, float& by, float& bz, float t0x, float t0y,
-                                         float t0z, float t1x, float t1y, float t1z, unsigned c, bool inp, int R1,
-                                         int R2, int R3, int iz, int hz) {
-    if (c >= a.wire_start) {
-        const float4 w0 = __ldg(a.tabW + 2 * c), w1 = __ldg(a.tabW + 2 * c + 1);
-        t0x = t0x * w0.x, t0y = t0y * w0.y, t0z = t0z * w0.z;
-        t1x = t1x * w0.w, t1y = t1y * w1.x, t1z = t1z * w1.y;
-    }
-    const float cx = t0x - t1x, cy = t0y - t1y, cz = t0z - t1z;
-    if (inp) {
-        const float2 kx = __ldg(a.pml_coef + R1 + hz), ky = __ldg(a.pml_coef + R2 + hz),
-                     kz = __ldg(a.pml_coef + R3 + iz);
-        bx = kx.x * bx - kx.y * cx;
-        by = ky.x * by - ky.y * cy;
-        bz = kz.x * bz - kz.y * cz;
-    } else {
-        const float dt = a.dt;
-        bx = bx - dt * cx;
-        by = by - dt * cy;
-        bz = bz - dt * cz;
-    }
-}
-
 // E^{n+1} of one cell from its curl (update_E.comp:41-64).
 __device__ __forceinline__ void e_update(const YeeArgs& a, float& ex, float& ey, float& ez, float cx, float cy,
                                          float cz, unsigned c, bool inp, int R1, int R2, int R4, int iz, int hz, int x,
@@ -551,21 +541,21 @@ __device__ __forceinline__ PairItem pair_item(const PairSched& ps, int nz, int i
     return it;
 }
 
-// Table rows of the depth classes of column (px, py): entry R1 + hz is (ix, hy, hz), R2 + hz is
-// (hx, iy, hz), R3 + iz is (hx, hy, iz), R4 + hz is (ix, iy, hz).
+// Places of the depth classes of column (px, py) in a z plane of the table: r1 is (ix, hy), r2 (hx, iy),
+// r3 (hx, hy), r4 (ix, iy).
 struct PmlRows {
     int r1, r2, r3, r4;
 };
 __device__ __forceinline__ PmlRows pml_rows(const unsigned char* pcx, int SX, int K, int px, int py) {
     const int ix = __ldg(pcx + px), iy = __ldg(pcx + SX + py), hx = __ldg(pcx + 3 * SX + px),
               hy = __ldg(pcx + 4 * SX + py);
-    return {(ix * K + hy) * K, (hx * K + iy) * K, (hx * K + hy) * K, (ix * K + iy) * K};
+    return {hy * K + ix, iy * K + hx, hy * K + hx, iy * K + ix};
 }
 
-// Plane classes along z, packed on the host: bit 0 in the absorber, bits 8-15 the integer depth
-// class, bits 16-23 the half-integer one.
-__device__ __forceinline__ int z_iz(unsigned v) { return (v >> 8) & 0xff; }
-__device__ __forceinline__ int z_hz(unsigned v) { return (v >> 16) & 0xff; }
+// A plane's absorber data, packed on the host: bit 0 in the absorber, bits 8-15 the integer depth
+// class, bits 16-23 the half-integer one; here as the table planes of those classes.
+__device__ __forceinline__ int z_iz(unsigned v, int K) { return (int)((v >> 8) & 0xff) * K * K; }
+__device__ __forceinline__ int z_hz(unsigned v, int K) { return (int)((v >> 16) & 0xff) * K * K; }
 
 template <int TY>
 __device__ __forceinline__ void plane_sync() {  // every warp of the CTA, once per plane
@@ -583,9 +573,7 @@ __device__ __forceinline__ void plane_sync() {  // every warp of the CTA, once p
 // registers at most.
 template <int TY, typename Idx>
 __global__ void __launch_bounds__(32 * (TY + 2), Layout2<TY, Idx>::CTAS)
-    yee_tma2(const __grid_constant__ CUtensorMap tex, const __grid_constant__ CUtensorMap tey,
-             const __grid_constant__ CUtensorMap tez, const __grid_constant__ CUtensorMap tbx,
-             const __grid_constant__ CUtensorMap tby, const __grid_constant__ CUtensorMap tbz,
+    yee_tma2(const __grid_constant__ CUtensorMap te, const __grid_constant__ CUtensorMap tb,
              const __grid_constant__ CUtensorMap tcls, YeeArgs a, PairSched ps, unsigned* err) {
     static_assert(TY == 4 || TY == 8 || TY == 16, "register budget assumes 6, 10 or 18 warps per CTA");
     using Lay = Layout2<TY, Idx>;
@@ -617,7 +605,7 @@ __global__ void __launch_bounds__(32 * (TY + 2), Layout2<TY, Idx>::CTAS)
     };
 
     if (warp == TY + 1) {
-        // ---- copies (lane 0) and the -x halo column: By, Bz of (x0-1, y0+lane), lanes 0 .. TY-1 ----
+        // ---- the copies (lane 0) ----
         const bool leader = lane == 0;
         int p_x = 0, p_y = 0, p_z = 0, p_end = -1;  // the next load: its tile and plane, the item's last plane
         int issued = 0, waited = -1, p_ord = 0;
@@ -632,12 +620,8 @@ __global__ void __launch_bounds__(32 * (TY + 2), Layout2<TY, Idx>::CTAS)
                 unsigned char* st = smem + (issued % S_) * Lay::STAGE;
                 uint64_t* bar = bars + issued % S_;
                 mbar_expect_tx(bar, Lay::TX_BYTES);
-                tma_load_3d(st + Lay::E_OFF + 0 * Lay::EP, &tex, p_x, p_y, p_z, bar);
-                tma_load_3d(st + Lay::E_OFF + 1 * Lay::EP, &tey, p_x, p_y, p_z, bar);
-                tma_load_3d(st + Lay::E_OFF + 2 * Lay::EP, &tez, p_x, p_y, p_z, bar);
-                tma_load_3d(st + Lay::B_OFF + 0 * Lay::BP, &tbx, p_x, p_y, p_z, bar);
-                tma_load_3d(st + Lay::B_OFF + 1 * Lay::BP, &tby, p_x, p_y, p_z, bar);
-                tma_load_3d(st + Lay::B_OFF + 2 * Lay::BP, &tbz, p_x, p_y, p_z, bar);
+                tma_load_3comp(st + Lay::E_OFF, &te, p_x, p_y, p_z, bar);
+                tma_load_3comp(st + Lay::B_OFF, &tb, p_x, p_y, p_z, bar);
                 tma_load_3d(st + Lay::C_OFF, &tcls, p_x - Lay::DC, p_y, p_z, bar);
                 ++issued;
                 // the ticket of the next item is drawn one load ahead (every item has at least two
@@ -679,41 +663,10 @@ __global__ void __launch_bounds__(32 * (TY + 2), Layout2<TY, Idx>::CTAS)
         }
         plane_sync<TY>();
         if (*stop == 0) return leave(true);
-        const int ce = (lane + 1) * W + 3;
         int k = 0, iter = 0;
         for (int ord = 0, item = queue[0]; item >= 0; item = queue[++ord & 7]) {
             const PairItem it = pair_item<TY>(ps, a.nz, item);
-            int snx, sny;
-            scene_size(it.scene, snx, sny);
-            const int cy = it.y0 + lane;
-            const bool live = lane < TY && it.x0 > 0 && cy < sny;
-            PmlRows r{};
-            bool inxy = false;
-            if (live) {
-                r = pml_rows(a.pml_cls_xy + (long long)it.scene * a.pml_xy_scene, SX, K, it.x0 - 1, cy);
-                inxy = it.x0 - 1 < L || cy < L || it.x0 - 1 >= snx - (L + 1) || cy >= sny - (L + 1);
-            }
-            unsigned zi = __ldg(a.pml_zi + it.zstart);
             for (int z = it.zstart; z < it.ze; ++z, ++k, ++iter) {
-                const unsigned char* st = smem + (k % S_) * Lay::STAGE;
-                const unsigned zn = __ldg(a.pml_zi + min(z + 1, a.nz - 1));
-                if (z >= it.zs && lane < TY) {
-                    float* sb = sB + (iter & 1) * 3 * SBC - 2;  // indexed by box element
-                    float hby = 0.0f, hbz = 0.0f, hbx = 0.0f;   // B below the lower face is 0
-                    if (live) {
-                        const float* Es = reinterpret_cast<const float*>(st + Lay::E_OFF);
-                        const float* E1 = reinterpret_cast<const float*>(smem + ((k + 1) % S_) * Lay::STAGE + Lay::E_OFF);
-                        const float* Bs = reinterpret_cast<const float*>(st + Lay::B_OFF);
-                        const Idx* Cs = reinterpret_cast<const Idx*>(st + Lay::C_OFF) + Lay::DC;
-                        const float f0x = Es[ce], f0y = Es[EPF + ce], f0z = Es[2 * EPF + ce];
-                        hby = Bs[BPF + ce], hbz = Bs[2 * BPF + ce];
-                        b_update(a, hbx, hby, hbz, 0.0f, E1[ce] - f0x, Es[EPF + ce + 1] - f0y, 0.0f,
-                                 Es[2 * EPF + ce + 1] - f0z, Es[ce + W] - f0x, (unsigned)Cs[ce], inxy || (zi & 1),
-                                 r.r1, r.r2, r.r3, z_iz(zi), z_hz(zi));
-                    }
-                    sb[SBC + ce] = hby;
-                    sb[2 * SBC + ce] = hbz;
-                }
                 // the next iteration reads loads k+1, k+2 (or k+2, k+3 at the start of the next item,
                 // which was taken when the last load of this one was issued)
                 if (leader) {
@@ -727,7 +680,6 @@ __global__ void __launch_bounds__(32 * (TY + 2), Layout2<TY, Idx>::CTAS)
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     issue_upto(k + S_);
                 }
-                zi = zn;
             }
             ++k;  // the item's last load (plane ze) was only read as the z+1 neighbour
         }
@@ -741,7 +693,7 @@ __global__ void __launch_bounds__(32 * (TY + 2), Layout2<TY, Idx>::CTAS)
     if (*stop == 0) return;
     // box element of the own / halo-row pair (E, B and 32-bit class boxes share it; the 16-bit class
     // box is DC elements further); B tile slot = element - 2
-    const bool row = warp == TY;  // the -y halo row: Bx, Bz of (xa, y0-1), (xa+1, y0-1)
+    const bool row = warp == TY;  // the halo warp; its row: Bx, Bz of (xa, y0-1), (xa+1, y0-1)
     const int me = (row ? 0 : warp + 1) * W + 2 * lane + 4;
     const pair_t dt2 = pk(a.dt, a.dt), mz = pk(a.minus_zero, a.minus_zero);
     int k = 0;     // load index of the current iteration's plane z
@@ -767,18 +719,39 @@ __global__ void __launch_bounds__(32 * (TY + 2), Layout2<TY, Idx>::CTAS)
         unsigned zi = __ldg(a.pml_zi + it.zstart);
 
         if (row) {
+            // the -x halo column too: By, Bz of (x0-1, y0 + lane), lanes 0 .. TY-1 (the others repeat the
+            // last one). Its cells always read the table: (1, dt) outside the layer
+            const int cl = min(lane, TY - 1), ce = (cl + 1) * W + 3;
+            const bool clive = it.x0 > 0 && it.y0 + cl < sny;
+            PmlRows C{};
+            if (clive) C = pml_rows(pcx, SX, K, it.x0 - 1, it.y0 + cl);
             for (int z = it.zstart; z < it.ze; ++z, ++k, ++iter) {
                 const unsigned char* st = smem + (k % S_) * Lay::STAGE;
                 const unsigned zn = __ldg(a.pml_zi + min(z + 1, a.nz - 1));
                 if (z >= it.zs) {
                     float* sb = sB + (iter & 1) * 3 * SBC - 2;
+                    const float* Es = reinterpret_cast<const float*>(st + Lay::E_OFF);
+                    const float* E1 = reinterpret_cast<const float*>(smem + ((k + 1) % S_) * Lay::STAGE + Lay::E_OFF);
+                    const float* Bs = reinterpret_cast<const float*>(st + Lay::B_OFF);
+                    const Idx* Cs = reinterpret_cast<const Idx*>(st + Lay::C_OFF) + Lay::DC;
+                    {
+                        const unsigned hc = (unsigned)Cs[ce];
+                        const float2 ky = __ldg(a.pml_coef + C.r2 + z_hz(zi, K)), kz = __ldg(a.pml_coef + C.r3 + z_iz(zi, K));
+                        const float f0x = Es[ce], f0y = Es[EPF + ce], f0z = Es[2 * EPF + ce];
+                        float t0y = E1[ce] - f0x, t0z = Es[EPF + ce + 1] - f0y, t1y = Es[2 * EPF + ce + 1] - f0z,
+                              t1z = Es[ce + W] - f0x;
+                        if (__any_sync(0xffffffffu, hc >= a.wire_start)) {
+                            const float4 w0 = __ldg(a.tabW + 2 * hc), w1 = __ldg(a.tabW + 2 * hc + 1);
+                            t0y = t0y * w0.y, t0z = t0z * w0.z, t1y = t1y * w1.x, t1z = t1z * w1.y;
+                        }
+                        const float hby = ky.x * Bs[BPF + ce] - ky.y * (t0y - t1y);
+                        const float hbz = kz.x * Bs[2 * BPF + ce] - kz.y * (t0z - t1z);
+                        if (lane < TY) sb[SBC + ce] = clive ? hby : 0.0f, sb[2 * SBC + ce] = clive ? hbz : 0.0f;
+                    }
                     pair_t hx2 = 0, hz2 = 0;  // B below the lower face is 0
                     if (rowok) {
-                        const float* Es = reinterpret_cast<const float*>(st + Lay::E_OFF);
-                        const float* E1 = reinterpret_cast<const float*>(smem + ((k + 1) % S_) * Lay::STAGE + Lay::E_OFF);
-                        const float* Bs = reinterpret_cast<const float*>(st + Lay::B_OFF);
                         unsigned ha, hb;
-                        load_class_pair<Idx>(reinterpret_cast<const Idx*>(st + Lay::C_OFF) + Lay::DC + me, ha, hb);
+                        load_class_pair<Idx>(Cs + me, ha, hb);
                         const pair_t f0x = lds2(Es + me), f0y = lds2(Es + EPF + me), f0z = lds2(Es + 2 * EPF + me);
                         pair_t t0x = sub2(lds2(Es + 2 * EPF + me + W), f0z), t1x = sub2(lds2(E1 + EPF + me), f0y);
                         pair_t t0z = sub2(pk(hi_of(f0y), Es[EPF + me + 2]), f0y), t1z = sub2(lds2(Es + me + W), f0x);
@@ -792,9 +765,9 @@ __global__ void __launch_bounds__(32 * (TY + 2), Layout2<TY, Idx>::CTAS)
                         hx2 = lds2(Bs + me), hz2 = lds2(Bs + 2 * BPF + me);
                         if (pmlrow || (zi & 1)) {
                             pair_t d, g;
-                            coef_pair(a, A.r1 + z_hz(zi), B.r1 + z_hz(zi), same, d, g);
+                            coef_pair(a, A.r1 + z_hz(zi, K), B.r1 + z_hz(zi, K), same, d, g);
                             hx2 = sub2(mul2(d, hx2, mz), mul2(g, cx, mz));
-                            coef_pair(a, A.r3 + z_iz(zi), B.r3 + z_iz(zi), same, d, g);
+                            coef_pair(a, A.r3 + z_iz(zi, K), B.r3 + z_iz(zi, K), same, d, g);
                             hz2 = sub2(mul2(d, hz2, mz), mul2(g, cz, mz));
                         } else {
                             hx2 = sub2(hx2, mul2(dt2, cx, mz));
@@ -813,6 +786,14 @@ __global__ void __launch_bounds__(32 * (TY + 2), Layout2<TY, Idx>::CTAS)
         }
 
         const bool full = __all_sync(0xffffffffu, o1);
+        ulonglong2* coef = reinterpret_cast<ulonglong2*>(smem + Lay::COEF_OFF) + warp * 32 + lane;  // + entry * 32 TY
+        if (pmlrow) {  // the thread's own slots: no other thread reads them
+            pair_t d, g;
+            coef_pair(a, A.r1, B.r1, same, d, g), coef[0] = make_ulonglong2(d, g);
+            coef_pair(a, A.r2, B.r2, same, d, g), coef[32 * TY] = make_ulonglong2(d, g);
+            coef_pair(a, A.r3, B.r3, same, d, g), coef[64 * TY] = make_ulonglong2(d, g);
+            coef_pair(a, A.r4, B.r4, same, d, g), coef[96 * TY] = make_ulonglong2(d, g);
+        }
         long long off = (long long)it.zstart * a.plane + (long long)y * a.pitch + xa;
         pair_t bpx = 0, bpy = 0;  // B^{n+1/2}(z-1).x, .y of the pair
         const float* E0 = reinterpret_cast<const float*>(smem + (k % S_) * Lay::STAGE + Lay::E_OFF) + me;
@@ -845,18 +826,25 @@ __global__ void __launch_bounds__(32 * (TY + 2), Layout2<TY, Idx>::CTAS)
             const bool pml = pmlrow || (zi & 1);
             {
                 const pair_t cx = sub2(t0x, t1x), cy = sub2(t0y, t1y), cz = sub2(t0z, t1z);
-                if (pml) {
-                    pair_t d, g;
-                    coef_pair(a, A.r1 + z_hz(zi), B.r1 + z_hz(zi), same, d, g);
-                    bx = sub2(mul2(d, bx, mz), mul2(g, cx, mz));
-                    coef_pair(a, A.r2 + z_hz(zi), B.r2 + z_hz(zi), same, d, g);
-                    by = sub2(mul2(d, by, mz), mul2(g, cy, mz));
-                    coef_pair(a, A.r3 + z_iz(zi), B.r3 + z_iz(zi), same, d, g);
-                    bz = sub2(mul2(d, bz, mz), mul2(g, cz, mz));
+                if (!(zi & 1)) {
+                    if (pmlrow) {
+                        const ulonglong2 k1 = coef[0], k2 = coef[32 * TY], k3 = coef[64 * TY];
+                        bx = sub2(mul2(k1.x, bx, mz), mul2(k1.y, cx, mz));
+                        by = sub2(mul2(k2.x, by, mz), mul2(k2.y, cy, mz));
+                        bz = sub2(mul2(k3.x, bz, mz), mul2(k3.y, cz, mz));
+                    } else {
+                        bx = sub2(bx, mul2(dt2, cx, mz));
+                        by = sub2(by, mul2(dt2, cy, mz));
+                        bz = sub2(bz, mul2(dt2, cz, mz));
+                    }
                 } else {
-                    bx = sub2(bx, mul2(dt2, cx, mz));
-                    by = sub2(by, mul2(dt2, cy, mz));
-                    bz = sub2(bz, mul2(dt2, cz, mz));
+                    pair_t d, g;
+                    coef_pair(a, A.r1 + z_hz(zi, K), B.r1 + z_hz(zi, K), same, d, g);
+                    bx = sub2(mul2(d, bx, mz), mul2(g, cx, mz));
+                    coef_pair(a, A.r2 + z_hz(zi, K), B.r2 + z_hz(zi, K), same, d, g);
+                    by = sub2(mul2(d, by, mz), mul2(g, cy, mz));
+                    coef_pair(a, A.r3 + z_iz(zi, K), B.r3 + z_iz(zi, K), same, d, g);
+                    bz = sub2(mul2(d, bz, mz), mul2(g, cz, mz));
                 }
             }
             sts2(sb, bx);
@@ -896,23 +884,28 @@ __global__ void __launch_bounds__(32 * (TY + 2), Layout2<TY, Idx>::CTAS)
                         ey = add2(mul2(pk(p0.y, q0.y), e0y, mz), mul2(pk(p1.x, q1.x), cy, mz));
                         ez = add2(mul2(pk(p0.z, q0.z), e0z, mz), mul2(pk(p1.y, q1.y), cz, mz));
                     }
+                } else if (!mat && !(zi & 1)) {
+                    const ulonglong2 k2 = coef[32 * TY], k1 = coef[0], k4 = coef[96 * TY];
+                    ex = add2(mul2(k2.x, e0x, mz), mul2(k2.y, cx, mz));
+                    ey = add2(mul2(k1.x, e0y, mz), mul2(k1.y, cy, mz));
+                    ez = add2(mul2(k4.x, e0z, mz), mul2(k4.y, cz, mz));
                 } else if (!mat) {
                     pair_t d, g;
-                    coef_pair(a, A.r2 + z_iz(zi), B.r2 + z_iz(zi), same, d, g);
+                    coef_pair(a, A.r2 + z_iz(zi, K), B.r2 + z_iz(zi, K), same, d, g);
                     ex = add2(mul2(d, e0x, mz), mul2(g, cx, mz));
-                    coef_pair(a, A.r1 + z_iz(zi), B.r1 + z_iz(zi), same, d, g);
+                    coef_pair(a, A.r1 + z_iz(zi, K), B.r1 + z_iz(zi, K), same, d, g);
                     ey = add2(mul2(d, e0y, mz), mul2(g, cy, mz));
-                    coef_pair(a, A.r4 + z_hz(zi), B.r4 + z_hz(zi), same, d, g);
+                    coef_pair(a, A.r4 + z_hz(zi, K), B.r4 + z_hz(zi, K), same, d, g);
                     ez = add2(mul2(d, e0z, mz), mul2(g, cz, mz));
                 } else {
                     float x0 = lo_of(e0x), y0 = lo_of(e0y), z0 = lo_of(e0z), x1 = hi_of(e0x), y1 = hi_of(e0y),
                           z1 = hi_of(e0z);
                     if (o0)
                         e_update(a, x0, y0, z0, lo_of(cx), lo_of(cy), lo_of(cz), ca, pxy0 || (zi & 1), A.r1, A.r2, A.r4,
-                                 z_iz(zi), z_hz(zi), xa, y, z, it.scene);
+                                 z_iz(zi, K), z_hz(zi, K), xa, y, z, it.scene);
                     if (o1)
                         e_update(a, x1, y1, z1, hi_of(cx), hi_of(cy), hi_of(cz), cb, pxy1 || (zi & 1), B.r1, B.r2, B.r4,
-                                 z_iz(zi), z_hz(zi), xa + 1, y, z, it.scene);
+                                 z_iz(zi, K), z_hz(zi, K), xa + 1, y, z, it.scene);
                     ex = pk(x0, x1), ey = pk(y0, y1), ez = pk(z0, z1);
                 }
                 const uint64_t evict_first = evict_first_policy();
@@ -969,6 +962,19 @@ bool encode(CUtensorMap* m, CUtensorMapDataType type, int elem, const void* base
 
 // tiling modes: 8, 16 = 32 x TY tiles of single cells (yee_tma); 64, 128 = 64 x 8 and 64 x 16 tiles
 // of cell pairs (yee_tma2)
+// The three component arrays from base, `comp` floats apart, as one map: the copies of the pair tiles.
+bool encode3(CUtensorMap* m, const float* base, long long comp, const YeeArgs& a, int box_h) {
+    EncodeFn fn = encode_fn();
+    if (!fn) return false;
+    const cuuint64_t dims[4] = {(cuuint64_t)a.nx, (cuuint64_t)a.ny, (cuuint64_t)a.nz, 3};
+    const cuuint64_t strides[3] = {(cuuint64_t)a.pitch * 4, (cuuint64_t)a.plane * 4, (cuuint64_t)comp * 4};
+    const cuuint32_t box[4] = {72, (cuuint32_t)box_h, 1, 3};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(base), dims, strides, box, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 int tile_rows(const YeeArgs& a) { return a.tile_rows == 16 || a.tile_rows == 128 ? 16 : (a.tile_rows == 32 ? 4 : 8); }
 bool pair_tiles(const YeeArgs& a) { return a.tile_rows == 32 || a.tile_rows == 64 || a.tile_rows == 128; }
 
@@ -1023,6 +1029,25 @@ PairSched pair_schedule(const YeeArgs& a, int TY, int G) {
     return ps;
 }
 
+// Grids too small for that balance (the rule above leaves fewer than kItemsPerCta items per CTA). An
+// item costs its planes plus about two and a half (the re-read plane and its start); r = items / G
+// rounds of them take a time between r (items of unequal cost even out over the tickets) and the
+// whole rounds, and the last item of a CTA sticks out by most of its length:
+//   cost = (zc + 2.5) (r / 2 + ceil(r) / 2 + 3/4).
+// Measured over thirteen sizes from 48 x 48 x 48 to 320 x 300 x 280 and chunks of 1 to 48 planes, the
+// chunk it picks is within 2.6 % of the best one (worst 13 %): 48 x 48 x 48 one plane (13.0 us a step
+// against 20.7 for the rule above), 211 x 147 x 93 eight (52.0 against 59.7), 192 x 192 x 128 eight
+// (61.0 against 75.2).
+void small_grid_schedule(PairSched& ps, int nz, int G) {
+    double best = -1.0;
+    for (int zc = 1; zc <= nz; ++zc) {
+        const long long items = (long long)((nz + zc - 1) / zc) * ps.tiles;
+        const double r = (double)items / G;
+        const double cost = (zc + 2.5) * (0.5 * r + 0.5 * (double)((items + G - 1) / G) + 0.75);
+        if (best < 0.0 || cost < best) best = cost, ps.zc = zc, ps.items = (int)items;
+    }
+}
+
 template <int TY, typename Idx>
 bool launch_p(const YeeArgs& a, const TmaMaps* m, int gen, unsigned* err, cudaStream_t s) {
     using Lay = Layout2<TY, Idx>;
@@ -1055,14 +1080,13 @@ bool launch_p(const YeeArgs& a, const TmaMaps* m, int gen, unsigned* err, cudaSt
         ps.tab = a.items;
     } else {
         ps = pair_schedule(a, TY, resident * sms);
+        if (ps.items < kItemsPerCta * resident * sms) small_grid_schedule(ps, a.nz, resident * sms);
         ps.tab = nullptr;
     }
     if (ps.items <= 0) return false;
     const int grid = std::min(ps.items, resident * sms);
     ps.work = a.work;
-    yee_tma2<TY, Idx><<<grid, dim3(32, TY + 2), Lay::SMEM, s>>>(m->e[gen][0], m->e[gen][1], m->e[gen][2],
-                                                               m->b[gen][0], m->b[gen][1], m->b[gen][2], m->cls, a,
-                                                               ps, err);
+    yee_tma2<TY, Idx><<<grid, dim3(32, TY + 2), Lay::SMEM, s>>>(m->e3[gen], m->b3[gen], m->cls, a, ps, err);
     return true;
 }
 
@@ -1074,13 +1098,18 @@ void tma_maps_destroy(TmaMaps* m) { delete m; }
 bool tma_maps_encode(TmaMaps* m, int gen, const YeeArgs& a, bool wide) {
     const int ty = tile_rows(a);
     const bool pair = pair_tiles(a);
-    const int ew = pair ? 72 : 40, bw = pair ? 72 : 36, cw16 = pair ? 72 : 40, cw32 = pair ? 72 : 36;
+    const int cw16 = pair ? 72 : 40, cw32 = pair ? 72 : 36;
     bool ok = (a.pitch % 4) == 0;
+    if (pair) {
+        const long long comp = a.ey - a.ex;  // the six arrays of a generation lie one after the other
+        ok = ok && a.ez - a.ex == 2 * comp && a.by - a.bx == comp && a.bz - a.bx == 2 * comp &&
+             encode3(&m->e3[gen], a.ex, comp, a, ty + 2) && encode3(&m->b3[gen], a.bx, comp, a, ty + 1);
+    }
     const float* e[3] = {a.ex, a.ey, a.ez};
     const float* b[3] = {a.bx, a.by, a.bz};
-    for (int c = 0; c < 3 && ok; ++c) {
-        ok = encode(&m->e[gen][c], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, e[c], a, ew, ty + 2) &&
-             encode(&m->b[gen][c], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, b[c], a, bw, ty + 1);
+    for (int c = 0; c < 3 && ok && !pair; ++c) {
+        ok = encode(&m->e[gen][c], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, e[c], a, 40, ty + 2) &&
+             encode(&m->b[gen][c], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, b[c], a, 36, ty + 1);
     }
     if (ok)
         ok = wide ? encode(&m->cls, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, a.cls, a, cw32, ty + 1)

@@ -460,7 +460,8 @@ int emlab_debug_set_wait_limit(int polls);
 /* Evaluates the device emlab_expf on n inputs (bit-exactness check against the host). */
 int emlab_debug_expf(const float* in, float* out, size_t n);
 /* Host-side schedule of the persistent pair kernel (no device needed), for `ctas` resident CTAs and
- * 64 x tile_rows tiles: on a single grid, the planes per z chunk and the number of work items;
+ * 64 x tile_rows tiles: on a single grid, the planes per z chunk and the number of work items (grids
+ * that give fewer than four items per CTA are split further by a rule of their own at the launch);
  * on a stack of scenes with their own cross-sections (emlab_stack_configure_scenes), the work items
  * themselves, 5 ints each (x0, y0, first plane, end plane, scene) in launch order. *n_items receives
  * the count; out may be NULL to query it, else it holds cap items. */
