@@ -3,13 +3,12 @@
 // The network (em_lab_gb300/extrap.py) is a 1-D convolutional encoder of the early port V(t), I(t)
 // and a 4-layer MLP head; every layer is a GEMM with BF16 operands and FP32 accumulation:
 //  * nn_gemm: C[M][N] = sum_k A(m, k) B(n, k) on the tcgen05 tensor cores (kind::f16 with BF16
-//    operands, FP32 accumulator in tensor memory). A CTA of four warps owns a 128 x 128 tile of C;
-//    for each 64-wide K chunk the threads stage A and B (strided loads: the same kernel serves the
-//    forward product X W^T and the backward products dZ W and dZ^T X) into the no-swizzle K-major
-//    core-matrix layout (8 rows x 16 bytes per core matrix, 128 B between core matrices along K,
-//    1024 B between 8-row groups), one thread issues four MMAs of K 16 and commits them to an
-//    mbarrier, and after the last chunk each warp reads its 32 accumulator lanes with tcgen05.ld.
-//    Waits are bounded; on expiry the CTA records an error, frees its tensor memory and leaves.
+//    operands, FP32 accumulator in tensor memory). Any strides: the same kernel serves the forward
+//    product X W^T and the backward products dZ W and dZ^T X. 64-wide K chunks are copied into a ring
+//    of shared-memory stages in the no-swizzle core-matrix layout (K-major, or row-major where the
+//    operand is contiguous along its rows), one thread issues four MMAs of K 16 per chunk and
+//    commits them to the stage's mbarrier. Waits are bounded; on expiry the CTA records an error,
+//    frees its tensor memory and leaves.
 //  * elementwise kernels: bias + ReLU with the BF16 copy for the next layer, ReLU backward, bias
 //    gradients, im2col / col2im of the strided convolutions, the MSE loss gradient, Adam (FP32
 //    master weights, BF16 copies for the GEMMs).
@@ -25,24 +24,45 @@
 namespace emlab {
 namespace {
 
-constexpr int kTM = 128, kTN = 128, kTK = 64;
-constexpr int kTileBytes = kTM * kTK * 2;  // 16 KB per operand tile
-constexpr int kResidencyPad = 24 * 1024;
+constexpr int kTM = 128, kTK = 64;  // tile rows, K chunk (tile columns: 64 or 128)
+constexpr int kThreads = 256;
+// Core matrices (8 x 16 bytes, 128 bytes) of a chunk. K-major (a piece is 8 elements along K of one
+// row): 144 bytes apart along K, 8 x 144 along the rows. Row-major (a piece is 8 rows of one k): 128
+// apart along K, 8 x 128 + 16 along the rows. The padding puts the pieces that eight neighbouring
+// threads copy into different banks.
+constexpr int kLboK = 144, kSboK = 8 * kLboK, kLboR = 128, kSboR = 8 * kLboR + 16;
+constexpr int kABytes = kTM / 8 * kSboK;  // the larger of the two
+constexpr int kMaxStages = 6;
 
 __device__ unsigned g_nn_err;  // nonzero: a bounded wait of nn_gemm expired
 
 __device__ __forceinline__ uint32_t saddr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-__device__ __forceinline__ uint64_t desc_kmajor(const void* p) {
-    // start >> 4, LBO 128 B >> 4 at bit 16, SBO 1024 B >> 4 at bit 32, descriptor version 1 at bit 46
+// start >> 4, leading (along K) offset >> 4 at bit 16, stride (along the rows) offset >> 4 at bit 32,
+// descriptor version 1 at bit 46; no swizzle
+__device__ __forceinline__ uint64_t operand_desc(const void* p, int lbo, int sbo) {
     const uint64_t a = saddr(p);
-    return ((a & 0x3FFFFull) >> 4) | ((uint64_t)(128 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46);
+    return ((a & 0x3FFFFull) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) | (1ull << 46);
 }
 
-// kind::f16 instruction descriptor: D FP32 (bits 4-5 = 1), A and B BF16 (bits 7-9, 10-12 = 1),
-// both K-major, N >> 3 at bits 17-22, M >> 4 at bits 24-28.
-__host__ __device__ constexpr uint32_t bf16_idesc(int m, int n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+// kind::f16 instruction descriptor: D FP32 (bits 4-5 = 1), A and B BF16 (bits 7-9, 10-12 = 1), bit 15 /
+// 16 set where A / B lies row-major (contiguous along M / N), N >> 3 at bits 17-22, M >> 4 at 24-28.
+__host__ __device__ constexpr uint32_t bf16_idesc(int m, int n, bool a_rows, bool b_rows) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | (a_rows ? 1u << 15 : 0u) | (b_rows ? 1u << 16 : 0u) |
+           ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+}
+
+// 16 bytes, of which the first `bytes` are read and the rest is zero.
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(saddr(dst)), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async4(void* dst, const void* src, int bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(saddr(dst)), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
 __device__ __forceinline__ bool wait_bounded(uint64_t* bar, uint32_t parity) {
@@ -73,78 +93,123 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
     for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
 }
 
-// One row (of A or B) of a 64-wide K chunk into the K-major core-matrix layout: the row's eight
-// 16-byte pieces go to (row / 8) * 1024 + piece * 128 + (row % 8) * 16. A row that is contiguous
-// along K and 16-byte aligned (vec) is read as eight 16-byte pieces, all in flight together; any
-// other stride, and the chunk that reaches past K, element by element.
-__device__ __forceinline__ void stage_row(unsigned char* tile, int row, const __nv_bfloat16* src, long long s_k,
-                                          bool live, int k0, int K, bool vec) {
-    const __nv_bfloat16 zero = __float2bfloat16(0.0f);
-    if (vec && k0 + kTK <= K) {
-        uint4 piece[kTK / 8];
+// How an operand (rows x K, element strides s_row, s_k) is read: kRowsK, contiguous along K in
+// 16-byte pieces; kColsK, contiguous along the rows in 16-byte pieces (the transposed products of the
+// backward pass; the tensor core reads it row-major); kAny, element by element.
+enum { kRowsK = 0, kColsK = 1, kAny = 2 };
+
+// One operand's 64-wide K chunk from k0, ROWS rows from row0 of its `rows`, into `tile`. Everything beyond
+// the operand's rows or K is zero; pieces beyond the rows stay so in a stage once `fresh` wrote them.
+template <int ROWS, int MODE>
+__device__ __forceinline__ void stage_operand(unsigned char* tile, const __nv_bfloat16* p, long long s_row,
+                                              long long s_k, int row0, int rows, int k0, int K, bool fresh) {
+    const int t = threadIdx.x;
+    if (MODE == kColsK) {  // piece (k, row block): a warp copies 32 (or 16) neighbouring row blocks of a k
 #pragma unroll
-        for (int j = 0; j < kTK / 8; ++j)
-            piece[j] = live ? __ldg(reinterpret_cast<const uint4*>(src + k0 + j * 8)) : make_uint4(0, 0, 0, 0);
-#pragma unroll
-        for (int j = 0; j < kTK / 8; ++j)
-            *reinterpret_cast<uint4*>(tile + (row >> 3) * 1024 + j * 128 + (row & 7) * 16) = piece[j];
-        return;
-    }
-#pragma unroll
-    for (int j = 0; j < kTK / 8; ++j) {
-        __align__(16) __nv_bfloat16 v[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int k = k0 + j * 8 + q;
-            v[q] = (live && k < K) ? src[(long long)k * s_k] : zero;
+        for (int i = 0; i < ROWS * kTK / 8 / kThreads; ++i) {
+            const int q = t + i * kThreads, block = q % (ROWS / 8), k = q / (ROWS / 8);
+            const int r = row0 + block * 8;
+            if (r >= rows && !fresh) continue;
+            const int live = k0 + k < K ? max(0, min(8, rows - r)) : 0;
+            cp_async16(tile + block * kSboR + (k >> 3) * kLboR + (k & 7) * 16,
+                       live ? p + (long long)(k0 + k) * s_k + r : p, 2 * live);
         }
-        *reinterpret_cast<uint4*>(tile + (row >> 3) * 1024 + j * 128 + (row & 7) * 16) = *reinterpret_cast<uint4*>(v);
+    } else {  // piece (row, K block): eight threads copy a row's 128 bytes
+#pragma unroll
+        for (int i = 0; i < ROWS * kTK / 8 / kThreads; ++i) {
+            const int q = t + i * kThreads, block = q & 7, r = q >> 3, k = k0 + block * 8;
+            if (row0 + r >= rows && !fresh) continue;
+            unsigned char* dst = tile + (r >> 3) * kSboK + block * kLboK + (r & 7) * 16;
+            const int live = row0 + r < rows ? max(0, min(8, K - k)) : 0;
+            const __nv_bfloat16* src = live ? p + (long long)(row0 + r) * s_row + (long long)k * s_k : p;
+            if (MODE == kRowsK) {
+                cp_async16(dst, src, 2 * live);
+            } else {
+                __align__(16) __nv_bfloat16 v[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) v[j] = j < live ? src[j * s_k] : __float2bfloat16(0.0f);
+                *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<uint4*>(v);
+            }
+        }
     }
 }
 
-__global__ void __launch_bounds__(128) nn_gemm_kernel(int M, int N, int K, const __nv_bfloat16* A, long long sam,
-                                                      long long sak, const __nv_bfloat16* B, long long sbn,
-                                                      long long sbk, float* C, long long ldc) {
-    __shared__ __align__(1024) unsigned char sa[kTileBytes];
-    __shared__ __align__(1024) unsigned char sb[kTileBytes];
-    __shared__ uint64_t bar;
+template <int TN>
+__host__ __device__ constexpr int gemm_stage() {
+    return kABytes + TN / 8 * kSboK;
+}
+
+// C[M][N] = sum_k A(m, k) B(n, k), a 128 x TN tile per CTA. What bounds it at the sizes of the network
+// (256 rows: a few CTAs of 4 to 21 chunks; the convolutions' weight gradients, one or four CTAs of 64
+// and 256) is the latency of a chunk's loads, so up to six chunks are in flight (asynchronous copies
+// into a ring, one mbarrier per stage that the MMAs reading it complete) and tiles are narrow where the
+// device is not full. Every layout is copied 16 bytes at a time. The K order of the sum is that of
+// the chunks whatever the tile or the ring, so results do not depend on either.
+template <int TN, int AM, int BM>
+__device__ __forceinline__ void gemm_tile(unsigned char* sm, int m0, int n0, int M, int N, int K,
+                                          const __nv_bfloat16* A, long long sam, long long sak,
+                                          const __nv_bfloat16* B, long long sbn, long long sbk, float* C,
+                                          long long ldc, int stages) {
+    __shared__ uint64_t bar[kMaxStages];  // the MMAs that read stage s have finished
     __shared__ uint32_t tslot;
+    // 1 + the chunk whose barrier everyone leaves after, once a wait ran out (a thread late to read it
+    // after one barrier may already see the next chunk's)
+    __shared__ volatile int stop;
+    constexpr int STAGE = gemm_stage<TN>();
+    constexpr bool ar = AM == kColsK, br = BM == kColsK;
+    constexpr int la = ar ? kLboR : kLboK, sa = ar ? kSboR : kSboK, lb = br ? kLboR : kLboK, sb = br ? kSboR : kSboK;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = blockIdx.x * kTM, n0 = blockIdx.y * kTN;
     if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(saddr(&bar)) : "memory");
+        for (int i = 0; i < stages; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(saddr(&bar[i])) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(&tslot)), "r"(kTN)
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(&tslot)), "r"(TN)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    const int chunks = (K + kTK - 1) / kTK;
+    auto load = [&](int c) {  // one group of copies per chunk, empty past the last
+        if (c < chunks) {
+            unsigned char* st = sm + (c % stages) * STAGE;
+            stage_operand<kTM, AM>(st, A, sam, sak, m0, M, c * kTK, K, c < stages);
+            stage_operand<TN, BM>(st + kABytes, B, sbn, sbk, n0, N, c * kTK, K, c < stages);
+        }
+        cp_commit();
+    };
+    for (int c = 0; c < kMaxStages - 2; ++c)
+        if (c < stages - 2) load(c);
+        else cp_commit();
+    if (tid == 0) stop = 0;
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tslot;
-    constexpr uint32_t idesc = bf16_idesc(kTM, kTN);
+    constexpr uint32_t idesc = bf16_idesc(kTM, TN, ar, br);
 
-    const int am = m0 + tid, bn = n0 + tid;  // the A row and the B row this thread stages
-    const __nv_bfloat16* arow = A + (long long)min(am, M - 1) * sam;
-    const __nv_bfloat16* brow = B + (long long)min(bn, N - 1) * sbn;
-    const bool vec_a = sak == 1 && (sam % 8) == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0;
-    const bool vec_b = sbk == 1 && (sbn % 8) == 0 && (reinterpret_cast<uintptr_t>(B) & 15) == 0;
-    uint32_t phase = 0;
     bool ok = true;
-    const int chunks = (K + kTK - 1) / kTK;
-    for (int c = 0; c < chunks && ok; ++c) {
-        stage_row(sa, tid, arow, sak, am < M, c * kTK, K, vec_a);
-        stage_row(sb, tid, brow, sbk, bn < N, c * kTK, K, vec_b);
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic stores -> tensor-core reads
+    int issued = 0;  // chunks handed to the tensor core
+    for (int c = 0; c < chunks; ++c) {
+        // chunk c - 2's stage takes chunk c - 2 + stages once its MMAs have read it (two chunks back, so
+        // that the wait is over when it is reached)
+        if (c >= 2 && c - 2 + stages < chunks && !wait_bounded(&bar[(c - 2) % stages], ((c - 2) / stages) & 1)) stop = c + 1;
+        load(c - 2 + stages);
+        // this thread's copies of chunk c have landed: those of at most stages - 2 later ones are open
+        if (stages == kMaxStages) cp_wait<kMaxStages - 2>();
+        else cp_wait<1>();
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the copies -> tensor-core reads
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncthreads();
+        if (stop == c + 1) {
+            ok = false;
+            break;
+        }
         if (tid == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            unsigned char* st = sm + (c % stages) * STAGE;
 #pragma unroll
             for (int s = 0; s < kTK / 16; ++s) {
-                const uint64_t ad = desc_kmajor(sa + s * 256), bd = desc_kmajor(sb + s * 256);
+                const uint64_t ad = operand_desc(st + s * 2 * la, la, sa), bd = operand_desc(st + kABytes + s * 2 * lb, lb, sb);
                 const uint32_t acc = (c > 0 || s > 0) ? 1u : 0u;
                 asm volatile(
                     "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -153,50 +218,87 @@ __global__ void __launch_bounds__(128) nn_gemm_kernel(int M, int N, int K, const
                     : "memory");
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                             saddr(&bar))
+                             saddr(&bar[c % stages]))
                          : "memory");
         }
-        ok = wait_bounded(&bar, phase);  // the MMAs have read the tiles: they may be restaged
-        phase ^= 1u;
-        if (__syncthreads_or(!ok)) {
-            ok = false;
-            if (tid == 0) {
-                atomicOr(&g_nn_err, 1u);
-                wait_bounded(&bar, phase ^ 1u);  // give the MMAs in flight a bounded time to finish
-            }
-        }
+        ++issued;
+    }
+    cp_wait<0>();
+    // every MMA has ended (commits complete in order: the last one's barrier covers all)
+    if (issued > 0 && !wait_bounded(&bar[(issued - 1) % stages], ((issued - 1) / stages) & 1)) ok = false;
+    if (__syncthreads_or(!ok)) {
+        ok = false;
+        if (tid == 0) atomicOr(&g_nn_err, 1u);
     }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (ok && chunks > 0) {
-        const int m = m0 + warp * 32 + lane;
-        for (int j = 0; j < kTN / 32; ++j) {
-            float d[32];
-            tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(j * 32), d);
-            if (m >= M) continue;
-            float* crow = C + (long long)m * ldc;
-            const int nb = n0 + j * 32;
-            if (nb + 32 <= N && (ldc % 4) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0) {
+    // warp w reads TMEM lanes 32 (w % 4) .. +31 (tile rows) of the columns of half w / 4
+    const int m = m0 + (warp & 3) * 32 + lane;
+    const bool vec_c = (ldc % 4) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
 #pragma unroll
-                for (int q = 0; q < 32; q += 4)
-                    *reinterpret_cast<float4*>(crow + nb + q) = make_float4(d[q], d[q + 1], d[q + 2], d[q + 3]);
-                continue;
-            }
+    for (int j = 0; j < TN / 64; ++j) {
+        const int col = (warp >> 2) * (TN / 2) + j * 32;
+        float d[32];
 #pragma unroll
-            for (int q = 0; q < 32; ++q) {
-                const int n = nb + q;
-                if (n < N) crow[n] = d[q];
-            }
+        for (int q = 0; q < 32; ++q) d[q] = 0.0f;
+        if (ok && issued > 0) tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)col, d);
+        const int nb = n0 + col;
+        if (!ok || m >= M) continue;
+        float* crow = C + (long long)m * ldc;
+        if (nb + 32 <= N && vec_c) {
+#pragma unroll
+            for (int q = 0; q < 32; q += 4)
+                *reinterpret_cast<float4*>(crow + nb + q) = make_float4(d[q], d[q + 1], d[q + 2], d[q + 3]);
+            continue;
         }
-    } else if (chunks == 0) {
-        const int m = m0 + warp * 32 + lane;
-        if (m < M)
-            for (int n = n0; n < min(N, n0 + kTN); ++n) C[(long long)m * ldc + n] = 0.0f;
+#pragma unroll
+        for (int q = 0; q < 32; ++q)
+            if (nb + q < N) crow[nb + q] = d[q];
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTN) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TN) : "memory");
+}
+
+template <int TN, int AM, int BM>
+__global__ void __launch_bounds__(kThreads) nn_gemm_kernel(int M, int N, int K, const __nv_bfloat16* A, long long sam,
+                                                           long long sak, const __nv_bfloat16* B, long long sbn,
+                                                           long long sbk, float* C, long long ldc, int stages) {
+    extern __shared__ __align__(1024) unsigned char sm[];
+    gemm_tile<TN, AM, BM>(sm, blockIdx.x * kTM, blockIdx.y * TN, M, N, K, A, sam, sak, B, sbn, sbk, C, ldc, stages);
+}
+
+template <int TN, int AM, int BM>
+cudaError_t launch_gemm(int M, int N, int K, const __nv_bfloat16* A, long long sam, long long sak,
+                        const __nv_bfloat16* B, long long sbn, long long sbk, float* C, long long ldc, int stages,
+                        cudaStream_t s) {
+    auto kernel = nn_gemm_kernel<TN, AM, BM>;
+    static const cudaError_t sized =  // once, thread-safe
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxStages * gemm_stage<TN>());
+    if (sized != cudaSuccess) return sized;
+    kernel<<<dim3((M + kTM - 1) / kTM, (N + TN - 1) / TN), kThreads, stages * gemm_stage<TN>(), s>>>(
+        M, N, K, A, sam, sak, B, sbn, sbk, C, ldc, stages);
+    return cudaGetLastError();
+}
+
+template <int TN>
+cudaError_t launch_gemm_modes(int M, int N, int K, const __nv_bfloat16* A, long long sam, long long sak,
+                              const __nv_bfloat16* B, long long sbn, long long sbk, float* C, long long ldc, int stages,
+                              cudaStream_t s) {
+    auto mode = [](const void* p, long long s_row, long long s_k) {
+        if (reinterpret_cast<uintptr_t>(p) & 15) return (int)kAny;
+        if (s_k == 1 && s_row % 8 == 0) return (int)kRowsK;
+        return s_row == 1 && s_k % 8 == 0 ? (int)kColsK : (int)kAny;
+    };
+    const int am = mode(A, sam, sak), bm = mode(B, sbn, sbk);
+    if (am == kRowsK && bm == kRowsK)
+        return launch_gemm<TN, kRowsK, kRowsK>(M, N, K, A, sam, sak, B, sbn, sbk, C, ldc, stages, s);
+    if (am == kRowsK && bm == kColsK)
+        return launch_gemm<TN, kRowsK, kColsK>(M, N, K, A, sam, sak, B, sbn, sbk, C, ldc, stages, s);
+    if (am == kColsK && bm == kColsK)
+        return launch_gemm<TN, kColsK, kColsK>(M, N, K, A, sam, sak, B, sbn, sbk, C, ldc, stages, s);
+    return launch_gemm<TN, kAny, kAny>(M, N, K, A, sam, sak, B, sbn, sbk, C, ldc, stages, s);
 }
 
 // z[m][n] = c[m][n] + bias[n % bias_n] (in place); a = relu ? max(z, 0) : z, as BF16 at
@@ -223,13 +325,79 @@ __global__ void nn_act_grad_kernel(const float* dy, long long ldy, int off, cons
     dz_bf[i] = __float2bfloat16(g);
 }
 
-// out[n] = sum_m d[m][n] (one thread per column, FP32 in row order)
-__global__ void nn_col_sum_kernel(const float* d, int M, int N, float* out) {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= N) return;
+// out[n] = sum_m d[m][n], added in row order. One CTA per 32 columns: warps 1 .. 7 copy blocks of 128 rows
+// into a ring of three, warp 0 adds them, one column per lane. Bound by the chain of additions (16384
+// rows of the first convolution), which the loads no longer interrupt: 871 us before, when one thread
+// per column loaded as it added.
+constexpr int kSumRows = 128, kSumStages = 3;
+constexpr int kSumBytes = kSumStages * kSumRows * 32 * 4;
+__device__ __forceinline__ void col_sum(float* ring, int n0, const float* d, int M, int N, float* out) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int n = n0 + lane;
+    const int blocks = (M + kSumRows - 1) / kSumRows;
+    auto load = [&](int b) {  // warps 1 .. 7: every seventh row
+        if (b < blocks)
+            for (int r = warp - 1; r < kSumRows; r += 7) {
+                const int m = b * kSumRows + r;
+                const bool live = m < M && n < N;
+                cp_async4(ring + ((b % kSumStages) * kSumRows + r) * 32 + lane, live ? d + (long long)m * N + n : d,
+                          live ? 4 : 0);
+            }
+        cp_commit();
+    };
+    if (warp)
+        for (int b = 0; b < kSumStages - 1; ++b) load(b);
     float s = 0.0f;
-    for (int m = 0; m < M; ++m) s += d[(long long)m * N + n];
-    out[n] = s;
+    for (int b = 0; b < blocks; ++b) {
+        if (warp) cp_wait<kSumStages - 2>();
+        __syncthreads();  // block b is there; warp 0 is done with block b - 1, whose place block b + 2 takes
+        if (warp) {
+            load(b + kSumStages - 1);
+        } else {
+            const float* v = ring + (b % kSumStages) * kSumRows * 32 + lane;
+            const int rows = min(kSumRows, M - b * kSumRows);
+            if (rows == kSumRows) {
+#pragma unroll
+                for (int r = 0; r < kSumRows; ++r) s += v[r * 32];
+            } else {
+                for (int r = 0; r < rows; ++r) s += v[r * 32];
+            }
+        }
+    }
+    if (warp) cp_wait<0>();
+    else if (n < N) out[n] = s;
+}
+
+__global__ void __launch_bounds__(kThreads) nn_col_sum_kernel(const float* d, int M, int N, float* out) {
+    __shared__ __align__(16) float ring[kSumBytes / 4];
+    col_sum(ring, blockIdx.x * 32, d, M, N, out);
+}
+
+// The weight and bias gradients of several layers in one launch: gW = dz^T x (M x N, K rows of dz and x)
+// and gb = the column sums of dz. They depend on nothing but the layers' dz, so the long chains (the
+// first convolution sums 16384 rows in one tile) run beside all the others instead of after them.
+constexpr int kMaxGrads = 16;
+struct GradItem {
+    int M, N, K, first;  // first: the layer's first CTA; its tiles, then its column sums
+    const __nv_bfloat16 *dz_bf, *x;
+    const float* dz;
+    float *gw, *gb;
+};
+struct GradList {
+    GradItem g[kMaxGrads];
+    int n;
+};
+__global__ void __launch_bounds__(kThreads) nn_weight_grads_kernel(const __grid_constant__ GradList list) {
+    extern __shared__ __align__(1024) unsigned char sm[];
+    int i = list.n - 1;
+    while (i > 0 && (int)blockIdx.x < list.g[i].first) --i;
+    const GradItem& g = list.g[i];
+    const int cols = (g.N + 63) / 64, tiles = (g.M + kTM - 1) / kTM * cols, t = (int)blockIdx.x - g.first;
+    if (t < tiles)
+        gemm_tile<64, kColsK, kColsK>(sm, t / cols * kTM, t % cols * 64, g.M, g.N, g.K, g.dz_bf, 1, g.M, g.x, 1, g.N,
+                                      g.gw, g.N, kMaxStages);
+    else
+        col_sum(reinterpret_cast<float*>(sm), (t - tiles) * 32, g.dz, g.K, g.M, g.gb);
 }
 
 // x: [B][Lin][C] (position-major); cols: [B * Lout][k * C], column (j, c) = x[b][l * stride - pad + j][c]
@@ -285,18 +453,28 @@ __global__ void nn_mse_kernel(const float* y, const float* t, long long n, float
     if (threadIdx.x == 0 && loss) atomicAdd(loss, red[0]);
 }
 
-// Adam (FP32 master weights); the BF16 copy is refreshed for the next GEMMs
-__global__ void nn_adam_kernel(float* w, float* m, float* v, const float* g, long long n, float lr, float b1, float b2,
-                               float eps, float bc1, float bc2, __nv_bfloat16* w_bf) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.0f - b1) * gi;
-    const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-    m[i] = mi, v[i] = vi;
-    const float wi = w[i] - lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
-    w[i] = wi;
-    if (w_bf) w_bf[i] = __float2bfloat16(wi);
+// Adam (FP32 master weights); the BF16 copy is refreshed for the next GEMMs. Several tensors in one
+// launch (a launch costs more than most of them): tensor i takes the blocks from first[i] on.
+constexpr int kMaxAdam = 32;
+struct AdamList {
+    emlab_nn_param p[kMaxAdam];
+    int first[kMaxAdam];
+    int n;
+};
+__global__ void nn_adam_kernel(const __grid_constant__ AdamList list, float lr, float b1, float b2, float eps, float bc1,
+                               float bc2) {
+    int t = list.n - 1;
+    while (t > 0 && (int)blockIdx.x < list.first[t]) --t;
+    const emlab_nn_param& p = list.p[t];
+    const long long i = ((int)blockIdx.x - list.first[t]) * (long long)blockDim.x + threadIdx.x;
+    if (i >= p.n) return;
+    const float gi = p.g[i];
+    const float mi = b1 * p.m[i] + (1.0f - b1) * gi;
+    const float vi = b2 * p.v[i] + (1.0f - b2) * gi * gi;
+    p.m[i] = mi, p.v[i] = vi;
+    const float wi = p.w[i] - lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
+    p.w[i] = wi;
+    if (p.w_bf16) static_cast<__nv_bfloat16*>(p.w_bf16)[i] = __float2bfloat16(wi);
 }
 
 __global__ void nn_to_bf16_kernel(const float* x, long long n, __nv_bfloat16* out, long long ldo, int cols, int off) {
@@ -325,14 +503,15 @@ extern "C" {
 int emlab_nn_gemm(int M, int N, int K, const void* A, long long sam, long long sak, const void* B, long long sbn,
                   long long sbk, float* C, long long ldc, void* stream) {
     if (M <= 0 || N <= 0 || K < 0 || !A || !B || !C) return report_error(EMLAB_ERR_INVALID, "bad GEMM arguments");
-    const dim3 grid((M + kTM - 1) / kTM, (N + kTN - 1) / kTN);
-    // 24 KB of unused dynamic shared memory holds residency to four CTAs per SM: 4 x 128 tensor-
-    // memory columns = the SM's 512, so no CTA waits in tcgen05.alloc
-    static const bool sized = cudaFuncSetAttribute(nn_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   kResidencyPad) == cudaSuccess;
-    if (!sized) return report_error(EMLAB_ERR_CUDA, "GEMM shared-memory attribute");
-    nn_gemm_kernel<<<grid, 128, kResidencyPad, NN_STREAM(stream)>>>(M, N, K, static_cast<const __nv_bfloat16*>(A), sam, sak,
-                                                        static_cast<const __nv_bfloat16*>(B), sbn, sbk, C, ldc);
+    const __nv_bfloat16* a = static_cast<const __nv_bfloat16*>(A);
+    const __nv_bfloat16* b = static_cast<const __nv_bfloat16*>(B);
+    // 128-column tiles once they fill the device (each operand row is then read half as often), with
+    // three chunks in the ring so that two CTAs share an SM; below that narrow tiles and all six chunks
+    const long long wide = (long long)((M + kTM - 1) / kTM) * ((N + 127) / 128);
+    const cudaError_t e =
+        wide >= 2 * 152 ? launch_gemm_modes<128>(M, N, K, a, sam, sak, b, sbn, sbk, C, ldc, 3, NN_STREAM(stream))
+                        : launch_gemm_modes<64>(M, N, K, a, sam, sak, b, sbn, sbk, C, ldc, kMaxStages, NN_STREAM(stream));
+    if (e != cudaSuccess) return report_error(EMLAB_ERR_CUDA, cudaGetErrorString(e));
     count_launches(1);
     NN_CHECK();
     return EMLAB_OK;
@@ -371,7 +550,7 @@ int emlab_nn_act_grad(const float* dy, long long ldy, int off, const float* z, i
 }
 
 int emlab_nn_col_sum(const float* d, int M, int N, float* out, void* stream) {
-    nn_col_sum_kernel<<<blocks(N, 128), 128, 0, NN_STREAM(stream)>>>(d, M, N, out);
+    nn_col_sum_kernel<<<(N + 31) / 32, kThreads, 0, NN_STREAM(stream)>>>(d, M, N, out);
     count_launches(1);
     NN_CHECK();
     return EMLAB_OK;
@@ -404,9 +583,58 @@ int emlab_nn_mse(const float* y, const float* t, long long n, float* dy, float* 
 
 int emlab_nn_adam(float* w, float* m, float* v, const float* g, long long n, float lr, float b1, float b2, float eps,
                   int t, void* w_bf16, void* stream) {
+    const emlab_nn_param p = {w, m, v, g, n, w_bf16};
+    return emlab_nn_adam_all(&p, 1, lr, b1, b2, eps, t, stream);
+}
+
+int emlab_nn_adam_all(const emlab_nn_param* params, int count, float lr, float b1, float b2, float eps, int t,
+                      void* stream) {
+    if (count < 0 || (count && !params)) return report_error(EMLAB_ERR_INVALID, "bad Adam arguments");
     const float bc1 = 1.0f - powf(b1, (float)t), bc2 = 1.0f - powf(b2, (float)t);
-    nn_adam_kernel<<<blocks(n), 256, 0, NN_STREAM(stream)>>>(w, m, v, g, n, lr, b1, b2, eps, bc1, bc2,
-                                                             static_cast<__nv_bfloat16*>(w_bf16));
+    for (int base = 0; base < count; base += kMaxAdam) {
+        AdamList list{};
+        unsigned total = 0;
+        for (int i = base; i < count && list.n < kMaxAdam; ++i) {
+            if (params[i].n <= 0) continue;
+            list.p[list.n] = params[i];
+            list.first[list.n++] = (int)total;
+            total += blocks(params[i].n);
+        }
+        if (!total) continue;
+        nn_adam_kernel<<<total, 256, 0, NN_STREAM(stream)>>>(list, lr, b1, b2, eps, bc1, bc2);
+        count_launches(1);
+        NN_CHECK();
+    }
+    return EMLAB_OK;
+}
+
+int emlab_nn_weight_grads(const emlab_nn_grad* grads, int count, void* stream) {
+    if (count < 0 || (count && !grads)) return report_error(EMLAB_ERR_INVALID, "bad gradient arguments");
+    auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+    GradList list{};
+    int total = 0;
+    for (int i = 0; i < count; ++i) {
+        const emlab_nn_grad& q = grads[i];
+        if (q.out_features <= 0 || q.in_features <= 0 || q.rows < 0 || !q.dz_bf16 || !q.x_bf16 || !q.dz || !q.gw || !q.gb)
+            return report_error(EMLAB_ERR_INVALID, "bad gradient arguments");
+        const int M = q.out_features, N = q.in_features;
+        if (list.n < kMaxGrads && M % 8 == 0 && N % 8 == 0 && aligned(q.dz_bf16) && aligned(q.x_bf16)) {
+            list.g[list.n++] = {M, N, q.rows, total, static_cast<const __nv_bfloat16*>(q.dz_bf16),
+                                static_cast<const __nv_bfloat16*>(q.x_bf16), q.dz, q.gw, q.gb};
+            total += (M + kTM - 1) / kTM * ((N + 63) / 64) + (M + 31) / 32;
+            continue;
+        }
+        // rows the tensor core cannot copy 16 bytes at a time: the separate products
+        if (int rc = emlab_nn_gemm(M, N, q.rows, q.dz_bf16, 1, M, q.x_bf16, 1, N, q.gw, N, stream)) return rc;
+        if (int rc = emlab_nn_col_sum(q.dz, q.rows, M, q.gb, stream)) return rc;
+    }
+    if (!total) return EMLAB_OK;
+    constexpr int smem = kMaxStages * gemm_stage<64>();
+    static_assert(smem >= kSumBytes, "the column sums' ring fits the tile's stages");
+    static const cudaError_t sized =
+        cudaFuncSetAttribute(nn_weight_grads_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (sized != cudaSuccess) return report_error(EMLAB_ERR_CUDA, cudaGetErrorString(sized));
+    nn_weight_grads_kernel<<<total, kThreads, smem, NN_STREAM(stream)>>>(list);
     count_launches(1);
     NN_CHECK();
     return EMLAB_OK;

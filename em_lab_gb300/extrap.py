@@ -255,33 +255,37 @@ class Net:
             dz, dzb = self.dz[name], self.dzb[name]
             _check(lib.emlab_nn_act_grad(self._fp(up), o, 0, self._fp(self.zh[name]), B, o, 1 if relu else 0,
                                          self._fp(dz), self._p(dzb), s))
-            self._gemm(o, i, B, dzb, 1, o, ins[name], 1, i, self.gW[name], i)
-            _check(lib.emlab_nn_col_sum(self._fp(dz), B, o, self._fp(self.gb[name]), s))
             self._gemm(B, i, o, dzb, o, 1, self.Wb[name], 1, i, self.dx[name], i)
             up = self.dx[name]
         c2 = CONV[1]
         # conv2: dz2 over rows (b, l) x 64 channels = the encoder part of d(X0)
         _check(lib.emlab_nn_act_grad(self._fp(up), ENC + AUX, 0, self._fp(self.z2), B, ENC, 1, self._fp(self.dz2),
                                      self._p(self.dz2b), s))
-        self._gemm(64, 256, B * 16, self.dz2b, 1, 64, self.cols2, 1, 256, self.gW["conv2"], 256)
-        _check(lib.emlab_nn_col_sum(self._fp(self.dz2), B * 16, 64, self._fp(self.gb["conv2"]), s))
         self._gemm(B * 16, 256, 64, self.dz2b, 64, 1, self.Wb["conv2"], 1, 256, self.dcols2, 256)
         _check(lib.emlab_nn_col2im(self._fp(self.dcols2), B, c2[6], c2[1], c2[3], c2[4], c2[5], c2[7],
                                    self._fp(self.da1), s))
         _check(lib.emlab_nn_act_grad(self._fp(self.da1), 32, 0, self._fp(self.z1), B * 64, 32, 1, self._fp(self.dz1),
                                      self._p(self.dz1b), s))
-        self._gemm(32, 16, B * 64, self.dz1b, 1, 32, self.cols1, 1, 16, self.gW["conv1"], 16)
-        _check(lib.emlab_nn_col_sum(self._fp(self.dz1), B * 64, 32, self._fp(self.gb["conv1"]), s))
+        # every layer's weight and bias gradients, the longest sums first
+        rows = [("conv1", B * 64, self.dz1b, self.cols1, self.dz1), ("conv2", B * 16, self.dz2b, self.cols2, self.dz2)]
+        rows += [(name, B, self.dzb[name], ins[name], self.dz[name]) for name, _, _, _ in HEAD]
+        grads = (_Grad * len(rows))()
+        for g, (name, n_rows, dzb, x, dz) in zip(grads, rows):
+            w = self.gW[name]
+            g.out_features, g.in_features, g.rows = w.shape[0], w.shape[1], n_rows
+            g.dz_bf16, g.x_bf16, g.dz = dzb.data_ptr(), x.data_ptr(), dz.data_ptr()
+            g.gw, g.gb = w.data_ptr(), self.gb[name].data_ptr()
+        _check(lib.emlab_nn_weight_grads(grads, len(grads), s))
 
     def step(self, lr=1e-3, b1=0.9, b2=0.999, eps=1e-8):
         self.t_step += 1
-        for name, o, i in layer_shapes():
-            _check(self.lib.emlab_nn_adam(self._fp(self.W[name]), self._fp(self.mW[name]), self._fp(self.vW[name]),
-                                          self._fp(self.gW[name]), o * i, lr, b1, b2, eps, self.t_step,
-                                          self._p(self.Wb[name]), self.stream))
-            _check(self.lib.emlab_nn_adam(self._fp(self.b[name]), self._fp(self.mb[name]), self._fp(self.vb[name]),
-                                          self._fp(self.gb[name]), o, lr, b1, b2, eps, self.t_step, None,
-                                          self.stream))
+        params = (_Param * (2 * len(self.W)))()
+        for k, name in enumerate(self.W):
+            for p, w, m, v, g, bf in ((params[2 * k], self.W, self.mW, self.vW, self.gW, self.Wb[name].data_ptr()),
+                                      (params[2 * k + 1], self.b, self.mb, self.vb, self.gb, None)):
+                p.w, p.m, p.v, p.g = (d[name].data_ptr() for d in (w, m, v, g))
+                p.n, p.w_bf16 = w[name].numel(), bf
+        _check(self.lib.emlab_nn_adam_all(params, len(params), lr, b1, b2, eps, self.t_step, self.stream))
 
     def status(self):
         _check(self.lib.emlab_nn_status(self.stream))
@@ -302,6 +306,18 @@ class Net:
         return {n: (self.gW[n].cpu().numpy(), self.gb[n].cpu().numpy()) for n, _, _ in layer_shapes()}
 
 
+class _Grad(C.Structure):
+    """emlab_nn_grad."""
+    _fields_ = [("out_features", C.c_int), ("in_features", C.c_int), ("rows", C.c_int), ("dz_bf16", C.c_void_p),
+                ("x_bf16", C.c_void_p), ("dz", C.c_void_p), ("gw", C.c_void_p), ("gb", C.c_void_p)]
+
+
+class _Param(C.Structure):
+    """emlab_nn_param."""
+    _fields_ = [("w", C.c_void_p), ("m", C.c_void_p), ("v", C.c_void_p), ("g", C.c_void_p), ("n", C.c_longlong),
+                ("w_bf16", C.c_void_p)]
+
+
 def _nn_lib():
     lib = load_library()
     if getattr(lib, "_nn_ready", False):
@@ -318,6 +334,8 @@ def _nn_lib():
         "emlab_nn_col2im": [fp, I, I, I, I, I, I, I, fp, P],
         "emlab_nn_mse": [fp, fp, L, fp, fp, P],
         "emlab_nn_adam": [fp, fp, fp, fp, L, F, F, F, F, I, P, P],
+        "emlab_nn_adam_all": [C.POINTER(_Param), I, F, F, F, F, I, P],
+        "emlab_nn_weight_grads": [C.POINTER(_Grad), I, P],
         "emlab_nn_to_bf16": [fp, L, P, L, I, I, P],
     }
     for name, args in sig.items():

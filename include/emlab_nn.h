@@ -12,7 +12,7 @@ extern "C" {
 #endif
 
 /* C[m * ldc + n] = sum_k A(m, k) B(n, k), A(m, k) = A[m * sam + k * sak], B(n, k) = B[n * sbn + k * sbk]
- * (BF16), FP32 accumulation on the tensor cores (tcgen05, 128 x 128 tiles). */
+ * (BF16), FP32 accumulation on the tensor cores (tcgen05, 128 x 64 or 128 x 128 tiles). */
 int emlab_nn_gemm(int M, int N, int K, const void* A, long long sam, long long sak, const void* B, long long sbn,
                   long long sbk, float* C, long long ldc, void* stream);
 /* Synchronises the stream; EMLAB_ERR_TIMEOUT if a GEMM gave up a bounded wait since the last call. */
@@ -38,6 +38,26 @@ int emlab_nn_adam(float* w, float* m, float* v, const float* g, long long n, flo
                   int t, void* w_bf16, void* stream);
 /* out_bf16[r * ldo + off + c] = x[r * cols + c] for the n = rows * cols values. */
 int emlab_nn_to_bf16(const float* x, long long n, void* out, long long ldo, int cols, int off, void* stream);
+
+/* Adam of several tensors in one launch (each as emlab_nn_adam does it; tensors of no elements are
+ * skipped). */
+typedef struct emlab_nn_param {
+    float *w, *m, *v;
+    const float* g;
+    long long n;
+    void* w_bf16; /* may be NULL */
+} emlab_nn_param;
+int emlab_nn_adam_all(const emlab_nn_param* params, int count, float lr, float b1, float b2, float eps, int t,
+                      void* stream);
+/* Weight and bias gradients of several layers in one launch: gw[o][i] = sum over rows of dz_bf16[r][o]
+ * x_bf16[r][i] (as emlab_nn_gemm), gb[o] = sum over rows of dz[r][o] in row order (as emlab_nn_col_sum). */
+typedef struct emlab_nn_grad {
+    int out_features, in_features, rows;
+    const void *dz_bf16, *x_bf16;
+    const float* dz;
+    float *gw, *gb;
+} emlab_nn_grad;
+int emlab_nn_weight_grads(const emlab_nn_grad* grads, int count, void* stream);
 
 #ifdef __cplusplus
 }
