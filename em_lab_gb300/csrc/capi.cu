@@ -1138,33 +1138,55 @@ int emlab_ntff_read_phasors(emlab_grid* g, float* out) {
     return emlab_grid_synchronize(g, 0);
 }
 
+}  // extern "C"
+
+namespace {
+// The pattern at n_dirs directions and nf frequencies into `out` (2 floats each): the scratch grows to
+// the largest request and stays (no allocation in a steady loop); launch(plan) queues the sums of the box
+// record `box`.
+template <class Launch>
+int evaluate_pattern(emlab_grid* g, const int* box, int nf, const float* directions, int n_dirs, float* out,
+                     Launch&& launch) {
+    const PatternPlan plan = pattern_plan(box, nf, n_dirs);
+    const size_t outs = (size_t)nf * n_dirs * 2;
+    if (g->d_spec_dirs.n < (size_t)n_dirs || g->d_spec_part.n < plan.scratch || g->d_spec_out.n < outs)
+        EMLAB_CUDA(cudaStreamSynchronize(g->stream));
+    if (g->d_spec_dirs.n < (size_t)n_dirs) EMLAB_CUDA(g->d_spec_dirs.alloc((size_t)n_dirs));
+    if (g->d_spec_part.n < plan.scratch) EMLAB_CUDA(g->d_spec_part.alloc(plan.scratch));
+    if (g->d_spec_out.n < outs) EMLAB_CUDA(g->d_spec_out.alloc(outs));
+    EMLAB_CUDA(cudaMemcpyAsync(g->d_spec_dirs.p, directions, (size_t)n_dirs * 16, cudaMemcpyHostToDevice, g->stream));
+    launch(plan);
+    g_launches += (uint64_t)plan.launches;
+    if (int rc = check_launch()) return rc;
+    EMLAB_CUDA(cudaMemcpyAsync(out, g->d_spec_out.p, outs * 4, cudaMemcpyDeviceToHost, g->stream));
+    return emlab_grid_synchronize(g, 0);
+}
+
+// The same from the far-field DFT's sums: frequencies f0 .. f0 + nf - 1 of one box.
+int evaluate_dft(emlab_grid* g, int box, int f0, int nf, const float* directions, int n_dirs, float* out) {
+    if (int rc = dft_fold_now(g)) return rc;
+    const uint64_t samples = g->dft_samples;
+    EMLAB_REQUIRE(samples > 0, "no far-field DFT samples yet");
+    const int* rec = g->dft_boxes.data() + (size_t)box * kDftBoxInts;
+    return evaluate_pattern(g, rec, nf, directions, n_dirs, out, [&](const PatternPlan& plan) {
+        launch_pattern_dft(g->d_dft_box.p + (size_t)box * kDftBoxInts, rec[14], g->d_dft_x.p, rec[13], g->dft_points,
+                           f0, nf, g->d_dft_omega.p, 2.0 / (double)samples, g->d_spec_dirs.p, n_dirs, plan, g->d_spec_part.p,
+                           g->d_spec_out.p, g->stream);
+    });
+}
+}  // namespace
+
+extern "C" {
+
 int emlab_ntff_evaluate(emlab_grid* g, const float* directions, int n_dirs, float* out) {
     if (int rc = require_grid(g)) return rc;
     EMLAB_REQUIRE(g->ntff_on, "far-field monitor is not configured");
     EMLAB_REQUIRE(directions && out && n_dirs > 0, "bad direction arguments");
     EMLAB_CUDA(cudaSetDevice(g->device));
-    const int slices = std::clamp((g->points + 4095) / 4096, 1, 64);  // FarField.cpp:297
-    const int chunk = 4096;
-    DevBuf<float4> d_dirs, d_part;
-    DevBuf<float> d_out;
-    EMLAB_CUDA(d_dirs.alloc((size_t)n_dirs));
-    EMLAB_CUDA(cudaMemcpyAsync(d_dirs.p, directions, (size_t)n_dirs * 16, cudaMemcpyHostToDevice, g->stream));
-    EMLAB_CUDA(d_part.alloc((size_t)chunk * slices * 4));
-    EMLAB_CUDA(d_out.alloc((size_t)n_dirs * 2));
-    const float k = (float)(6.28318530717958647692 / (double)g->ntff_wl);
-    for (int first = 0; first < n_dirs; first += chunk) {
-        const int count = std::min(chunk, n_dirs - first);
-        launch_ntff_pattern(g->d_box.p, g->points, g->d_ntff.p, d_dirs.p, first, count, slices, k, d_part.p, g->stream);
-        launch_ntff_reduce(d_dirs.p, d_part.p, first, count, slices, d_out.p, g->stream);
-        g_launches += 2;
-        if (int rc = check_launch()) return rc;
-    }
-    std::vector<float> tmp((size_t)n_dirs * 2);
-    EMLAB_CUDA(cudaMemcpyAsync(tmp.data(), d_out.p, tmp.size() * 4, cudaMemcpyDeviceToHost, g->stream));
-    if (int rc = emlab_grid_synchronize(g, 0)) return rc;
-    // only the dispatch starting at direction 0 carries the power (ntff_pattern.comp:52)
-    for (int d = 0; d < n_dirs; ++d) out[2 * d] = tmp[2 * (size_t)d], out[2 * d + 1] = d == 0 ? tmp[1] : 0.0f;
-    return EMLAB_OK;
+    return evaluate_pattern(g, g->box, 1, directions, n_dirs, out, [&](const PatternPlan& plan) {
+        launch_pattern_phasors(g->d_box.p, g->points, g->d_ntff.p, 6.28318530717958647692 / (double)g->ntff_wl, g->d_spec_dirs.p,
+                               n_dirs, plan, g->d_spec_part.p, g->d_spec_out.p, g->stream);
+    });
 }
 
 // ---- multi-frequency far-field DFT ----------------------------------------------------------------
@@ -1326,35 +1348,7 @@ int emlab_ntff_dft_evaluate(emlab_grid* g, int f, const float* directions, int n
     EMLAB_REQUIRE(g->dft_nbox == 1, "the DFT has several boxes: evaluate them one by one with emlab_ntff_dft_spectra");
     EMLAB_REQUIRE(directions && out && n_dirs > 0, "bad direction arguments");
     EMLAB_CUDA(cudaSetDevice(g->device));
-    if (int rc = dft_fold(g)) return rc;
-    const uint64_t samples = g->dft_samples;
-    EMLAB_REQUIRE(samples > 0, "no far-field DFT samples yet");
-    DevBuf<float> ph;
-    EMLAB_CUDA(ph.alloc((size_t)g->dft_points * 32));
-    launch_dft_to_phasor(g->d_dft_x.p, g->dft_points, f, 2.0 / (double)samples, ph.p, g->stream);
-    const int slices = std::clamp((g->dft_points + 4095) / 4096, 1, 64);
-    const int chunk = 4096;
-    DevBuf<float4> d_dirs, d_part;
-    DevBuf<float> d_out;
-    EMLAB_CUDA(d_dirs.alloc((size_t)n_dirs));
-    EMLAB_CUDA(cudaMemcpyAsync(d_dirs.p, directions, (size_t)n_dirs * 16, cudaMemcpyHostToDevice, g->stream));
-    EMLAB_CUDA(d_part.alloc((size_t)chunk * slices * 4));
-    EMLAB_CUDA(d_out.alloc((size_t)n_dirs * 2));
-    const float k = (float)g->dft_omega[(size_t)f];
-    for (int first = 0; first < n_dirs; first += chunk) {
-        const int count = std::min(chunk, n_dirs - first);
-        launch_ntff_pattern(g->d_dft_box.p, g->dft_points, ph.p, d_dirs.p, first, count, slices, k, d_part.p,
-                            g->stream);
-        launch_ntff_reduce(d_dirs.p, d_part.p, first, count, slices, d_out.p, g->stream);
-        g_launches += 2;
-    }
-    g_launches += 1;
-    if (int rc = check_launch()) return rc;
-    std::vector<float> tmp((size_t)n_dirs * 2);
-    EMLAB_CUDA(cudaMemcpyAsync(tmp.data(), d_out.p, tmp.size() * 4, cudaMemcpyDeviceToHost, g->stream));
-    if (int rc = emlab_grid_synchronize(g, 0)) return rc;
-    for (int d = 0; d < n_dirs; ++d) out[2 * d] = tmp[2 * (size_t)d], out[2 * d + 1] = d == 0 ? tmp[1] : 0.0f;
-    return EMLAB_OK;
+    return evaluate_dft(g, 0, f, 1, directions, n_dirs, out);
 }
 
 int emlab_ntff_dft_evaluate_all(emlab_grid* g, const float* directions, int n_dirs, float* out) {
@@ -1363,36 +1357,7 @@ int emlab_ntff_dft_evaluate_all(emlab_grid* g, const float* directions, int n_di
     EMLAB_REQUIRE(g->dft_nbox == 1, "the DFT has several boxes: evaluate them one by one with emlab_ntff_dft_spectra");
     EMLAB_REQUIRE(directions && out && n_dirs > 0, "bad direction arguments");
     EMLAB_CUDA(cudaSetDevice(g->device));
-    if (int rc = dft_fold(g)) return rc;
-    const uint64_t samples = g->dft_samples;
-    EMLAB_REQUIRE(samples > 0, "no far-field DFT samples yet");
-    const int slices = std::clamp((g->dft_points + 4095) / 4096, 1, 64);
-    const int chunk = 8192;
-    DevBuf<float> ph, d_out;
-    DevBuf<float4> d_dirs, d_part;
-    EMLAB_CUDA(ph.alloc((size_t)g->dft_points * 32));
-    EMLAB_CUDA(d_dirs.alloc((size_t)n_dirs));
-    EMLAB_CUDA(cudaMemcpyAsync(d_dirs.p, directions, (size_t)n_dirs * 16, cudaMemcpyHostToDevice, g->stream));
-    EMLAB_CUDA(d_part.alloc((size_t)chunk * slices * 4));
-    EMLAB_CUDA(d_out.alloc((size_t)g->dft_nf * n_dirs * 2));
-    for (int f = 0; f < g->dft_nf; ++f) {
-        launch_dft_to_phasor(g->d_dft_x.p, g->dft_points, f, 2.0 / (double)samples, ph.p, g->stream);
-        const float k = (float)g->dft_omega[(size_t)f];
-        for (int first = 0; first < n_dirs; first += chunk) {
-            const int count = std::min(chunk, n_dirs - first);
-            launch_ntff_pattern_fast(g->d_dft_box.p, g->dft_points, ph.p, d_dirs.p, first, count, slices, k,
-                                     d_part.p, g->stream);
-            launch_ntff_reduce(d_dirs.p, d_part.p, first, count, slices, d_out.p + (size_t)f * n_dirs * 2, g->stream);
-            g_launches += 2;
-        }
-        g_launches += 1;
-    }
-    if (int rc = check_launch()) return rc;
-    EMLAB_CUDA(cudaMemcpyAsync(out, d_out.p, (size_t)g->dft_nf * n_dirs * 8, cudaMemcpyDeviceToHost, g->stream));
-    if (int rc = emlab_grid_synchronize(g, 0)) return rc;
-    for (int f = 0; f < g->dft_nf; ++f)  // the radiated power is reported once per frequency (first direction)
-        for (int d = 1; d < n_dirs; ++d) out[((size_t)f * n_dirs + d) * 2 + 1] = 0.0f;
-    return EMLAB_OK;
+    return evaluate_dft(g, 0, 0, g->dft_nf, directions, n_dirs, out);
 }
 
 int emlab_ntff_dft_spectra(emlab_grid* g, int box, const float* directions, int n_dirs, float* out) {
@@ -1401,29 +1366,7 @@ int emlab_ntff_dft_spectra(emlab_grid* g, int box, const float* directions, int 
     EMLAB_REQUIRE(box >= 0 && box < g->dft_nbox, "no such far-field DFT box");
     EMLAB_REQUIRE(directions && out && n_dirs > 0 && n_dirs <= 8192, "bad direction arguments (1 to 8192 directions)");
     EMLAB_CUDA(cudaSetDevice(g->device));
-    if (int rc = dft_fold(g)) return rc;
-    const uint64_t samples = g->dft_samples;
-    EMLAB_REQUIRE(samples > 0, "no far-field DFT samples yet");
-    const int* rec = g->dft_boxes.data() + (size_t)box * kDftBoxInts;
-    const int first = rec[13], points = rec[14];
-    const int slices = std::clamp((points + 4095) / 4096, 1, 64);
-    const size_t part = (size_t)g->dft_nf * n_dirs * slices * 4, outs = (size_t)g->dft_nf * n_dirs * 2;
-    // the scratch grows to the largest request and stays (no allocation in a steady loop)
-    if (g->d_spec_dirs.n < (size_t)n_dirs) EMLAB_CUDA(g->d_spec_dirs.alloc((size_t)n_dirs));
-    if (g->d_spec_part.n < part) EMLAB_CUDA(g->d_spec_part.alloc(part));
-    if (g->d_spec_out.n < outs) EMLAB_CUDA(g->d_spec_out.alloc(outs));
-    EMLAB_CUDA(cudaMemcpyAsync(g->d_spec_dirs.p, directions, (size_t)n_dirs * 16, cudaMemcpyHostToDevice, g->stream));
-    launch_ntff_spectra(g->d_dft_box.p + (size_t)box * kDftBoxInts, first, points, g->dft_points, g->d_dft_x.p,
-                        g->dft_nf, g->d_dft_omega.p, 2.0 / (double)samples, g->d_spec_dirs.p, n_dirs, slices,
-                        g->d_spec_part.p, g->stream);
-    launch_ntff_reduce_multi(g->d_spec_dirs.p, g->d_spec_part.p, n_dirs, slices, g->dft_nf, g->d_spec_out.p, g->stream);
-    g_launches += 2;
-    if (int rc = check_launch()) return rc;
-    EMLAB_CUDA(cudaMemcpyAsync(out, g->d_spec_out.p, outs * 4, cudaMemcpyDeviceToHost, g->stream));
-    if (int rc = emlab_grid_synchronize(g, 0)) return rc;
-    for (int f = 0; f < g->dft_nf; ++f)  // the radiated power is reported once per frequency (first direction)
-        for (int d = 1; d < n_dirs; ++d) out[((size_t)f * n_dirs + d) * 2 + 1] = 0.0f;
-    return EMLAB_OK;
+    return evaluate_dft(g, box, 0, g->dft_nf, directions, n_dirs, out);
 }
 
 }  // extern "C"

@@ -127,12 +127,21 @@ void launch_probe_gather(const MonitorArgs& m, const int4* origins, int n, float
                          const float* cell_eps, cudaStream_t s);
 void launch_flux_plane(const MonitorArgs& m, int axis, int index, int rmin0, int rmin1, int rs0, int rs1,
                        float* partials, cudaStream_t s);
-void launch_ntff_pattern(const int* box, int points, const float* phasors, const float4* dirs, int first, int count,
-                         int slices, float k, float4* partials, cudaStream_t s);
-void launch_ntff_pattern_fast(const int* box, int points, const float* phasors, const float4* dirs, int first,
-                              int count, int slices, float k, float4* partials, cudaStream_t s);
-void launch_ntff_reduce(const float4* dirs, const float4* partials, int first, int count, int slices, float* out,
-                        cudaStream_t s);
+// The far-field pattern of a box (pattern.cu) at n_dirs directions and nf frequencies (box: the host's
+// record): slices of the surface, directions and frequencies per launch, kernel launches, floats of scratch.
+struct PatternPlan {
+    int slices, chunk, freqs, launches;
+    size_t scratch;
+};
+PatternPlan pattern_plan(const int* box, int nf, int n_dirs);
+// out[(f * n_dirs + d) * 2] = |N_perp - r x L|^2, out[f * n_dirs * 2 + 1] = radiated power (0 at the other
+// directions), from the single-frequency monitor's phasors (wavenumber k), or from the DFT sums of
+// frequencies f0 .. f0 + nf - 1 scaled by `scale` (the box's `points` nodes from `first` of X's total_points)
+void launch_pattern_phasors(const int* dbox, int points, const float* phasors, double k, const float4* dirs, int n_dirs,
+                            const PatternPlan& plan, float* scratch, float* out, cudaStream_t s);
+void launch_pattern_dft(const int* dbox, int points, const double* X, int first, int total_points, int f0, int nf,
+                        const double* omega, double scale, const float4* dirs, int n_dirs, const PatternPlan& plan,
+                        float* scratch, float* out, cudaStream_t s);
 void launch_port_residuals(const float* series, long long steps, int nports, double* out, cudaStream_t s);
 void launch_sweep_sums(const float* series, long long steps, int nports, double nu_lo, double nu_hi, int points,
                        double dt, double* out, cudaStream_t s);
@@ -143,21 +152,11 @@ void launch_check_finite(const MonitorArgs& m, unsigned* flag, cudaStream_t s);
 constexpr int kDftBoxInts = 16;
 void launch_dft_sample(const MonitorArgs& m, const int* boxes, int nbox, int box_max, int points, float* blk, int t,
                        cudaStream_t s);
-// far-field spectra of one box (`points` nodes from point `first` of X's `total_points`) straight
-// from the DFT sums scaled by `scale`: per frequency the partial sums of the pattern over direction
-// chunks and surface slices, then the per-direction reduction (|N_perp - r x L|^2 and the radiated
-// power at direction 0), one launch each for all frequencies; out[(f * count + d) * 2 + {0, 1}]
-void launch_ntff_spectra(const int* box, int first, int points, int total_points, const double* X, int nf,
-                         const double* omega, double scale, const float4* dirs, int count, int slices,
-                         float4* partials, cudaStream_t s);
-void launch_ntff_reduce_multi(const float4* dirs, const float4* partials, int count, int slices, int nf, float* out,
-                              cudaStream_t s);
 // X_new[f][c][j] = X_old[f][c][map[j]] for the carried boxes of a stack compaction
 void launch_dft_gather(const double* x_old, int old_points, const int* map, int new_points, int nf, double* x_new,
                        cudaStream_t s);
 void launch_dft_fold(const float* blk, int T, int points, int nf, const float2* W, const double* omega, long long n0,
                      double dt, double* X, cudaStream_t s);
-void launch_dft_to_phasor(const double* X, int points, int f, double scale, float* ph, cudaStream_t s);
 void launch_raymarch(const MonitorArgs& m, const float* sigma, const float* eps, const emlab_render_params& p,
                      unsigned char* img, cudaStream_t s);
 // tensor-core fold (dft_tc.cu): MMA N for nf frequencies, host twiddle tables (hi, lo) in the

@@ -187,9 +187,9 @@ struct emlab_grid {
     DevBuf<float> d_dft_blk;
     DevBuf<float> d_dft_bhi, d_dft_blo;  // tensor-core twiddles (split hi/lo, MMA operand layout)
     int dft_engine = EMLAB_DFT_TENSOR;
-    // far-field spectra scratch (emlab_ntff_dft_spectra), grown on demand and kept
-    DevBuf<float4> d_spec_dirs, d_spec_part;
-    DevBuf<float> d_spec_out;
+    // far-field pattern scratch (directions, partial sums, results), grown on demand and kept
+    DevBuf<float4> d_spec_dirs;
+    DevBuf<float> d_spec_part, d_spec_out;
     // opt-in convolutional PML (cpml.cu): parameters, per-axis coefficient tables, slab psi arrays
     bool cpml_on = false;
     emlab_cpml cpml{};

@@ -4,7 +4,6 @@
 // with -fmad=false so its per-step FP32 arithmetic matches the CPU restatement bit for bit.
 // Monitors read the field generation that the step just produced.
 #include "emlab_internal.h"
-#include "sincos_reduced.cuh"
 
 namespace emlab {
 
@@ -244,260 +243,6 @@ __global__ void __launch_bounds__(256) flux_kernel(MonitorArgs m, int axis, int 
     if (lid == 0) partials[blockIdx.y * gridDim.x + blockIdx.x] = sp[0];
 }
 
-// ntff_pattern.comp:45-110 (128 directions x one surface slice per block)
-__global__ void __launch_bounds__(128) ntff_pattern_kernel(const int* box, int points, const float4* ph,
-                                                           const float4* dirs, int first, int count, int slices,
-                                                           float kw, float4* partials) {
-    __shared__ float4 sPos[128], sJr[128], sJi[128], sMr[128], sMi[128];
-    __shared__ float sP[128];
-    __shared__ int sbox[13];
-    const int lid = threadIdx.x;
-    if (lid < 13) sbox[lid] = box[lid];
-    __syncthreads();
-    const int local = blockIdx.x * 128 + lid;
-    const int d = first + local;
-    const int slice = blockIdx.y;
-    const bool inRange = d < first + count;
-    const float4 rr = inRange ? dirs[d] : make_float4(0.0f, 0.0f, 1.0f, 0.0f);
-    const bool power = blockIdx.x == 0 && first == 0;
-    const float cx = 0.5f * (float)(sbox[0] + sbox[3]), cy = 0.5f * (float)(sbox[1] + sbox[4]),
-                cz = 0.5f * (float)(sbox[2] + sbox[5]);
-    const int per = (points + slices - 1) / slices;
-    const int f0 = slice * per, last = min(f0 + per, points);
-    float Nr[3] = {0, 0, 0}, Ni[3] = {0, 0, 0}, Lr[3] = {0, 0, 0}, Li[3] = {0, 0, 0};
-    float P = 0.0f;
-    for (int base = f0; base < last; base += 128) {
-        const int i = base + lid;
-        if (i < last) {
-            int node[3];
-            float n[3], w;
-            ntff_point(sbox, i, node, n, w);
-            const float4* s2 = ph + 8 * (long long)i + 4;
-            const float4 eR = s2[0], eI = s2[1], hR = s2[2], hI = s2[3];
-            sPos[lid] = make_float4((float)node[0] - cx, (float)node[1] - cy, (float)node[2] - cz, 0.0f);
-            // cross(n, v) = (n1 v2 - v1 n2, n2 v0 - v2 n0, n0 v1 - v0 n1)
-#define EMLAB_CROSS(A0, A1, A2, B0, B1, B2) \
-    make_float4(A1 * B2 - B1 * A2, A2 * B0 - B2 * A0, A0 * B1 - B0 * A1, 0.0f)
-            const float4 jr = EMLAB_CROSS(n[0], n[1], n[2], hR.x, hR.y, hR.z);
-            const float4 ji = EMLAB_CROSS(n[0], n[1], n[2], hI.x, hI.y, hI.z);
-            const float4 mr = EMLAB_CROSS(n[0], n[1], n[2], eR.x, eR.y, eR.z);
-            const float4 mi = EMLAB_CROSS(n[0], n[1], n[2], eI.x, eI.y, eI.z);
-            sJr[lid] = make_float4(w * jr.x, w * jr.y, w * jr.z, 0.0f);
-            sJi[lid] = make_float4(w * ji.x, w * ji.y, w * ji.z, 0.0f);
-            sMr[lid] = make_float4(-w * mr.x, -w * mr.y, -w * mr.z, 0.0f);
-            sMi[lid] = make_float4(-w * mi.x, -w * mi.y, -w * mi.z, 0.0f);
-            if (power) {
-                const float4 c1 = EMLAB_CROSS(eR.x, eR.y, eR.z, hR.x, hR.y, hR.z);
-                const float4 c2 = EMLAB_CROSS(eI.x, eI.y, eI.z, hI.x, hI.y, hI.z);
-                const float s0 = c1.x + c2.x, s1 = c1.y + c2.y, s2v = c1.z + c2.z;
-                P = P + w * (s0 * n[0] + s1 * n[1] + s2v * n[2]);
-            }
-#undef EMLAB_CROSS
-        }
-        __syncthreads();
-        const int cnt = min(128, last - base);
-        for (int q = 0; q < cnt; ++q) {
-            const float4 pos = sPos[q];
-            const float psi = kw * (rr.x * pos.x + rr.y * pos.y + rr.z * pos.z);
-            float sn, cs;
-            sincosf(psi, &sn, &cs);
-            const float4 jr = sJr[q], ji = sJi[q], mr = sMr[q], mi = sMi[q];
-            Nr[0] = Nr[0] + (jr.x * cs - ji.x * sn), Nr[1] = Nr[1] + (jr.y * cs - ji.y * sn), Nr[2] = Nr[2] + (jr.z * cs - ji.z * sn);
-            Ni[0] = Ni[0] + (jr.x * sn + ji.x * cs), Ni[1] = Ni[1] + (jr.y * sn + ji.y * cs), Ni[2] = Ni[2] + (jr.z * sn + ji.z * cs);
-            Lr[0] = Lr[0] + (mr.x * cs - mi.x * sn), Lr[1] = Lr[1] + (mr.y * cs - mi.y * sn), Lr[2] = Lr[2] + (mr.z * cs - mi.z * sn);
-            Li[0] = Li[0] + (mr.x * sn + mi.x * cs), Li[1] = Li[1] + (mr.y * sn + mi.y * cs), Li[2] = Li[2] + (mr.z * sn + mi.z * cs);
-        }
-        __syncthreads();
-    }
-    sP[lid] = P;
-    __syncthreads();
-    for (int stride = 64; stride > 0; stride >>= 1) {
-        if (lid < stride) sP[lid] = sP[lid] + sP[lid + stride];
-        __syncthreads();
-    }
-    if (inRange) {
-        const long long o = 4ll * ((long long)local * slices + slice);
-        partials[o + 0] = make_float4(Nr[0], Nr[1], Nr[2], (power && lid == 0) ? sP[0] : 0.0f);
-        partials[o + 1] = make_float4(Ni[0], Ni[1], Ni[2], 0.0f);
-        partials[o + 2] = make_float4(Lr[0], Lr[1], Lr[2], 0.0f);
-        partials[o + 3] = make_float4(Li[0], Li[1], Li[2], 0.0f);
-    }
-}
-
-
-// Surface sources of the fast pattern sums. PhasorSource: the stage-2 phasors of ntff_pattern.comp's
-// layout (8 float4 per point). DftSource: the far-field DFT sums of frequency f straight from X
-// ([f][c][i] complex FP64), scaled and rounded to FP32 as dft_to_phasor_kernel stages them, for a
-// box whose first point in X is `first`.
-struct PhasorSource {
-    const float4* ph;
-    float k;
-    __device__ float kw(int) const { return k; }
-    __device__ void load(int, int i, float4& eR, float4& eI, float4& hR, float4& hI) const {
-        const float4* s2 = ph + 8 * (long long)i + 4;
-        eR = s2[0], eI = s2[1], hR = s2[2], hI = s2[3];
-    }
-};
-struct DftSource {
-    const double* X;
-    long long total;
-    int first;
-    const double* omega;
-    double scale;
-    __device__ float kw(int f) const { return (float)omega[f]; }
-    __device__ void load(int f, int i, float4& eR, float4& eI, float4& hR, float4& hI) const {
-        const double2* x = reinterpret_cast<const double2*>(X) + (size_t)f * 6 * total + first + i;
-        double2 v[6];
-#pragma unroll
-        for (int c = 0; c < 6; ++c) v[c] = x[(size_t)c * total];
-        eR = make_float4((float)(v[0].x * scale), (float)(v[1].x * scale), (float)(v[2].x * scale), 0.0f);
-        eI = make_float4((float)(v[0].y * scale), (float)(v[1].y * scale), (float)(v[2].y * scale), 0.0f);
-        hR = make_float4((float)(v[3].x * scale), (float)(v[4].x * scale), (float)(v[5].x * scale), 0.0f);
-        hI = make_float4((float)(v[3].y * scale), (float)(v[4].y * scale), (float)(v[5].y * scale), 0.0f);
-    }
-};
-
-// The same sums as ntff_pattern_kernel for 256 directions per block (two per thread, sharing every
-// staged surface point), with sincos_reduced and explicit multiply-adds: the far-field DFT's
-// pattern over large angle grids. blockIdx.z is the source's frequency; each frequency has its own
-// block of partials (count * slices * 4 float4).
-template <class Src>
-__global__ void __launch_bounds__(128) ntff_pattern_fast_kernel(const int* box, int points, Src src,
-                                                                const float4* dirs, int first, int count, int slices,
-                                                                float4* partials) {
-    __shared__ float4 sPos[128], sJr[128], sJi[128], sMr[128], sMi[128];
-    __shared__ float sP[128];
-    __shared__ int sbox[13];
-    const int lid = threadIdx.x;
-    const int fq = blockIdx.z;
-    const float kw = src.kw(fq);
-    partials += (size_t)fq * count * slices * 4;
-    if (lid < 13) sbox[lid] = box[lid];
-    __syncthreads();
-    const int local0 = blockIdx.x * 256 + lid, local1 = local0 + 128;
-    const int slice = blockIdx.y;
-    const bool in0 = local0 < count, in1 = local1 < count;
-    const float4 r0 = in0 ? dirs[first + local0] : make_float4(0.0f, 0.0f, 1.0f, 0.0f);
-    const float4 r1 = in1 ? dirs[first + local1] : make_float4(0.0f, 0.0f, 1.0f, 0.0f);
-    const bool power = blockIdx.x == 0 && first == 0;
-    const float cx = 0.5f * (float)(sbox[0] + sbox[3]), cy = 0.5f * (float)(sbox[1] + sbox[4]),
-                cz = 0.5f * (float)(sbox[2] + sbox[5]);
-    const int per = (points + slices - 1) / slices;
-    const int f0 = slice * per, last = min(f0 + per, points);
-    float a[2][12];
-#pragma unroll
-    for (int t = 0; t < 2; ++t)
-#pragma unroll
-        for (int j = 0; j < 12; ++j) a[t][j] = 0.0f;
-    float P = 0.0f;
-    const float k0x = kw * r0.x, k0y = kw * r0.y, k0z = kw * r0.z, k1x = kw * r1.x, k1y = kw * r1.y, k1z = kw * r1.z;
-    for (int base = f0; base < last; base += 128) {
-        const int i = base + lid;
-        if (i < last) {
-            int node[3];
-            float n[3], w;
-            ntff_point(sbox, i, node, n, w);
-            float4 eR, eI, hR, hI;
-            src.load(fq, i, eR, eI, hR, hI);
-            sPos[lid] = make_float4((float)node[0] - cx, (float)node[1] - cy, (float)node[2] - cz, 0.0f);
-#define EMLAB_CROSS(A0, A1, A2, B0, B1, B2) \
-    make_float4(A1 * B2 - B1 * A2, A2 * B0 - B2 * A0, A0 * B1 - B0 * A1, 0.0f)
-            const float4 jr = EMLAB_CROSS(n[0], n[1], n[2], hR.x, hR.y, hR.z);
-            const float4 ji = EMLAB_CROSS(n[0], n[1], n[2], hI.x, hI.y, hI.z);
-            const float4 mr = EMLAB_CROSS(n[0], n[1], n[2], eR.x, eR.y, eR.z);
-            const float4 mi = EMLAB_CROSS(n[0], n[1], n[2], eI.x, eI.y, eI.z);
-            sJr[lid] = make_float4(w * jr.x, w * jr.y, w * jr.z, 0.0f);
-            sJi[lid] = make_float4(w * ji.x, w * ji.y, w * ji.z, 0.0f);
-            sMr[lid] = make_float4(-w * mr.x, -w * mr.y, -w * mr.z, 0.0f);
-            sMi[lid] = make_float4(-w * mi.x, -w * mi.y, -w * mi.z, 0.0f);
-            if (power) {
-                const float4 c1 = EMLAB_CROSS(eR.x, eR.y, eR.z, hR.x, hR.y, hR.z);
-                const float4 c2 = EMLAB_CROSS(eI.x, eI.y, eI.z, hI.x, hI.y, hI.z);
-                P = P + w * ((c1.x + c2.x) * n[0] + (c1.y + c2.y) * n[1] + (c1.z + c2.z) * n[2]);
-            }
-#undef EMLAB_CROSS
-        }
-        __syncthreads();
-        const int cnt = min(128, last - base);
-        for (int q = 0; q < cnt; ++q) {
-            const float4 pos = sPos[q];
-            const float4 jr = sJr[q], ji = sJi[q], mr = sMr[q], mi = sMi[q];
-            float sn[2], cs[2];
-            sincos_reduced(fmaf(k0x, pos.x, fmaf(k0y, pos.y, k0z * pos.z)), &sn[0], &cs[0]);
-            sincos_reduced(fmaf(k1x, pos.x, fmaf(k1y, pos.y, k1z * pos.z)), &sn[1], &cs[1]);
-#pragma unroll
-            for (int t = 0; t < 2; ++t) {
-                const float c = cs[t], s = sn[t];
-                a[t][0] = fmaf(jr.x, c, fmaf(-ji.x, s, a[t][0]));
-                a[t][1] = fmaf(jr.y, c, fmaf(-ji.y, s, a[t][1]));
-                a[t][2] = fmaf(jr.z, c, fmaf(-ji.z, s, a[t][2]));
-                a[t][3] = fmaf(jr.x, s, fmaf(ji.x, c, a[t][3]));
-                a[t][4] = fmaf(jr.y, s, fmaf(ji.y, c, a[t][4]));
-                a[t][5] = fmaf(jr.z, s, fmaf(ji.z, c, a[t][5]));
-                a[t][6] = fmaf(mr.x, c, fmaf(-mi.x, s, a[t][6]));
-                a[t][7] = fmaf(mr.y, c, fmaf(-mi.y, s, a[t][7]));
-                a[t][8] = fmaf(mr.z, c, fmaf(-mi.z, s, a[t][8]));
-                a[t][9] = fmaf(mr.x, s, fmaf(mi.x, c, a[t][9]));
-                a[t][10] = fmaf(mr.y, s, fmaf(mi.y, c, a[t][10]));
-                a[t][11] = fmaf(mr.z, s, fmaf(mi.z, c, a[t][11]));
-            }
-        }
-        __syncthreads();
-    }
-    sP[lid] = P;
-    __syncthreads();
-    for (int stride = 64; stride > 0; stride >>= 1) {
-        if (lid < stride) sP[lid] = sP[lid] + sP[lid + stride];
-        __syncthreads();
-    }
-#pragma unroll
-    for (int t = 0; t < 2; ++t) {
-        const int local = t ? local1 : local0;
-        if (!(t ? in1 : in0)) continue;
-        const long long o = 4ll * ((long long)local * slices + slice);
-        partials[o + 0] = make_float4(a[t][0], a[t][1], a[t][2], (power && lid == 0 && t == 0) ? sP[0] : 0.0f);
-        partials[o + 1] = make_float4(a[t][3], a[t][4], a[t][5], 0.0f);
-        partials[o + 2] = make_float4(a[t][6], a[t][7], a[t][8], 0.0f);
-        partials[o + 3] = make_float4(a[t][9], a[t][10], a[t][11], 0.0f);
-    }
-}
-
-// ntff_reduce.comp:19-39 (blockIdx.y: the frequency of a multi-frequency pattern, each with its own
-// partials and outputs)
-__global__ void ntff_reduce_kernel(const float4* dirs, const float4* partials, int first, int count, int slices,
-                                   float* out) {
-    partials += (size_t)blockIdx.y * count * slices * 4;
-    out += (size_t)blockIdx.y * count * 2;
-    const int local = blockIdx.x * blockDim.x + threadIdx.x;
-    const int d = first + local;
-    if (local >= count) return;
-    const float4 r = dirs[d];
-    float N[2][3] = {{0, 0, 0}, {0, 0, 0}}, L[2][3] = {{0, 0, 0}, {0, 0, 0}};
-    float P = 0.0f;
-    for (int s = 0; s < slices; ++s) {
-        const long long o = 4ll * ((long long)local * slices + s);
-        const float4 a = partials[o], b = partials[o + 1], c = partials[o + 2], e = partials[o + 3];
-        N[0][0] = N[0][0] + a.x, N[0][1] = N[0][1] + a.y, N[0][2] = N[0][2] + a.z;
-        P = P + a.w;
-        N[1][0] = N[1][0] + b.x, N[1][1] = N[1][1] + b.y, N[1][2] = N[1][2] + b.z;
-        L[0][0] = L[0][0] + c.x, L[0][1] = L[0][1] + c.y, L[0][2] = L[0][2] + c.z;
-        L[1][0] = L[1][0] + e.x, L[1][1] = L[1][1] + e.y, L[1][2] = L[1][2] + e.z;
-    }
-    const float rv[3] = {r.x, r.y, r.z};
-    float F2 = 0.0f;
-    for (int part = 0; part < 2; ++part) {
-        const float dn = N[part][0] * rv[0] + N[part][1] * rv[1] + N[part][2] * rv[2];
-        const float rl0 = rv[1] * L[part][2] - L[part][1] * rv[2];
-        const float rl1 = rv[2] * L[part][0] - L[part][2] * rv[0];
-        const float rl2 = rv[0] * L[part][1] - L[part][0] * rv[1];
-        const float F0 = (N[part][0] - dn * rv[0]) - rl0, F1 = (N[part][1] - dn * rv[1]) - rl1,
-                    F2c = (N[part][2] - dn * rv[2]) - rl2;
-        F2 = F2 + (F0 * F0 + F1 * F1 + F2c * F2c);
-    }
-    out[2 * d] = F2;
-    out[2 * d + 1] = 0.5f * P;
-}
-
 // PortMonitor::evaluateSweep sums (Ports.cpp:215-242) in FP64: one block per (port, frequency)
 __global__ void __launch_bounds__(256) sweep_kernel(const float* series, long long steps, int nports, double nu_lo,
                                                     double nu_hi, int points, double dt, double* out) {
@@ -627,21 +372,6 @@ __global__ void dft_gather_kernel(const double2* x_old, int old_points, const in
     x_new[fc * new_points + j] = x_old[fc * old_points + map[j]];
 }
 
-// Stage-2 phasor layout of ntff_pattern.comp (PhasorPair, 8 float4 per node) from the DFT sums of
-// one frequency, scaled by `scale` (2 / samples turns a sum into the amplitude of a steady tone).
-__global__ void dft_to_phasor_kernel(const double* X, int points, int f, double scale, float4* ph) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= points) return;
-    const double2* x = reinterpret_cast<const double2*>(X) + (size_t)f * 6 * points + i;
-    double2 v[6];
-    for (int c = 0; c < 6; ++c) v[c] = x[(size_t)c * points];
-    float4* p = ph + 8 * (size_t)i;
-    p[4] = make_float4((float)(v[0].x * scale), (float)(v[1].x * scale), (float)(v[2].x * scale), 0.0f);  // E re
-    p[5] = make_float4((float)(v[0].y * scale), (float)(v[1].y * scale), (float)(v[2].y * scale), 0.0f);  // E im
-    p[6] = make_float4((float)(v[3].x * scale), (float)(v[4].x * scale), (float)(v[5].x * scale), 0.0f);  // H re
-    p[7] = make_float4((float)(v[3].y * scale), (float)(v[4].y * scale), (float)(v[5].y * scale), 0.0f);  // H im
-}
-
 __global__ void expf_kernel(const float* in, float* out, size_t n) {
     const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     if (i < n) out[i] = emlab_expf(in[i]);
@@ -675,38 +405,6 @@ void launch_flux_plane(const MonitorArgs& m, int axis, int index, int rmin0, int
                        float* partials, cudaStream_t s) {
     const dim3 grid((rs0 + 15) / 16, (rs1 + 15) / 16);
     flux_kernel<<<grid, dim3(16, 16), 0, s>>>(m, axis, index, rmin0, rmin1, rs0, rs1, partials);
-}
-
-void launch_ntff_pattern(const int* box, int points, const float* phasors, const float4* dirs, int first, int count,
-                         int slices, float k, float4* partials, cudaStream_t s) {
-    const dim3 grid((count + 127) / 128, slices);
-    ntff_pattern_kernel<<<grid, 128, 0, s>>>(box, points, reinterpret_cast<const float4*>(phasors), dirs, first, count,
-                                             slices, k, partials);
-}
-
-void launch_ntff_pattern_fast(const int* box, int points, const float* phasors, const float4* dirs, int first,
-                              int count, int slices, float k, float4* partials, cudaStream_t s) {
-    const dim3 grid((count + 255) / 256, slices);
-    ntff_pattern_fast_kernel<<<grid, 128, 0, s>>>(box, points, PhasorSource{reinterpret_cast<const float4*>(phasors), k},
-                                                  dirs, first, count, slices, partials);
-}
-
-void launch_ntff_spectra(const int* box, int first, int points, int total_points, const double* X, int nf,
-                         const double* omega, double scale, const float4* dirs, int count, int slices,
-                         float4* partials, cudaStream_t s) {
-    const dim3 grid((count + 255) / 256, slices, nf);
-    ntff_pattern_fast_kernel<<<grid, 128, 0, s>>>(box, points, DftSource{X, total_points, first, omega, scale}, dirs,
-                                                  0, count, slices, partials);
-}
-
-void launch_ntff_reduce_multi(const float4* dirs, const float4* partials, int count, int slices, int nf, float* out,
-                              cudaStream_t s) {
-    ntff_reduce_kernel<<<dim3((count + 63) / 64, nf), 64, 0, s>>>(dirs, partials, 0, count, slices, out);
-}
-
-void launch_ntff_reduce(const float4* dirs, const float4* partials, int first, int count, int slices, float* out,
-                        cudaStream_t s) {
-    ntff_reduce_kernel<<<(count + 63) / 64, 64, 0, s>>>(dirs, partials, first, count, slices, out);
 }
 
 void launch_sweep_sums(const float* series, long long steps, int nports, double nu_lo, double nu_hi, int points,
@@ -767,10 +465,6 @@ void launch_dft_fold(const float* blk, int T, int points, int nf, const float2* 
         cudaFuncSetAttribute(dft_fold_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess)
         smem_set = smem;
     dft_fold_kernel<<<(unsigned)((cols + 127) / 128), 128, smem, s>>>(blk, T, points, nf, W, omega, n0, dt, X);
-}
-
-void launch_dft_to_phasor(const double* X, int points, int f, double scale, float* ph, cudaStream_t s) {
-    dft_to_phasor_kernel<<<(points + 255) / 256, 256, 0, s>>>(X, points, f, scale, reinterpret_cast<float4*>(ph));
 }
 
 void launch_debug_expf(const float* in, float* out, size_t n, cudaStream_t s) {

@@ -8,7 +8,7 @@ of its own (a 384 x 384 x 256 scene fills the GPU by itself), stepped with the f
 attached, then evaluated at every frequency over the full angle grid by emlab_ntff_dft_pattern_gemm
 (the sums of ntff_pattern.comp / ntff_reduce.comp split per face into a u and a v factor: the sum over
 v one complex GEMM on the tcgen05 tensor cores, csrc/pattern_tc.cu) or, with pattern="direct",
-emlab_ntff_dft_evaluate_all (the direct sums with range-reduced hardware sin/cos, csrc/monitors.cu).
+emlab_ntff_dft_evaluate_all (the FP32 sums of csrc/pattern.cu).
 """
 from __future__ import annotations
 

@@ -279,9 +279,8 @@ int emlab_ntff_dft_read(emlab_grid* g, double* out);
  * (the amplitude of a steady tone): out[2d] = |N_perp - r x L|^2, out[1] = radiated power. */
 int emlab_ntff_dft_evaluate(emlab_grid* g, int f, const float* directions, int n_dirs, float* out);
 /* The pattern at every configured frequency: out[(f * n_dirs + d) * 2] = |N_perp - r x L|^2,
- * out[f * n_dirs * 2 + 1] = radiated power at f. Same sums as emlab_ntff_dft_evaluate with the
- * surface phases from a 2-pi range reduction and hardware sin/cos (relative difference about 1e-5),
- * two directions per thread: for large angle grids. */
+ * out[f * n_dirs * 2 + 1] = radiated power at f. The same sums as emlab_ntff_dft_evaluate, all
+ * frequencies together. */
 int emlab_ntff_dft_evaluate_all(emlab_grid* g, const float* directions, int n_dirs, float* out);
 /* The far-field DFT on several Huygens boxes at once (the boxes of the scenes of a stack): boxes[6k ..
  * 6k + 5] = min xyz, max xyz of box k in grid coordinates, each inside [1, n - 2] on every axis with
@@ -296,7 +295,7 @@ int emlab_ntff_dft_configure_boxes(emlab_grid* g, const int* boxes, int n_boxes,
                                    int n_freq, int block);
 /* The pattern of box `box` at every configured frequency (1 to 8192 directions, 4 floats each, xyz
  * used), in the layout of emlab_ntff_dft_evaluate_all: out[(f * n_dirs + d) * 2] = |N_perp - r x L|^2,
- * out[f * n_dirs * 2 + 1] = radiated power at f, from the sums scaled by 2 / samples. Two launches
+ * out[f * n_dirs * 2 + 1] = radiated power at f, from the sums scaled by 2 / samples. A few launches
  * for all frequencies; the device scratch grows to the largest request and is kept. */
 int emlab_ntff_dft_spectra(emlab_grid* g, int box, const float* directions, int n_dirs, float* out);
 /* The same pattern as emlab_ntff_dft_spectra (all frequencies, one box, out in its layout), the sums
