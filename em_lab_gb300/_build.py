@@ -29,7 +29,8 @@ NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-fmad=false", "-Xcompiler", HOS
               "-I", str(ROOT / "include"), "-I", str(CSRC)]
 
 SOURCES = ["yee.cu", "yee_tma.cu", "monitors.cu", "capi.cu", "noalloc.cu", "dft_tc.cu", "render.cu", "stack.cu", "learn.cu", "radar.cu", "cpml.cu", "pattern.cu", "pattern_tc.cu", "setup.cpp"]
-HEADERS = ["emlab_math.h", "emlab_internal.h", "setup.h", "yee_common.cuh", "grid_state.h", "twiddle.cuh"]
+HEADERS = ["emlab_math.h", "emlab_internal.h", "setup.h", "yee_common.cuh", "grid_state.h", "twiddle.cuh",
+           "chain.cuh"]
 
 
 def _nvcc() -> str:

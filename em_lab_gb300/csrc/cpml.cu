@@ -71,6 +71,8 @@ __device__ __forceinline__ float cpml_term(const CpmlArgs& p, const YeeArgs& a, 
 // half-integer positions; E beyond the upper faces is 0 as in update_B.comp:27-29).
 template <typename Idx>
 __global__ void __launch_bounds__(128) cpml_b_kernel(YeeArgs a, CpmlArgs p) {
+    chain_wait();
+    chain_next();
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y, z = blockIdx.z;
     if (x >= a.nx) return;
     const long long o = (long long)z * a.plane + (long long)y * a.pitch + x;
@@ -105,6 +107,8 @@ __global__ void __launch_bounds__(128) cpml_b_kernel(YeeArgs a, CpmlArgs p) {
 // material (no absorber conductivity).
 template <typename Idx>
 __global__ void __launch_bounds__(128) cpml_e_kernel(YeeArgs a, CpmlArgs p) {
+    chain_wait();
+    chain_next();
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y, z = blockIdx.z;
     if (x >= a.nx) return;
     const long long o = (long long)z * a.plane + (long long)y * a.pitch + x;
@@ -179,15 +183,15 @@ int cpml_clear(emlab_grid* g) {
     return EMLAB_OK;
 }
 
-void launch_cpml(emlab_grid* g, const YeeArgs& a, bool wide, cudaStream_t s) {
+void launch_cpml(emlab_grid* g, const YeeArgs& a, bool wide, const Chain& s) {
     const CpmlArgs p = cpml_args(g);
     const dim3 grid((a.nx + 127) / 128, a.ny, a.nz);
     if (wide) {
-        cpml_b_kernel<uint32_t><<<grid, 128, 0, s>>>(a, p);
-        cpml_e_kernel<uint32_t><<<grid, 128, 0, s>>>(a, p);
+        launch_chained(s, cpml_b_kernel<uint32_t>, grid, 128, 0, a, p);
+        launch_chained({s.stream, true}, cpml_e_kernel<uint32_t>, grid, 128, 0, a, p);
     } else {
-        cpml_b_kernel<uint16_t><<<grid, 128, 0, s>>>(a, p);
-        cpml_e_kernel<uint16_t><<<grid, 128, 0, s>>>(a, p);
+        launch_chained(s, cpml_b_kernel<uint16_t>, grid, 128, 0, a, p);
+        launch_chained({s.stream, true}, cpml_e_kernel<uint16_t>, grid, 128, 0, a, p);
     }
 }
 

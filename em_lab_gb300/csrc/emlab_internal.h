@@ -15,6 +15,7 @@
 
 #include <vector>
 
+#include "chain.cuh"
 #include "emlab.h"
 #include "emlab_math.h"
 
@@ -94,7 +95,7 @@ struct MonitorArgs {
     const float* bx; const float* by; const float* bz;
 };
 
-void launch_yee_fused(const YeeArgs& a, bool wide, cudaStream_t s);
+void launch_yee_fused(const YeeArgs& a, bool wide, const Chain& s);
 
 // TMA-staged fused kernel: tensor maps of one field generation and the class index.
 struct TmaMaps;
@@ -111,18 +112,18 @@ std::vector<int4> ragged_items(const std::vector<int>& z0, const std::vector<int
 // the uniform grid's pair-kernel schedule for g CTAs: planes per z chunk and work items
 void pair_schedule_shape(int nx, int ny, int nz, int ty, int g, int* zc, int* items);
 // Launches the TMA kernel reading generation `gen`; err receives a nonzero word if a wait timed out.
-bool launch_yee_tma(const YeeArgs& a, const TmaMaps* m, int gen, bool wide, unsigned* err, cudaStream_t s);
-void launch_yee_split(const YeeArgs& a, bool wide, cudaStream_t s);
-void launch_sources(const YeeArgs& a, const SourceArgs& sa, int k, bool wide, cudaStream_t s);
+bool launch_yee_tma(const YeeArgs& a, const TmaMaps* m, int gen, bool wide, unsigned* err, const Chain& s);
+void launch_yee_split(const YeeArgs& a, bool wide, const Chain& s);
+void launch_sources(const YeeArgs& a, const SourceArgs& sa, int k, bool wide, const Chain& s);
 
 // ports: ports[2i] = (x, y, z, axis), ports[2i+1] = (edges, sign, 0, 0); phasors 8 per port;
 // params[k] = (cos wtE, sin wtE, cos wtH, sin wtH) and blend for sub-step k.
 void launch_ports(const MonitorArgs& m, const int4* ports, int n, float* phasors, float* series, long long rec_index,
-                  const float4* rot, const float* blend, int k, cudaStream_t s);
+                  const float4* rot, const float* blend, int k, const Chain& s);
 void launch_ntff(const MonitorArgs& m, const int* box, int points, float* phasors, const float4* rot,
-                 const float* blend, int k, cudaStream_t s);
+                 const float* blend, int k, const Chain& s);
 void launch_lines(const MonitorArgs& m, const int4* q, int nq, const int4* terms, const float* weights,
-                  float* phasors, float* now, const float4* rot, const float* blend, int k, cudaStream_t s);
+                  float* phasors, float* now, const float4* rot, const float* blend, int k, const Chain& s);
 void launch_probe_gather(const MonitorArgs& m, const int4* origins, int n, float4* out, const float* cell_sig,
                          const float* cell_eps, cudaStream_t s);
 void launch_flux_plane(const MonitorArgs& m, int axis, int index, int rmin0, int rmin1, int rs0, int rs1,
@@ -151,7 +152,7 @@ void launch_check_finite(const MonitorArgs& m, unsigned* flag, cudaStream_t s);
 // box's first point in the concatenated point list, its point count.
 constexpr int kDftBoxInts = 16;
 void launch_dft_sample(const MonitorArgs& m, const int* boxes, int nbox, int box_max, int points, float* blk, int t,
-                       cudaStream_t s);
+                       const Chain& s);
 // X_new[f][c][j] = X_old[f][c][map[j]] for the carried boxes of a stack compaction
 void launch_dft_gather(const double* x_old, int old_points, const int* map, int new_points, int nf, double* x_new,
                        cudaStream_t s);

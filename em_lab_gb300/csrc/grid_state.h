@@ -238,7 +238,7 @@ int ensure_cell_materials(emlab_grid* g);
 // cpml.cu: tables and psi arrays for the configured size, psi reset, and the two in-place passes
 int cpml_prepare(emlab_grid* g);
 int cpml_clear(emlab_grid* g);
-void launch_cpml(emlab_grid* g, const YeeArgs& a, bool wide, cudaStream_t s);
+void launch_cpml(emlab_grid* g, const YeeArgs& a, bool wide, const Chain& s);
 // capi.cu: the far-field DFT across a stack compaction. dft_carry_take folds the partial block and
 // keeps the sums of the boxes that lie inside kept scenes (old scene idx[k] becomes scene k at
 // new_z0[k]); dft_carry_restore re-attaches those boxes at their new planes with their sums.

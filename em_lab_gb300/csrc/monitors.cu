@@ -54,6 +54,12 @@ __global__ void ports_kernel(MonitorArgs m, const int4* ports, int n, float* ph,
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int4 p = ports[2 * i], info = ports[2 * i + 1];
+    const float4 r = __ldcg(rot + k);
+    const float b = __ldcg(blend + k);
+    float* q = ph + 8 * i;
+    float4 s1 = __ldcg(reinterpret_cast<const float4*>(q)), s2 = __ldcg(reinterpret_cast<const float4*>(q) + 1);
+    chain_wait();
+    chain_next();
     const int a = p.w;
     const float s = (float)info.y;
     float V = 0.0f, I = 0.0f;
@@ -77,18 +83,16 @@ __global__ void ports_kernel(MonitorArgs m, const int4* ports, int n, float* ph,
         series[(rec * n + i) * 2 + 0] = V;
         series[(rec * n + i) * 2 + 1] = I;
     }
-    const float4 r = rot[k];
-    const float b = blend[k];
     const float o0 = (2.0f * r.x) * V, o1 = (-2.0f * r.y) * V, o2 = (2.0f * r.z) * I, o3 = (-2.0f * r.w) * I;
-    float* q = ph + 8 * i;
-    q[0] = q[0] + b * (o0 - q[0]);
-    q[1] = q[1] + b * (o1 - q[1]);
-    q[2] = q[2] + b * (o2 - q[2]);
-    q[3] = q[3] + b * (o3 - q[3]);
-    q[4] = q[4] + b * (q[0] - q[4]);
-    q[5] = q[5] + b * (q[1] - q[5]);
-    q[6] = q[6] + b * (q[2] - q[6]);
-    q[7] = q[7] + b * (q[3] - q[7]);
+    s1.x = s1.x + b * (o0 - s1.x);
+    s1.y = s1.y + b * (o1 - s1.y);
+    s1.z = s1.z + b * (o2 - s1.z);
+    s1.w = s1.w + b * (o3 - s1.w);
+    s2.x = s2.x + b * (s1.x - s2.x);
+    s2.y = s2.y + b * (s1.y - s2.y);
+    s2.z = s2.z + b * (s1.z - s2.z);
+    s2.w = s2.w + b * (s1.w - s2.w);
+    reinterpret_cast<float4*>(q)[0] = s1, reinterpret_cast<float4*>(q)[1] = s2;
 }
 
 // ntff_common.glsl:30-53; box = (min xyz, max xyz, face offsets[7])
@@ -113,9 +117,9 @@ __device__ __forceinline__ void ntff_point(const int* box, int index, int node[3
 // ntff_accumulate.comp:30-52: 32 floats per point (stage1 eRe, eIm, hRe, hIm, stage2 ...). The
 // block's 128 x 128 B of state move between HBM and shared memory as one contiguous chunk
 // (consecutive threads, consecutive float4s), rows padded to 9 float4s against bank conflicts;
-// each thread then updates its own point there. Every load a thread makes (its eight float4s of
-// the block's state and the 18 field values of its node) is issued before the first is used, so
-// the kernel waits one memory round trip instead of nine. Same arithmetic per point.
+// each thread then updates its own point there. The state is read ahead of the wait (this kernel's
+// own stores of the step before), the 18 field values of a node in one round trip after it. Same
+// arithmetic per point.
 constexpr int kNtffThreads = 128;
 __global__ void __launch_bounds__(kNtffThreads) ntff_kernel(MonitorArgs m, const int* box, int points, float4* ph,
                                                             const float4* rot, const float* blend, int k) {
@@ -129,16 +133,19 @@ __global__ void __launch_bounds__(kNtffThreads) ntff_kernel(MonitorArgs m, const
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
         const int j = threadIdx.x + q * kNtffThreads;
-        if (j < 8 * count) v[q] = base[j];
+        if (j < 8 * count) v[q] = __ldcg(base + j);
     }
     __syncthreads();  // sbox
     const int i = first + threadIdx.x;
     const bool live = i < points;
     float E[3], Hh[3];
+    int node[3];
+    float n[3], w;
+    if (live) ntff_point(sbox, i, node, n, w);
+    const float4 r = __ldcg(rot + k);
+    const float b = __ldcg(blend + k);
+    chain_wait();
     if (live) {
-        int node[3];
-        float n[3], w;
-        ntff_point(sbox, i, node, n, w);
         e_at_node(m, node[0], node[1], node[2], E[0], E[1], E[2]);
         b_at_node(m, node[0], node[1], node[2], Hh[0], Hh[1], Hh[2]);
     }
@@ -149,8 +156,6 @@ __global__ void __launch_bounds__(kNtffThreads) ntff_kernel(MonitorArgs m, const
     }
     __syncthreads();
     if (live) {
-        const float4 r = rot[k];
-        const float b = blend[k];
         float4* p = st + 9 * threadIdx.x;
         float4 s1[4] = {p[0], p[1], p[2], p[3]}, s2[4] = {p[4], p[5], p[6], p[7]};
         const float f[4] = {2.0f * r.x, -2.0f * r.y, 2.0f * r.z, -2.0f * r.w};
@@ -179,6 +184,8 @@ __global__ void __launch_bounds__(kNtffThreads) ntff_kernel(MonitorArgs m, const
 __global__ void lines_kernel(MonitorArgs m, const int4* qs, int nq, const int4* terms, const float* weights, float4* ph,
                              float* now, const float4* rot, const float* blend, int k) {
     const int qi = blockIdx.x * blockDim.x + threadIdx.x;
+    chain_wait();
+    chain_next();
     if (qi >= nq) return;
     const int4 info = qs[qi];
     float sum = 0.0f;
@@ -294,6 +301,7 @@ __global__ void finite_kernel(MonitorArgs m, unsigned* flag) {
 __global__ void __launch_bounds__(256) dft_sample_kernel(MonitorArgs m, const int* boxes, int points, float* blk,
                                                          int t) {
     __shared__ int sbox[kDftBoxInts];
+    chain_next();  // the last kernel of a step: the next solver pass may come in
     if (threadIdx.x < kDftBoxInts) sbox[threadIdx.x] = boxes[(size_t)blockIdx.y * kDftBoxInts + threadIdx.x];
     __syncthreads();
     const int local = blockIdx.x * blockDim.x + threadIdx.x;
@@ -302,6 +310,7 @@ __global__ void __launch_bounds__(256) dft_sample_kernel(MonitorArgs m, const in
     int node[3];
     float n[3], w;
     ntff_point(sbox, local, node, n, w);
+    chain_wait();
     float E[3], Hh[3];
     e_at_node(m, node[0], node[1], node[2], E[0], E[1], E[2]);
     b_at_node(m, node[0], node[1], node[2], Hh[0], Hh[1], Hh[2]);
@@ -380,20 +389,20 @@ __global__ void expf_kernel(const float* in, float* out, size_t n) {
 }  // namespace
 
 void launch_ports(const MonitorArgs& m, const int4* ports, int n, float* phasors, float* series, long long rec,
-                  const float4* rot, const float* blend, int k, cudaStream_t s) {
-    ports_kernel<<<(n + 63) / 64, 64, 0, s>>>(m, ports, n, phasors, series, rec, rot, blend, k);
+                  const float4* rot, const float* blend, int k, const Chain& s) {
+    launch_chained(s, ports_kernel, (n + 63) / 64, 64, 0, m, ports, n, phasors, series, rec, rot, blend, k);
 }
 
 void launch_ntff(const MonitorArgs& m, const int* box, int points, float* phasors, const float4* rot,
-                 const float* blend, int k, cudaStream_t s) {
-    ntff_kernel<<<(points + kNtffThreads - 1) / kNtffThreads, kNtffThreads, 0, s>>>(
-        m, box, points, reinterpret_cast<float4*>(phasors), rot, blend, k);
+                 const float* blend, int k, const Chain& s) {
+    launch_chained(s, ntff_kernel, (points + kNtffThreads - 1) / kNtffThreads, kNtffThreads, 0, m, box, points,
+                   reinterpret_cast<float4*>(phasors), rot, blend, k);
 }
 
 void launch_lines(const MonitorArgs& m, const int4* q, int nq, const int4* terms, const float* weights,
-                  float* phasors, float* now, const float4* rot, const float* blend, int k, cudaStream_t s) {
-    lines_kernel<<<(nq + 63) / 64, 64, 0, s>>>(m, q, nq, terms, weights, reinterpret_cast<float4*>(phasors), now, rot,
-                                                blend, k);
+                  float* phasors, float* now, const float4* rot, const float* blend, int k, const Chain& s) {
+    launch_chained(s, lines_kernel, (nq + 63) / 64, 64, 0, m, q, nq, terms, weights, reinterpret_cast<float4*>(phasors),
+                   now, rot, blend, k);
 }
 
 void launch_probe_gather(const MonitorArgs& m, const int4* origins, int n, float4* out, const float*, const float*,
@@ -446,8 +455,8 @@ void launch_check_finite(const MonitorArgs& m, unsigned* flag, cudaStream_t s) {
 }
 
 void launch_dft_sample(const MonitorArgs& m, const int* boxes, int nbox, int box_max, int points, float* blk, int t,
-                       cudaStream_t s) {
-    dft_sample_kernel<<<dim3((box_max + 255) / 256, nbox), 256, 0, s>>>(m, boxes, points, blk, t);
+                       const Chain& s) {
+    launch_chained(s, dft_sample_kernel, dim3((box_max + 255) / 256, nbox), 256, 0, m, boxes, points, blk, t);
 }
 
 void launch_dft_gather(const double* x_old, int old_points, const int* map, int new_points, int nf, double* x_new,

@@ -146,6 +146,8 @@ __global__ void __launch_bounds__(32 * (TY + 1), TY <= 8 ? 3 : 1)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+    chain_wait();
+    chain_next();
     bool failed = false;
     int issued_hi = zstart - 1;  // leader: last plane whose loads were issued
     int waited_ok = zstart - 1;  // leader: last plane whose loads were seen complete
@@ -594,6 +596,8 @@ __global__ void __launch_bounds__(32 * (TY + 2), Layout2<TY, Idx>::CTAS)
         *stop = -1;
     }
     __syncthreads();
+    chain_wait();
+    chain_next();
 
     // the absorber of an item's scene (common.glsl:40-43 with the scene's own nx, ny)
     auto scene_size = [&](int scene, int& snx, int& sny) {
@@ -979,7 +983,7 @@ int tile_rows(const YeeArgs& a) { return a.tile_rows == 16 || a.tile_rows == 128
 bool pair_tiles(const YeeArgs& a) { return a.tile_rows == 32 || a.tile_rows == 64 || a.tile_rows == 128; }
 
 template <int TY, typename Idx>
-bool launch_t(const YeeArgs& a, const TmaMaps* m, int gen, unsigned* err, cudaStream_t s) {
+bool launch_t(const YeeArgs& a, const TmaMaps* m, int gen, unsigned* err, const Chain& s) {
     using Lay = Layout<TY, Idx>;
     static bool configured = false;
     {
@@ -992,8 +996,8 @@ bool launch_t(const YeeArgs& a, const TmaMaps* m, int gen, unsigned* err, cudaSt
         }
     }
     const dim3 grid((a.nx + 31) / 32, (a.ny + TY - 1) / TY, (a.nz + a.zchunk - 1) / a.zchunk);
-    yee_tma<TY, Idx><<<grid, dim3(32, TY + 1), Lay::SMEM, s>>>(m->e[gen][0], m->e[gen][1], m->e[gen][2], m->b[gen][0],
-                                                           m->b[gen][1], m->b[gen][2], m->cls, a, err);
+    launch_chained(s, yee_tma<TY, Idx>, grid, dim3(32, TY + 1), Lay::SMEM, m->e[gen][0], m->e[gen][1], m->e[gen][2],
+                   m->b[gen][0], m->b[gen][1], m->b[gen][2], m->cls, a, err);
     return true;
 }
 
@@ -1049,7 +1053,7 @@ void small_grid_schedule(PairSched& ps, int nz, int G) {
 }
 
 template <int TY, typename Idx>
-bool launch_p(const YeeArgs& a, const TmaMaps* m, int gen, unsigned* err, cudaStream_t s) {
+bool launch_p(const YeeArgs& a, const TmaMaps* m, int gen, unsigned* err, const Chain& s) {
     using Lay = Layout2<TY, Idx>;
     static int resident = 0, sms = 0;  // per process: one device model
     std::unique_lock<std::mutex> lk(g_launch_setup);
@@ -1086,7 +1090,7 @@ bool launch_p(const YeeArgs& a, const TmaMaps* m, int gen, unsigned* err, cudaSt
     if (ps.items <= 0) return false;
     const int grid = std::min(ps.items, resident * sms);
     ps.work = a.work;
-    yee_tma2<TY, Idx><<<grid, dim3(32, TY + 2), Lay::SMEM, s>>>(m->e3[gen], m->b3[gen], m->cls, a, ps, err);
+    launch_chained(s, yee_tma2<TY, Idx>, grid, dim3(32, TY + 2), Lay::SMEM, m->e3[gen], m->b3[gen], m->cls, a, ps, err);
     return true;
 }
 
@@ -1167,7 +1171,7 @@ std::vector<int4> ragged_items(const std::vector<int>& z0, const std::vector<int
     return out;
 }
 
-bool launch_yee_tma(const YeeArgs& a, const TmaMaps* m, int gen, bool wide, unsigned* err, cudaStream_t s) {
+bool launch_yee_tma(const YeeArgs& a, const TmaMaps* m, int gen, bool wide, unsigned* err, const Chain& s) {
     if (!m || !m->ok[gen] || !m->cls_ok) return false;
     if (pair_tiles(a) && tile_rows(a) == 16)
         return wide ? launch_p<16, uint32_t>(a, m, gen, err, s)
