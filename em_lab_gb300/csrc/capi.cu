@@ -302,6 +302,44 @@ float blend_of(float avg, float wl, double dt) {
     return (float)(1.0 - std::exp(-dt / (0.5 * tau)));
 }
 
+// Polls until query() is no longer cudaErrorNotReady or the time (60 s by default) is over. The first
+// 10 ms only yield: a sleep of 50 us lasts some 110 and ends late by half of that on average, which a
+// frame of a small scene paid three times (272 us a frame of a 48 cube, 86 us without the
+// sleeps, the copies of the error word and the allocations of the read-backs).
+template <class Query>
+cudaError_t wait_until(Query&& query, int timeout_ms) {
+    const auto limit = std::chrono::milliseconds(timeout_ms > 0 ? timeout_ms : 60000);
+    const auto t0 = std::chrono::steady_clock::now();
+    for (;;) {
+        const cudaError_t e = query();
+        if (e != cudaErrorNotReady) return e;
+        const auto spent = std::chrono::steady_clock::now() - t0;
+        if (spent > limit) return e;
+        if (spent < std::chrono::milliseconds(10)) std::this_thread::yield();
+        else std::this_thread::sleep_for(std::chrono::microseconds(50));
+    }
+}
+
+// The grid's pinned scratch of at least `bytes` (at most kHostScratch), for one synchronous call; null where it
+// cannot be had.
+unsigned char* host_scratch(emlab_grid* g, size_t bytes) {
+    if (bytes > kHostScratch) return nullptr;
+    if (g->h_scratch_busy && cudaStreamSynchronize(g->stream) != cudaSuccess) return nullptr;  // left by a failed wait
+    if (g->h_scratch_bytes < bytes) {
+        const size_t want = std::max<size_t>(2 * bytes, 16 << 10);
+        if (g->h_scratch) cudaFreeHost(g->h_scratch);
+        g->h_scratch = nullptr, g->h_scratch_bytes = 0;
+        if (cudaMallocHost(&g->h_scratch, std::min(want, kHostScratch)) != cudaSuccess) {
+            cudaGetLastError();
+            g->h_scratch = nullptr;
+            return nullptr;
+        }
+        g->h_scratch_bytes = std::min(want, kHostScratch);
+    }
+    g->h_scratch_busy = true;
+    return g->h_scratch;
+}
+
 int ensure_stage(emlab_grid* g, size_t bytes) {
     if (bytes <= g->stage_bytes) return EMLAB_OK;
     invalidate_graphs(g);
@@ -361,7 +399,7 @@ int dft_fold(emlab_grid* g) {
     const double dt = (double)g->cfg.courant;
     if (g->dft_engine == EMLAB_DFT_TENSOR &&
         launch_dft_fold_tc(g->d_dft_blk.p, g->dft_t, g->dft_points, g->dft_nf, g->d_dft_bhi.p, g->d_dft_blo.p,
-                           g->d_dft_omega.p, g->dft_n0, dt, g->d_dft_x.p, g->d_err.p, g->stream)) {
+                           g->d_dft_omega.p, g->dft_n0, dt, g->d_dft_x.p, const_cast<unsigned*>(g->h_err), g->stream)) {
         ++g_launches;
     } else {
         // CUDA-core folds of 64 samples each, every one with the phase of its own first sample
@@ -412,7 +450,7 @@ uint64_t enqueue_step(emlab_grid* g, int k, bool graph, const float* d_sig, cons
         launched += 2;
     } else {
         const bool tma = g->kernel == EMLAB_KERNEL_FUSED &&
-                         launch_yee_tma(a, g->tma, g->cur, g->wide, g->d_err.p, first);
+                         launch_yee_tma(a, g->tma, g->cur, g->wide, const_cast<unsigned*>(g->h_err), first);
         if (!tma && g->stack.ragged) g->launch_failed = true;  // no kernel here knows the scenes' cross-sections
         else if (!tma) launch_yee_fused(a, g->wide, first);
         launched += 1;
@@ -485,12 +523,13 @@ int emlab_grid_create(emlab_grid** out) {
     if (cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&g->stage_done[0], cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&g->stage_done[1], cudaEventDisableTiming) != cudaSuccess ||
-        g->d_flag.alloc(1) != cudaSuccess || g->d_err.alloc(1) != cudaSuccess ||
-        cudaMemsetAsync(g->d_err.p, 0, 4, g->stream) != cudaSuccess || g->d_work.alloc(2) != cudaSuccess ||
-        cudaMemsetAsync(g->d_work.p, 0, 16, g->stream) != cudaSuccess) {
+        g->d_flag.alloc(1) != cudaSuccess || cudaMallocHost((void**)&g->h_err, 4) != cudaSuccess ||
+        g->d_work.alloc(2) != cudaSuccess || cudaMemsetAsync(g->d_work.p, 0, 16, g->stream) != cudaSuccess) {
+        if (g->h_err) cudaFreeHost(const_cast<unsigned*>(g->h_err));
         delete g;
         return fail(EMLAB_ERR_CUDA, "stream or event creation failed");
     }
+    *g->h_err = 0;
     *out = g;
     return EMLAB_OK;
 }
@@ -508,6 +547,8 @@ int emlab_grid_destroy(emlab_grid* g) {
     for (size_t i = 0; i < g->ev_start.size(); ++i) cudaEventDestroy(g->ev_start[i]), cudaEventDestroy(g->ev_stop[i]);
     if (g->tma) tma_maps_destroy(g->tma);
     invalidate_graphs(g);
+    cudaFreeHost(const_cast<unsigned*>(g->h_err));
+    if (g->h_scratch) cudaFreeHost(g->h_scratch);
     for (auto& a : g->analyzer) {
         if (a.h_probe) cudaFreeHost(a.h_probe);
         if (a.h_part) cudaFreeHost(a.h_part);
@@ -768,23 +809,14 @@ int emlab_grid_set_graph(emlab_grid* g, int chunk) {
 
 int emlab_grid_synchronize(emlab_grid* g, int timeout_ms) {
     if (!g) return fail(EMLAB_ERR_INVALID, "null grid handle");
-    const auto limit = std::chrono::milliseconds(timeout_ms > 0 ? timeout_ms : 60000);
-    const auto t0 = std::chrono::steady_clock::now();
-    for (;;) {
-        cudaError_t e = cudaStreamQuery(g->stream);
-        if (e == cudaSuccess) {
-            unsigned err = 0;
-            EMLAB_CUDA(cudaMemcpy(&err, g->d_err.p, 4, cudaMemcpyDeviceToHost));
-            if (err) {
-                EMLAB_CUDA(cudaMemsetAsync(g->d_err.p, 0, 4, g->stream));
-                return fail(EMLAB_ERR_TIMEOUT, "a solver kernel gave up a bounded wait on the device");
-            }
-            return EMLAB_OK;
-        }
-        if (e != cudaErrorNotReady) return fail(EMLAB_ERR_CUDA, std::string("stream: ") + cudaGetErrorString(e));
-        if (std::chrono::steady_clock::now() - t0 > limit) return fail(EMLAB_ERR_TIMEOUT, "grid stream wait timed out");
-        std::this_thread::sleep_for(std::chrono::microseconds(50));
+    const cudaError_t e = wait_until([&] { return cudaStreamQuery(g->stream); }, timeout_ms);
+    if (e == cudaErrorNotReady) return fail(EMLAB_ERR_TIMEOUT, "grid stream wait timed out");
+    if (e != cudaSuccess) return fail(EMLAB_ERR_CUDA, std::string("stream: ") + cudaGetErrorString(e));
+    if (*g->h_err) {
+        *g->h_err = 0;
+        return fail(EMLAB_ERR_TIMEOUT, "a solver kernel gave up a bounded wait on the device");
     }
+    return EMLAB_OK;
 }
 
 int emlab_grid_get_state(const emlab_grid* g, emlab_grid_state* out) {
@@ -1026,19 +1058,10 @@ int emlab_ports_collect_series(emlab_grid* g, int slot, float* out, size_t max_s
     EMLAB_REQUIRE(g->series_busy[slot], "the series slot holds no pending take");
     EMLAB_REQUIRE(out || max_steps == 0, "null output");
     EMLAB_CUDA(cudaSetDevice(g->device));
-    const auto limit = std::chrono::milliseconds(timeout_ms > 0 ? timeout_ms : 60000);
-    const auto t0 = std::chrono::steady_clock::now();
-    for (;;) {
-        const cudaError_t e = cudaEventQuery(g->series_done[slot]);
-        if (e == cudaSuccess) break;
-        if (e != cudaErrorNotReady) return fail(EMLAB_ERR_CUDA, std::string("series copy: ") + cudaGetErrorString(e));
-        if (std::chrono::steady_clock::now() - t0 > limit)
-            return fail(EMLAB_ERR_TIMEOUT, "series copy did not complete within the timeout");
-        std::this_thread::sleep_for(std::chrono::microseconds(50));
-    }
-    unsigned err = 0;
-    EMLAB_CUDA(cudaMemcpy(&err, g->d_err.p, 4, cudaMemcpyDeviceToHost));
-    if (err) return fail(EMLAB_ERR_TIMEOUT, "a solver kernel's bounded wait ran out");
+    const cudaError_t e = wait_until([&] { return cudaEventQuery(g->series_done[slot]); }, timeout_ms);
+    if (e == cudaErrorNotReady) return fail(EMLAB_ERR_TIMEOUT, "series copy did not complete within the timeout");
+    if (e != cudaSuccess) return fail(EMLAB_ERR_CUDA, std::string("series copy: ") + cudaGetErrorString(e));
+    if (*g->h_err) return fail(EMLAB_ERR_TIMEOUT, "a solver kernel's bounded wait ran out");
     const size_t s = std::min(max_steps, g->h_series_rows[slot]);
     if (s) std::memcpy(out, g->h_series[slot], s * (size_t)g->nports * 8);
     g->series_busy[slot] = false;
@@ -1435,16 +1458,28 @@ int emlab_probe_gather(emlab_grid* g, const int* origins, int n_probes, float* o
     if (int rc = require_grid(g)) return rc;
     EMLAB_REQUIRE(origins && out && n_probes > 0, "bad probe arguments");
     EMLAB_CUDA(cudaSetDevice(g->device));
-    DevBuf<int4> d_o;
-    DevBuf<float4> d_out;
-    EMLAB_CUDA(d_o.alloc((size_t)n_probes));
-    EMLAB_CUDA(d_out.alloc((size_t)n_probes * 54));
-    EMLAB_CUDA(cudaMemcpyAsync(d_o.p, origins, (size_t)n_probes * 16, cudaMemcpyHostToDevice, g->stream));
-    launch_probe_gather(monitor_args(g), d_o.p, n_probes, d_out.p, nullptr, nullptr, g->stream);
-    ++g_launches;
-    if (int rc = check_launch()) return rc;
-    EMLAB_CUDA(cudaMemcpyAsync(out, d_out.p, (size_t)n_probes * 54 * 16, cudaMemcpyDeviceToHost, g->stream));
-    if (int rc = emlab_grid_synchronize(g, 0)) return rc;
+    const size_t in = (size_t)n_probes * 16, bytes = (size_t)n_probes * 54 * 16;
+    if (unsigned char* h = host_scratch(g, in + bytes)) {  // the kernel reads and writes host memory
+        std::memcpy(h, origins, in);
+        launch_probe_gather(monitor_args(g), reinterpret_cast<int4*>(h), n_probes, reinterpret_cast<float4*>(h + in),
+                            nullptr, nullptr, g->stream);
+        ++g_launches;
+        if (int rc = check_launch()) return rc;
+        if (int rc = emlab_grid_synchronize(g, 0)) return rc;
+        g->h_scratch_busy = false;
+        std::memcpy(out, h + in, bytes);
+    } else {
+        DevBuf<int4> d_o;
+        DevBuf<float4> d_out;
+        EMLAB_CUDA(d_o.alloc((size_t)n_probes));
+        EMLAB_CUDA(d_out.alloc((size_t)n_probes * 54));
+        EMLAB_CUDA(cudaMemcpyAsync(d_o.p, origins, in, cudaMemcpyHostToDevice, g->stream));
+        launch_probe_gather(monitor_args(g), d_o.p, n_probes, d_out.p, nullptr, nullptr, g->stream);
+        ++g_launches;
+        if (int rc = check_launch()) return rc;
+        EMLAB_CUDA(cudaMemcpyAsync(out, d_out.p, bytes, cudaMemcpyDeviceToHost, g->stream));
+        if (int rc = emlab_grid_synchronize(g, 0)) return rc;
+    }
     if (int rc = ensure_cell_materials(g)) return rc;
     const int nx = g->cfg.nx, ny = g->cfg.ny, nz = g->cfg.nz;
     for (int id = 0; id < n_probes * 54; ++id) {
@@ -1494,38 +1529,29 @@ int emlab_flux_planes(emlab_grid* g, const emlab_flux_plane* planes, int n_plane
     EMLAB_REQUIRE(planes && out && n_planes >= 0, "bad flux arguments");
     EMLAB_CUDA(cudaSetDevice(g->device));
     const int size[3] = {g->cfg.nx, g->cfg.ny, g->cfg.nz};
-    struct Rect {
-        int axis, index, m0, m1, r0, r1;
-        size_t groups, offset;
-    };
-    std::vector<Rect> rects;
+    std::vector<FluxRect> rects;
     size_t total = 0;
     for (int i = 0; i < n_planes; ++i) {
-        const emlab_flux_plane& p = planes[i];
-        Rect r{std::clamp(p.axis, 0, 2), p.index, 0, 0, 0, 0, 0, total};
-        const int u = r.axis == 0 ? 1 : 0, v = r.axis == 2 ? 1 : 2;
-        r.m0 = std::max(p.rect_min[0], 0), r.m1 = std::max(p.rect_min[1], 0);
-        r.r0 = std::min(p.rect_max[0], size[u]) - r.m0, r.r1 = std::min(p.rect_max[1], size[v]) - r.m1;
-        if (p.index < 0 || p.index >= size[r.axis] || r.r0 <= 0 || r.r1 <= 0) r.groups = 0;
-        else r.groups = (size_t)((r.r0 + 15) / 16) * ((r.r1 + 15) / 16);
-        total += r.groups;
-        rects.push_back(r);
+        rects.push_back(flux_rect(planes[i], size, (long long)total));
+        total += (size_t)rects.back().groups;
     }
     DevBuf<float> d_part;
-    EMLAB_CUDA(d_part.alloc(std::max<size_t>(total, 1)));
-    const MonitorArgs m = monitor_args(g);
-    for (const Rect& r : rects) {
-        if (!r.groups) continue;
-        launch_flux_plane(m, r.axis, r.index, r.m0, r.m1, r.r0, r.r1, d_part.p + r.offset, g->stream);
-        ++g_launches;
+    std::vector<float> h_part;
+    float* part = reinterpret_cast<float*>(host_scratch(g, std::max<size_t>(total, 1) * 4));
+    const bool direct = part != nullptr;  // the kernel writes host memory
+    if (!direct) {
+        EMLAB_CUDA(d_part.alloc(std::max<size_t>(total, 1)));
+        h_part.resize(std::max<size_t>(total, 1));
+        part = h_part.data();
     }
+    g_launches += (uint64_t)launch_flux_planes(monitor_args(g), rects.data(), n_planes, direct ? part : d_part.p, g->stream);
     if (int rc = check_launch()) return rc;
-    std::vector<float> part(std::max<size_t>(total, 1));
-    EMLAB_CUDA(cudaMemcpyAsync(part.data(), d_part.p, part.size() * 4, cudaMemcpyDeviceToHost, g->stream));
+    if (!direct) EMLAB_CUDA(cudaMemcpyAsync(part, d_part.p, h_part.size() * 4, cudaMemcpyDeviceToHost, g->stream));
     if (int rc = emlab_grid_synchronize(g, 0)) return rc;
+    if (direct) g->h_scratch_busy = false;
     for (int i = 0; i < n_planes; ++i) {
         double s = 0.0;  // FP64 sum of the FP32 workgroup partials (FieldAnalyzer.cpp:356-357)
-        for (size_t k = 0; k < rects[i].groups; ++k) s += (double)part[rects[i].offset + k];
+        for (int k = 0; k < rects[i].groups; ++k) s += (double)part[(size_t)rects[i].first + k];
         out[i] = s;
     }
     return EMLAB_OK;
@@ -1544,19 +1570,11 @@ int emlab_analyzer_submit(emlab_grid* g, const int* origins, int n_probes, const
     const int size[3] = {g->cfg.nx, g->cfg.ny, g->cfg.nz};
     a.planes.clear();
     size_t total = 0;
-    std::vector<int> geo;  // axis, index, m0, m1, r0, r1 per plane with partials
+    std::vector<FluxRect> rects;
     for (int i = 0; i < n_planes; ++i) {
-        const emlab_flux_plane& p = planes[i];
-        const int axis = std::clamp(p.axis, 0, 2);
-        const int u = axis == 0 ? 1 : 0, v = axis == 2 ? 1 : 2;
-        const int m0 = std::max(p.rect_min[0], 0), m1 = std::max(p.rect_min[1], 0);
-        const int r0 = std::min(p.rect_max[0], size[u]) - m0, r1 = std::min(p.rect_max[1], size[v]) - m1;
-        size_t groups = 0;
-        if (p.index >= 0 && p.index < size[axis] && r0 > 0 && r1 > 0)
-            groups = (size_t)((r0 + 15) / 16) * ((r1 + 15) / 16);
-        a.planes.emplace_back(total, groups);
-        geo.insert(geo.end(), {axis, p.index, m0, m1, r0, r1});
-        total += groups;
+        rects.push_back(flux_rect(planes[i], size, (long long)total));
+        a.planes.emplace_back(total, (size_t)rects.back().groups);
+        total += (size_t)rects.back().groups;
     }
     if ((size_t)n_probes > a.probe_cap) {
         if (a.h_probe) cudaFreeHost(a.h_probe);
@@ -1586,12 +1604,7 @@ int emlab_analyzer_submit(emlab_grid* g, const int* origins, int n_probes, const
         EMLAB_CUDA(cudaMemcpyAsync(a.h_probe, a.d_probe.p, (size_t)n_probes * 54 * 16, cudaMemcpyDeviceToHost,
                                    g->stream));
     }
-    for (int i = 0; i < n_planes; ++i) {
-        if (!a.planes[(size_t)i].second) continue;
-        const int* q = &geo[(size_t)i * 6];
-        launch_flux_plane(m, q[0], q[1], q[2], q[3], q[4], q[5], a.d_part.p + a.planes[(size_t)i].first, g->stream);
-        ++g_launches;
-    }
+    g_launches += (uint64_t)launch_flux_planes(m, rects.data(), n_planes, a.d_part.p, g->stream);
     if (total) EMLAB_CUDA(cudaMemcpyAsync(a.h_part, a.d_part.p, total * 4, cudaMemcpyDeviceToHost, g->stream));
     if (int rc = check_launch()) return rc;
     EMLAB_CUDA(cudaEventRecord(a.done, g->stream));

@@ -126,8 +126,16 @@ void launch_lines(const MonitorArgs& m, const int4* q, int nq, const int4* terms
                   float* phasors, float* now, const float4* rot, const float* blend, int k, const Chain& s);
 void launch_probe_gather(const MonitorArgs& m, const int4* origins, int n, float4* out, const float* cell_sig,
                          const float* cell_eps, cudaStream_t s);
-void launch_flux_plane(const MonitorArgs& m, int axis, int index, int rmin0, int rmin1, int rs0, int rs1,
-                       float* partials, cudaStream_t s);
+// One flux plane clipped to the grid (FieldAnalyzer::dispatchPlane, src/FieldAnalyzer.cpp:100-124): groups 16 x 16
+// workgroups, none for an empty rectangle or an index outside the grid, whose partials start at `first`.
+struct FluxRect {
+    int axis, index, m0, m1, r0, r1;
+    int groups;
+    long long first;
+};
+FluxRect flux_rect(const emlab_flux_plane& p, const int size[3], long long first);
+// The partials of n planes; returns the number of launches.
+int launch_flux_planes(const MonitorArgs& m, const FluxRect* rects, int n, float* partials, cudaStream_t s);
 // The far-field pattern of a box (pattern.cu) at n_dirs directions and nf frequencies (box: the host's
 // record): slices of the surface, directions and frequencies per launch, kernel launches, floats of scratch.
 struct PatternPlan {

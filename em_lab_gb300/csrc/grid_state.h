@@ -48,6 +48,7 @@ struct DevBuf {
     }
 };
 
+constexpr size_t kHostScratch = 1 << 20;
 constexpr int kChunk = 1024;  // sub-steps whose host-side scalars are uploaded together
 
 // One queued FieldAnalyzer measurement: device outputs, pinned host copies, the event that ends it.
@@ -112,7 +113,12 @@ struct emlab_grid {
     DevBuf<unsigned> pml_zi;  // per plane: that bit and the z depth classes, packed (YeeArgs::pml_zi)
     int pml_K = 0;
     emlab::TmaMaps* tma = nullptr;
-    DevBuf<unsigned> d_err;  // set by a solver kernel whose bounded on-device wait ran out
+    volatile unsigned* h_err = nullptr;  // pinned, written by a kernel whose bounded on-device wait ran out
+    // pinned scratch of the synchronous read-backs, which kernels read and write directly: at most
+    // kHostScratch bytes, free again when the call's synchronize has succeeded
+    unsigned char* h_scratch = nullptr;
+    size_t h_scratch_bytes = 0;
+    bool h_scratch_busy = false;
     DevBuf<unsigned long long> d_work;  // persistent Yee kernel: tickets drawn, CTAs that have left
     std::vector<float> cell_sigma, cell_eps;  // alpha channels of the textures (read-back only)
     // sources

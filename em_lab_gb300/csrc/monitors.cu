@@ -9,7 +9,7 @@ namespace emlab {
 
 namespace {
 
-__device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
+__host__ __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 
 __device__ __forceinline__ long long cidx(const MonitorArgs& m, int x, int y, int z) {
     x = clampi(x, 0, m.nx - 1), y = clampi(y, 0, m.ny - 1), z = clampi(z, 0, m.nz - 1);
@@ -218,11 +218,22 @@ __global__ void probe_kernel(MonitorArgs m, const int4* origins, int n, float4* 
     out[id] = k < 27 ? make_float4(m.ex[j], m.ey[j], m.ez[j], 0.0f) : make_float4(m.bx[j], m.by[j], m.bz[j], 0.0f);
 }
 
-// poynting_flux.comp:32-63: one partial per 16x16 workgroup, tree reduction in the shader's order
-__global__ void __launch_bounds__(256) flux_kernel(MonitorArgs m, int axis, int index, int rmin0, int rmin1, int rs0,
-                                                   int rs1, float* partials) {
+// poynting_flux.comp:32-63: one partial per 16x16 workgroup, tree reduction in the shader's order. The
+// workgroups of up to kFluxPlanes planes in one launch (a box's six planes of 16 x 16 nodes are six
+// workgroups: launches, not work, bounded them one plane at a time).
+constexpr int kFluxPlanes = 16;
+struct FluxList {
+    FluxRect r[kFluxPlanes];
+    int n;
+};
+__global__ void __launch_bounds__(256) flux_kernel(MonitorArgs m, const __grid_constant__ FluxList list,
+                                                   float* partials) {
     __shared__ float sp[256];
-    const int lu = blockIdx.x * 16 + threadIdx.x, lv = blockIdx.y * 16 + threadIdx.y;
+    int q = 0, group = blockIdx.x;
+    while (group >= list.r[q].groups) group -= list.r[q++].groups;
+    const int axis = list.r[q].axis, index = list.r[q].index, rmin0 = list.r[q].m0, rmin1 = list.r[q].m1;
+    const int rs0 = list.r[q].r0, rs1 = list.r[q].r1, across = (rs0 + 15) / 16;
+    const int lu = group % across * 16 + threadIdx.x, lv = group / across * 16 + threadIdx.y;
     const int lid = threadIdx.y * 16 + threadIdx.x;
     float flux = 0.0f;
     if (lu < rs0 && lv < rs1) {
@@ -247,7 +258,7 @@ __global__ void __launch_bounds__(256) flux_kernel(MonitorArgs m, int axis, int 
         if (lid < stride) sp[lid] = sp[lid] + sp[lid + stride];
         __syncthreads();
     }
-    if (lid == 0) partials[blockIdx.y * gridDim.x + blockIdx.x] = sp[0];
+    if (lid == 0) partials[list.r[q].first + group] = sp[0];
 }
 
 // PortMonitor::evaluateSweep sums (Ports.cpp:215-242) in FP64: one block per (port, frequency)
@@ -410,10 +421,27 @@ void launch_probe_gather(const MonitorArgs& m, const int4* origins, int n, float
     probe_kernel<<<(n * 54 + 63) / 64, 64, 0, s>>>(m, origins, n, out);
 }
 
-void launch_flux_plane(const MonitorArgs& m, int axis, int index, int rmin0, int rmin1, int rs0, int rs1,
-                       float* partials, cudaStream_t s) {
-    const dim3 grid((rs0 + 15) / 16, (rs1 + 15) / 16);
-    flux_kernel<<<grid, dim3(16, 16), 0, s>>>(m, axis, index, rmin0, rmin1, rs0, rs1, partials);
+FluxRect flux_rect(const emlab_flux_plane& p, const int size[3], long long first) {
+    FluxRect r{clampi(p.axis, 0, 2), p.index, max(p.rect_min[0], 0), max(p.rect_min[1], 0), 0, 0, 0, first};
+    const int u = r.axis == 0 ? 1 : 0, v = r.axis == 2 ? 1 : 2;
+    r.r0 = min(p.rect_max[0], size[u]) - r.m0, r.r1 = min(p.rect_max[1], size[v]) - r.m1;
+    if (p.index >= 0 && p.index < size[r.axis] && r.r0 > 0 && r.r1 > 0) r.groups = (r.r0 + 15) / 16 * ((r.r1 + 15) / 16);
+    return r;
+}
+
+int launch_flux_planes(const MonitorArgs& m, const FluxRect* rects, int n, float* partials, cudaStream_t s) {
+    int launches = 0;
+    for (int i = 0; i < n;) {
+        FluxList list;
+        int groups = 0;
+        list.n = 0;
+        for (; i < n && list.n < kFluxPlanes; ++i)
+            if (rects[i].groups) list.r[list.n++] = rects[i], groups += rects[i].groups;
+        if (!groups) continue;
+        flux_kernel<<<groups, dim3(16, 16), 0, s>>>(m, list, partials);
+        ++launches;
+    }
+    return launches;
 }
 
 void launch_sweep_sums(const float* series, long long steps, int nports, double nu_lo, double nu_hi, int points,

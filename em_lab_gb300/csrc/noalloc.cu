@@ -1,10 +1,11 @@
 // noalloc.cu - Poynting flux through planes without any memory allocation.
 //
-// emlab_flux_planes allocates its per-workgroup partial sums with cudaMalloc and frees them again
-// on every call. Some callers cannot accept that: a frame loop that measures flux every other
-// frame, like the reference's, while the solver keeps stepping (cudaFree waits for the whole
-// device, so every measurement would stall the solver), and applications that budget all device
-// memory themselves (an allocation they did not plan for can fail part-way through a run). This
+// emlab_flux_planes sums in a pinned host scratch that its grid keeps, allocated by the first call, and
+// past a megabyte of workgroup partials in device memory of the call. Some callers cannot accept that: a
+// frame loop that measures flux every other frame, like the reference's, while the solver keeps stepping
+// (cudaFree waits for the whole device, so such a measurement would stall the solver), and applications
+// that budget all device memory themselves (an allocation they did not plan for can fail part-way
+// through a run). This
 // variant keeps its scratch in fixed file-scope device arrays instead: kMaxPartials workgroup
 // partials (256 KB) and kMaxPlanes FP64 sums, held by every device that loads the library until
 // the process exits. The first call on a device looks their addresses up; every call shares them,
@@ -90,40 +91,24 @@ extern "C" int emlab_flux_planes_noalloc(emlab_grid* g, const emlab_flux_plane* 
         return report_error(EMLAB_ERR_INVALID, "emlab_flux_planes_noalloc: more planes than its fixed scratch holds "
                                                "(EMLAB_FLUX_NOALLOC_MAX_PLANES)");
     if (n_planes == 0) return EMLAB_OK;
-    // the rectangle clipping of FieldAnalyzer::dispatchPlane (src/FieldAnalyzer.cpp:100-124)
     const int size[3] = {m.nx, m.ny, m.nz};
     PlaneSums ps{};
-    int axis[kMaxPlanes], m0[kMaxPlanes], m1[kMaxPlanes], r0[kMaxPlanes], r1[kMaxPlanes];
+    FluxRect rects[kMaxPlanes];
     int total = 0;
     for (int i = 0; i < n_planes; ++i) {
-        const emlab_flux_plane& p = planes[i];
-        const int a = p.axis < 0 ? 0 : (p.axis > 2 ? 2 : p.axis);
-        const int u = a == 0 ? 1 : 0, v = a == 2 ? 1 : 2;
-        axis[i] = a;
-        m0[i] = p.rect_min[0] > 0 ? p.rect_min[0] : 0;
-        m1[i] = p.rect_min[1] > 0 ? p.rect_min[1] : 0;
-        r0[i] = (p.rect_max[0] < size[u] ? p.rect_max[0] : size[u]) - m0[i];
-        r1[i] = (p.rect_max[1] < size[v] ? p.rect_max[1] : size[v]) - m1[i];
-        long long groups = 0;
-        if (p.index >= 0 && p.index < size[a] && r0[i] > 0 && r1[i] > 0)
-            groups = (long long)((r0[i] + 15) / 16) * ((r1[i] + 15) / 16);
-        if (total + groups > kMaxPartials)
+        const FluxRect& r = rects[i] = flux_rect(planes[i], size, total);
+        if ((long long)total + r.groups > kMaxPartials)
             return report_error(EMLAB_ERR_INVALID, "emlab_flux_planes_noalloc: the planes need more workgroup partials "
                                                    "than its fixed scratch holds (EMLAB_FLUX_NOALLOC_MAX_PARTIALS)");
         ps.offset[i] = total;
-        ps.groups[i] = (int)groups;
-        total += (int)groups;
+        ps.groups[i] = r.groups;
+        total += r.groups;
     }
     ps.n = n_planes;
     Scratch s;
     if (scratch_for(device, s) != EMLAB_OK)
         return report_error(EMLAB_ERR_CUDA, "emlab_flux_planes_noalloc: device scratch lookup failed");
-    int launched = 0;
-    for (int i = 0; i < n_planes; ++i) {
-        if (!ps.groups[i]) continue;
-        launch_flux_plane(m, axis[i], planes[i].index, m0[i], m1[i], r0[i], r1[i], s.partials + ps.offset[i], stream);
-        ++launched;
-    }
+    const int launched = launch_flux_planes(m, rects, n_planes, s.partials, stream);
     flux_sum_kernel<<<1, kMaxPlanes, 0, stream>>>(s.partials, ps, s.sums);
     count_launches(launched + 1);
     cudaError_t e = cudaGetLastError();

@@ -510,8 +510,8 @@ extern "C" int emlab_ntff_dft_pattern_gemm(emlab_grid* g, int box, const float* 
         face_tiles_kernel<<<dim3(field_blocks, 6 * n), kFieldThreads, 0, g->stream>>>(bx, X, g->dft_points, f0, scale, B, power);
         const int items = n * ((D + kDirs - 1) / kDirs);
         pattern_kernel<<<std::min(items, sms), kThreads, kSmem, g->stream>>>(
-            bx, B, power, g->d_dft_omega.p + f0, n, g->d_spec_dirs.p, D, g->d_spec_out.p + (size_t)f0 * D * 2, g->d_err.p,
-            wait_limit());
+            bx, B, power, g->d_dft_omega.p + f0, n, g->d_spec_dirs.p, D, g->d_spec_out.p + (size_t)f0 * D * 2,
+            const_cast<unsigned*>(g->h_err), wait_limit());
         count_launches(2);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return fail(EMLAB_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
