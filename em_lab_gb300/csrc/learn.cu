@@ -25,7 +25,7 @@ namespace emlab {
 namespace {
 
 constexpr int kTM = 128, kTK = 64;  // tile rows, K chunk (tile columns: 64 or 128)
-constexpr int kThreads = 256;
+constexpr int kThreads = 256, kLoaders = kThreads - 32;  // warp 0 issues the MMAs, the others copy
 // Core matrices (8 x 16 bytes, 128 bytes) of a chunk. K-major (a piece is 8 elements along K of one
 // row): 144 bytes apart along K, 8 x 144 along the rows. Row-major (a piece is 8 rows of one k): 128
 // apart along K, 8 x 128 + 16 along the rows. The padding puts the pieces that eight neighbouring
@@ -98,26 +98,25 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
 // backward pass; the tensor core reads it row-major); kAny, element by element.
 enum { kRowsK = 0, kColsK = 1, kAny = 2 };
 
-// One operand's 64-wide K chunk from k0, ROWS rows from row0 of its `rows`, into `tile`. Everything beyond
-// the operand's rows or K is zero; pieces beyond the rows stay so in a stage once `fresh` wrote them.
+// One operand's 64-wide K chunk from k0, ROWS rows from row0 of its `rows`, into `tile`, by the loading
+// threads (t of kLoaders). Everything beyond the operand's rows or K is zero; pieces beyond the rows stay so
+// in a stage once `fresh` wrote them.
 template <int ROWS, int MODE>
-__device__ __forceinline__ void stage_operand(unsigned char* tile, const __nv_bfloat16* p, long long s_row,
+__device__ __forceinline__ void stage_operand(int t, unsigned char* tile, const __nv_bfloat16* p, long long s_row,
                                               long long s_k, int row0, int rows, int k0, int K, bool fresh) {
-    const int t = threadIdx.x;
-    if (MODE == kColsK) {  // piece (k, row block): a warp copies 32 (or 16) neighbouring row blocks of a k
 #pragma unroll
-        for (int i = 0; i < ROWS * kTK / 8 / kThreads; ++i) {
-            const int q = t + i * kThreads, block = q % (ROWS / 8), k = q / (ROWS / 8);
+    for (int i = 0; i < (ROWS * kTK / 8 + kLoaders - 1) / kLoaders; ++i) {
+        const int q = t + i * kLoaders;
+        if (q >= ROWS * kTK / 8) break;
+        if (MODE == kColsK) {  // piece (k, row block): a warp copies 32 (or 16) neighbouring row blocks of a k
+            const int block = q % (ROWS / 8), k = q / (ROWS / 8);
             const int r = row0 + block * 8;
             if (r >= rows && !fresh) continue;
             const int live = k0 + k < K ? max(0, min(8, rows - r)) : 0;
             cp_async16(tile + block * kSboR + (k >> 3) * kLboR + (k & 7) * 16,
                        live ? p + (long long)(k0 + k) * s_k + r : p, 2 * live);
-        }
-    } else {  // piece (row, K block): eight threads copy a row's 128 bytes
-#pragma unroll
-        for (int i = 0; i < ROWS * kTK / 8 / kThreads; ++i) {
-            const int q = t + i * kThreads, block = q & 7, r = q >> 3, k = k0 + block * 8;
+        } else {  // piece (row, K block): eight threads copy a row's 128 bytes
+            const int block = q & 7, r = q >> 3, k = k0 + block * 8;
             if (row0 + r >= rows && !fresh) continue;
             unsigned char* dst = tile + (r >> 3) * kSboK + block * kLboK + (r & 7) * 16;
             const int live = row0 + r < rows ? max(0, min(8, K - k)) : 0;
@@ -134,158 +133,256 @@ __device__ __forceinline__ void stage_operand(unsigned char* tile, const __nv_bf
     }
 }
 
+// What becomes of a product C. kStore: C itself. kBiasAct: z = C + bias to C, and its activation as BF16 for the
+// next layer (`group` rows of C make one row there: the positions of a convolution). kActGrad: the first `cols`
+// columns are the gradient after an activation whose argument was z; dz and its BF16 copy, contiguous.
+// In the tile's epilogue each of these costs a few hundred nanoseconds where a launch of its own took 3.4 us
+// on the device and 10 on the host; same arithmetic, element by element.
+enum { kStore = 0, kBiasAct = 1, kActGrad = 2 };
+struct Epilogue {
+    int kind;
+    float* C;
+    long long ldc;
+    const float* in;  // bias, or z
+    __nv_bfloat16* bf;
+    long long ldo;
+    int off, group, relu, cols;
+};
+
+__device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+__device__ __forceinline__ void store_bf16(__nv_bfloat16* out, const float (&v)[32]) {
+#pragma unroll
+    for (int q = 0; q < 32; q += 8) {
+        __align__(16) __nv_bfloat16 b[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) b[j] = __float2bfloat16(v[q + j]);
+        *reinterpret_cast<uint4*>(out + q) = *reinterpret_cast<uint4*>(b);
+    }
+}
+
+// 32 columns from nb of row m of an N-column product
+__device__ __forceinline__ void store_row(const Epilogue& e, int m, int nb, int N, float (&d)[32]) {
+    if (e.kind == kActGrad) {
+        const long long at = (long long)m * e.cols + nb;
+        const int n = min(N, e.cols) - nb;
+        if (n >= 32 && e.cols % 8 == 0 && aligned16(e.C) && aligned16(e.in) && aligned16(e.bf)) {
+            float z[32];
+#pragma unroll
+            for (int q = 0; q < 32; q += 4) *reinterpret_cast<float4*>(z + q) = *reinterpret_cast<const float4*>(e.in + at + q);
+#pragma unroll
+            for (int q = 0; q < 32; ++q)
+                if (e.relu && !(z[q] > 0.0f)) d[q] = 0.0f;
+#pragma unroll
+            for (int q = 0; q < 32; q += 4)
+                *reinterpret_cast<float4*>(e.C + at + q) = make_float4(d[q], d[q + 1], d[q + 2], d[q + 3]);
+            store_bf16(e.bf + at, d);
+            return;
+        }
+#pragma unroll
+        for (int q = 0; q < 32; ++q)
+            if (q < n) {
+                if (e.relu && !(e.in[at + q] > 0.0f)) d[q] = 0.0f;
+                e.C[at + q] = d[q];
+                e.bf[at + q] = __float2bfloat16(d[q]);
+            }
+        return;
+    }
+    if (e.kind == kBiasAct) {
+#pragma unroll
+        for (int q = 0; q < 32; ++q)
+            if (nb + q < N) d[q] = d[q] + (e.in ? e.in[nb + q] : 0.0f);
+    }
+    float* crow = e.C + (long long)m * e.ldc;
+    if (nb + 32 <= N && e.ldc % 4 == 0 && aligned16(e.C)) {
+#pragma unroll
+        for (int q = 0; q < 32; q += 4)
+            *reinterpret_cast<float4*>(crow + nb + q) = make_float4(d[q], d[q + 1], d[q + 2], d[q + 3]);
+    } else {
+#pragma unroll
+        for (int q = 0; q < 32; ++q)
+            if (nb + q < N) crow[nb + q] = d[q];
+    }
+    if (e.kind != kBiasAct || !e.bf) return;
+#pragma unroll
+    for (int q = 0; q < 32; ++q) d[q] = e.relu && d[q] < 0.0f ? 0.0f : d[q];
+    __nv_bfloat16* out = e.bf + (long long)(m / e.group) * e.ldo + e.off + (long long)(m % e.group) * N + nb;
+    if (nb + 32 <= N && aligned16(out)) {
+        store_bf16(out, d);
+        return;
+    }
+#pragma unroll
+    for (int q = 0; q < 32; ++q)
+        if (nb + q < N) out[q] = __float2bfloat16(d[q]);
+}
+
 template <int TN>
 __host__ __device__ constexpr int gemm_stage() {
     return kABytes + TN / 8 * kSboK;
 }
 
-// C[M][N] = sum_k A(m, k) B(n, k), a 128 x TN tile per CTA. What bounds it at the sizes of the network
-// (256 rows: a few CTAs of 4 to 21 chunks; the convolutions' weight gradients, one or four CTAs of 64
-// and 256) is the latency of a chunk's loads, so up to six chunks are in flight (asynchronous copies
-// into a ring, one mbarrier per stage that the MMAs reading it complete) and tiles are narrow where the
-// device is not full. Every layout is copied 16 bytes at a time. The K order of the sum is that of
-// the chunks whatever the tile or the ring, so results do not depend on either.
-template <int TN, int AM, int BM>
-__device__ __forceinline__ void gemm_tile(unsigned char* sm, int m0, int n0, int M, int N, int K,
-                                          const __nv_bfloat16* A, long long sam, long long sak,
-                                          const __nv_bfloat16* B, long long sbn, long long sbk, float* C,
-                                          long long ldc, int stages) {
-    __shared__ uint64_t bar[kMaxStages];  // the MMAs that read stage s have finished
-    __shared__ uint32_t tslot;
-    // 1 + the chunk whose barrier everyone leaves after, once a wait ran out (a thread late to read it
-    // after one barrier may already see the next chunk's)
-    __shared__ volatile int stop;
-    constexpr int STAGE = gemm_stage<TN>();
-    constexpr bool ar = AM == kColsK, br = BM == kColsK;
-    constexpr int la = ar ? kLboR : kLboK, sa = ar ? kSboR : kSboK, lb = br ? kLboR : kLboK, sb = br ? kSboR : kSboK;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (tid == 0) {
-        for (int i = 0; i < stages; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(saddr(&bar[i])) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+// The ring of a tile: warps 1 .. 7 copy `rounds` rounds of operands into STAGES stages (load(c, stage)), a lane of
+// warp 0 hands each round that has landed to the tensor core (mma(c, stage)) and a commit frees its stage.
+// A copying thread waits for nothing but a free stage: its copies arrive at the stage's barrier by themselves, and
+// the proxy fence between them and the tensor core's reads is the issuing lane's. With the whole CTA at a
+// barrier each round the copies of the next waited for the issue of this one: the first head layer (256 x 256,
+// K 1344) took 29.6 us, 23.2 us this way.
+// False if a wait ran out; every copy and MMA of the caller has ended on return.
+template <int STAGES>
+struct Ring {
+    uint64_t full[STAGES], empty[STAGES];
+};
+template <int STAGES>
+__device__ __forceinline__ void ring_init(Ring<STAGES>& ring) {  // one thread, before a barrier
+    for (int i = 0; i < STAGES; ++i) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(saddr(&ring.full[i])), "r"(kLoaders) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(saddr(&ring.empty[i])) : "memory");
     }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+template <int STAGES, bool kAsync, class Load, class Mma>
+__device__ __forceinline__ bool ring_run(Ring<STAGES>& ring, int rounds, Load&& load, Mma&& mma) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    bool ok = true;
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(&tslot)), "r"(TN)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    const int chunks = (K + kTK - 1) / kTK;
-    auto load = [&](int c) {  // one group of copies per chunk, empty past the last
-        if (c < chunks) {
-            unsigned char* st = sm + (c % stages) * STAGE;
-            stage_operand<kTM, AM>(st, A, sam, sak, m0, M, c * kTK, K, c < stages);
-            stage_operand<TN, BM>(st + kABytes, B, sbn, sbk, n0, N, c * kTK, K, c < stages);
+        if (lane == 0) {
+            int c = 0;
+            for (; c < rounds; ++c) {
+                ok = wait_bounded(&ring.full[c % STAGES], (c / STAGES) & 1);
+                if (!ok) break;
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the copies -> tensor-core reads
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                mma(c, c % STAGES);
+                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                                 saddr(&ring.empty[c % STAGES]))
+                             : "memory");
+            }
+            // commits complete in order: the last one's barrier covers all
+            if (c > 0 && !wait_bounded(&ring.empty[(c - 1) % STAGES], ((c - 1) / STAGES) & 1)) ok = false;
         }
-        cp_commit();
-    };
-    for (int c = 0; c < kMaxStages - 2; ++c)
-        if (c < stages - 2) load(c);
-        else cp_commit();
-    if (tid == 0) stop = 0;
+        __syncwarp();
+    } else {
+        for (int c = 0; c < rounds; ++c) {
+            // the warp leaves together, also if some lanes' waits just made it
+            if (c >= STAGES) ok = wait_bounded(&ring.empty[c % STAGES], (c / STAGES - 1) & 1);
+            if (!__all_sync(0xffffffffu, ok)) {
+                ok = false;
+                break;
+            }
+            load(c, c % STAGES);
+            const uint32_t full = saddr(&ring.full[c % STAGES]);
+            if (kAsync)  // arrives once this thread's copies so far have landed
+                asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(full) : "memory");
+            else
+                asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.shared::cta.b64 t, [%0];\n\t}" ::"r"(full) : "memory");
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    }
+    return ok;
+}
+
+// Tensor memory of a tile's accumulator, and the barriers before it is read and given back
+__device__ __forceinline__ void tmem_alloc(uint32_t* slot, int cols) {  // warp 0
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(slot)), "r"(cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_sync() {
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = tslot;
-    constexpr uint32_t idesc = bf16_idesc(kTM, TN, ar, br);
-
-    bool ok = true;
-    int issued = 0;  // chunks handed to the tensor core
-    for (int c = 0; c < chunks; ++c) {
-        // chunk c - 2's stage takes chunk c - 2 + stages once its MMAs have read it (two chunks back, so
-        // that the wait is over when it is reached)
-        if (c >= 2 && c - 2 + stages < chunks && !wait_bounded(&bar[(c - 2) % stages], ((c - 2) / stages) & 1)) stop = c + 1;
-        load(c - 2 + stages);
-        // this thread's copies of chunk c have landed: those of at most stages - 2 later ones are open
-        if (stages == kMaxStages) cp_wait<kMaxStages - 2>();
-        else cp_wait<1>();
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the copies -> tensor-core reads
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
-        if (stop == c + 1) {
-            ok = false;
-            break;
-        }
-        if (tid == 0) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            unsigned char* st = sm + (c % stages) * STAGE;
-#pragma unroll
-            for (int s = 0; s < kTK / 16; ++s) {
-                const uint64_t ad = operand_desc(st + s * 2 * la, la, sa), bd = operand_desc(st + kABytes + s * 2 * lb, lb, sb);
-                const uint32_t acc = (c > 0 || s > 0) ? 1u : 0u;
-                asm volatile(
-                    "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
-                    "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
-                    : "memory");
-            }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                             saddr(&bar[c % stages]))
-                         : "memory");
-        }
-        ++issued;
-    }
-    cp_wait<0>();
-    // every MMA has ended (commits complete in order: the last one's barrier covers all)
-    if (issued > 0 && !wait_bounded(&bar[(issued - 1) % stages], ((issued - 1) / stages) & 1)) ok = false;
+}
+__device__ __forceinline__ void mma_bf16(uint32_t tmem, uint64_t ad, uint64_t bd, uint32_t idesc, bool accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
+        "l"(ad), "l"(bd), "r"(idesc), "r"(accumulate ? 1u : 0u)
+        : "memory");
+}
+// The epilogue: warp w reads TMEM lanes 32 (w % 4) .. +31 (tile rows) of the columns of half w / 4.
+template <int TN>
+__device__ __forceinline__ void tile_out(bool ok, bool any, uint32_t tmem, int m0, int n0, int M, int N, const Epilogue& e) {
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     if (__syncthreads_or(!ok)) {
         ok = false;
-        if (tid == 0) atomicOr(&g_nn_err, 1u);
+        if (threadIdx.x == 0) atomicOr(&g_nn_err, 1u);
     }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    // warp w reads TMEM lanes 32 (w % 4) .. +31 (tile rows) of the columns of half w / 4
-    const int m = m0 + (warp & 3) * 32 + lane;
-    const bool vec_c = (ldc % 4) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
+    const int warp = threadIdx.x >> 5, m = m0 + (warp & 3) * 32 + (threadIdx.x & 31);
 #pragma unroll
     for (int j = 0; j < TN / 64; ++j) {
         const int col = (warp >> 2) * (TN / 2) + j * 32;
         float d[32];
 #pragma unroll
         for (int q = 0; q < 32; ++q) d[q] = 0.0f;
-        if (ok && issued > 0) tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)col, d);
-        const int nb = n0 + col;
-        if (!ok || m >= M) continue;
-        float* crow = C + (long long)m * ldc;
-        if (nb + 32 <= N && vec_c) {
-#pragma unroll
-            for (int q = 0; q < 32; q += 4)
-                *reinterpret_cast<float4*>(crow + nb + q) = make_float4(d[q], d[q + 1], d[q + 2], d[q + 3]);
-            continue;
-        }
-#pragma unroll
-        for (int q = 0; q < 32; ++q)
-            if (nb + q < N) crow[nb + q] = d[q];
+        if (ok && any) tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)col, d);
+        if (ok && m < M && n0 + col < N) store_row(e, m, n0 + col, N, d);
     }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    tmem_sync();
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TN) : "memory");
 }
 
-template <int TN, int AM, int BM>
-__global__ void __launch_bounds__(kThreads) nn_gemm_kernel(int M, int N, int K, const __nv_bfloat16* A, long long sam,
-                                                           long long sak, const __nv_bfloat16* B, long long sbn,
-                                                           long long sbk, float* C, long long ldc, int stages) {
-    extern __shared__ __align__(1024) unsigned char sm[];
-    gemm_tile<TN, AM, BM>(sm, blockIdx.x * kTM, blockIdx.y * TN, M, N, K, A, sam, sak, B, sbn, sbk, C, ldc, stages);
+// C[M][N] = sum_k A(m, k) B(n, k), a 128 x TN tile per CTA. What bounds it at the sizes of the network
+// (256 rows: a few CTAs of 4 to 21 chunks) is the latency of a chunk's loads, so up to six chunks are in
+// flight and tiles are narrow where the device is not full. Every layout is copied 16 bytes at a time.
+// The K order of the sum is that of the chunks whatever the tile or the ring, so results do not depend
+// on either.
+template <int TN, int STAGES, int AM, int BM>
+__device__ __forceinline__ void gemm_tile(unsigned char* sm, int m0, int n0, int M, int N, int K,
+                                          const __nv_bfloat16* A, long long sam, long long sak,
+                                          const __nv_bfloat16* B, long long sbn, long long sbk, const Epilogue& e) {
+    __shared__ Ring<STAGES> ring;
+    __shared__ uint32_t tslot;
+    constexpr int STAGE = gemm_stage<TN>();
+    constexpr bool ar = AM == kColsK, br = BM == kColsK;
+    constexpr int la = ar ? kLboR : kLboK, sa = ar ? kSboR : kSboK, lb = br ? kLboR : kLboK, sb = br ? kSboR : kSboK;
+    if (threadIdx.x == 0) ring_init(ring);
+    if (threadIdx.x < 32) tmem_alloc(&tslot, TN);
+    tmem_sync();
+    const uint32_t tmem = tslot;
+    constexpr uint32_t idesc = bf16_idesc(kTM, TN, ar, br);
+    const int chunks = (K + kTK - 1) / kTK;
+    const bool ok = ring_run<STAGES, AM != kAny && BM != kAny>(
+        ring, chunks,
+        [&](int c, int s) {
+            unsigned char* st = sm + s * STAGE;
+            const int t = threadIdx.x - 32;
+            stage_operand<kTM, AM>(t, st, A, sam, sak, m0, M, c * kTK, K, c < STAGES);
+            stage_operand<TN, BM>(t, st + kABytes, B, sbn, sbk, n0, N, c * kTK, K, c < STAGES);
+        },
+        [&](int c, int s) {
+            unsigned char* st = sm + s * STAGE;
+#pragma unroll
+            for (int k = 0; k < kTK / 16; ++k)
+                mma_bf16(tmem, operand_desc(st + k * 2 * la, la, sa), operand_desc(st + kABytes + k * 2 * lb, lb, sb), idesc,
+                         c > 0 || k > 0);
+        });
+    tile_out<TN>(ok, chunks > 0, tmem, m0, n0, M, N, e);
 }
 
-template <int TN, int AM, int BM>
+template <int TN, int STAGES, int AM, int BM>
+__global__ void __launch_bounds__(kThreads) nn_gemm_kernel(int M, int N, int K, const __nv_bfloat16* A, long long sam,
+                                                           long long sak, const __nv_bfloat16* B, long long sbn,
+                                                           long long sbk, const __grid_constant__ Epilogue e) {
+    extern __shared__ __align__(1024) unsigned char sm[];
+    gemm_tile<TN, STAGES, AM, BM>(sm, blockIdx.x * kTM, blockIdx.y * TN, M, N, K, A, sam, sak, B, sbn, sbk, e);
+}
+
+template <int TN, int STAGES, int AM, int BM>
 cudaError_t launch_gemm(int M, int N, int K, const __nv_bfloat16* A, long long sam, long long sak,
-                        const __nv_bfloat16* B, long long sbn, long long sbk, float* C, long long ldc, int stages,
-                        cudaStream_t s) {
-    auto kernel = nn_gemm_kernel<TN, AM, BM>;
+                        const __nv_bfloat16* B, long long sbn, long long sbk, const Epilogue& e, cudaStream_t s) {
+    auto kernel = nn_gemm_kernel<TN, STAGES, AM, BM>;
     static const cudaError_t sized =  // once, thread-safe
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxStages * gemm_stage<TN>());
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, STAGES * gemm_stage<TN>());
     if (sized != cudaSuccess) return sized;
-    kernel<<<dim3((M + kTM - 1) / kTM, (N + TN - 1) / TN), kThreads, stages * gemm_stage<TN>(), s>>>(
-        M, N, K, A, sam, sak, B, sbn, sbk, C, ldc, stages);
+    kernel<<<dim3((M + kTM - 1) / kTM, (N + TN - 1) / TN), kThreads, STAGES * gemm_stage<TN>(), s>>>(
+        M, N, K, A, sam, sak, B, sbn, sbk, e);
     return cudaGetLastError();
 }
 
-template <int TN>
+template <int TN, int STAGES>
 cudaError_t launch_gemm_modes(int M, int N, int K, const __nv_bfloat16* A, long long sam, long long sak,
-                              const __nv_bfloat16* B, long long sbn, long long sbk, float* C, long long ldc, int stages,
-                              cudaStream_t s) {
+                              const __nv_bfloat16* B, long long sbn, long long sbk, const Epilogue& e, cudaStream_t s) {
     auto mode = [](const void* p, long long s_row, long long s_k) {
         if (reinterpret_cast<uintptr_t>(p) & 15) return (int)kAny;
         if (s_k == 1 && s_row % 8 == 0) return (int)kRowsK;
@@ -293,12 +390,12 @@ cudaError_t launch_gemm_modes(int M, int N, int K, const __nv_bfloat16* A, long 
     };
     const int am = mode(A, sam, sak), bm = mode(B, sbn, sbk);
     if (am == kRowsK && bm == kRowsK)
-        return launch_gemm<TN, kRowsK, kRowsK>(M, N, K, A, sam, sak, B, sbn, sbk, C, ldc, stages, s);
+        return launch_gemm<TN, STAGES, kRowsK, kRowsK>(M, N, K, A, sam, sak, B, sbn, sbk, e, s);
     if (am == kRowsK && bm == kColsK)
-        return launch_gemm<TN, kRowsK, kColsK>(M, N, K, A, sam, sak, B, sbn, sbk, C, ldc, stages, s);
+        return launch_gemm<TN, STAGES, kRowsK, kColsK>(M, N, K, A, sam, sak, B, sbn, sbk, e, s);
     if (am == kColsK && bm == kColsK)
-        return launch_gemm<TN, kColsK, kColsK>(M, N, K, A, sam, sak, B, sbn, sbk, C, ldc, stages, s);
-    return launch_gemm<TN, kAny, kAny>(M, N, K, A, sam, sak, B, sbn, sbk, C, ldc, stages, s);
+        return launch_gemm<TN, STAGES, kColsK, kColsK>(M, N, K, A, sam, sak, B, sbn, sbk, e, s);
+    return launch_gemm<TN, STAGES, kAny, kAny>(M, N, K, A, sam, sak, B, sbn, sbk, e, s);
 }
 
 // z[m][n] = c[m][n] + bias[n % bias_n] (in place); a = relu ? max(z, 0) : z, as BF16 at
@@ -326,17 +423,26 @@ __global__ void nn_act_grad_kernel(const float* dy, long long ldy, int off, cons
 }
 
 // out[n] = sum_m d[m][n], added in row order. One CTA per 32 columns: warps 1 .. 7 copy blocks of 128 rows
-// into a ring of three, warp 0 adds them, one column per lane. Bound by the chain of additions (16384
-// rows of the first convolution), which the loads no longer interrupt: 871 us before, when one thread
-// per column loaded as it added.
-constexpr int kSumRows = 128, kSumStages = 3;
-constexpr int kSumBytes = kSumStages * kSumRows * 32 * 4;
+// into a ring, warp 0 adds them, one column per lane. The chain of additions is the floor (four cycles each:
+// 34 us for the 16384 rows of the first convolution); 121 us with copies of four bytes a thread, 64 us
+// with sixteen, 871 us when one thread per column loaded as it added.
+constexpr int kSumRows = 128;
+__host__ __device__ constexpr int sum_bytes(int stages) { return stages * kSumRows * 32 * 4; }
+template <int kSumStages>
 __device__ __forceinline__ void col_sum(float* ring, int n0, const float* d, int M, int N, float* out) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int n = n0 + lane;
     const int blocks = (M + kSumRows - 1) / kSumRows;
-    auto load = [&](int b) {  // warps 1 .. 7: every seventh row
-        if (b < blocks)
+    const bool wide = N % 4 == 0 && aligned16(d);
+    auto load = [&](int b) {  // warps 1 .. 7: four columns of a row a thread, or every seventh row a warp
+        if (b < blocks && wide) {
+            for (int q = threadIdx.x - 32; q < kSumRows * 8; q += kThreads - 32) {
+                const int r = q >> 3, c = (q & 7) * 4, m = b * kSumRows + r;
+                const bool live = m < M && n0 + c < N;
+                cp_async16(ring + ((b % kSumStages) * kSumRows + r) * 32 + c, live ? d + (long long)m * N + n0 + c : d,
+                           live ? 16 : 0);
+            }
+        } else if (b < blocks)
             for (int r = warp - 1; r < kSumRows; r += 7) {
                 const int m = b * kSumRows + r;
                 const bool live = m < M && n < N;
@@ -369,14 +475,80 @@ __device__ __forceinline__ void col_sum(float* ring, int n0, const float* d, int
 }
 
 __global__ void __launch_bounds__(kThreads) nn_col_sum_kernel(const float* d, int M, int N, float* out) {
-    __shared__ __align__(16) float ring[kSumBytes / 4];
-    col_sum(ring, blockIdx.x * 32, d, M, N, out);
+    __shared__ __align__(16) float ring[sum_bytes(3) / 4];  // what a launch gets without asking
+    col_sum<3>(ring, blockIdx.x * 32, d, M, N, out);
+}
+
+// The product of two operands contiguous along their rows (kColsK) where at most 64 rows of A are left:
+// gw = dz^T x of a convolution sums thousands of rows into one small tile, and what a round costs beside its
+// data (a chunk of the ring above: 0.9 us) bounds it. A chunk holds only the rows there are, so `group`
+// chunks share a round: the first convolution (32 x 16, 16384 rows) takes 43 rounds of six instead of 256,
+// 70 us instead of 242 by itself. The MMAs still read 128 rows and a multiple of 16 columns; what they
+// find beyond the operand's rows is other data of the ring and ends in accumulator rows and columns that
+// are not stored. Same K order.
+constexpr int kNarrowStages = 4;
+__device__ __forceinline__ void narrow_tile(unsigned char* sm, int smem, int m0, int n0, int M, int N, int K,
+                                            const __nv_bfloat16* A, const __nv_bfloat16* B, const Epilogue& e) {
+    __shared__ Ring<kNarrowStages> ring;
+    __shared__ uint32_t tslot;
+    const int ra = (min(kTM, M - m0) + 7) / 8, rb = (min(64, N - n0) + 7) / 8;  // row blocks
+    const int chunk = (ra + rb) * kSboR;
+    // the last chunk's MMAs read 16 row blocks of A and up to eight of B from its start on: inside the ring
+    const int slots = (smem - (max(16, ra + 8) * kSboR - chunk)) / chunk;
+    const int group = min(8, slots / kNarrowStages), stage = group * chunk;
+    if (threadIdx.x == 0) ring_init(ring);
+    if (threadIdx.x < 32) tmem_alloc(&tslot, 64);
+    tmem_sync();
+    const uint32_t tmem = tslot;
+    const int chunks = (K + kTK - 1) / kTK, rounds = (chunks + group - 1) / group;
+    // this thread's pieces (k, row block) of a chunk, the same in every chunk: up to three of each operand
+    struct Piece {
+        const __nv_bfloat16* src;
+        int dst, k, bytes;  // k: kTK and more where there is no piece
+    };
+    constexpr int kPieces = (8 * kTK + kLoaders - 1) / kLoaders;
+    Piece piece[2 * kPieces];
+#pragma unroll
+    for (int i = 0; i < 2 * kPieces; ++i) {
+        const bool of_a = i < kPieces;
+        const int blocks = of_a ? ra : rb, q = max(0, (int)threadIdx.x - 32) + i % kPieces * kLoaders;
+        const int block = q % blocks, k = q / blocks, rows = of_a ? M : N, row = (of_a ? m0 : n0) + block * 8;
+        piece[i] = {(of_a ? A : B) + (long long)min(k, K - 1) * rows + row,
+                    (of_a ? 0 : ra * kSboR) + block * kSboR + (k >> 3) * kLboR + (k & 7) * 16, k, 2 * min(8, rows - row)};
+    }
+    // columns beyond the rows there are (to a multiple of 16) need not be formed
+    const uint32_t idesc = bf16_idesc(kTM, (rb + 1) / 2 * 16, true, true);
+    const bool ok = ring_run<kNarrowStages, true>(
+        ring, rounds,
+        [&](int c, int s) {
+            for (int g = 0; g < group && c * group + g < chunks; ++g) {
+                unsigned char* st = sm + s * stage + g * chunk;
+                const int k0 = (c * group + g) * kTK;
+#pragma unroll
+                for (int i = 0; i < 2 * kPieces; ++i) {
+                    if (piece[i].k >= kTK) continue;
+                    const bool live = k0 + piece[i].k < K;
+                    cp_async16(st + piece[i].dst, live ? piece[i].src + (long long)k0 * (i < kPieces ? M : N) : piece[i].src,
+                               live ? piece[i].bytes : 0);
+                }
+            }
+        },
+        [&](int c, int s) {
+            for (int g = 0; g < group && c * group + g < chunks; ++g) {
+                unsigned char* st = sm + s * stage + g * chunk;
+#pragma unroll
+                for (int k = 0; k < kTK / 16; ++k)
+                    mma_bf16(tmem, operand_desc(st + k * 2 * kLboR, kLboR, kSboR),
+                             operand_desc(st + ra * kSboR + k * 2 * kLboR, kLboR, kSboR), idesc, c > 0 || g > 0 || k > 0);
+            }
+        });
+    tile_out<64>(ok, chunks > 0, tmem, m0, n0, M, N, e);
 }
 
 // The weight and bias gradients of several layers in one launch: gW = dz^T x (M x N, K rows of dz and x)
 // and gb = the column sums of dz. They depend on nothing but the layers' dz, so the long chains (the
 // first convolution sums 16384 rows in one tile) run beside all the others instead of after them.
-constexpr int kMaxGrads = 16;
+constexpr int kMaxGrads = 16, kGradSumStages = 9;
 struct GradItem {
     int M, N, K, first;  // first: the layer's first CTA; its tiles, then its column sums
     const __nv_bfloat16 *dz_bf, *x;
@@ -393,11 +565,15 @@ __global__ void __launch_bounds__(kThreads) nn_weight_grads_kernel(const __grid_
     while (i > 0 && (int)blockIdx.x < list.g[i].first) --i;
     const GradItem& g = list.g[i];
     const int cols = (g.N + 63) / 64, tiles = (g.M + kTM - 1) / kTM * cols, t = (int)blockIdx.x - g.first;
-    if (t < tiles)
-        gemm_tile<64, kColsK, kColsK>(sm, t / cols * kTM, t % cols * 64, g.M, g.N, g.K, g.dz_bf, 1, g.M, g.x, 1, g.N,
-                                      g.gw, g.N, kMaxStages);
+    const Epilogue e = {kStore, g.gw, g.N, nullptr, nullptr, 0, 0, 1, 0, 0};
+    const int m0 = t / cols * kTM, n0 = t % cols * 64;
+    // up to 64 rows the ring holds at least two chunks a round; more rows and the six single chunks serve
+    if (t < tiles && g.M - m0 <= 64)
+        narrow_tile(sm, kMaxStages * gemm_stage<64>(), m0, n0, g.M, g.N, g.K, g.dz_bf, g.x, e);
+    else if (t < tiles)
+        gemm_tile<64, kMaxStages, kColsK, kColsK>(sm, m0, n0, g.M, g.N, g.K, g.dz_bf, 1, g.M, g.x, 1, g.N, e);
     else
-        col_sum(reinterpret_cast<float*>(sm), (t - tiles) * 32, g.dz, g.K, g.M, g.gb);
+        col_sum<kGradSumStages>(reinterpret_cast<float*>(sm), (t - tiles) * 32, g.dz, g.K, g.M, g.gb);
 }
 
 // x: [B][Lin][C] (position-major); cols: [B * Lout][k * C], column (j, c) = x[b][l * stride - pad + j][c]
@@ -415,8 +591,9 @@ __global__ void nn_im2col_kernel(const __nv_bfloat16* x, int B, int Lin, int Cc,
 }
 
 // dx[b][p][c] = sum over (l, j) with l * stride - pad + j = p of dcols[(b, l)][(j, c)] (FP32)
+// With z: the gradient after the activation whose argument was z, and its BF16 copy.
 __global__ void nn_col2im_kernel(const float* dcols, int B, int Lin, int Cc, int k, int stride, int pad, int Lout,
-                                 float* dx) {
+                                 float* dx, const float* z, __nv_bfloat16* dz_bf) {
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     const long long total = (long long)B * Lin * Cc;
     if (i >= total) return;
@@ -431,18 +608,23 @@ __global__ void nn_col2im_kernel(const float* dcols, int B, int Lin, int Cc, int
         if (l >= Lout) continue;
         s += dcols[((long long)b * Lout + l) * ((long long)k * Cc) + (long long)j * Cc + c];
     }
+    if (z && !(z[i] > 0.0f)) s = 0.0f;
     dx[i] = s;
+    if (z) dz_bf[i] = __float2bfloat16(s);
 }
 
-// mean squared error over n values: dy = 2 (y - t) / n, loss += sum (y - t)^2 / n (per block, atomic)
-__global__ void nn_mse_kernel(const float* y, const float* t, long long n, float* dy, float* loss) {
+// mean squared error over n values: dy = 2 (y - t) / n, loss += sum (y - t)^2 / n (per block, atomic). With
+// dy_bf: its BF16 copy, and zeros in both from n to total.
+__global__ void nn_mse_kernel(const float* y, const float* t, long long n, long long total, float* dy, __nv_bfloat16* dy_bf,
+                              float* loss) {
     __shared__ float red[256];
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     float e = 0.0f;
-    if (i < n) {
-        const float d = y[i] - t[i];
-        dy[i] = 2.0f * d / (float)n;
-        e = d * d / (float)n;
+    if (i < total) {
+        const float d = i < n ? y[i] - t[i] : 0.0f, g = i < n ? 2.0f * d / (float)n : 0.0f;
+        dy[i] = g;
+        if (dy_bf) dy_bf[i] = __float2bfloat16(g);
+        if (i < n) e = d * d / (float)n;
     }
     red[threadIdx.x] = e;
     __syncthreads();
@@ -450,7 +632,7 @@ __global__ void nn_mse_kernel(const float* y, const float* t, long long n, float
         if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
         __syncthreads();
     }
-    if (threadIdx.x == 0 && loss) atomicAdd(loss, red[0]);
+    if (threadIdx.x == 0 && loss && (long long)blockIdx.x * blockDim.x < n) atomicAdd(loss, red[0]);
 }
 
 // Adam (FP32 master weights); the BF16 copy is refreshed for the next GEMMs. Several tensors in one
@@ -477,11 +659,13 @@ __global__ void nn_adam_kernel(const __grid_constant__ AdamList list, float lr, 
     if (p.w_bf16) static_cast<__nv_bfloat16*>(p.w_bf16)[i] = __float2bfloat16(wi);
 }
 
-__global__ void nn_to_bf16_kernel(const float* x, long long n, __nv_bfloat16* out, long long ldo, int cols, int off) {
+// The first `given` of n values are read, the rest is zero.
+__global__ void nn_to_bf16_kernel(const float* x, long long given, long long n, __nv_bfloat16* out, long long ldo,
+                                  int cols, int off) {
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const long long r = i / cols, c = i - r * cols;
-    out[r * ldo + off + c] = __float2bfloat16(x[i]);
+    out[r * ldo + off + c] = __float2bfloat16(i < given ? x[i] : 0.0f);
 }
 
 inline unsigned blocks(long long n, int t = 256) { return (unsigned)((n + t - 1) / t); }
@@ -498,23 +682,47 @@ using namespace emlab;
         if (e_ != cudaSuccess) return report_error(EMLAB_ERR_CUDA, cudaGetErrorString(e_)); \
     } while (0)
 
-extern "C" {
 
-int emlab_nn_gemm(int M, int N, int K, const void* A, long long sam, long long sak, const void* B, long long sbn,
-                  long long sbk, float* C, long long ldc, void* stream) {
-    if (M <= 0 || N <= 0 || K < 0 || !A || !B || !C) return report_error(EMLAB_ERR_INVALID, "bad GEMM arguments");
+namespace {
+int gemm(int M, int N, int K, const void* A, long long sam, long long sak, const void* B, long long sbn, long long sbk,
+         const Epilogue& e, void* stream) {
+    if (M <= 0 || N <= 0 || K < 0 || !A || !B) return report_error(EMLAB_ERR_INVALID, "bad GEMM arguments");
     const __nv_bfloat16* a = static_cast<const __nv_bfloat16*>(A);
     const __nv_bfloat16* b = static_cast<const __nv_bfloat16*>(B);
     // 128-column tiles once they fill the device (each operand row is then read half as often), with
     // three chunks in the ring so that two CTAs share an SM; below that narrow tiles and all six chunks
     const long long wide = (long long)((M + kTM - 1) / kTM) * ((N + 127) / 128);
-    const cudaError_t e =
-        wide >= 2 * 152 ? launch_gemm_modes<128>(M, N, K, a, sam, sak, b, sbn, sbk, C, ldc, 3, NN_STREAM(stream))
-                        : launch_gemm_modes<64>(M, N, K, a, sam, sak, b, sbn, sbk, C, ldc, kMaxStages, NN_STREAM(stream));
-    if (e != cudaSuccess) return report_error(EMLAB_ERR_CUDA, cudaGetErrorString(e));
+    const cudaError_t err =
+        wide >= 2 * 152 ? launch_gemm_modes<128, 3>(M, N, K, a, sam, sak, b, sbn, sbk, e, NN_STREAM(stream))
+                        : launch_gemm_modes<64, kMaxStages>(M, N, K, a, sam, sak, b, sbn, sbk, e, NN_STREAM(stream));
+    if (err != cudaSuccess) return report_error(EMLAB_ERR_CUDA, cudaGetErrorString(err));
     count_launches(1);
     NN_CHECK();
     return EMLAB_OK;
+}
+}  // namespace
+
+extern "C" {
+
+int emlab_nn_gemm(int M, int N, int K, const void* A, long long sam, long long sak, const void* B, long long sbn,
+                  long long sbk, float* C, long long ldc, void* stream) {
+    if (!C) return report_error(EMLAB_ERR_INVALID, "bad GEMM arguments");
+    return gemm(M, N, K, A, sam, sak, B, sbn, sbk, {kStore, C, ldc, nullptr, nullptr, 0, 0, 1, 0, 0}, stream);
+}
+
+int emlab_nn_gemm_bias_act(int M, int N, int K, const void* A, long long sam, long long sak, const void* B, long long sbn,
+                           long long sbk, float* Z, long long ldz, const float* bias, int relu, void* out_bf16,
+                           long long ldo, int off, int group, void* stream) {
+    if (!Z || group < 1) return report_error(EMLAB_ERR_INVALID, "bad GEMM arguments");
+    return gemm(M, N, K, A, sam, sak, B, sbn, sbk,
+                {kBiasAct, Z, ldz, bias, static_cast<__nv_bfloat16*>(out_bf16), ldo, off, group, relu, 0}, stream);
+}
+
+int emlab_nn_gemm_act_grad(int M, int N, int K, const void* A, long long sam, long long sak, const void* B, long long sbn,
+                           long long sbk, const float* z, int cols, int relu, float* dz, void* dz_bf16, void* stream) {
+    if (!z || !dz || !dz_bf16 || cols < 1 || cols > N) return report_error(EMLAB_ERR_INVALID, "bad GEMM arguments");
+    return gemm(M, N, K, A, sam, sak, B, sbn, sbk,
+                {kActGrad, dz, 0, z, static_cast<__nv_bfloat16*>(dz_bf16), 0, 0, 1, relu, cols}, stream);
 }
 
 int emlab_nn_status(void* stream) {
@@ -568,14 +776,35 @@ int emlab_nn_im2col(const void* x, int B, int Lin, int C, int k, int stride, int
 int emlab_nn_col2im(const float* dcols, int B, int Lin, int C, int k, int stride, int pad, int Lout, float* dx,
                     void* stream) {
     nn_col2im_kernel<<<blocks((long long)B * Lin * C), 256, 0, NN_STREAM(stream)>>>(dcols, B, Lin, C, k, stride, pad,
-                                                                                    Lout, dx);
+                                                                                    Lout, dx, nullptr, nullptr);
     count_launches(1);
     NN_CHECK();
     return EMLAB_OK;
 }
 
 int emlab_nn_mse(const float* y, const float* t, long long n, float* dy, float* loss, void* stream) {
-    nn_mse_kernel<<<blocks(n), 256, 0, NN_STREAM(stream)>>>(y, t, n, dy, loss);
+    nn_mse_kernel<<<blocks(n), 256, 0, NN_STREAM(stream)>>>(y, t, n, n, dy, nullptr, loss);
+    count_launches(1);
+    NN_CHECK();
+    return EMLAB_OK;
+}
+
+int emlab_nn_mse_grad(const float* y, const float* t, long long n, long long total, float* dy, void* dy_bf16, float* loss,
+                      void* stream) {
+    if (!y || !t || !dy || !dy_bf16 || n < 1 || total < n)
+        return report_error(EMLAB_ERR_INVALID, "bad loss arguments");
+    nn_mse_kernel<<<blocks(total), 256, 0, NN_STREAM(stream)>>>(y, t, n, total, dy, static_cast<__nv_bfloat16*>(dy_bf16),
+                                                                loss);
+    count_launches(1);
+    NN_CHECK();
+    return EMLAB_OK;
+}
+
+int emlab_nn_col2im_act_grad(const float* dcols, int B, int Lin, int C, int k, int stride, int pad, int Lout,
+                             const float* z, float* dz, void* dz_bf16, void* stream) {
+    if (!z || !dz || !dz_bf16) return report_error(EMLAB_ERR_INVALID, "bad gradient arguments");
+    nn_col2im_kernel<<<blocks((long long)B * Lin * C), 256, 0, NN_STREAM(stream)>>>(
+        dcols, B, Lin, C, k, stride, pad, Lout, dz, z, static_cast<__nv_bfloat16*>(dz_bf16));
     count_launches(1);
     NN_CHECK();
     return EMLAB_OK;
@@ -630,7 +859,7 @@ int emlab_nn_weight_grads(const emlab_nn_grad* grads, int count, void* stream) {
     }
     if (!total) return EMLAB_OK;
     constexpr int smem = kMaxStages * gemm_stage<64>();
-    static_assert(smem >= kSumBytes, "the column sums' ring fits the tile's stages");
+    static_assert(smem >= sum_bytes(kGradSumStages), "the column sums' ring fits the tile's stages");
     static const cudaError_t sized =
         cudaFuncSetAttribute(nn_weight_grads_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (sized != cudaSuccess) return report_error(EMLAB_ERR_CUDA, cudaGetErrorString(sized));
@@ -641,7 +870,13 @@ int emlab_nn_weight_grads(const emlab_nn_grad* grads, int count, void* stream) {
 }
 
 int emlab_nn_to_bf16(const float* x, long long n, void* out, long long ldo, int cols, int off, void* stream) {
-    nn_to_bf16_kernel<<<blocks(n), 256, 0, NN_STREAM(stream)>>>(x, n, static_cast<__nv_bfloat16*>(out), ldo, cols, off);
+    return emlab_nn_pad_to_bf16(x, n, n, out, ldo, cols, off, stream);
+}
+
+int emlab_nn_pad_to_bf16(const float* x, long long given, long long n, void* out, long long ldo, int cols, int off,
+                         void* stream) {
+    nn_to_bf16_kernel<<<blocks(n), 256, 0, NN_STREAM(stream)>>>(x, given, n, static_cast<__nv_bfloat16*>(out), ldo, cols,
+                                                                off);
     count_launches(1);
     NN_CHECK();
     return EMLAB_OK;

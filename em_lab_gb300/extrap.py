@@ -164,14 +164,11 @@ class Net:
         self.ah = {n: z(B, o, dt=bf16) for n, i, o, r in HEAD if r}
         self.y = self.zh["out"]
         self.t = z(B, OUT)
-        self.dy = z(B, OUT)
         self.dz = {n: z(B, o) for n, i, o, _ in HEAD}
         self.dzb = {n: z(B, o, dt=bf16) for n, i, o, _ in HEAD}
-        self.dx = {n: z(B, i) for n, i, o, _ in HEAD}
         self.dz2 = z(B * 16, 64)
         self.dz2b = z(B * 16, 64, dt=bf16)
         self.dcols2 = z(B * 16, 256)
-        self.da1 = z(B * 64, 32)
         self.dz1 = z(B * 64, 32)
         self.dz1b = z(B * 64, 32, dt=bf16)
         self.loss = z(1)
@@ -198,74 +195,68 @@ class Net:
         _check(self.lib.emlab_nn_gemm(M, N, K, self._p(A), sam, sak, self._p(B), sbn, sbk, self._fp(Cc), ldc,
                                       self.stream))
 
-    def _bias_act(self, z, bias, M, N, relu, out, ldo, off, bias_n):
-        _check(self.lib.emlab_nn_bias_act(self._fp(z), self._fp(bias), M, N, bias_n, 1 if relu else 0,
-                                          self._p(out) if out is not None else None, ldo, off, self.stream))
-
     def load(self, x, zt, t=None):
         """A batch: x (n, T_IN, 2), head inputs zt (n, AUX), targets t (n, OUT) (float32 host arrays)."""
         torch = self.torch
         n = x.shape[0]
         assert n <= self.B
         self.n = n
-        xs = torch.zeros((self.B, T_IN, 2), dtype=torch.float32, device=self.dev)
-        xs[:n] = torch.from_numpy(np.ascontiguousarray(x, np.float32)).to(self.dev)
-        zs = torch.zeros((self.B, AUX), dtype=torch.float32, device=self.dev)
-        zs[:n] = torch.from_numpy(np.ascontiguousarray(zt, np.float32)).to(self.dev)
-        self._conv(xs.view(self.B * T_IN, 2), self.x0.view(self.B * T_IN, 2))
-        self._conv(zs, self.X0, ldo=ENC + AUX, cols=AUX, off=ENC)
-        self.t.zero_()
-        if t is not None:
-            self.t[:n] = torch.from_numpy(np.ascontiguousarray(t, np.float32)).to(self.dev)
+        # rows beyond n are zero inputs (their targets and gradients are left out)
+        for src, row, out, ldo, cols, off in ((x, T_IN * 2, self.x0, 2, 2, 0), (zt, AUX, self.X0, ENC + AUX, AUX, ENC)):
+            d = torch.from_numpy(np.ascontiguousarray(src, np.float32)).to(self.dev)
+            _check(self.lib.emlab_nn_pad_to_bf16(d.data_ptr(), n * row, self.B * row, out.data_ptr(), ldo, cols, off,
+                                                 self.stream))
+        if t is None:
+            self.t.zero_()
+        else:
+            self.t[:n].copy_(torch.from_numpy(np.ascontiguousarray(t, np.float32)))
 
     # -- forward / backward
+    def _gemm_bias_act(self, M, N, K, A, name, z, relu, out, ldo, group, s):
+        """z = A W^T + b of a layer, and its activation as BF16 at out (`group` rows of z to a row)."""
+        _check(self.lib.emlab_nn_gemm_bias_act(M, N, K, A.data_ptr(), K, 1, self.Wb[name].data_ptr(), K, 1, z.data_ptr(),
+                                               N, self.b[name].data_ptr(), int(relu),
+                                               None if out is None else out.data_ptr(), ldo, 0, group, s))
+
     def forward(self):
         B, lib, s = self.B, self.lib, self.stream
         c1, c2 = CONV
         _check(lib.emlab_nn_im2col(self._p(self.x0), B, c1[6], c1[1], c1[3], c1[4], c1[5], c1[7], self._p(self.cols1), s))
-        self._gemm(B * 64, 32, 16, self.cols1, 16, 1, self.Wb["conv1"], 16, 1, self.z1, 32)
-        self._bias_act(self.z1, self.b["conv1"], B * 64, 32, True, self.a1, 32, 0, 32)
+        self._gemm_bias_act(B * 64, 32, 16, self.cols1, "conv1", self.z1, True, self.a1, 32, 1, s)
         _check(lib.emlab_nn_im2col(self._p(self.a1), B, c2[6], c2[1], c2[3], c2[4], c2[5], c2[7], self._p(self.cols2), s))
-        self._gemm(B * 16, 64, 256, self.cols2, 256, 1, self.Wb["conv2"], 256, 1, self.z2, 64)
         # rows (b, l) of z2 are the encoder features of sample b at columns l * 64 + c
-        self._bias_act(self.z2, self.b["conv2"], B, ENC, True, self.X0, ENC + AUX, 0, 64)
+        self._gemm_bias_act(B * 16, 64, 256, self.cols2, "conv2", self.z2, True, self.X0, ENC + AUX, 16, s)
         x = self.X0
         for name, i, o, relu in HEAD:
-            self._gemm(B, o, i, x, i, 1, self.Wb[name], i, 1, self.zh[name], o)
             out = self.ah.get(name)
-            self._bias_act(self.zh[name], self.b[name], B, o, relu, out, o, 0, o)
+            self._gemm_bias_act(B, o, i, x, name, self.zh[name], relu, out, o, 1, s)
             x = out
         return self.y
 
     def backward(self):
-        """MSE gradients of every weight and bias (loss over the loaded rows; padding rows carry zero
-        targets and zero outputs' gradient is masked by the row count)."""
+        """MSE gradients of every weight and bias (loss over the loaded rows; the gradient of padding
+        rows is zero)."""
         B, lib, s = self.B, self.lib, self.stream
         n = self.n
         self.loss.zero_()
-        # only the loaded rows contribute: gradient rows beyond n are zero
-        self.dy.zero_()
-        _check(lib.emlab_nn_mse(self._fp(self.y), self._fp(self.t), n * OUT, self._fp(self.dy),
-                                self._fp(self.loss), s))
-        up = self.dy
+        last = HEAD[-1][0]
+        _check(lib.emlab_nn_mse_grad(self.y.data_ptr(), self.t.data_ptr(), n * OUT, B * OUT, self.dz[last].data_ptr(),
+                                     self.dzb[last].data_ptr(), self.loss.data_ptr(), s))
         ins = {"fc1": self.X0}
         for k in range(1, len(HEAD)):
             ins[HEAD[k][0]] = self.ah[HEAD[k - 1][0]]
-        for name, i, o, relu in reversed(HEAD):
-            dz, dzb = self.dz[name], self.dzb[name]
-            _check(lib.emlab_nn_act_grad(self._fp(up), o, 0, self._fp(self.zh[name]), B, o, 1 if relu else 0,
-                                         self._fp(dz), self._p(dzb), s))
-            self._gemm(B, i, o, dzb, o, 1, self.Wb[name], 1, i, self.dx[name], i)
-            up = self.dx[name]
+        # the gradient of a layer's input through the activation before it; below fc1 that is conv2's, whose
+        # rows (b, l) x 64 channels are the encoder part of d(X0)
+        for k in range(len(HEAD) - 1, -1, -1):
+            name, i, o, _ = HEAD[k]
+            z, dz, dzb, cols = (self.z2, self.dz2, self.dz2b, ENC) if k == 0 else \
+                (self.zh[HEAD[k - 1][0]], self.dz[HEAD[k - 1][0]], self.dzb[HEAD[k - 1][0]], i)
+            _check(lib.emlab_nn_gemm_act_grad(B, i, o, self.dzb[name].data_ptr(), o, 1, self.Wb[name].data_ptr(), 1, i,
+                                              z.data_ptr(), cols, 1, dz.data_ptr(), dzb.data_ptr(), s))
         c2 = CONV[1]
-        # conv2: dz2 over rows (b, l) x 64 channels = the encoder part of d(X0)
-        _check(lib.emlab_nn_act_grad(self._fp(up), ENC + AUX, 0, self._fp(self.z2), B, ENC, 1, self._fp(self.dz2),
-                                     self._p(self.dz2b), s))
         self._gemm(B * 16, 256, 64, self.dz2b, 64, 1, self.Wb["conv2"], 1, 256, self.dcols2, 256)
-        _check(lib.emlab_nn_col2im(self._fp(self.dcols2), B, c2[6], c2[1], c2[3], c2[4], c2[5], c2[7],
-                                   self._fp(self.da1), s))
-        _check(lib.emlab_nn_act_grad(self._fp(self.da1), 32, 0, self._fp(self.z1), B * 64, 32, 1, self._fp(self.dz1),
-                                     self._p(self.dz1b), s))
+        _check(lib.emlab_nn_col2im_act_grad(self.dcols2.data_ptr(), B, c2[6], c2[1], c2[3], c2[4], c2[5], c2[7],
+                                            self.z1.data_ptr(), self.dz1.data_ptr(), self.dz1b.data_ptr(), s))
         # every layer's weight and bias gradients, the longest sums first
         rows = [("conv1", B * 64, self.dz1b, self.cols1, self.dz1), ("conv2", B * 16, self.dz2b, self.cols2, self.dz2)]
         rows += [(name, B, self.dzb[name], ins[name], self.dz[name]) for name, _, _, _ in HEAD]
@@ -326,6 +317,11 @@ def _nn_lib():
     fp = C.POINTER(C.c_float)
     sig = {
         "emlab_nn_gemm": [I, I, I, P, L, L, P, L, L, fp, L, P],
+        "emlab_nn_gemm_bias_act": [I, I, I, P, L, L, P, L, L, P, L, P, I, P, L, I, I, P],
+        "emlab_nn_gemm_act_grad": [I, I, I, P, L, L, P, L, L, P, I, I, P, P, P],
+        "emlab_nn_col2im_act_grad": [P, I, I, I, I, I, I, I, P, P, P, P],
+        "emlab_nn_mse_grad": [P, P, L, L, P, P, P, P],
+        "emlab_nn_pad_to_bf16": [P, L, L, P, L, I, I, P],
         "emlab_nn_status": [P],
         "emlab_nn_bias_act": [fp, fp, I, I, I, I, P, L, I, P],
         "emlab_nn_act_grad": [fp, L, I, fp, I, I, I, fp, P, P],
