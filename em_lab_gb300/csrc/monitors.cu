@@ -114,6 +114,50 @@ __device__ __forceinline__ void ntff_point(const int* box, int index, int node[3
     n[a] = side == 1 ? 1.0f : -1.0f;
 }
 
+// E and H of consecutive surface nodes, one a lane of a full warp (live: the lane has one; xface: it lies on a
+// face of constant x; first: the first node of a row of its face, whose neighbour in y is not the lane
+// before). On the x faces consecutive nodes lie rows apart, so every load is a sector a lane and the
+// kernels wait for their number: nine of them here instead of eighteen (the values one row back come from
+// the lane before, x and x - 1 are one load where they share eight bytes). The same sums as above. A step of
+// 128 x 128 x 128 cells with the per-step accumulation 37.5 us before, 36.8 here; of 80 x 80 x 647 cells with
+// the surface DFT 91.6 and 90.0; on large grids DRAM bounds the x faces either way.
+__device__ __forceinline__ float2 at_x_pair(const float* f, const MonitorArgs& m, int x, int y, int z) {  // (x - 1, x)
+    const long long i = cidx(m, x, y, z), j = cidx(m, x - 1, y, z);
+    if ((i & 1) && j == i - 1) return *reinterpret_cast<const float2*>(f + j);
+    return make_float2(f[j], f[i]);
+}
+__device__ __forceinline__ void surface_fields(const MonitorArgs& m, bool live, bool xface, bool first, const int p[3],
+                                               float E[3], float H[3]) {
+    const unsigned all = 0xffffffffu;
+    const int x = p[0], y = p[1], z = p[2];
+    if (__any_sync(all, live && xface)) {
+        float2 ex{}, by{}, bym{}, bz{}, bzy{};
+        float ey = 0.0f, bx = 0.0f, bxm = 0.0f, ez = 0.0f, ezm = 0.0f;
+        if (live && xface) {
+            ex = at_x_pair(m.ex, m, x, y, z), by = at_x_pair(m.by, m, x, y, z), bym = at_x_pair(m.by, m, x, y, z - 1);
+            bz = at_x_pair(m.bz, m, x, y, z);
+            ey = m.ey[cidx(m, x, y, z)], ez = m.ez[cidx(m, x, y, z)], ezm = m.ez[cidx(m, x, y, z - 1)];
+            bx = m.bx[cidx(m, x, y, z)], bxm = m.bx[cidx(m, x, y, z - 1)];
+        }
+        float eyy = __shfl_up_sync(all, ey, 1), bxy = __shfl_up_sync(all, bx, 1), bxmy = __shfl_up_sync(all, bxm, 1);
+        bzy.x = __shfl_up_sync(all, bz.x, 1), bzy.y = __shfl_up_sync(all, bz.y, 1);
+        if (live && xface) {
+            if (first || threadIdx.x % 32 == 0) {
+                eyy = m.ey[cidx(m, x, y - 1, z)], bxy = m.bx[cidx(m, x, y - 1, z)], bxmy = m.bx[cidx(m, x, y - 1, z - 1)];
+                bzy = at_x_pair(m.bz, m, x, y - 1, z);
+            }
+            E[0] = 0.5f * (ex.y + ex.x), E[1] = 0.5f * (ey + eyy), E[2] = 0.5f * (ez + ezm);
+            H[0] = 0.25f * (bx + bxy + bxm + bxmy);
+            H[1] = 0.25f * (by.y + by.x + bym.y + bym.x);
+            H[2] = 0.25f * (bz.y + bz.x + bzy.y + bzy.x);
+        }
+    }
+    if (live && !xface) {
+        e_at_node(m, x, y, z, E[0], E[1], E[2]);
+        b_at_node(m, x, y, z, H[0], H[1], H[2]);
+    }
+}
+
 // ntff_accumulate.comp:30-52: 32 floats per point (stage1 eRe, eIm, hRe, hIm, stage2 ...). The
 // block's 128 x 128 B of state move between HBM and shared memory as one contiguous chunk
 // (consecutive threads, consecutive float4s), rows padded to 9 float4s against bank conflicts;
@@ -139,16 +183,13 @@ __global__ void __launch_bounds__(kNtffThreads) ntff_kernel(MonitorArgs m, const
     const int i = first + threadIdx.x;
     const bool live = i < points;
     float E[3], Hh[3];
-    int node[3];
-    float n[3], w;
+    int node[3] = {0, 0, 0};
+    float n[3] = {0.0f, 0.0f, 0.0f}, w;
     if (live) ntff_point(sbox, i, node, n, w);
     const float4 r = __ldcg(rot + k);
     const float b = __ldcg(blend + k);
     chain_wait();
-    if (live) {
-        e_at_node(m, node[0], node[1], node[2], E[0], E[1], E[2]);
-        b_at_node(m, node[0], node[1], node[2], Hh[0], Hh[1], Hh[2]);
-    }
+    surface_fields(m, live, n[0] != 0.0f, node[1] == sbox[1], node, E, Hh);
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
         const int j = threadIdx.x + q * kNtffThreads;
@@ -316,15 +357,15 @@ __global__ void __launch_bounds__(256) dft_sample_kernel(MonitorArgs m, const in
     if (threadIdx.x < kDftBoxInts) sbox[threadIdx.x] = boxes[(size_t)blockIdx.y * kDftBoxInts + threadIdx.x];
     __syncthreads();
     const int local = blockIdx.x * blockDim.x + threadIdx.x;
-    if (local >= sbox[14]) return;
+    const bool live = local < sbox[14];
     const int i = sbox[13] + local;
-    int node[3];
-    float n[3], w;
-    ntff_point(sbox, local, node, n, w);
+    int node[3] = {0, 0, 0};
+    float n[3] = {0.0f, 0.0f, 0.0f}, w;
+    if (live) ntff_point(sbox, local, node, n, w);
     chain_wait();
     float E[3], Hh[3];
-    e_at_node(m, node[0], node[1], node[2], E[0], E[1], E[2]);
-    b_at_node(m, node[0], node[1], node[2], Hh[0], Hh[1], Hh[2]);
+    surface_fields(m, live, n[0] != 0.0f, node[1] == sbox[1], node, E, Hh);
+    if (!live) return;
     float* o = blk + (size_t)t * 6 * points + i;
     o[0] = E[0], o[(size_t)points] = E[1], o[2 * (size_t)points] = E[2];
     o[3 * (size_t)points] = Hh[0], o[4 * (size_t)points] = Hh[1], o[5 * (size_t)points] = Hh[2];
