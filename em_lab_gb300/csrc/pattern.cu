@@ -6,16 +6,18 @@
 //
 // What bounds it is the arithmetic per (direction, node) pair. A face is a lattice (iu, iv) at a fixed
 // height, so the phase is a product of three factors and the sum is
-//   e^{jk r_a p_a} sum_iu U(iu) [ sum_iv V(iv) F_q(iu, iv) ],  q = the two tangential components of J, of M:
-// 16 multiply-adds per pair (four complex products with V) where the direct sum has 24 and a sine and a
-// cosine; V serves all columns iu of a strip and U a whole column. One thread holds two directions and
-// a strip of four columns (64 sums); the strip's fields pass through shared memory as pairs of
-// columns, so the products are packed .f32x2 multiply-adds. (One direction and eight columns need
-// the same registers but two shared loads for each here, and their 512 bytes a warp then bound the SM
-// at half the multiply-add rate.) V advances from row to row by one complex product and is evaluated
-// anew every 32 rows. Strips are grouped into slices;
-// every slice leaves its share of N and L for the reduction. The direct sums took 2650 us for the 10550
-// directions of a console report on 57624 nodes, 871 us for 650 directions at 32 frequencies on 23064.
+//   e^{jk r_a p_a} sum_iu U(iu) [ sum_iv V(iv) F_q(iu, iv) ],  q = the two tangential components of J, of M.
+// Positions are taken from the box centre, so V at the mirror row is the conjugate of V, and a row and its
+// mirror need two real factors for their sum S and difference D instead of two complex ones:
+//   V F(p) + conj(V) F(-p) = cos S + j sin D.
+// That is 8 multiply-adds per pair where the direct sum has 24 and a sine and a cosine; V serves all columns iu
+// of a strip and U a whole column. One thread holds two directions and a strip of four columns (64 sums);
+// S and D pass through shared memory as pairs of columns, so the products are packed .f32x2 multiply-adds.
+// (One direction and eight columns need the same registers but twice the shared loads a multiply-add, and
+// those then bound the SM.) V advances from row to row by one complex product and is evaluated anew every
+// 32 rows. Strips are grouped into slices; every slice leaves its share of N and L for the reduction.
+// The 10550 directions of a console report on 57624 nodes: 2650 us as direct sums, 424 us with both rows of a
+// pair multiplied, 236 us folded; 650 directions at 32 frequencies on 224664 nodes: 3671 and 1990 us.
 #include <algorithm>
 
 #include "emlab_internal.h"
@@ -27,7 +29,8 @@ namespace {
 constexpr int kThreads = 128;
 constexpr int kDirs = 2;    // directions of a thread
 constexpr int kStrip = 4;   // columns iu of a strip
-constexpr int kRows = 32;   // rows iv staged at a time: kRows * kStrip = one node per thread
+constexpr int kRows = 32;   // rows (with their mirrors) staged at a time: kRows * kStrip = one pair of nodes per thread
+constexpr int kRowFloats = 4 * 4 * kStrip + 4;  // [q][S re, S im, D re, D im][column], and padding against bank conflicts
 
 using pair_t = unsigned long long;
 __device__ __forceinline__ pair_t pk(float a, float b) {
@@ -132,7 +135,7 @@ __host__ __device__ inline int face_strips(const int* box, int f) {
 // directions ([direction][component]{re, im}).
 template <int A>
 __device__ __forceinline__ void strip_sums(const int* box, const float4* cur, int face, int iu0,
-                                           const Turns (&turns)[kDirs][3], float (*sF)[kRows][4][2][kStrip], int& buf,
+                                           const Turns (&turns)[kDirs][3], float (*sF)[kRows * kRowFloats], int& buf,
                                            float (&N)[kDirs][3][2], float (&L)[kDirs][3][2]) {
     constexpr int U = A == 0 ? 1 : 0, V = A == 2 ? 1 : 2;
     const int nu1 = box[3 + U] - box[U] + 1, nv1 = box[3 + V] - box[V] + 1, base = box[6 + face];
@@ -151,21 +154,30 @@ __device__ __forceinline__ void strip_sums(const int* box, const float4* cur, in
 #pragma unroll
             for (int c = 0; c < kStrip / 2; ++c) acc[t][q][0][c] = 0, acc[t][q][1][c] = 0;
     }
-    for (int iv0 = 0; iv0 < nv1; iv0 += kRows) {
-        const int iv = iv0 + rv;
-        float4 j4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), m4 = j4;
-        if (iu < nu1 && iv < nv1) {
+    const int folded = (nv1 + 1) / 2;
+    for (int iv0 = 0; iv0 < folded; iv0 += kRows) {
+        const int iv = iv0 + rv, mirror = nv1 - 1 - iv;
+        float4 j4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), m4 = j4, jm = j4, mm = j4;
+        if (iu < nu1 && iv < folded) {
             const float4* p = cur + 2 * (size_t)(base + iv * nu1 + iu);
             j4 = __ldg(p), m4 = __ldg(p + 1);
+            if (mirror != iv) {  // the middle row is its own mirror: S its fields, D 0 (and the sine there 0)
+                p = cur + 2 * (size_t)(base + mirror * nu1 + iu);
+                jm = __ldg(p), mm = __ldg(p + 1);
+            }
         }
-        float (*row)[2][kStrip] = sF[buf][rv];
-        row[0][0][cu] = j4.x, row[0][1][cu] = j4.y, row[1][0][cu] = j4.z, row[1][1][cu] = j4.w;
-        row[2][0][cu] = m4.x, row[2][1][cu] = m4.y, row[3][0][cu] = m4.z, row[3][1][cu] = m4.w;
+        float* row = sF[buf] + rv * kRowFloats + cu;
+        auto put = [&](int q, float re, float im, float mre, float mim) {
+            row[(4 * q + 0) * kStrip] = re + mre, row[(4 * q + 1) * kStrip] = im + mim;
+            row[(4 * q + 2) * kStrip] = re - mre, row[(4 * q + 3) * kStrip] = im - mim;
+        };
+        put(0, j4.x, j4.y, jm.x, jm.y), put(1, j4.z, j4.w, jm.z, jm.w);
+        put(2, m4.x, m4.y, mm.x, mm.y), put(3, m4.z, m4.w, mm.z, mm.w);
         float vs[kDirs], vc[kDirs];
 #pragma unroll
         for (int t = 0; t < kDirs; ++t) twiddle(turns[t][V], pv0 + (float)iv0, vs[t], vc[t]);
         __syncthreads();  // the other buffer's readers are past it since the last barrier
-        const int rows = min(kRows, nv1 - iv0);
+        const int rows = min(kRows, folded - iv0);
         for (int j = 0; j < rows; ++j) {
             pair_t c2[kDirs], s2[kDirs], m2[kDirs];
 #pragma unroll
@@ -176,14 +188,14 @@ __device__ __forceinline__ void strip_sums(const int* box, const float4* cur, in
             }
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(sF[buf][j][q][0]);
-                const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(sF[buf][j][q][1]);
+                const ulonglong2* f = reinterpret_cast<const ulonglong2*>(sF[buf] + j * kRowFloats + 4 * q * kStrip);
+                const ulonglong2 sr = f[0], si = f[1], dr = f[2], di = f[3];
 #pragma unroll
                 for (int t = 0; t < kDirs; ++t) {
-                    fma2(acc[t][q][0][0], c2[t], a.x), fma2(acc[t][q][0][0], m2[t], b.x);
-                    fma2(acc[t][q][1][0], s2[t], a.x), fma2(acc[t][q][1][0], c2[t], b.x);
-                    fma2(acc[t][q][0][1], c2[t], a.y), fma2(acc[t][q][0][1], m2[t], b.y);
-                    fma2(acc[t][q][1][1], s2[t], a.y), fma2(acc[t][q][1][1], c2[t], b.y);
+                    fma2(acc[t][q][0][0], c2[t], sr.x), fma2(acc[t][q][0][0], m2[t], di.x);
+                    fma2(acc[t][q][1][0], c2[t], si.x), fma2(acc[t][q][1][0], s2[t], dr.x);
+                    fma2(acc[t][q][0][1], c2[t], sr.y), fma2(acc[t][q][0][1], m2[t], di.y);
+                    fma2(acc[t][q][1][1], c2[t], si.y), fma2(acc[t][q][1][1], s2[t], dr.y);
                 }
             }
         }
@@ -223,7 +235,7 @@ constexpr int kBlockDirs = kThreads * kDirs;
 __global__ void __launch_bounds__(kThreads, 3) ntff_pattern_kernel(const int* box, const float4* cur, int points,
                                                                    const double* k, double k0, const float4* dirs,
                                                                    int count, int slices, float* partials) {
-    __shared__ __align__(16) float sF[2][kRows][4][2][kStrip];
+    __shared__ __align__(16) float sF[2][kRows * kRowFloats];
     __shared__ int sbox[13];
     const int tid = threadIdx.x, slice = blockIdx.y, fq = blockIdx.z;
     if (tid < 13) sbox[tid] = box[tid];
