@@ -190,8 +190,8 @@ def _watch(sc, dt: float) -> RingDown:
     return RingDown(min_steps=int(math.ceil(4.0 * period)), max_steps=int(math.ceil(MAX_PERIODS * period)))
 
 
-TILINGS = (64, 32, 128, 8)  # 64 x 8, 64 x 4, 64 x 16 pair tiles; 32 x 8 single-cell tiles
-PAIR_TILINGS = (64, 32, 128)  # a stack of scenes with their own cross-sections: pair tiles only
+TILINGS = (0, 32, 128, 8)  # 64 x 8 or 32 x 16 (automatic), 64 x 4, 64 x 16 pair tiles; 32 x 8 single-cell tiles
+PAIR_TILINGS = (0, 32, 128)  # a stack of scenes with their own cross-sections: pair tiles only
 
 
 def autotune_tiling(grid, modes=TILINGS, steps=4):

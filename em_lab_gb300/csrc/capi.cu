@@ -65,8 +65,8 @@ YeeArgs yee_args(emlab_grid* g) {
     a.minus_zero = -0.0f;
     // tile height and z chunks: enough CTAs for ~4 per SM, but at least 8 planes each (the first
     // plane of a chunk is recomputed)
-    const int mode = g->tile_rows == 0 ? 64 : g->tile_rows;  // automatic: 64 x 8 pair tiles
-    const int ty = mode == 16 || mode == 128 ? 16 : (mode == 32 ? 4 : 8);
+    const int mode = g->tile_rows == 0 ? g->auto_tiling : g->tile_rows;
+    const int ty = mode == 16 || mode == 128 || mode == kNarrowPairTiles ? 16 : (mode == 32 ? 4 : 8);
     const int tx = (mode == 32 || mode == 64 || mode == 128) && g->kernel == EMLAB_KERNEL_FUSED ? 64 : 32;
     a.tile_rows = g->kernel == EMLAB_KERNEL_FUSED ? mode : ty;
     const long long xy = (long long)((a.nx + tx - 1) / tx) * ((a.ny + ty - 1) / ty);
@@ -80,7 +80,7 @@ YeeArgs yee_args(emlab_grid* g) {
     a.pml_cls_xy = g->pml_cls.p, a.pml_xy = g->pml.p, a.pml_xy_stride = g->pml_stride, a.pml_xy_scene = 0;
     a.items = nullptr, a.n_items = 0, a.scene_xy = nullptr;
     if (g->stack.ragged) {
-        const int ti = ty == 4 ? 0 : (ty == 8 ? 1 : 2);
+        const int ti = mode == kNarrowPairTiles ? 3 : (ty == 4 ? 0 : (ty == 8 ? 1 : 2));
         a.pml_cls_xy = g->d_pml_cls_xy.p, a.pml_xy = g->d_pml_xy.p;
         a.pml_xy_stride = g->pml_xy_stride, a.pml_xy_scene = 6 * g->pml_xy_stride;
         a.items = g->d_items[ti].p, a.n_items = g->n_items[ti];
@@ -138,9 +138,28 @@ int emlab::upload_class_table(emlab_grid* g, const ClassTable& t) {
 }
 
 // Tensor maps of both field generations and the class index (the TMA kernel's inputs).
+// The pair tiles of the automatic tiling: 64 x 8, or 32 x 16 (as many cells and warps) where those cover at
+// least 7 % fewer cells. Where both cover the same the narrow tile is within 4 % either way: its rows have
+// twice the halo along x, but fewer of them touch the x layers (microseconds a step, wide and narrow:
+// 128 cube 30.7 and 29.6, 256 x 256 x 176 117.9 and 118.7, 512 cube 1214 and 1240). With 8 to 25 % fewer
+// cells it takes 2 to 13 % less: 96 cube 27.5 and 24.8, 150 cube 56.0 and 52.6, 211 x 147 x 93 56.2 and 53.0, 200
+// cube 108.5 and 101.4, 16 scenes of 48 to 160 cells an edge 295 and 263, 8 of 80 71.1 and 62.2.
+static int auto_tiling(const emlab_grid* g) {
+    long long wide = 0, narrow = 0;
+    auto count = [&](long long nx, long long ny, long long nz) {
+        wide += (nx + 63) / 64 * 64 * ((ny + 7) / 8 * 8) * nz;
+        narrow += (nx + 31) / 32 * 32 * ((ny + 15) / 16 * 16) * nz;
+    };
+    if (g->stack.ragged)
+        for (int i = 0; i < g->stack.scenes(); ++i) count(g->stack.nx[(size_t)i], g->stack.ny[(size_t)i], g->stack.nz[(size_t)i]);
+    else count(g->cfg.nx, g->cfg.ny, 1);
+    return 100 * narrow <= 93 * wide ? kNarrowPairTiles : 64;
+}
+
 void emlab::refresh_tma(emlab_grid* g) {
     invalidate_graphs(g);
     if (!g->tma) g->tma = tma_maps_create();
+    g->auto_tiling = auto_tiling(g);
     const int cur = g->cur;
     for (int gen = 0; gen < 2; ++gen) {
         g->cur = gen;
@@ -233,9 +252,9 @@ int emlab::upload_pml(emlab_grid* g) {
         int dev = 0, sms = 0;
         EMLAB_CUDA(cudaGetDevice(&dev));
         EMLAB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        const int tys[3] = {4, 8, 16}, per_sm[3] = {3, 2, 1};
-        for (int t = 0; t < 3; ++t) {
-            const std::vector<int4> items = ragged_items(st.z0, st.nx, st.ny, st.nz, tys[t], per_sm[t] * sms);
+        const int tys[4] = {4, 8, 16, 16}, per_sm[4] = {3, 2, 1, 2}, xts[4] = {64, 64, 64, 32};
+        for (int t = 0; t < 4; ++t) {
+            const std::vector<int4> items = ragged_items(st.z0, st.nx, st.ny, st.nz, tys[t], per_sm[t] * sms, xts[t]);
             EMLAB_REQUIRE(!items.empty(), "stack: no work items");
             EMLAB_CUDA(g->d_items[t].alloc(items.size()));
             EMLAB_CUDA(cudaMemcpyAsync(g->d_items[t].p, items.data(), items.size() * 16, cudaMemcpyHostToDevice, g->stream));
@@ -243,7 +262,7 @@ int emlab::upload_pml(emlab_grid* g) {
         }
     } else {
         for (auto& d : g->d_items) d.release();
-        g->n_items[0] = g->n_items[1] = g->n_items[2] = 0;
+        for (int& n : g->n_items) n = 0;
         g->d_scene_xy.release(), g->d_pml_cls_xy.release(), g->d_pml_xy.release();
     }
     EMLAB_CUDA(g->pml.alloc(pt.size()));

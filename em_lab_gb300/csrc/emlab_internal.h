@@ -26,6 +26,10 @@ namespace emlab {
 //   tabM[2c]   = (sig.x, sig.y, sig.z, eps.x) tabM[2c+1] = (eps.y, eps.z, 0, 0)
 //   tabW[2c]   = (w0.x, w0.y, w0.z, w1.x)     tabW[2c+1] = (w1.y, w1.z, 0, 0)
 // Classes >= wire_start carry thin-wire factors other than 1.
+// Tiling mode of the pair kernel's 32 x 16 tiles, two rows a warp: not one a caller can ask for, the automatic
+// tiling's choice beside 64 (64 x 8).
+constexpr int kNarrowPairTiles = 48;
+
 struct YeeArgs {
     int nx, ny, nz;
     int pitch;          // floats per row
@@ -54,7 +58,7 @@ struct YeeArgs {
     float dt;
     float minus_zero;  // -0, for the packed products of the pair kernel (mul2)
     int zchunk;
-    int tile_rows;   // tiling mode of the fused kernels (8, 16: single-cell tiles; 64, 128: pair tiles)
+    int tile_rows;   // tiling mode of the fused kernels (8, 16: single-cell tiles; 32, 64, 128, kNarrowPairTiles: pair tiles)
     unsigned long long* work;      // work-item tickets and leaver count of the persistent kernel (zero between launches)
     int wait_polls;                // polls of a plane's copy barrier before the CTA gives up (wait_limit())
     // x / y absorber lookups of the pair kernel: rows 0 (I_x), 1 (I_y), 3 (H_x), 4 (H_y) of a
@@ -108,7 +112,7 @@ bool tma_maps_ready(const TmaMaps* m, int gen);
 // chunk by chunk, tile by tile): tiles of 64 x ty cells over each scene's nx x ny, z chunks of one
 // length for all scenes, chosen for g CTAs as the uniform schedule chooses it
 std::vector<int4> ragged_items(const std::vector<int>& z0, const std::vector<int>& nx, const std::vector<int>& ny,
-                               const std::vector<int>& nz, int ty, int g);
+                               const std::vector<int>& nz, int ty, int g, int xt = 64);
 // the uniform grid's pair-kernel schedule for g CTAs: planes per z chunk and work items
 void pair_schedule_shape(int nx, int ny, int nz, int ty, int g, int* zc, int* items);
 // Launches the TMA kernel reading generation `gen`; err receives a nonzero word if a wait timed out.

@@ -100,6 +100,7 @@ struct emlab_grid {
     int cur = 0;
     int kernel = EMLAB_KERNEL_FUSED;
     int tile_rows = 0;  // 0: automatic
+    int auto_tiling = 64;  // what that means for the grid or stack: set with the tensor maps
     // materials
     DevBuf<uint8_t> cls;
     bool wide = false;
@@ -133,10 +134,10 @@ struct emlab_grid {
     // stack of scenes (empty: a single scene)
     emlab::StackLayout stack;
     uint32_t stack_sep = 0;  // class of the separator planes
-    // ragged stack: pair-kernel work items per tile height (4, 8, 16 rows), every scene's nx, ny,
+    // ragged stack: pair-kernel work items per tile (64 x 4, 8, 16; 32 x 16), every scene's nx, ny,
     // and per-scene x / y absorber tables
-    DevBuf<int4> d_items[3];
-    int n_items[3] = {0, 0, 0};
+    DevBuf<int4> d_items[4];
+    int n_items[4] = {0, 0, 0, 0};
     DevBuf<int2> d_scene_xy;
     DevBuf<uint8_t> d_pml_cls_xy;
     DevBuf<float> d_pml_xy;

@@ -30,6 +30,7 @@ struct TmaMaps {
     CUtensorMap cls;
     bool ok[2] = {false, false};
     bool cls_ok = false;
+    int tiling = -1;  // YeeArgs::tile_rows that the boxes were made for
 };
 
 namespace {
@@ -350,7 +351,8 @@ __global__ void __launch_bounds__(32 * (TY + 1), TY <= 8 ? 3 : 1)
 
 // ------------------------------------------------------------------------------------------------
 // Two cells per thread along x: a CTA owns a 64 x TY tile (warp w = row y0+w, lane l = cells
-// x0+2l and x0+2l+1) and marches it along z. Same arithmetic per cell as above, bit for bit.
+// x0+2l and x0+2l+1) or a 32 x 2 TY tile (two rows a warp, XL = 16 lanes each) and marches it along z.
+// Same arithmetic per cell as above, bit for bit.
 //
 // What bounds it: HBM on large grids (48.6 bytes of traffic per cell-step), and before that the
 // instructions issued per cell, so the own warps' inner loop is written for few of them:
@@ -368,15 +370,16 @@ __global__ void __launch_bounds__(32 * (TY + 1), TY <= 8 ? 3 : 1)
 //    copy takes its thread about a hundred cycles, so a plane's E and B are one copy each (the three
 //    components are the fourth dimension of the tensor map): three copies a plane instead of seven,
 //    and nothing else in that warp's way; it was the longest chain of the plane.
-template <int TY, typename Idx>
+template <int TY, typename Idx, int XL = 32>
 struct Layout2 {
     static constexpr int STAGES = 4;
-    static constexpr int W = 72;                        // box row width of E, B and the class index
+    static constexpr int ROWS = TY * 32 / XL;           // a warp holds 32 / XL rows of 2 XL cells
+    static constexpr int W = 2 * XL + 8;                // box row width of E, B and the class index
     static constexpr int CX = sizeof(Idx) == 2 ? 8 : 4;  // boxes start at x0 - 4 (16-bit class: x0 - 8)
     static constexpr int DC = CX - 4;                   // class element offset from the E/B element
-    static constexpr int EP = W * (TY + 2) * 4;         // one component: rows y0-1 .. y0+TY
-    static constexpr int BP = W * (TY + 1) * 4;         // rows y0-1 .. y0+TY-1
-    static constexpr int C_BYTES = W * (TY + 1) * (int)sizeof(Idx);
+    static constexpr int EP = W * (ROWS + 2) * 4;       // one component: rows y0-1 .. y0+ROWS
+    static constexpr int BP = W * (ROWS + 1) * 4;       // rows y0-1 .. y0+ROWS-1
+    static constexpr int C_BYTES = W * (ROWS + 1) * (int)sizeof(Idx);
     static constexpr int E_OFF = 0;                     // the three components of a copy lie back to back
     static constexpr int B_OFF = (3 * EP + 127) / 128 * 128;
     static constexpr int C_OFF = B_OFF + (3 * BP + 127) / 128 * 128;
@@ -384,7 +387,7 @@ struct Layout2 {
     static constexpr uint32_t TX_BYTES = 3 * EP + 3 * BP + C_BYTES;
     // B tile row: element e of a box row maps to slot e - 2 (col 1 = x0-1, col 2+i = x0+i)
     static constexpr int SB_OFF = STAGES * STAGE;
-    static constexpr int SB_BYTES = 2 * 3 * (TY + 1) * W * 4;
+    static constexpr int SB_BYTES = 2 * 3 * (ROWS + 1) * W * 4;
     // absorber coefficients of every own pair outside the z layers: [entry r1..r4][thread]{decay, gain}
     static constexpr int COEF_OFF = (SB_OFF + SB_BYTES + 127) / 128 * 128;
     static constexpr int COEF_BYTES = 4 * 32 * TY * 16;
@@ -513,7 +516,7 @@ __device__ __forceinline__ void e_update(const YeeArgs& a, float& ex, float& ey,
 // planes apart from their neighbours. work[0] counts tickets, work[1] the CTAs that have left: the
 // last to leave, also after a wait that ran out, clears both, so every launch starts at zero.
 struct PairSched {
-    int tiles_x;  // 64-cell tiles along x
+    int tiles_x;  // tiles along x
     int tiles;    // tiles per z chunk
     int items;    // tiles * z chunks
     int zc;       // planes per z chunk
@@ -525,7 +528,7 @@ struct PairItem {
     int x0, y0, zs, ze, zstart, scene;
 };
 
-template <int TY>
+template <int XT, int ROWS>
 __device__ __forceinline__ PairItem pair_item(const PairSched& ps, int nz, int item) {
     PairItem it;
     if (ps.tab) {
@@ -533,8 +536,8 @@ __device__ __forceinline__ PairItem pair_item(const PairSched& ps, int nz, int i
         it.x0 = t.x & 0xffff, it.y0 = (int)((unsigned)t.x >> 16), it.zs = t.y, it.ze = t.z, it.scene = t.w;
     } else {
         const int c = item / ps.tiles, t = item - c * ps.tiles;
-        it.x0 = (t % ps.tiles_x) * 64;
-        it.y0 = (t / ps.tiles_x) * TY;
+        it.x0 = (t % ps.tiles_x) * XT;
+        it.y0 = (t / ps.tiles_x) * ROWS;
         it.zs = c * ps.zc;
         it.ze = min(nz, it.zs + ps.zc);
         it.scene = 0;
@@ -570,17 +573,18 @@ __device__ __forceinline__ void plane_sync() {  // every warp of the CTA, once p
 // on across item boundaries, so the pipeline never drains inside a launch. The leader (lane 0 of
 // warp TY+1) takes the next item when its loads near it and posts the item number in a small
 // shared ring that the other warps read at their item boundary (always at least one barrier later).
-// 64 x 4 tiles: three 192-thread CTAs per SM; 64 x 8: two 320-thread CTAs; 64 x 16: one 576-thread
+// 64 x 4 tiles: three 192-thread CTAs per SM; 64 x 8 and 32 x 16: two 320-thread CTAs; 64 x 16: one 576-thread
 // CTA. Registers are allocated per SM quadrant and 18-20 warps put 5 warps on one quadrant: 96
 // registers at most.
-template <int TY, typename Idx>
-__global__ void __launch_bounds__(32 * (TY + 2), Layout2<TY, Idx>::CTAS)
+template <int TY, typename Idx, int XL>
+__global__ void __launch_bounds__(32 * (TY + 2), Layout2<TY, Idx, XL>::CTAS)
     yee_tma2(const __grid_constant__ CUtensorMap te, const __grid_constant__ CUtensorMap tb,
              const __grid_constant__ CUtensorMap tcls, YeeArgs a, PairSched ps, unsigned* err) {
     static_assert(TY == 4 || TY == 8 || TY == 16, "register budget assumes 6, 10 or 18 warps per CTA");
-    using Lay = Layout2<TY, Idx>;
-    constexpr int S_ = Lay::STAGES;
-    constexpr int EPF = Lay::EP / 4, BPF = Lay::BP / 4, W = Lay::W, SBC = (TY + 1) * W;
+    using Lay = Layout2<TY, Idx, XL>;
+    static_assert(XL == 32 || XL == 16, "a warp holds one row or two");
+    constexpr int S_ = Lay::STAGES, ROWS = Lay::ROWS;
+    constexpr int EPF = Lay::EP / 4, BPF = Lay::BP / 4, W = Lay::W, SBC = (ROWS + 1) * W;
     extern __shared__ __align__(128) unsigned char smem[];
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Lay::BAR_OFF);
     float* sB = reinterpret_cast<float*>(smem + Lay::SB_OFF);
@@ -616,7 +620,7 @@ __global__ void __launch_bounds__(32 * (TY + 2), Layout2<TY, Idx>::CTAS)
         bool more = true;
         unsigned long long ticket = 0;
         auto seek = [&](int item) {
-            const PairItem it = pair_item<TY>(ps, a.nz, item);
+            const PairItem it = pair_item<2 * XL, Lay::ROWS>(ps, a.nz, item);
             p_x = it.x0 - 4, p_y = it.y0 - 1, p_z = it.zstart, p_end = it.ze;
         };
         auto issue_upto = [&](int last) {  // issue loads up to index `last` while the sequence lasts
@@ -669,7 +673,7 @@ __global__ void __launch_bounds__(32 * (TY + 2), Layout2<TY, Idx>::CTAS)
         if (*stop == 0) return leave(true);
         int k = 0, iter = 0;
         for (int ord = 0, item = queue[0]; item >= 0; item = queue[++ord & 7]) {
-            const PairItem it = pair_item<TY>(ps, a.nz, item);
+            const PairItem it = pair_item<2 * XL, Lay::ROWS>(ps, a.nz, item);
             for (int z = it.zstart; z < it.ze; ++z, ++k, ++iter) {
                 // the next iteration reads loads k+1, k+2 (or k+2, k+3 at the start of the next item,
                 // which was taken when the last load of this one was issued)
@@ -698,18 +702,20 @@ __global__ void __launch_bounds__(32 * (TY + 2), Layout2<TY, Idx>::CTAS)
     // box element of the own / halo-row pair (E, B and 32-bit class boxes share it; the 16-bit class
     // box is DC elements further); B tile slot = element - 2
     const bool row = warp == TY;  // the halo warp; its row: Bx, Bz of (xa, y0-1), (xa+1, y0-1)
-    const int me = (row ? 0 : warp + 1) * W + 2 * lane + 4;
+    // two rows a warp: the halo warp's upper half repeats its lower half
+    const int lx = lane % XL, mine = warp * (32 / XL) + lane / XL;  // the pair's place in its row, the own row
+    const int me = (row ? 0 : mine + 1) * W + 2 * lx + 4;
     const pair_t dt2 = pk(a.dt, a.dt), mz = pk(a.minus_zero, a.minus_zero);
     int k = 0;     // load index of the current iteration's plane z
     int iter = 0;  // iteration counter: parity selects the B tile buffer
     for (int ord = 0, item = queue[0]; item >= 0; item = queue[++ord & 7]) {
-        const PairItem it = pair_item<TY>(ps, a.nz, item);
+        const PairItem it = pair_item<2 * XL, Lay::ROWS>(ps, a.nz, item);
         int snx, sny;
         scene_size(it.scene, snx, sny);
         // cells outside the item's scene (a ragged stack's frozen cells) are neither updated nor
         // written: they keep their initial 0 in both field generations
-        const int xa = it.x0 + 2 * lane;
-        const int y = row ? it.y0 - 1 : it.y0 + warp;
+        const int xa = it.x0 + 2 * lx;
+        const int y = row ? it.y0 - 1 : it.y0 + mine;
         const bool rowok = row ? it.y0 > 0 : y < sny;
         const bool o0 = rowok && xa < snx, o1 = rowok && xa + 1 < snx;
         const unsigned char* pcx = a.pml_cls_xy + (long long)it.scene * a.pml_xy_scene;
@@ -723,9 +729,9 @@ __global__ void __launch_bounds__(32 * (TY + 2), Layout2<TY, Idx>::CTAS)
         unsigned zi = __ldg(a.pml_zi + it.zstart);
 
         if (row) {
-            // the -x halo column too: By, Bz of (x0-1, y0 + lane), lanes 0 .. TY-1 (the others repeat the
+            // the -x halo column too: By, Bz of (x0-1, y0 + lane), lanes 0 .. ROWS-1 (the others repeat the
             // last one). Its cells always read the table: (1, dt) outside the layer
-            const int cl = min(lane, TY - 1), ce = (cl + 1) * W + 3;
+            const int cl = min(lane, ROWS - 1), ce = (cl + 1) * W + 3;
             const bool clive = it.x0 > 0 && it.y0 + cl < sny;
             PmlRows C{};
             if (clive) C = pml_rows(pcx, SX, K, it.x0 - 1, it.y0 + cl);
@@ -750,7 +756,7 @@ __global__ void __launch_bounds__(32 * (TY + 2), Layout2<TY, Idx>::CTAS)
                         }
                         const float hby = ky.x * Bs[BPF + ce] - ky.y * (t0y - t1y);
                         const float hbz = kz.x * Bs[2 * BPF + ce] - kz.y * (t0z - t1z);
-                        if (lane < TY) sb[SBC + ce] = clive ? hby : 0.0f, sb[2 * SBC + ce] = clive ? hbz : 0.0f;
+                        if (lane < ROWS) sb[SBC + ce] = clive ? hby : 0.0f, sb[2 * SBC + ce] = clive ? hbz : 0.0f;
                     }
                     pair_t hx2 = 0, hz2 = 0;  // B below the lower face is 0
                     if (rowok) {
@@ -964,23 +970,28 @@ bool encode(CUtensorMap* m, CUtensorMapDataType type, int elem, const void* base
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// tiling modes: 8, 16 = 32 x TY tiles of single cells (yee_tma); 64, 128 = 64 x 8 and 64 x 16 tiles
-// of cell pairs (yee_tma2)
+// tiling modes: 8, 16 = 32 x TY tiles of single cells (yee_tma); 32, 64, 128 = 64 x 4, 64 x 8 and 64 x 16
+// tiles of cell pairs, kNarrowPairTiles = 32 x 16 (yee_tma2)
 // The three component arrays from base, `comp` floats apart, as one map: the copies of the pair tiles.
-bool encode3(CUtensorMap* m, const float* base, long long comp, const YeeArgs& a, int box_h) {
+bool encode3(CUtensorMap* m, const float* base, long long comp, const YeeArgs& a, int box_w, int box_h) {
     EncodeFn fn = encode_fn();
     if (!fn) return false;
     const cuuint64_t dims[4] = {(cuuint64_t)a.nx, (cuuint64_t)a.ny, (cuuint64_t)a.nz, 3};
     const cuuint64_t strides[3] = {(cuuint64_t)a.pitch * 4, (cuuint64_t)a.plane * 4, (cuuint64_t)comp * 4};
-    const cuuint32_t box[4] = {72, (cuuint32_t)box_h, 1, 3};
+    const cuuint32_t box[4] = {(cuuint32_t)box_w, (cuuint32_t)box_h, 1, 3};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(base), dims, strides, box, estr,
               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-int tile_rows(const YeeArgs& a) { return a.tile_rows == 16 || a.tile_rows == 128 ? 16 : (a.tile_rows == 32 ? 4 : 8); }
-bool pair_tiles(const YeeArgs& a) { return a.tile_rows == 32 || a.tile_rows == 64 || a.tile_rows == 128; }
+bool narrow_tiles(const YeeArgs& a) { return a.tile_rows == kNarrowPairTiles; }
+int tile_rows(const YeeArgs& a) {
+    return a.tile_rows == 16 || a.tile_rows == 128 || narrow_tiles(a) ? 16 : (a.tile_rows == 32 ? 4 : 8);
+}
+bool pair_tiles(const YeeArgs& a) {
+    return a.tile_rows == 32 || a.tile_rows == 64 || a.tile_rows == 128 || narrow_tiles(a);
+}
 
 template <int TY, typename Idx>
 bool launch_t(const YeeArgs& a, const TmaMaps* m, int gen, unsigned* err, const Chain& s) {
@@ -1010,10 +1021,10 @@ bool launch_t(const YeeArgs& a, const TmaMaps* m, int gen, unsigned* err, const 
 constexpr int kItemsPerCta = 4;
 constexpr int kMinBalancedPlanes = 16;
 
-PairSched pair_schedule(const YeeArgs& a, int TY, int G) {
+PairSched pair_schedule(const YeeArgs& a, int xt, int rows, int G) {
     PairSched ps;
-    ps.tiles_x = (a.nx + 63) / 64;
-    ps.tiles = ps.tiles_x * ((a.ny + TY - 1) / TY);
+    ps.tiles_x = (a.nx + xt - 1) / xt;
+    ps.tiles = ps.tiles_x * ((a.ny + rows - 1) / rows);
     const int max_chunks = std::max(1, a.nz / 4);
     const long long want = std::min((long long)kItemsPerCta * G,
                                     (long long)std::max(1, a.nz / kMinBalancedPlanes) * ps.tiles);
@@ -1052,9 +1063,9 @@ void small_grid_schedule(PairSched& ps, int nz, int G) {
     }
 }
 
-template <int TY, typename Idx>
+template <int TY, int XL, typename Idx>
 bool launch_p(const YeeArgs& a, const TmaMaps* m, int gen, unsigned* err, const Chain& s) {
-    using Lay = Layout2<TY, Idx>;
+    using Lay = Layout2<TY, Idx, XL>;
     static int resident = 0, sms = 0;  // per process: one device model
     std::unique_lock<std::mutex> lk(g_launch_setup);
     if (!resident) {
@@ -1065,12 +1076,12 @@ bool launch_p(const YeeArgs& a, const TmaMaps* m, int gen, unsigned* err, const 
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
             cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
             smem_sm <= 0 ||
-            cudaFuncSetAttribute(yee_tma2<TY, Idx>, cudaFuncAttributeMaxDynamicSharedMemorySize, Lay::SMEM) !=
+            cudaFuncSetAttribute(yee_tma2<TY, Idx, XL>, cudaFuncAttributeMaxDynamicSharedMemorySize, Lay::SMEM) !=
                 cudaSuccess ||
-            cudaFuncSetAttribute(yee_tma2<TY, Idx>, cudaFuncAttributePreferredSharedMemoryCarveout,
+            cudaFuncSetAttribute(yee_tma2<TY, Idx, XL>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  std::min(100, (100 * Lay::CTAS * (Lay::SMEM + 1024) +
                                                 smem_sm - 1) / smem_sm)) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, yee_tma2<TY, Idx>, 32 * (TY + 2), Lay::SMEM) !=
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, yee_tma2<TY, Idx, XL>, 32 * (TY + 2), Lay::SMEM) !=
                 cudaSuccess ||
             resident < 1) {
             resident = 0;
@@ -1083,14 +1094,14 @@ bool launch_p(const YeeArgs& a, const TmaMaps* m, int gen, unsigned* err, const 
         ps.items = a.n_items;
         ps.tab = a.items;
     } else {
-        ps = pair_schedule(a, TY, resident * sms);
+        ps = pair_schedule(a, 2 * XL, Lay::ROWS, resident * sms);
         if (ps.items < kItemsPerCta * resident * sms) small_grid_schedule(ps, a.nz, resident * sms);
         ps.tab = nullptr;
     }
     if (ps.items <= 0) return false;
     const int grid = std::min(ps.items, resident * sms);
     ps.work = a.work;
-    launch_chained(s, yee_tma2<TY, Idx>, grid, dim3(32, TY + 2), Lay::SMEM, m->e3[gen], m->b3[gen], m->cls, a, ps, err);
+    launch_chained(s, yee_tma2<TY, Idx, XL>, grid, dim3(32, TY + 2), Lay::SMEM, m->e3[gen], m->b3[gen], m->cls, a, ps, err);
     return true;
 }
 
@@ -1102,12 +1113,14 @@ void tma_maps_destroy(TmaMaps* m) { delete m; }
 bool tma_maps_encode(TmaMaps* m, int gen, const YeeArgs& a, bool wide) {
     const int ty = tile_rows(a);
     const bool pair = pair_tiles(a);
-    const int cw16 = pair ? 72 : 40, cw32 = pair ? 72 : 36;
+    const int pair_w = narrow_tiles(a) ? 40 : 72;
+    const int cw16 = pair ? pair_w : 40, cw32 = pair ? pair_w : 36;
     bool ok = (a.pitch % 4) == 0;
     if (pair) {
         const long long comp = a.ey - a.ex;  // the six arrays of a generation lie one after the other
         ok = ok && a.ez - a.ex == 2 * comp && a.by - a.bx == comp && a.bz - a.bx == 2 * comp &&
-             encode3(&m->e3[gen], a.ex, comp, a, ty + 2) && encode3(&m->b3[gen], a.bx, comp, a, ty + 1);
+             encode3(&m->e3[gen], a.ex, comp, a, pair_w, ty + 2) &&
+             encode3(&m->b3[gen], a.bx, comp, a, pair_w, ty + 1);
     }
     const float* e[3] = {a.ex, a.ey, a.ez};
     const float* b[3] = {a.bx, a.by, a.bz};
@@ -1120,6 +1133,7 @@ bool tma_maps_encode(TmaMaps* m, int gen, const YeeArgs& a, bool wide) {
                   : encode(&m->cls, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, a.cls, a, cw16, ty + 1);
     m->ok[gen] = ok;
     m->cls_ok = ok;
+    m->tiling = a.tile_rows;
     return ok;
 }
 
@@ -1128,17 +1142,17 @@ bool tma_maps_ready(const TmaMaps* m, int gen) { return m && m->ok[gen] && m->cl
 void pair_schedule_shape(int nx, int ny, int nz, int ty, int g, int* zc, int* items) {
     YeeArgs a{};
     a.nx = nx, a.ny = ny, a.nz = nz;
-    const PairSched ps = pair_schedule(a, ty, g);
+    const PairSched ps = pair_schedule(a, 64, ty, g);
     *zc = ps.zc, *items = ps.items;
 }
 
 std::vector<int4> ragged_items(const std::vector<int>& z0, const std::vector<int>& nx, const std::vector<int>& ny,
-                               const std::vector<int>& nz, int ty, int g) {
+                               const std::vector<int>& nz, int ty, int g, int xt) {
     const size_t n = z0.size();
     std::vector<long long> tiles(n);
     int deepest = 1;
     for (size_t i = 0; i < n; ++i) {
-        tiles[i] = (long long)((nx[i] + 63) / 64) * ((ny[i] + ty - 1) / ty);
+        tiles[i] = (long long)((nx[i] + xt - 1) / xt) * ((ny[i] + ty - 1) / ty);
         deepest = std::max(deepest, nz[i]);
     }
     // one chunk length for every scene: the CTA with the most items bounds the launch, and every
@@ -1162,26 +1176,29 @@ std::vector<int4> ragged_items(const std::vector<int>& z0, const std::vector<int
     }
     std::vector<int4> out;
     for (size_t i = 0; i < n; ++i) {
-        const int tx = (nx[i] + 63) / 64, tyn = (ny[i] + ty - 1) / ty;
+        const int tx = (nx[i] + xt - 1) / xt, tyn = (ny[i] + ty - 1) / ty;
         for (int zs = 0; zs < nz[i]; zs += zc_best)
             for (int t = 0; t < tx * tyn; ++t)
-                out.push_back(make_int4((t % tx) * 64 | ((t / tx) * ty) << 16, z0[i] + zs,
+                out.push_back(make_int4((t % tx) * xt | ((t / tx) * ty) << 16, z0[i] + zs,
                                         z0[i] + std::min(nz[i], zs + zc_best), (int)i));
     }
     return out;
 }
 
 bool launch_yee_tma(const YeeArgs& a, const TmaMaps* m, int gen, bool wide, unsigned* err, const Chain& s) {
-    if (!m || !m->ok[gen] || !m->cls_ok) return false;
+    if (!m || !m->ok[gen] || !m->cls_ok || m->tiling != a.tile_rows) return false;
+    if (narrow_tiles(a))
+        return wide ? launch_p<8, 16, uint32_t>(a, m, gen, err, s)
+                    : launch_p<8, 16, uint16_t>(a, m, gen, err, s);
     if (pair_tiles(a) && tile_rows(a) == 16)
-        return wide ? launch_p<16, uint32_t>(a, m, gen, err, s)
-                    : launch_p<16, uint16_t>(a, m, gen, err, s);
+        return wide ? launch_p<16, 32, uint32_t>(a, m, gen, err, s)
+                    : launch_p<16, 32, uint16_t>(a, m, gen, err, s);
     if (pair_tiles(a) && tile_rows(a) == 4)
-        return wide ? launch_p<4, uint32_t>(a, m, gen, err, s)
-                    : launch_p<4, uint16_t>(a, m, gen, err, s);
+        return wide ? launch_p<4, 32, uint32_t>(a, m, gen, err, s)
+                    : launch_p<4, 32, uint16_t>(a, m, gen, err, s);
     if (pair_tiles(a))
-        return wide ? launch_p<8, uint32_t>(a, m, gen, err, s)
-                    : launch_p<8, uint16_t>(a, m, gen, err, s);
+        return wide ? launch_p<8, 32, uint32_t>(a, m, gen, err, s)
+                    : launch_p<8, 32, uint16_t>(a, m, gen, err, s);
     if (tile_rows(a) == 16) return wide ? launch_t<16, uint32_t>(a, m, gen, err, s) : launch_t<16, uint16_t>(a, m, gen, err, s);
     return wide ? launch_t<8, uint32_t>(a, m, gen, err, s) : launch_t<8, uint16_t>(a, m, gen, err, s);
 }
