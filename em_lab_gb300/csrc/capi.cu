@@ -65,7 +65,7 @@ YeeArgs yee_args(emlab_grid* g) {
     a.minus_zero = -0.0f;
     // tile height and z chunks: enough CTAs for ~4 per SM, but at least 8 planes each (the first
     // plane of a chunk is recomputed)
-    const int mode = g->tile_rows == 0 ? g->auto_tiling : g->tile_rows;
+    const int mode = g->tile_rows ? g->tile_rows : (g->kernel == EMLAB_KERNEL_FUSED ? g->auto_tiling : 64);
     const int ty = mode == 16 || mode == 128 || mode == kNarrowPairTiles ? 16 : (mode == 32 ? 4 : 8);
     const int tx = (mode == 32 || mode == 64 || mode == 128) && g->kernel == EMLAB_KERNEL_FUSED ? 64 : 32;
     a.tile_rows = g->kernel == EMLAB_KERNEL_FUSED ? mode : ty;

@@ -5,9 +5,8 @@
 // frame loop that measures flux every other frame, like the reference's, while the solver keeps stepping
 // (cudaFree waits for the whole device, so such a measurement would stall the solver), and applications
 // that budget all device memory themselves (an allocation they did not plan for can fail part-way
-// through a run). This
-// variant keeps its scratch in fixed file-scope device arrays instead: kMaxPartials workgroup
-// partials (256 KB) and kMaxPlanes FP64 sums, held by every device that loads the library until
+// through a run). This variant keeps its scratch in fixed file-scope device arrays instead: kMaxPartials
+// workgroup partials (256 KB) and kMaxPlanes FP64 sums, held by every device that loads the library until
 // the process exits. The first call on a device looks their addresses up; every call shares them,
 // so calls whose kernels overlap on the GPU race. The call returns once the sums are on the host.
 #include <cuda_runtime.h>
