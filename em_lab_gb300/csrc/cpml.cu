@@ -27,9 +27,10 @@
 // cells of a row through a chunk of planes, copies the next plane's operands into shared memory of its own
 // while it works on one, keeps the plane neighbour in registers and takes the row neighbour from the next
 // lane. The E pass takes the chunks from the top down, so that it starts on what the B pass left in L2 and
-// the next B pass on what it leaves. A step of 192 x 168 x 144 cells with sources, of 20 waited for together: 124 us with a cell a
-// thread, whose stores of psi and of one component stood before the loads of the next; 106 us with two
-// cells in registers, 88 us with the copies ahead, 80 us with the E pass turned round.
+// the next B pass on what it leaves. A step of 192 x 168 x 144 cells with sources, of 20 waited for
+// together: 124 us with a cell a thread, whose stores of psi and of one component stood before the loads
+// of the next; 106 us with two cells in registers, 88 us with the copies ahead, 80 us with the E pass
+// turned round.
 #include <cuda_runtime.h>
 
 #include <algorithm>
