@@ -201,15 +201,27 @@ class Net:
         n = x.shape[0]
         assert n <= self.B
         self.n = n
+
+        def host(src, *shape):
+            """src as a float32 tensor of exactly that shape: assignment broadcasts it or raises."""
+            v = torch.from_numpy(np.ascontiguousarray(src, np.float32))
+            if v.shape != shape:
+                full = torch.empty(shape, dtype=torch.float32)
+                full[:] = v
+                v = full
+            return v
+
+        # the kernel reads n rows through a pointer: the shapes are settled here
+        parts = ((host(x, n, T_IN, 2), T_IN * 2, self.x0, 2, 2, 0), (host(zt, n, AUX), AUX, self.X0, ENC + AUX, AUX, ENC))
         # rows beyond n are zero inputs (their targets and gradients are left out)
-        for src, row, out, ldo, cols, off in ((x, T_IN * 2, self.x0, 2, 2, 0), (zt, AUX, self.X0, ENC + AUX, AUX, ENC)):
-            d = torch.from_numpy(np.ascontiguousarray(src, np.float32)).to(self.dev)
+        for src, row, out, ldo, cols, off in parts:
+            d = src.to(self.dev)
             _check(self.lib.emlab_nn_pad_to_bf16(d.data_ptr(), n * row, self.B * row, out.data_ptr(), ldo, cols, off,
                                                  self.stream))
         if t is None:
             self.t.zero_()
         else:
-            self.t[:n].copy_(torch.from_numpy(np.ascontiguousarray(t, np.float32)))
+            self.t[:n].copy_(host(t, n, OUT))
 
     # -- forward / backward
     def _gemm_bias_act(self, M, N, K, A, name, z, relu, out, ldo, group, s):
