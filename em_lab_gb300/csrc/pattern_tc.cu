@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(kThreads, 1) pattern_kernel(const __grid_const
         for (int s = 0; s < kStages; ++s) mbar_init(full + s, 1), mbar_init(empty + s, 1);
         mbar_init(a_full, 32 * kComputeWarps);
         for (int s = 0; s < 2; ++s) mbar_init(t_full + s, 1), mbar_init(t_empty + s, 32 * kComputeWarps);
-        mbar_init(bars + 15, 1);  // the tensor core's last commit after a failure
+        mbar_init(bars + 15, 1);  // the tensor core's last commit
         *abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -322,10 +322,10 @@ __global__ void __launch_bounds__(kThreads, 1) pattern_kernel(const __grid_const
                                 commit(t_full + half);
                             }
                     }
-            if (!ok) {  // the MMAs issued so far end before tensor and shared memory go
-                commit(bars + 15);
-                drain(bars + 15, 0);
-            }
+            // The MMAs issued so far end before tensor and shared memory go: also where another role gave up its
+            // wait for them after the last one was issued.
+            commit(bars + 15);
+            drain(bars + 15, 0);
         }
         __syncwarp();
     } else {
@@ -382,7 +382,10 @@ __global__ void __launch_bounds__(kThreads, 1) pattern_kernel(const __grid_const
                         float g[4][2] = {};
                         for (int b = 0; b < box.f[f].blocks; ++b, ++blk) {
                             const uint32_t half = blk & 1;
-                            if (!(ok = mbar_wait(t_full + half, (blk >> 1) & 1, abort, polls))) break;
+                            // one verdict a warp, whatever its lanes saw (a lane may find the barrier complete and
+                            // another the abort word): what follows is for whole warps
+                            const bool landed = mbar_wait(t_full + half, (blk >> 1) & 1, abort, polls);
+                            if (!(ok = __all_sync(0xffffffffu, landed))) break;
                             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                             const int iu0 = b * kCols + half_cols * (kCols / 2);
                             float s, c;
@@ -430,6 +433,7 @@ __global__ void __launch_bounds__(kThreads, 1) pattern_kernel(const __grid_const
                 for (int k = 0; k < 12; ++k) combine[k] = (&NL[0][0][0])[k];
             {  // all of them leave after the same item: one that gave up takes the others along
                 uint32_t failed;
+                __syncwarp();
                 asm volatile(
                     "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\tbar.red.or.pred q, 1, %2, p;\n\t"
                     "selp.u32 %0, 1, 0, q;\n\t}"
@@ -460,6 +464,7 @@ __global__ void __launch_bounds__(kThreads, 1) pattern_kernel(const __grid_const
                     o[0] = F2, o[1] = 0.5f * P;
                 }
             }
+            __syncwarp();
             asm volatile("bar.sync 1, %0;" ::"n"(32 * kComputeWarps) : "memory");  // `combine` is free again
         }
     }
