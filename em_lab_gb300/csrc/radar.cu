@@ -26,8 +26,10 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <cstdint>
 #include <cstring>
-#include <vector>
+#include <memory>
+#include <new>
 
 #include "../../include/emlab.h"
 #include "emlab_internal.h"
@@ -316,23 +318,32 @@ extern "C" int emlab_radar_backproject(const emlab_radar_geometry* geo, const fl
         return report_error(EMLAB_ERR_INVALID, "bad radar back-projection arguments");
     const long long total = (long long)geo->nr * geo->nel * geo->naz;
     if (total > (1ll << 31)) return report_error(EMLAB_ERR_INVALID, "radar image too large");
-    // inputs in one buffer, one copy: z, the weights and amplitudes in FP64 and as pairs, the positions
+    // device memory first: sizes that cannot be had end here, before anything is read. One buffer: z, the weights
+    // and amplitudes in FP64 and as pairs, the positions, the image
     const size_t zb = (size_t)M * C * 8, nb = ((size_t)C + ntx) * 8, pb = ((size_t)C + ntx) * 12;
     const size_t bytes = (zb + 2 * nb + pb + 15) / 16 * 16;
-    std::vector<unsigned char> host;
-    try {
-        host.resize(bytes);
-    } catch (const std::bad_alloc&) {
+    unsigned char* buf = nullptr;
+    if ((size_t)M > SIZE_MAX / 16 / (size_t)C || cudaMalloc(&buf, bytes + (size_t)total * 8) != cudaSuccess) {
+        cudaGetLastError();
+        return report_error(EMLAB_ERR_OOM, "radar: device allocation failed");
+    }
+    // One copy for all inputs where z is short. A longer z goes from the caller's array by a copy of its own, which
+    // costs less than bringing it together with the rest from about this size on.
+    const size_t packed_z = zb <= (128u << 10) ? zb : 0;
+    std::unique_ptr<unsigned char[]> host(new (std::nothrow) unsigned char[packed_z + 2 * nb + pb]);
+    if (!host) {
+        cudaFree(buf);
         return report_error(EMLAB_ERR_OOM, "radar: host allocation failed");
     }
-    std::memcpy(host.data(), z, zb);
-    std::memcpy(host.data() + zb, weights, (size_t)C * 8);
-    std::memcpy(host.data() + zb + (size_t)C * 8, tx_amp, (size_t)ntx * 8);
-    FF* pairs = reinterpret_cast<FF*>(host.data() + zb + nb);
+    unsigned char* rest = host.get() + packed_z;
+    if (packed_z) std::memcpy(host.get(), z, zb);
+    std::memcpy(rest, weights, (size_t)C * 8);
+    std::memcpy(rest + (size_t)C * 8, tx_amp, (size_t)ntx * 8);
+    FF* pairs = reinterpret_cast<FF*>(rest + nb);
     for (int i = 0; i < C; ++i) pairs[i] = to_ff(weights[i]);
     for (int j = 0; j < ntx; ++j) pairs[C + j] = to_ff(tx_amp[j]);
-    std::memcpy(host.data() + zb + 2 * nb, elem_pos, (size_t)C * 12);
-    std::memcpy(host.data() + zb + 2 * nb + (size_t)C * 12, tx_pos, (size_t)ntx * 12);
+    std::memcpy(rest + 2 * nb, elem_pos, (size_t)C * 12);
+    std::memcpy(rest + 2 * nb + (size_t)C * 12, tx_pos, (size_t)ntx * 12);
     RadarTable table;
     for (int k = 0; k < kTable; ++k) {
         const double t = 6.28318530717958647692 * k / kTable;
@@ -342,13 +353,11 @@ extern "C" int emlab_radar_backproject(const emlab_radar_geometry* geo, const fl
     const double turns = geo->omega / 6.28318530717958647692;
     const FF w2 = to_ff(turns);
     const Turns wt = {w2.h, w2.l, (float)(turns - (double)w2.h - (double)w2.l)};
-    unsigned char* buf = nullptr;
-    if (cudaMalloc(&buf, bytes + (size_t)total * 8) != cudaSuccess) {
-        cudaGetLastError();
-        return report_error(EMLAB_ERR_OOM, "radar: device allocation failed");
-    }
     double* dp = reinterpret_cast<double*>(buf + bytes);
-    cudaError_t e = cudaMemcpy(buf, host.data(), bytes, cudaMemcpyHostToDevice);
+    cudaError_t e = cudaSuccess;
+    if (!packed_z) e = cudaMemcpy(buf, z, zb, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess)
+        e = cudaMemcpy(buf + zb - packed_z, host.get(), packed_z + 2 * nb + pb, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) {
         const double* d64 = reinterpret_cast<const double*>(buf + zb);
         const FF* dff = reinterpret_cast<const FF*>(buf + zb + nb);
