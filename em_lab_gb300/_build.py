@@ -30,7 +30,7 @@ NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-fmad=false", "-Xcompiler", HOS
 
 SOURCES = ["yee.cu", "yee_tma.cu", "monitors.cu", "capi.cu", "noalloc.cu", "dft_tc.cu", "render.cu", "stack.cu", "learn.cu", "radar.cu", "cpml.cu", "pattern.cu", "pattern_tc.cu", "setup.cpp"]
 HEADERS = ["emlab_math.h", "emlab_internal.h", "setup.h", "yee_common.cuh", "grid_state.h", "twiddle.cuh",
-           "chain.cuh"]
+           "chain.cuh", "radar_pairs.cuh"]
 
 
 def _nvcc() -> str:

@@ -11,18 +11,19 @@
 // The reference's sums are FP64, and the FP64 pipe (two multiply-adds per SM and cycle against 128 in
 // FP32) bounded the image: two sincos, three divisions and about forty other FP64 operations per
 // element and point. Here every FP64 quantity inside the element loops is an unevaluated pair of FP32
-// (about 47 significant bits): distances are FP32 already, phases are reduced in turns exactly, sin and
+// (48 bits, radar_pairs.cuh): distances are FP32 already, phases are reduced in turns exactly, sin and
 // cos come from a 512-entry table of pairs and a short series, delays are summed as differences from
 // the array centre's, and the common factor e^{j w t_out} of the receive sum is left out (it does not
 // change the power). The weighted mean delay is formed in FP64 once per point.
 //
 // What the pairs cannot decide is the rounding of the interpolation weight to FP32 and whether a delay
-// reaches the last sample. So each point carries a bound of its delay's error, and a point for which a
-// rounding within that bound could move the power by more than 2e-8 of itself, or whose sums are out
-// of the pairs' range or not finite, is formed again in FP64, in the reference's order, by its whole
-// warp. Images of 9 to 64 elements agree with the FP64 kernel's to 1e-14 of their power (2% of the points
-// with 36 elements, 7% with 64, take the second way). One call, 64 x 61 x 41 points and 36 elements:
-// 1558 us before, 428 us here; 90 x 61 x 61 points and 64 elements: 4734 and 934 us.
+// reaches the last sample. So each position carries a bound of its distance from the FP64 sums', derived
+// beside the code that forms it, and a point for which a rounding within that bound and the pairs' own errors
+// could move the power by more than 2e-10 of itself, or whose sums are out of the pairs' range or not finite,
+// is formed again in FP64, in the reference's order, by its whole warp. The power is thus within 2e-10 of the
+// FP64 sums'.
+// One call, 64 x 61 x 41 points and 36 elements: 1560 us with FP64 sums, 415 us here (the kernel 197 us, about 1 % of the
+// points the second way); 90 x 61 x 61 points and 64 elements: 4930 and 780 us.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -33,86 +34,14 @@
 
 #include "../../include/emlab.h"
 #include "emlab_internal.h"
+#include "radar_pairs.cuh"
 
 namespace emlab {
 namespace {
 
-struct F3 {
-    float x, y, z;
-};
-__device__ __forceinline__ F3 sub(F3 a, F3 b) { return {a.x - b.x, a.y - b.y, a.z - b.z}; }
-__device__ __forceinline__ F3 add(F3 a, F3 b) { return {a.x + b.x, a.y + b.y, a.z + b.z}; }
-__device__ __forceinline__ F3 mul(F3 a, float s) { return {a.x * s, a.y * s, a.z * s}; }
-__device__ __forceinline__ float dot(F3 a, F3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
-__device__ __forceinline__ float len(F3 a) { return sqrtf(dot(a, a)); }
-__device__ __forceinline__ F3 ld3(const float* p) { return {p[0], p[1], p[2]}; }
+using namespace radar;
 
-// Unevaluated sums hi + lo of two floats (Dekker, Numer. Math. 18, 1971; Knuth, TAOCP 2, 4.2.2).
-struct FF {
-    float h, l;
-};
-__host__ __device__ __forceinline__ FF to_ff(double v) {
-    const float h = (float)v;
-    return {h, (float)(v - (double)h)};
-}
-__device__ __forceinline__ double to_f64(FF a) { return (double)a.h + (double)a.l; }
-__device__ __forceinline__ FF fast_sum(float a, float b) {  // |a| >= |b|
-    const float s = a + b;
-    return {s, b - (s - a)};
-}
-__device__ __forceinline__ FF two_sum(float a, float b) {
-    const float s = a + b, t = s - a;
-    return {s, (a - (s - t)) + (b - t)};
-}
-__device__ __forceinline__ FF operator+(FF a, FF b) {
-    const FF s = two_sum(a.h, b.h);
-    return fast_sum(s.h, s.l + (a.l + b.l));
-}
-__device__ __forceinline__ FF operator+(FF a, float b) {
-    const FF s = two_sum(a.h, b);
-    return fast_sum(s.h, s.l + a.l);
-}
-__device__ __forceinline__ FF operator-(FF a) { return {-a.h, -a.l}; }
-__device__ __forceinline__ FF operator*(FF a, FF b) {
-    const float p = a.h * b.h;
-    return fast_sum(p, fmaf(a.l, b.h, fmaf(a.h, b.l, fmaf(a.h, b.h, -p))));
-}
-__device__ __forceinline__ FF operator*(FF a, float b) {
-    const float p = a.h * b;
-    return fast_sum(p, fmaf(a.l, b, fmaf(a.h, b, -p)));
-}
-
-// e^{j w d}, d >= 0 in FP32, from wt = w / 2 pi in turns per unit as a sum of three floats: the turns are
-// reduced to the nearest table entry (exactly: the products with d are kept in full), the rest r,
-// |r| <= pi / 512, enters through sin r = r - r^3/6 + r^5/120 and cos r = 1 - r^2/2 + r^4/24 (truncation
-// below 1e-16).
-constexpr int kTable = 512, kThreads = 128;
-constexpr float kTurns = 4096.0f;  // the rest e below stays under 2^-12 of a turn
-struct Turns {
-    float h, m, l;
-};
-struct Phase {
-    FF c, s;
-};
-__device__ __forceinline__ Phase phase(const float4* table, Turns wt, float d) {
-    const float p = wt.h * d, u = wt.m * d;
-    const FF e = two_sum(fmaf(wt.h, d, -p), u);
-    const float el = e.l + fmaf(wt.l, d, fmaf(wt.m, d, -u));
-    const float f = p - rintf(p);  // exact
-    const float k = rintf(f * (float)kTable);
-    FF t = two_sum(fmaf(k, -1.0f / kTable, f), e.h);  // turns beyond the entry; the first term is exact
-    t = fast_sum(t.h, t.l + el);
-    constexpr float two_pi_h = 6.28318548f, two_pi_l = -1.74845553e-7f;
-    const FF r = t * FF{two_pi_h, two_pi_l};
-    const float r2 = r.h * r.h;
-    const FF sr = fast_sum(r.h, fmaf(r.h * r2, fmaf(r2, 8.33333377e-3f, -0.166666672f), r.l));
-    const float r2l = fmaf(2.0f * r.h, r.l, fmaf(r.h, r.h, -r2));
-    const FF cm = {-0.5f * r2, fmaf(r2 * r2, 4.16666679e-2f, -0.5f * r2l)};  // cos r - 1
-    const float4 v = table[(int)k & (kTable - 1)];
-    const FF ct = {v.x, v.y}, st = {v.z, v.w};
-    // ct cos r - st sin r = ct + (ct (cos r - 1) - st sin r)
-    return {ct + (ct * cm + -(st * sr)), st + (st * cm + ct * sr)};
-}
+constexpr int kThreads = 128;
 
 struct Geo {
     F3 tx, ax0, ax1, ax2, lo, hi;
@@ -124,10 +53,8 @@ struct Inputs {
     const float *elem_pos, *tx_pos;
     const FF *weights, *tx_amp;              // as pairs,
     const double *weights64, *tx_amp64;      // and as they came
+    bool pairs;                              // the weights can be held as pairs
 };
-
-// Sums whose squares and low parts stay normal numbers; false for a NaN.
-__device__ __forceinline__ bool in_range(float v) { return v > 1e-18f && v < 1e18f; }
 
 // The power at p in FP64 by one warp: the lanes form the terms of 32 elements, and one lane per sum adds
 // them in the order of the elements. terms: 32 x 5 doubles of this warp.
@@ -192,49 +119,9 @@ __device__ __noinline__ double point64(const Geo& g, F3 p, const Inputs& in, dou
     return sr * sr + si * si;
 }
 
-struct Delay {
-    double t;
-    float err;  // bound of the difference from the FP64 sums; negative: to be formed in FP64
-};
-
-// RadarMonitor::txDelay (Radar.cpp:87-103). The bound scales with the cancellation in the array factor
-// and was fitted on the CPU against FP64 and extended sums: arrays of 1 to 256 elements half a wavelength
-// apart, 2 to 1000 cells away, with a factor of two and more in hand; cancellation beyond 100 goes to FP64.
-__device__ __forceinline__ Delay tx_delay(const Geo& g, F3 p, const float4* table, Turns wt, const Inputs& in) {
-    FF ar = {0, 0}, ai = ar, adr = ar, adi = ar, mag = ar;
-    const float d0 = len(sub(p, g.tx));
-    float spread = 0.0f, far = 0.0f;
-    for (int j = 0; j < in.ntx; ++j) {
-        const F3 v = sub(p, ld3(in.tx_pos + 3 * j));
-        const float d = fmaxf(len(v), 0.5f);
-        const float q = 1.0f / d;
-        const FF inv = {q, q * fmaf(-q, d, 1.0f)};
-        const FF a = (in.tx_amp[j] * (inv * inv)) * fmaxf(dot(v, g.ax2), 0.0f);  // amp (g / d) / d
-        const Phase e = phase(table, wt, d);
-        const FF tr = a * e.c, ti = a * e.s;  // the conjugate of a e^{-j w d}
-        const FF dd = two_sum(d, -d0);
-        ar = ar + tr, ai = ai + ti;
-        adr = adr + tr * dd, adi = adi + ti * dd;
-        mag = mag + a;
-        spread = fmaxf(spread, fabsf(dd.h)), far = fmaxf(far, d);
-    }
-    if (!in_range(mag.h) || !in_range(fmaxf(fabsf(ar.h), fabsf(ai.h))) || !(fabsf(wt.h) * far < kTurns))
-        return {0.0, -1.0f};
-    const double r = to_f64(ar), i = to_f64(ai);
-    const double t = (double)d0 + (to_f64(adr) * r + to_f64(adi) * i) / (r * r + i * i);  // real(ad / a)
-    const float over = rsqrtf(ar.h * ar.h + ai.h * ai.h), k = mag.h * over;
-    const float rest = sqrtf(adr.h * adr.h + adi.h * adi.h) * over;
-    const float err = k * (0x1p-47f * (spread + rest) + 0x1p-52f * (fabsf((float)t) + d0));
-    return {t, k < 100.0f && fabs(t) < 1e18 ? err : -1.0f};
-}
-
-struct RadarTable {
-    float4 v[kTable];  // cos, sin of 2 pi k / kTable, each as a pair
-};
-
 __global__ void __launch_bounds__(kThreads) backproject_kernel(const __grid_constant__ emlab_radar_geometry geo,
-                                                          const __grid_constant__ RadarTable tab, Turns wt, FF half_dt,
-                                                          FF inv_sdt, const __grid_constant__ Inputs in, double* power) {
+                                                          const __grid_constant__ RadarTable tab, Triple wt, Triple inv_sdt,
+                                                          const __grid_constant__ Inputs in, double* power) {
     __shared__ float4 table[kTable];
     __shared__ double terms[kThreads / 32][32][5];
     for (int k = threadIdx.x; k < kTable; k += kThreads) table[k] = tab.v[k];
@@ -260,40 +147,37 @@ __global__ void __launch_bounds__(kThreads) backproject_kernel(const __grid_cons
     double result = -1.0;
     bool again = false;
     if (inside) {
-        const Delay delay = tx_delay(g, P, table, wt, in);
-        const FF outbound = to_ff(delay.t) + half_dt;  // with the half step
-        const float err = fabsf(delay.err * inv_sdt.h);
+        const Delay delay = tx_delay(g.tx, g.ax2, P, table, wt, {in.tx_pos, in.tx_amp, in.ntx});
+        const Record rec = record_of(delay, geo.dt, geo.sample_dt, inv_sdt);
         FF sr = {0, 0}, si = sr;
         bool any = false;
-        float doubt = 0.0f;  // by how much roundings within the error could move the sum
-        const int n = delay.err < 0.0f ? 0 : in.C;
+        // by how much the roundings within the bounds could move the sum; and what the pairs' errors scale with: the
+        // magnitudes of the terms and of the running sums, the largest distance
+        float doubt = 0.0f, terms32 = 0.0f, sums = 0.0f, far = 0.0f;
+        const int n = delay.err < 0.0f || !in.pairs ? 0 : in.C;
         for (int i = 0; i < n; ++i) {
             const float d = len(sub(P, ld3(in.elem_pos + 3 * i)));  // path delay beyond the outbound one
-            const FF s = (outbound + d) * inv_sdt;                   // decimated sample
-            float m = floorf(s.h);
-            if (m == s.h && s.l < 0.0f) m -= 1.0f;
-            const float part = s.h - m, eps = err + 0x1p-47f * fabsf(s.h);
-            const float f = part + s.l, above = part + (s.l + eps), below = part + (s.l - eps);
-            if (above >= 1.0f || below < 0.0f || !(fabsf(s.h) < 1e9f) || !(fabsf(wt.h * d) < kTurns)) doubt = INFINITY;
-            if (!(m >= 0.0f && m < (float)(in.M - 1))) continue;
-            const int m0 = (int)m;
-            const float2 z0 = in.z[(long long)m0 * in.C + i], z1 = in.z[(long long)(m0 + 1) * in.C + i];
+            const Sample at = sample_at(rec, d);
+            if (!at.clear || !(fabsf(wt.h) * d < kTurns)) doubt = INFINITY;
+            if (at.m < 0 || at.m >= in.M - 1) continue;
+            const float f = at.f;
+            const float2 z0 = in.z[(long long)at.m * in.C + i], z1 = in.z[(long long)(at.m + 1) * in.C + i];
             const float vr = z0.x * (1.0f - f) + z1.x * f, vi = z0.y * (1.0f - f) + z1.y * f;
-            if (above != below) {
-                // a unit in the last place of f and of 1 - f, and the roundings that follow from it
-                const float a0 = sqrtf(z0.x * z0.x + z0.y * z0.y), a1 = sqrtf(z1.x * z1.x + z1.y * z1.y);
-                doubt += fabsf(in.weights[i].h) * (0x1p-23f * (a0 + a1));
-            }
+            if (at.above != at.below)  // the interpolated value's range, part by part
+                doubt += fabsf(in.weights[i].h) * (interpolation_range(z0.x, z1.x, at) + interpolation_range(z0.y, z1.y, at));
             const Phase q = phase(table, wt, d);
             const FF wr = in.weights[i] * vr, wi = in.weights[i] * vi;
             sr = sr + (wr * q.c + -(wi * q.s));
             si = si + (wr * q.s + wi * q.c);
             any |= vr != 0.0f || vi != 0.0f;
+            terms32 += fabsf(wr.h) + fabsf(wi.h), sums += fabsf(sr.h) + fabsf(si.h), far = fmaxf(far, d);
         }
         const double pr = to_f64(sr), pi = to_f64(si);
         result = pr * pr + pi * pi;
         const float top = fmaxf(fabsf(sr.h), fabsf(si.h));
-        again = delay.err < 0.0f || doubt > 1e-8f * top || (any && !in_range(top));
+        // a term: weight 3 u^2, phase 7, products 5, additions 3 each, as in tx_delay's; FP64's w t: 2^-53 of its radians
+        doubt += 0x1p-48f * (36.0f * terms32 + 3.0f * sums) + 0x1p-53f * 6.3f * (fabsf(wt.h) * far) * terms32;
+        again = delay.err < 0.0f || !in.pairs || !(doubt <= 1e-10f * top) || (any && !in_range(top));
     }
     const unsigned all = 0xffffffffu;
     for (unsigned todo = __ballot_sync(all, again); todo; todo &= todo - 1) {
@@ -344,15 +228,6 @@ extern "C" int emlab_radar_backproject(const emlab_radar_geometry* geo, const fl
     for (int j = 0; j < ntx; ++j) pairs[C + j] = to_ff(tx_amp[j]);
     std::memcpy(rest + 2 * nb, elem_pos, (size_t)C * 12);
     std::memcpy(rest + 2 * nb + (size_t)C * 12, tx_pos, (size_t)ntx * 12);
-    RadarTable table;
-    for (int k = 0; k < kTable; ++k) {
-        const double t = 6.28318530717958647692 * k / kTable;
-        const FF c = to_ff(std::cos(t)), s = to_ff(std::sin(t));
-        table.v[k] = make_float4(c.h, c.l, s.h, s.l);
-    }
-    const double turns = geo->omega / 6.28318530717958647692;
-    const FF w2 = to_ff(turns);
-    const Turns wt = {w2.h, w2.l, (float)(turns - (double)w2.h - (double)w2.l)};
     double* dp = reinterpret_cast<double*>(buf + bytes);
     cudaError_t e = cudaSuccess;
     if (!packed_z) e = cudaMemcpy(buf, z, zb, cudaMemcpyHostToDevice);
@@ -362,14 +237,39 @@ extern "C" int emlab_radar_backproject(const emlab_radar_geometry* geo, const fl
         const double* d64 = reinterpret_cast<const double*>(buf + zb);
         const FF* dff = reinterpret_cast<const FF*>(buf + zb + nb);
         const float* pos = reinterpret_cast<const float*>(buf + zb + 2 * nb);
-        const Inputs in = {reinterpret_cast<const float2*>(buf), M, C, ntx, pos, pos + 3 * (size_t)C, dff, dff + C, d64, d64 + C};
+        const Inputs in = {reinterpret_cast<const float2*>(buf), M, C, ntx, pos, pos + 3 * (size_t)C, dff, dff + C, d64, d64 + C,
+                           pairs_hold(weights, C)};
         backproject_kernel<<<(unsigned)((total + kThreads - 1) / kThreads), kThreads>>>(
-            *geo, table, wt, to_ff(0.5 * geo->dt), to_ff(1.0 / geo->sample_dt), in, dp);
+            *geo, make_table(), turns_of(geo->omega), quotient(1.0, geo->sample_dt, 0.0), in, dp);
         count_launches(1);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpy(power, dp, (size_t)total * 8, cudaMemcpyDeviceToHost);
     cudaFree(buf);
     if (e != cudaSuccess) return report_error(EMLAB_ERR_CUDA, cudaGetErrorString(e));
+    return EMLAB_OK;
+}
+
+extern "C" int emlab_debug_radar_delays(const emlab_radar_geometry* geo, const float* points, int n_points,
+                                        const float* elem_pos, int C, const float* tx_pos, const double* tx_amp, int ntx,
+                                        double* delays, double* samples) {
+    if (!geo || !points || !elem_pos || !tx_pos || !tx_amp || !delays || !samples || n_points < 0 || C < 1 || ntx < 1)
+        return report_error(EMLAB_ERR_INVALID, "bad radar delay arguments");
+    const RadarTable table = make_table();
+    const Triple wt = turns_of(geo->omega), inv = quotient(1.0, geo->sample_dt, 0.0);
+    const std::unique_ptr<FF[]> amp(new (std::nothrow) FF[ntx]);
+    if (!amp) return report_error(EMLAB_ERR_OOM, "radar: host allocation failed");
+    for (int j = 0; j < ntx; ++j) amp[j] = to_ff(tx_amp[j]);
+    for (int k = 0; k < n_points; ++k) {
+        const F3 p = ld3(points + 3 * (size_t)k);
+        const Delay delay = tx_delay(ld3(geo->tx), ld3(geo->axes + 6), p, table.v, wt, {tx_pos, amp.get(), ntx});
+        const Record rec = record_of(delay, geo->dt, geo->sample_dt, inv);
+        delays[2 * (size_t)k] = delay.t, delays[2 * (size_t)k + 1] = (double)delay.err;
+        for (int i = 0; i < C; ++i) {
+            const Sample at = sample_at(rec, len(sub(p, ld3(elem_pos + 3 * (size_t)i))));
+            double* o = samples + 5 * ((size_t)k * C + i);
+            o[0] = at.clear ? 1.0 : 0.0, o[1] = at.m, o[2] = at.f, o[3] = at.below, o[4] = at.above;
+        }
+    }
     return EMLAB_OK;
 }

@@ -340,7 +340,9 @@ typedef struct emlab_radar_geometry {
 } emlab_radar_geometry;
 /* power[(ir * nel + ie) * naz + ia] = |sum_i w_i z_i(t_i) e^{j omega t_i}|^2 (-1 outside the volume);
  * z: M decimated complex baseband samples of C elements ([m][i] as float pairs); elem_pos (C x 3),
- * weights (C); tx_pos (ntx x 3) and tx_amp (ntx): the transmitting elements. Host arrays. */
+ * weights (C); tx_pos (ntx x 3) and tx_amp (ntx): the transmitting elements. Host arrays. Positions and
+ * distances are FP32 as the reference's; the sums over the elements are pairs of FP32, formed again in FP64
+ * where it matters: every power is within 2e-10 of itself of the one that FP64 sums give. */
 int emlab_radar_backproject(const emlab_radar_geometry* geo, const float* z, int M, int C, const float* elem_pos,
                             const double* weights, const float* tx_pos, const double* tx_amp, int ntx,
                             double* power);
@@ -456,6 +458,12 @@ int emlab_source_lists(const emlab_source* sources, size_t n, int nx, int ny, in
  * waiting, with the full bound, for the copies it already issued); values above the default (about a
  * second of polling) are clamped to it. Restore with emlab_debug_set_wait_limit(1 << 20). */
 int emlab_debug_set_wait_limit(int polls);
+/* On the host, with the radar kernel's arithmetic, for n_points points (xyz each): delays[2 k] the transmit delay
+ * (RadarMonitor::txDelay) and delays[2 k + 1] the bound of its distance from the FP64 sums' (negative: the kernel
+ * forms the point in FP64); samples[5 (k C + i)] for element i: 1 where the sample index is certain, the
+ * index m, the FP32 interpolation weight f, and f rounded from either end of the interval that holds it. */
+int emlab_debug_radar_delays(const emlab_radar_geometry* geo, const float* points, int n_points, const float* elem_pos,
+                             int C, const float* tx_pos, const double* tx_amp, int ntx, double* delays, double* samples);
 /* Evaluates the device emlab_expf on n inputs (bit-exactness check against the host). */
 int emlab_debug_expf(const float* in, float* out, size_t n);
 /* Host-side schedule of the persistent pair kernel (no device needed), for `ctas` resident CTAs and
