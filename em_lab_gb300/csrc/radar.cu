@@ -56,11 +56,53 @@ struct Inputs {
     bool pairs;                              // the weights can be held as pairs
 };
 
-// The power at p in FP64 by one warp: the lanes form the terms of 32 elements, and one lane per sum adds
-// them in the order of the elements. terms: 32 x 5 doubles of this warp.
-__device__ __noinline__ double point64(const Geo& g, F3 p, const Inputs& in, double w, double dt, double sdt,
-                                       double (*terms)[5]) {
-    const int lane = threadIdx.x & 31;
+// The reference's sums at a point in FP64: the terms of a transmitting and of a receiving element, and the delay from
+// the former's sums.
+struct Point64 {
+    const Geo& g;
+    F3 p;
+    const Inputs& in;
+    double w, dt, sdt;
+
+    // RadarMonitor::txDelay (Radar.cpp:87-103)
+    __device__ void tx_term(int j, double (&t)[5]) const {
+        const F3 v = sub(p, ld3(in.tx_pos + 3 * j));
+        const double d = fmax((double)len(v), 0.5);
+        const double gj = fmax((double)dot(v, g.ax2) / d, 0.0);
+        const double a = in.tx_amp64[j] * gj / d;
+        double s, c;
+        sincos(-w * d, &s, &c);
+        t[0] = a * c, t[1] = a * s;
+        t[2] = d * t[0], t[3] = d * t[1];
+        t[4] = a;
+    }
+    __device__ double outbound(double ar, double ai, double adr, double adi, double mag) const {
+        const double absa = sqrt(ar * ar + ai * ai);
+        return absa < 1e-3 * mag ? (double)len(sub(p, g.tx)) : (adr * ar + adi * ai) / (ar * ar + ai * ai);  // real(ad / a)
+    }
+    __device__ void rx_term(int i, double outbound, double (&o)[2]) const {
+        o[0] = o[1] = 0.0;
+        const double t = outbound + (double)len(sub(p, ld3(in.elem_pos + 3 * i)));  // path delay
+        const double s = (t + 0.5 * dt) / sdt;                                       // decimated sample
+        if (s != s) o[0] = o[1] = s;
+        if (s >= 0.0 && s < (double)(in.M - 1)) {
+            const int m0 = (int)s;
+            const float f = (float)(s - (double)m0);
+            const float2 z0 = in.z[(long long)m0 * in.C + i], z1 = in.z[(long long)(m0 + 1) * in.C + i];
+            const float vr = z0.x * (1.0f - f) + z1.x * f, vi = z0.y * (1.0f - f) + z1.y * f;
+            double sn, cs;
+            sincos(w * t, &sn, &cs);
+            const double wr = in.weights64[i] * (double)vr, wi = in.weights64[i] * (double)vi;
+            o[0] = wr * cs - wi * sn;
+            o[1] = wr * sn + wi * cs;
+        }
+    }
+};
+
+// The power by one warp: the lanes form the terms of 32 elements, and one lane per sum adds them in the order of the
+// elements. terms: 32 x 5 doubles of this warp.
+__device__ __noinline__ double point_by_warp(const Point64& q, double (*terms)[5]) {
+    const int lane = threadIdx.x & 31, ntx = q.in.ntx, C = q.in.C;
     auto add_terms = [&](double acc, int sums, int n) {
         __syncwarp();
         if (lane < sums)
@@ -68,54 +110,44 @@ __device__ __noinline__ double point64(const Geo& g, F3 p, const Inputs& in, dou
         __syncwarp();
         return acc;
     };
-    // RadarMonitor::txDelay (Radar.cpp:87-103)
     double acc = 0.0;
-    for (int j0 = 0; j0 < in.ntx; j0 += 32) {
-        const int j = j0 + lane;
-        if (j < in.ntx) {
-            const F3 v = sub(p, ld3(in.tx_pos + 3 * j));
-            const double d = fmax((double)len(v), 0.5);
-            const double gj = fmax((double)dot(v, g.ax2) / d, 0.0);
-            const double a = in.tx_amp64[j] * gj / d;
-            double s, c;
-            sincos(-w * d, &s, &c);
-            const double tr = a * c, ti = a * s;
-            terms[lane][0] = tr, terms[lane][1] = ti;
-            terms[lane][2] = d * tr, terms[lane][3] = d * ti;
-            terms[lane][4] = a;
+    for (int j0 = 0; j0 < ntx; j0 += 32) {
+        if (j0 + lane < ntx) {
+            double t[5];
+            q.tx_term(j0 + lane, t);
+            for (int k = 0; k < 5; ++k) terms[lane][k] = t[k];
         }
-        acc = add_terms(acc, 5, min(32, in.ntx - j0));
+        acc = add_terms(acc, 5, min(32, ntx - j0));
     }
     const unsigned all = 0xffffffffu;
     const double ar = __shfl_sync(all, acc, 0), ai = __shfl_sync(all, acc, 1), adr = __shfl_sync(all, acc, 2),
                  adi = __shfl_sync(all, acc, 3), mag = __shfl_sync(all, acc, 4);
-    const double absa = sqrt(ar * ar + ai * ai);
-    const double outbound = absa < 1e-3 * mag ? (double)len(sub(p, g.tx))
-                                              : (adr * ar + adi * ai) / (ar * ar + ai * ai);  // real(ad / a)
+    const double outbound = q.outbound(ar, ai, adr, adi, mag);
     acc = 0.0;
-    for (int i0 = 0; i0 < in.C; i0 += 32) {
-        const int i = i0 + lane;
-        if (i < in.C) {
-            double tr = 0.0, ti = 0.0;
-            const double t = outbound + (double)len(sub(p, ld3(in.elem_pos + 3 * i)));  // path delay
-            const double s = (t + 0.5 * dt) / sdt;                                       // decimated sample
-            if (s != s) tr = ti = s;
-            if (s >= 0.0 && s < (double)(in.M - 1)) {
-                const int m0 = (int)s;
-                const float f = (float)(s - (double)m0);
-                const float2 z0 = in.z[(long long)m0 * in.C + i], z1 = in.z[(long long)(m0 + 1) * in.C + i];
-                const float vr = z0.x * (1.0f - f) + z1.x * f, vi = z0.y * (1.0f - f) + z1.y * f;
-                double sn, cs;
-                sincos(w * t, &sn, &cs);
-                const double wr = in.weights64[i] * (double)vr, wi = in.weights64[i] * (double)vi;
-                tr = wr * cs - wi * sn;
-                ti = wr * sn + wi * cs;
-            }
-            terms[lane][0] = tr, terms[lane][1] = ti;
+    for (int i0 = 0; i0 < C; i0 += 32) {
+        if (i0 + lane < C) {
+            double o[2];
+            q.rx_term(i0 + lane, outbound, o);
+            terms[lane][0] = o[0], terms[lane][1] = o[1];
         }
-        acc = add_terms(acc, 2, min(32, in.C - i0));
+        acc = add_terms(acc, 2, min(32, C - i0));
     }
     const double sr = __shfl_sync(all, acc, 0), si = __shfl_sync(all, acc, 1);
+    return sr * sr + si * si;
+}
+
+// The same by one lane.
+__device__ __noinline__ double point_by_lane(const Point64& q) {
+    double sum[5] = {}, t[5], sr = 0.0, si = 0.0, o[2];
+    for (int j = 0; j < q.in.ntx; ++j) {
+        q.tx_term(j, t);
+        for (int k = 0; k < 5; ++k) sum[k] += t[k];
+    }
+    const double outbound = q.outbound(sum[0], sum[1], sum[2], sum[3], sum[4]);
+    for (int i = 0; i < q.in.C; ++i) {
+        q.rx_term(i, outbound, o);
+        sr += o[0], si += o[1];
+    }
     return sr * sr + si * si;
 }
 
@@ -179,11 +211,20 @@ __global__ void __launch_bounds__(kThreads) backproject_kernel(const __grid_cons
         doubt += 0x1p-48f * (36.0f * terms32 + 3.0f * sums) + 0x1p-53f * 6.3f * (fabsf(wt.h) * far) * terms32;
         again = delay.err < 0.0f || !in.pairs || !(doubt <= 1e-10f * top) || (any && !in_range(top));
     }
+    // Few points of a warp are formed again by all its lanes together, one after the other: rounds of 32 terms for each.
+    // Where that is more rounds than the terms of one point, each lane takes its own (an array with an element at its
+    // centre and bins a whole number of samples away has rows of such points: 64 x 61 x 41 points and one element
+    // 314 us with FP64 sums, 459 with such points by the warp, 245 here).
     const unsigned all = 0xffffffffu;
-    for (unsigned todo = __ballot_sync(all, again); todo; todo &= todo - 1) {
+    unsigned todo = __ballot_sync(all, again);
+    if (__popc(todo) * ((in.ntx + 31) / 32 + (in.C + 31) / 32) > in.ntx + in.C) {
+        if (again) result = point_by_lane({g, P, in, geo.omega, geo.dt, geo.sample_dt});
+        todo = 0;
+    }
+    for (; todo; todo &= todo - 1) {
         const int lane = __ffs(todo) - 1;
         const F3 p = {__shfl_sync(all, P.x, lane), __shfl_sync(all, P.y, lane), __shfl_sync(all, P.z, lane)};
-        const double v = point64(g, p, in, geo.omega, geo.dt, geo.sample_dt, terms[threadIdx.x / 32]);
+        const double v = point_by_warp({g, p, in, geo.omega, geo.dt, geo.sample_dt}, terms[threadIdx.x / 32]);
         if ((threadIdx.x & 31) == lane) result = v;
     }
     if (idx < total) power[idx] = result;
