@@ -26,6 +26,8 @@ namespace {
 thread_local std::string g_last_error;
 std::atomic<uint64_t> g_launches{0};
 std::atomic<int> g_wait_polls{kWaitPolls};
+constexpr int kHostWaitMs = 60000;
+std::atomic<int> g_host_wait_ms{kHostWaitMs};
 
 }  // namespace
 
@@ -327,7 +329,7 @@ float blend_of(float avg, float wl, double dt) {
 // sleeps, the copies of the error word and the allocations of the read-backs).
 template <class Query>
 cudaError_t wait_until(Query&& query, int timeout_ms) {
-    const auto limit = std::chrono::milliseconds(timeout_ms > 0 ? timeout_ms : 60000);
+    const auto limit = std::chrono::milliseconds(timeout_ms > 0 ? timeout_ms : g_host_wait_ms.load());
     const auto t0 = std::chrono::steady_clock::now();
     for (;;) {
         const cudaError_t e = query();
@@ -339,11 +341,13 @@ cudaError_t wait_until(Query&& query, int timeout_ms) {
     }
 }
 
-// The grid's pinned scratch of at least `bytes` (at most kHostScratch), for one synchronous call; null where it
-// cannot be had.
-unsigned char* host_scratch(emlab_grid* g, size_t bytes) {
-    if (bytes > kHostScratch) return nullptr;
-    if (g->h_scratch_busy && cudaStreamSynchronize(g->stream) != cudaSuccess) return nullptr;  // left by a failed wait
+// The grid's pinned scratch of at least `bytes` (at most kHostScratch), for one synchronous call; *out is null where
+// it cannot be had. Scratch that a call left in use when its wait ran out is waited for, with the same limit.
+int host_scratch(emlab_grid* g, size_t bytes, unsigned char** out) {
+    *out = nullptr;
+    if (bytes > kHostScratch) return EMLAB_OK;
+    if (g->h_scratch_busy)
+        if (int rc = emlab_grid_synchronize(g, 0)) return rc;
     if (g->h_scratch_bytes < bytes) {
         const size_t want = std::max<size_t>(2 * bytes, 16 << 10);
         if (g->h_scratch) cudaFreeHost(g->h_scratch);
@@ -351,12 +355,13 @@ unsigned char* host_scratch(emlab_grid* g, size_t bytes) {
         if (cudaMallocHost(&g->h_scratch, std::min(want, kHostScratch)) != cudaSuccess) {
             cudaGetLastError();
             g->h_scratch = nullptr;
-            return nullptr;
+            return EMLAB_OK;
         }
         g->h_scratch_bytes = std::min(want, kHostScratch);
     }
     g->h_scratch_busy = true;
-    return g->h_scratch;
+    *out = g->h_scratch;
+    return EMLAB_OK;
 }
 
 int ensure_stage(emlab_grid* g, size_t bytes) {
@@ -1197,7 +1202,7 @@ int evaluate_pattern(emlab_grid* g, const int* box, int nf, const float* directi
     const PatternPlan plan = pattern_plan(box, nf, n_dirs);
     const size_t outs = (size_t)nf * n_dirs * 2;
     if (g->d_spec_dirs.n < (size_t)n_dirs || g->d_spec_part.n < plan.scratch || g->d_spec_out.n < outs)
-        EMLAB_CUDA(cudaStreamSynchronize(g->stream));
+        if (int rc = emlab_grid_synchronize(g, 0)) return rc;
     if (g->d_spec_dirs.n < (size_t)n_dirs) EMLAB_CUDA(g->d_spec_dirs.alloc((size_t)n_dirs));
     if (g->d_spec_part.n < plan.scratch) EMLAB_CUDA(g->d_spec_part.alloc(plan.scratch));
     if (g->d_spec_out.n < outs) EMLAB_CUDA(g->d_spec_out.alloc(outs));
@@ -1478,7 +1483,9 @@ int emlab_probe_gather(emlab_grid* g, const int* origins, int n_probes, float* o
     EMLAB_REQUIRE(origins && out && n_probes > 0, "bad probe arguments");
     EMLAB_CUDA(cudaSetDevice(g->device));
     const size_t in = (size_t)n_probes * 16, bytes = (size_t)n_probes * 54 * 16;
-    if (unsigned char* h = host_scratch(g, in + bytes)) {  // the kernel reads and writes host memory
+    unsigned char* h = nullptr;
+    if (int rc = host_scratch(g, in + bytes, &h)) return rc;
+    if (h) {  // the kernel reads and writes host memory
         std::memcpy(h, origins, in);
         launch_probe_gather(monitor_args(g), reinterpret_cast<int4*>(h), n_probes, reinterpret_cast<float4*>(h + in),
                             nullptr, nullptr, g->stream);
@@ -1556,7 +1563,9 @@ int emlab_flux_planes(emlab_grid* g, const emlab_flux_plane* planes, int n_plane
     }
     DevBuf<float> d_part;
     std::vector<float> h_part;
-    float* part = reinterpret_cast<float*>(host_scratch(g, std::max<size_t>(total, 1) * 4));
+    unsigned char* scratch = nullptr;
+    if (int rc = host_scratch(g, std::max<size_t>(total, 1) * 4, &scratch)) return rc;
+    float* part = reinterpret_cast<float*>(scratch);
     const bool direct = part != nullptr;  // the kernel writes host memory
     if (!direct) {
         EMLAB_CUDA(d_part.alloc(std::max<size_t>(total, 1)));
@@ -1762,6 +1771,12 @@ int emlab_source_lists(const emlab_source* sources, size_t n, int nx, int ny, in
 int emlab_debug_set_wait_limit(int polls) {
     EMLAB_REQUIRE(polls >= 0, "negative poll count");
     g_wait_polls = polls > 0 ? std::min(polls, kWaitPolls) : 0;
+    return EMLAB_OK;
+}
+
+int emlab_debug_set_host_wait(int ms) {
+    EMLAB_REQUIRE(ms >= 0, "negative wait");
+    g_host_wait_ms = ms > 0 ? std::min(ms, kHostWaitMs) : kHostWaitMs;
     return EMLAB_OK;
 }
 

@@ -499,7 +499,7 @@ extern "C" int emlab_ntff_dft_pattern_gemm(emlab_grid* g, int box, const float* 
     const int group = (int)std::clamp<size_t>((256ull << 20) / per_f, 1, (size_t)nf);
     const size_t scratch = (group * per_f) / 4 + (size_t)group * bx.parts, outs = (size_t)nf * D * 2;
     if (g->d_spec_dirs.n < (size_t)D || g->d_spec_part.n < scratch || g->d_spec_out.n < outs)
-        EMLAB_CUDA(cudaStreamSynchronize(g->stream));
+        if (int rc = emlab_grid_synchronize(g, 0)) return rc;
     if (g->d_spec_dirs.n < (size_t)D) EMLAB_CUDA(g->d_spec_dirs.alloc((size_t)D));
     if (g->d_spec_part.n < scratch) EMLAB_CUDA(g->d_spec_part.alloc(scratch));
     if (g->d_spec_out.n < outs) EMLAB_CUDA(g->d_spec_out.alloc(outs));

@@ -106,6 +106,7 @@ def load_library() -> C.CDLL:
         "emlab_lines_read": ([P, fp, fp], I),
         "emlab_debug_expf": ([fp, fp, SZ], I),
         "emlab_debug_set_wait_limit": ([I], I),
+        "emlab_debug_set_host_wait": ([I], I),
         "emlab_debug_pair_schedule": ([I, I, I, I, I, ip, ip], I),
         "emlab_debug_ragged_items": ([ip, ip, ip, ip, I, I, I, ip, SZ, C.POINTER(SZ)], I),
         "emlab_grid_set_cpml": ([P, C.POINTER(abi.Cpml)], I),
@@ -150,6 +151,11 @@ def debug_set_wait_limit(polls: int) -> None:
     """Test hook: polls of an on-device barrier wait before a kernel gives up and the grid reports
     EMLAB_ERR_TIMEOUT (0: the first wait of every launch gives up; WAIT_POLLS_DEFAULT restores)."""
     _check(load_library().emlab_debug_set_wait_limit(int(polls)))
+
+
+def debug_set_host_wait(ms: int) -> None:
+    """Test hook: the limit in milliseconds of the calls that wait for their own result (0: the usual 60 s)."""
+    _check(load_library().emlab_debug_set_host_wait(int(ms)))
 
 
 def pair_schedule(nx: int, ny: int, nz: int, tile_rows: int, ctas: int):

@@ -458,6 +458,9 @@ int emlab_source_lists(const emlab_source* sources, size_t n, int nx, int ny, in
  * waiting, with the full bound, for the copies it already issued); values above the default (about a
  * second of polling) are clamped to it. Restore with emlab_debug_set_wait_limit(1 << 20). */
 int emlab_debug_set_wait_limit(int polls);
+/* Test hook of the host-side waits: the limit in milliseconds of the calls that wait for their own result
+ * (probes, flux planes, patterns, reads) in this process; 0 restores the 60 s, more are clamped to them. */
+int emlab_debug_set_host_wait(int ms);
 /* On the host, with the radar kernel's arithmetic, for n_points points (xyz each): delays[2 k] the transmit delay
  * (RadarMonitor::txDelay) and delays[2 k + 1] the bound of its distance from the FP64 sums' (negative: the kernel
  * forms the point in FP64); samples[5 (k C + i)] for element i: 1 where the sample index is certain, the
