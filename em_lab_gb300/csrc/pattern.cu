@@ -157,11 +157,12 @@ __device__ __forceinline__ void strip_sums(const int* box, const float4* cur, in
     const int folded = (nv1 + 1) / 2;
     for (int iv0 = 0; iv0 < folded; iv0 += kRows) {
         const int iv = iv0 + rv, mirror = nv1 - 1 - iv;
+        const bool middle = mirror == iv;  // its own mirror: S its fields, D 0
         float4 j4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), m4 = j4, jm = j4, mm = j4;
         if (iu < nu1 && iv < folded) {
             const float4* p = cur + 2 * (size_t)(base + iv * nu1 + iu);
             j4 = __ldg(p), m4 = __ldg(p + 1);
-            if (mirror != iv) {  // the middle row is its own mirror: S its fields, D 0 (and the sine there 0)
+            if (!middle) {
                 p = cur + 2 * (size_t)(base + mirror * nu1 + iu);
                 jm = __ldg(p), mm = __ldg(p + 1);
             }
@@ -169,7 +170,7 @@ __device__ __forceinline__ void strip_sums(const int* box, const float4* cur, in
         float* row = sF[buf] + rv * kRowFloats + cu;
         auto put = [&](int q, float re, float im, float mre, float mim) {
             row[(4 * q + 0) * kStrip] = re + mre, row[(4 * q + 1) * kStrip] = im + mim;
-            row[(4 * q + 2) * kStrip] = re - mre, row[(4 * q + 3) * kStrip] = im - mim;
+            row[(4 * q + 2) * kStrip] = middle ? 0.0f : re - mre, row[(4 * q + 3) * kStrip] = middle ? 0.0f : im - mim;
         };
         put(0, j4.x, j4.y, jm.x, jm.y), put(1, j4.z, j4.w, jm.z, jm.w);
         put(2, m4.x, m4.y, mm.x, mm.y), put(3, m4.z, m4.w, mm.z, mm.w);
