@@ -1789,16 +1789,34 @@ int emlab_debug_pair_schedule(int nx, int ny, int nz, int tile_rows, int ctas, i
     return EMLAB_OK;
 }
 
+static bool pair_tile(int cols, int rows) {
+    return cols == 64 ? rows == 4 || rows == 8 || rows == 16 : cols == 32 && rows == 16;
+}
+
+int emlab_debug_pair_launch(int nx, int ny, int nz, int tile_cols, int tile_rows, int ctas, int* zc, int* items) {
+    EMLAB_REQUIRE(zc && items, "null output");
+    EMLAB_REQUIRE(nx > 0 && ny > 0 && nz > 0, "empty grid");
+    EMLAB_REQUIRE(pair_tile(tile_cols, tile_rows), "pair tiles have 64 x 4, 64 x 8, 64 x 16 or 32 x 16 cells");
+    EMLAB_REQUIRE(ctas > 0, "no CTAs");
+    pair_launch_shape(nx, ny, nz, tile_cols, tile_rows, ctas, zc, items);
+    return EMLAB_OK;
+}
+
 int emlab_debug_ragged_items(const int* z0, const int* nx, const int* ny, const int* nz, int n_scenes, int tile_rows,
                              int ctas, int* out, size_t cap, size_t* n_items) {
+    return emlab_debug_ragged_tiles(z0, nx, ny, nz, n_scenes, 64, tile_rows, ctas, out, cap, n_items);
+}
+
+int emlab_debug_ragged_tiles(const int* z0, const int* nx, const int* ny, const int* nz, int n_scenes, int tile_cols,
+                             int tile_rows, int ctas, int* out, size_t cap, size_t* n_items) {
     EMLAB_REQUIRE(z0 && nx && ny && nz && n_items && n_scenes > 0, "null argument or no scenes");
-    EMLAB_REQUIRE(tile_rows == 4 || tile_rows == 8 || tile_rows == 16, "pair tiles have 4, 8 or 16 rows");
+    EMLAB_REQUIRE(pair_tile(tile_cols, tile_rows), "pair tiles have 64 x 4, 64 x 8, 64 x 16 or 32 x 16 cells");
     EMLAB_REQUIRE(ctas > 0, "no CTAs");
     std::vector<int> vz0(z0, z0 + n_scenes), vnx(nx, nx + n_scenes), vny(ny, ny + n_scenes), vnz(nz, nz + n_scenes);
     for (int i = 0; i < n_scenes; ++i)
         EMLAB_REQUIRE(vnx[i] > 0 && vny[i] > 0 && vnz[i] > 0 && vnx[i] < 65536 && vny[i] < 65536 && vz0[i] >= 0,
                       "scene extents out of range");
-    const std::vector<int4> items = ragged_items(vz0, vnx, vny, vnz, tile_rows, ctas);
+    const std::vector<int4> items = ragged_items(vz0, vnx, vny, vnz, tile_rows, ctas, tile_cols);
     *n_items = items.size();
     if (!out) return EMLAB_OK;
     EMLAB_REQUIRE(cap >= items.size(), "output too small");

@@ -113,8 +113,10 @@ bool tma_maps_ready(const TmaMaps* m, int gen);
 // length for all scenes, chosen for g CTAs as the uniform schedule chooses it
 std::vector<int4> ragged_items(const std::vector<int>& z0, const std::vector<int>& nx, const std::vector<int>& ny,
                                const std::vector<int>& nz, int ty, int g, int xt = 64);
-// the uniform grid's pair-kernel schedule for g CTAs: planes per z chunk and work items
+// the uniform grid's pair-kernel schedule for g CTAs: planes per z chunk and work items; of 64 x ty tiles by the
+// rule for grids of at least four items per CTA, and of xt x ty tiles as launched (with the rule for smaller grids)
 void pair_schedule_shape(int nx, int ny, int nz, int ty, int g, int* zc, int* items);
+void pair_launch_shape(int nx, int ny, int nz, int xt, int ty, int g, int* zc, int* items);
 // Launches the TMA kernel reading generation `gen`; err receives a nonzero word if a wait timed out.
 bool launch_yee_tma(const YeeArgs& a, const TmaMaps* m, int gen, bool wide, unsigned* err, const Chain& s);
 void launch_yee_split(const YeeArgs& a, bool wide, const Chain& s);

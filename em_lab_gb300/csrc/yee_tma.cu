@@ -1063,6 +1063,13 @@ void small_grid_schedule(PairSched& ps, int nz, int G) {
     }
 }
 
+// What is launched on a single grid: the first rule, or the second where it leaves fewer than kItemsPerCta items per CTA.
+PairSched uniform_schedule(const YeeArgs& a, int xt, int rows, int G) {
+    PairSched ps = pair_schedule(a, xt, rows, G);
+    if (ps.items < kItemsPerCta * G) small_grid_schedule(ps, a.nz, G);
+    return ps;
+}
+
 template <int TY, int XL, typename Idx>
 bool launch_p(const YeeArgs& a, const TmaMaps* m, int gen, unsigned* err, const Chain& s) {
     using Lay = Layout2<TY, Idx, XL>;
@@ -1094,8 +1101,7 @@ bool launch_p(const YeeArgs& a, const TmaMaps* m, int gen, unsigned* err, const 
         ps.items = a.n_items;
         ps.tab = a.items;
     } else {
-        ps = pair_schedule(a, 2 * XL, Lay::ROWS, resident * sms);
-        if (ps.items < kItemsPerCta * resident * sms) small_grid_schedule(ps, a.nz, resident * sms);
+        ps = uniform_schedule(a, 2 * XL, Lay::ROWS, resident * sms);
         ps.tab = nullptr;
     }
     if (ps.items <= 0) return false;
@@ -1143,6 +1149,13 @@ void pair_schedule_shape(int nx, int ny, int nz, int ty, int g, int* zc, int* it
     YeeArgs a{};
     a.nx = nx, a.ny = ny, a.nz = nz;
     const PairSched ps = pair_schedule(a, 64, ty, g);
+    *zc = ps.zc, *items = ps.items;
+}
+
+void pair_launch_shape(int nx, int ny, int nz, int xt, int ty, int g, int* zc, int* items) {
+    YeeArgs a{};
+    a.nx = nx, a.ny = ny, a.nz = nz;
+    const PairSched ps = uniform_schedule(a, xt, ty, g);
     *zc = ps.zc, *items = ps.items;
 }
 

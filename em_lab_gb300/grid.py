@@ -108,7 +108,9 @@ def load_library() -> C.CDLL:
         "emlab_debug_set_wait_limit": ([I], I),
         "emlab_debug_set_host_wait": ([I], I),
         "emlab_debug_pair_schedule": ([I, I, I, I, I, ip, ip], I),
+        "emlab_debug_pair_launch": ([I, I, I, I, I, I, ip, ip], I),
         "emlab_debug_ragged_items": ([ip, ip, ip, ip, I, I, I, ip, SZ, C.POINTER(SZ)], I),
+        "emlab_debug_ragged_tiles": ([ip, ip, ip, ip, I, I, I, I, ip, SZ, C.POINTER(SZ)], I),
         "emlab_grid_set_cpml": ([P, C.POINTER(abi.Cpml)], I),
         "emlab_edge_materials": ([fp, fp, I, I, I, C.POINTER(abi.EdgeOverride), SZ, C.POINTER(abi.WireTerm), SZ,
                                   fp, fp, fp, fp, C.POINTER(C.c_uint32)], I),
@@ -159,24 +161,32 @@ def debug_set_host_wait(ms: int) -> None:
 
 
 def pair_schedule(nx: int, ny: int, nz: int, tile_rows: int, ctas: int):
-    """The persistent pair kernel's schedule on a single grid (host arithmetic): (planes per z chunk,
-    work items)."""
+    """The persistent pair kernel's schedule on a single grid of at least four work items per CTA (host
+    arithmetic): (planes per z chunk, work items) of 64-column tiles."""
     zc, items = C.c_int(), C.c_int()
     _check(load_library().emlab_debug_pair_schedule(int(nx), int(ny), int(nz), int(tile_rows), int(ctas),
                                                     C.byref(zc), C.byref(items)))
     return zc.value, items.value
 
 
-def ragged_items(z0, nx, ny, nz, tile_rows: int, ctas: int) -> np.ndarray:
+def pair_launch(nx: int, ny: int, nz: int, tile_cols: int, tile_rows: int, ctas: int):
+    """The schedule that is launched on a single grid, whatever its size: (planes per z chunk, work items)."""
+    zc, items = C.c_int(), C.c_int()
+    _check(load_library().emlab_debug_pair_launch(int(nx), int(ny), int(nz), int(tile_cols), int(tile_rows), int(ctas),
+                                                  C.byref(zc), C.byref(items)))
+    return zc.value, items.value
+
+
+def ragged_items(z0, nx, ny, nz, tile_rows: int, ctas: int, tile_cols: int = 64) -> np.ndarray:
     """The persistent pair kernel's work items on a stack of scenes with their own cross-sections
     (host arithmetic): (items, 5) int32 rows (x0, y0, first plane, end plane, scene)."""
     arrs = [np.ascontiguousarray(v, np.int32) for v in (z0, nx, ny, nz)]
     ptr = [a.ctypes.data_as(C.POINTER(C.c_int)) for a in arrs]
     lib, n = load_library(), C.c_size_t()
-    _check(lib.emlab_debug_ragged_items(*ptr, len(arrs[0]), int(tile_rows), int(ctas), None, 0, C.byref(n)))
+    head = (*ptr, len(arrs[0]), int(tile_cols), int(tile_rows), int(ctas))
+    _check(lib.emlab_debug_ragged_tiles(*head, None, 0, C.byref(n)))
     out = np.zeros((n.value, 5), np.int32)
-    _check(lib.emlab_debug_ragged_items(*ptr, len(arrs[0]), int(tile_rows), int(ctas),
-                                        out.ctypes.data_as(C.POINTER(C.c_int)), n.value, C.byref(n)))
+    _check(lib.emlab_debug_ragged_tiles(*head, out.ctypes.data_as(C.POINTER(C.c_int)), n.value, C.byref(n)))
     return out
 
 

@@ -469,15 +469,19 @@ int emlab_debug_radar_delays(const emlab_radar_geometry* geo, const float* point
                              int C, const float* tx_pos, const double* tx_amp, int ntx, double* delays, double* samples);
 /* Evaluates the device emlab_expf on n inputs (bit-exactness check against the host). */
 int emlab_debug_expf(const float* in, float* out, size_t n);
-/* Host-side schedule of the persistent pair kernel (no device needed), for `ctas` resident CTAs and
- * 64 x tile_rows tiles: on a single grid, the planes per z chunk and the number of work items (grids
- * that give fewer than four items per CTA are split further by a rule of their own at the launch);
- * on a stack of scenes with their own cross-sections (emlab_stack_configure_scenes), the work items
- * themselves, 5 ints each (x0, y0, first plane, end plane, scene) in launch order. *n_items receives
- * the count; out may be NULL to query it, else it holds cap items. */
+/* Host-side schedule of the persistent pair kernel (no device needed), for `ctas` resident CTAs: on a single
+ * grid, the planes per z chunk and the number of work items; on a stack of scenes with their own
+ * cross-sections (emlab_stack_configure_scenes), the work items themselves, 5 ints each (x0, y0, first
+ * plane, end plane, scene) in launch order. *n_items receives the count; out may be NULL to query it, else
+ * it holds cap items. Tiles of tile_cols x tile_rows cells (64 x 4, 64 x 8, 64 x 16 or 32 x 16; 64 columns without the
+ * argument). emlab_debug_pair_launch gives what is launched; emlab_debug_pair_schedule the rule for grids of at
+ * least four items per CTA, which smaller grids replace by one of their own. */
 int emlab_debug_pair_schedule(int nx, int ny, int nz, int tile_rows, int ctas, int* zc, int* items);
+int emlab_debug_pair_launch(int nx, int ny, int nz, int tile_cols, int tile_rows, int ctas, int* zc, int* items);
 int emlab_debug_ragged_items(const int* z0, const int* nx, const int* ny, const int* nz, int n_scenes, int tile_rows,
                              int ctas, int* out, size_t cap, size_t* n_items);
+int emlab_debug_ragged_tiles(const int* z0, const int* nx, const int* ny, const int* nz, int n_scenes, int tile_cols,
+                             int tile_rows, int ctas, int* out, size_t cap, size_t* n_items);
 
 #ifdef __cplusplus
 }
