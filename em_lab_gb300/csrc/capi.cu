@@ -33,6 +33,17 @@ std::atomic<int> g_host_wait_ms{kHostWaitMs};
 
 int emlab::wait_limit() { return g_wait_polls.load(); }
 
+int emlab::sm_count() {
+    constexpr int kDevices = 64;
+    static std::atomic<int> known[kDevices];  // a property of the device: asked for once
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) dev = 0;
+    if (dev < kDevices && (n = known[dev].load(std::memory_order_relaxed)) > 0) return n;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) return 1;
+    if (dev < kDevices) known[dev].store(n, std::memory_order_relaxed);
+    return n;
+}
+
 int emlab::fail(int code, const std::string& msg) {
     g_last_error = msg;
     return code;
@@ -72,7 +83,7 @@ YeeArgs yee_args(emlab_grid* g) {
     const int tx = (mode == 32 || mode == 64 || mode == 128) && g->kernel == EMLAB_KERNEL_FUSED ? 64 : 32;
     a.tile_rows = g->kernel == EMLAB_KERNEL_FUSED ? mode : ty;
     const long long xy = (long long)((a.nx + tx - 1) / tx) * ((a.ny + ty - 1) / ty);
-    const long long want = 152 * 4;
+    const long long want = 4 * sm_count();
     int chunks = (int)std::max<long long>(1, (want + xy - 1) / xy);
     int zc = (a.nz + chunks - 1) / chunks;
     zc = std::max(zc, std::min(8, a.nz));

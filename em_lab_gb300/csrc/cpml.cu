@@ -261,7 +261,7 @@ void launch_pass(const YeeArgs& a, const CpmlArgs& p, const Chain& s) {
     const dim3 tiles((a.nx + 2 * LX - 1) / (2 * LX), (a.ny + rows - 1) / rows);
     // Chunks re-read the plane neighbour of their first plane, and a launch wants its blocks (five to an SM) to
     // come out in several waves: the deepest chunk of at most eight planes with four waves, or single planes.
-    const int want = 4 * 5 * 152, least = (int)std::min<long long>(a.nz, (want + tiles.x * tiles.y - 1) / (tiles.x * tiles.y));
+    const int want = 4 * 5 * sm_count(), least = (int)std::min<long long>(a.nz, (want + tiles.x * tiles.y - 1) / (tiles.x * tiles.y));
     const int zc = std::max(1, std::min(8, a.nz / least));
     launch_chained(s, cpml_kernel<Idx, LX, kB>, dim3(tiles.x, tiles.y, (a.nz + zc - 1) / zc), kCpmlThreads, kStages * kStageBytes, a, p, zc);
 }

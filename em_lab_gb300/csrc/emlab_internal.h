@@ -80,6 +80,10 @@ struct YeeArgs {
 // out; the waits that drain copies already in flight before a CTA leaves always keep the default.
 constexpr int kWaitPolls = 1 << 20;
 int wait_limit();
+// multiprocessors of the current device, which the launch rules count their blocks by
+int sm_count();
+// multiprocessors of the current device
+int sm_count();
 
 struct SourceArgs {
     const int4* cells;       // xyz = cell (scene coordinates), w = first list entry; entry n is the sentinel

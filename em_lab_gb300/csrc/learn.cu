@@ -693,7 +693,7 @@ int gemm(int M, int N, int K, const void* A, long long sam, long long sak, const
     // three chunks in the ring so that two CTAs share an SM; below that narrow tiles and all six chunks
     const long long wide = (long long)((M + kTM - 1) / kTM) * ((N + 127) / 128);
     const cudaError_t err =
-        wide >= 2 * 152 ? launch_gemm_modes<128, 3>(M, N, K, a, sam, sak, b, sbn, sbk, e, NN_STREAM(stream))
+        wide >= 2 * sm_count() ? launch_gemm_modes<128, 3>(M, N, K, a, sam, sak, b, sbn, sbk, e, NN_STREAM(stream))
                         : launch_gemm_modes<64, kMaxStages>(M, N, K, a, sam, sak, b, sbn, sbk, e, NN_STREAM(stream));
     if (err != cudaSuccess) return report_error(EMLAB_ERR_CUDA, cudaGetErrorString(err));
     count_launches(1);

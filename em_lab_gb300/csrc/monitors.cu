@@ -520,7 +520,7 @@ void launch_port_residuals(const float* series, long long steps, int nports, dou
 }
 
 void launch_check_finite(const MonitorArgs& m, unsigned* flag, cudaStream_t s) {
-    finite_kernel<<<152 * 8, 256, 0, s>>>(m, flag);
+    finite_kernel<<<sm_count() * 8, 256, 0, s>>>(m, flag);
 }
 
 void launch_dft_sample(const MonitorArgs& m, const int* boxes, int nbox, int box_max, int points, float* blk, int t,

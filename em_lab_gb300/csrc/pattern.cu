@@ -362,10 +362,10 @@ PatternPlan pattern_plan(const int* box, int nf, int n_dirs) {
     for (int f = 0; f < 6; ++f) strips += face_strips(box, f);
     // frequencies whose currents (32 bytes a node) take 256 MB together
     p.freqs = (int)std::clamp<long long>((256ll << 20) / (32 * points), 1, nf);
-    // slices: just under four blocks for each of the 456 that the device holds, so that the last wave is
+    // slices: just under four blocks for each that the device holds (three to an SM), so that the last wave is
     // nearly full, but no more than there are strips, and 64 at most (the reduction reads all of them)
     const long long blocks = (long long)((n_dirs + kBlockDirs - 1) / kBlockDirs) * p.freqs;
-    p.slices = (int)std::max<long long>(1, std::min<long long>(std::min(strips, 64), 4 * 456 / blocks));
+    p.slices = (int)std::max<long long>(1, std::min<long long>(std::min(strips, 64), 4 * 3 * sm_count() / blocks));
     // directions per launch: all of them unless their partial sums would pass 256 MB
     const long long per_dir = 48ll * p.slices * p.freqs;
     p.chunk = (int)std::max<long long>(kBlockDirs, std::min<long long>(n_dirs, (256ll << 20) / per_dir / kBlockDirs * kBlockDirs));
