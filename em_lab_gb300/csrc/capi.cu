@@ -1145,6 +1145,12 @@ int emlab_ports_residuals(emlab_grid* g, double* out) {
 }
 
 // ---- far field -----------------------------------------------------------------------------
+// The scratch of the patterns goes back with the last far-field monitor (the stream is idle then).
+static void release_pattern_scratch(emlab_grid* g) {
+    if (g->ntff_on || g->dft_on) return;
+    g->d_spec_dirs.release(), g->d_spec_part.release(), g->d_spec_out.release();
+}
+
 int emlab_ntff_configure(emlab_grid* g, const int box_min[3], const int box_max[3], float wavelength,
                          float averaging_periods, int box_out[6]) {
     if (int rc = require_grid(g)) return rc;
@@ -1153,7 +1159,10 @@ int emlab_ntff_configure(emlab_grid* g, const int box_min[3], const int box_max[
     invalidate_graphs(g);
     g->ntff_on = false;
     g->d_ntff.release();
-    if (!(wavelength > 0.0f)) return EMLAB_OK;
+    if (!(wavelength > 0.0f)) {
+        release_pattern_scratch(g);
+        return EMLAB_OK;
+    }
     EMLAB_REQUIRE(box_min && box_max, "null box");
     const int n[3] = {g->cfg.nx, g->cfg.ny, g->cfg.nz};
     const int L = g->cfg.pml_thickness;
@@ -1328,7 +1337,10 @@ int emlab_ntff_dft_configure(emlab_grid* g, const int box_min[3], const int box_
                              int n_freq, int box_out[6]) {
     if (int rc = require_grid(g)) return rc;
     if (int rc = dft_detach(g)) return rc;
-    if (n_freq <= 0) return EMLAB_OK;
+    if (n_freq <= 0) {
+        release_pattern_scratch(g);
+        return EMLAB_OK;
+    }
     EMLAB_REQUIRE(box_min && box_max && wavelengths, "null DFT argument");
     EMLAB_REQUIRE(n_freq <= 128, "at most 128 DFT frequencies");
     const int n[3] = {g->cfg.nx, g->cfg.ny, g->cfg.nz};
@@ -1350,7 +1362,10 @@ int emlab_ntff_dft_configure_boxes(emlab_grid* g, const int* boxes, int n_boxes,
                                    int n_freq, int block) {
     if (int rc = require_grid(g)) return rc;
     if (int rc = dft_detach(g)) return rc;
-    if (n_freq <= 0 || n_boxes <= 0) return EMLAB_OK;
+    if (n_freq <= 0 || n_boxes <= 0) {
+        release_pattern_scratch(g);
+        return EMLAB_OK;
+    }
     EMLAB_REQUIRE(boxes && wavelengths, "null DFT argument");
     EMLAB_REQUIRE(n_freq <= 128, "at most 128 DFT frequencies");
     EMLAB_REQUIRE(n_boxes <= 65535, "too many far-field DFT boxes");

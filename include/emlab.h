@@ -253,7 +253,9 @@ int emlab_ntff_point_count(emlab_grid* g, int* points);
 /* PhasorPair per point (ntff_common.glsl:17-28): 32 floats each. */
 int emlab_ntff_read_phasors(emlab_grid* g, float* out);
 /* ntff_pattern.comp + ntff_reduce.comp (FarField.cpp:226-243, 294-335): for each direction
- * (4 floats, xyz used) out[2d] = |N_perp - r x L|^2 and out[1] = radiated power P. */
+ * (4 floats, xyz used) out[2d] = |N_perp - r x L|^2 and out[1] = radiated power P. The device scratch of this and
+ * the other pattern calls grows to the largest request (frequencies and directions are taken in groups of 256 MB of
+ * surface currents and of partial sums) and is kept until the grid's last far-field monitor is disabled. */
 int emlab_ntff_evaluate(emlab_grid* g, const float* directions, int n_dirs, float* out);
 
 /* Multi-frequency far-field DFT on a Huygens box (the reference's far-field monitor tracks one
