@@ -26,7 +26,8 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 if ROOT not in sys.path:
     sys.path.insert(0, ROOT)
 
-BYTES_PER_CELL_STEP = 60  # E and B read + write in FP32 (48 B) + six binary16 edge materials (12 B)
+FIELD_BYTES = 48  # E and B read + written in FP32, per cell-step; the pass also reads the cell's class index (2 or 4 B)
+MATERIAL_BYTES = 12  # the reference layout's six binary16 edge materials, which this pass does not read
 METRIC = "Yee Mcells/s (cell-steps per second, 1e6)"
 
 
@@ -639,7 +640,10 @@ def main():
     elapsed_ms = elapsed_s * 1e3
     peak, peak_kind = _peaks()
     per_launch_ms = kernel_ms / max(kernel_n, 1)
-    achieved = BYTES_PER_CELL_STEP * cells / (per_launch_ms * 1e-3) / 1e9
+    # what the pass cannot do without; and the same cell-steps at the reference layout's bytes (effective bandwidth)
+    bytes_per_cell = FIELD_BYTES + grid.class_bytes()
+    achieved = bytes_per_cell * cells / (per_launch_ms * 1e-3) / 1e9
+    effective = (FIELD_BYTES + MATERIAL_BYTES) * cells / (per_launch_ms * 1e-3) / 1e9
 
     # --- end-to-end leg through the C ABI with host buffers ------------------------------------
     # The headless frame loop of the reference (Main.cpp:1074-1099): each frame steps the grid
@@ -708,7 +712,7 @@ def main():
             "warmup": args.warmup, "ms_per_step": elapsed_ms / args.steps, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic",
             "config": {"workload": workload_text(args, sc, dft_points), "cells": int(cells), "kernel": args.kernel,
-                       "tiling": args.tile_rows or "auto (64x8 pair tiles)",
+                       "tiling": args.tile_rows or "auto (64x8 or 32x16 pair tiles, whichever covers fewer cells)",
                        "l2": (f"inputs larger than L2 ({state_gb:.1f} GB of field state per step)" if state_gb > 0.129
                               else f"field state {state_gb * 1e3:.0f} MB fits in L2 (129 MB); no flush between steps"),
                        "e2e_extra": "probe + 6-plane flux box read every 2 steps; " + (
@@ -718,10 +722,12 @@ def main():
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "traffic": traffic, "peak_source": peak_kind,
                          "traffic_source": ("DRAM bytes read + written per launch from one ncu capture of the "
-                                            "256^3 case, scaled by the cells a launch updates (profiles/traffic.txt); "
+                                            "256^3 case, scaled by the cells a launch updates, and 2 B a cell more "
+                                            "where the class index has 32 bits (profiles/traffic.txt); "
                                             "not measured in this run") if traffic else None,
                          "kernel": kname, "kernel_ms_per_launch": per_launch_ms,
-                         "algorithmic_bytes_per_cell_step": BYTES_PER_CELL_STEP},
+                         "algorithmic_bytes_per_cell_step": bytes_per_cell,
+                         "effective_at_60_bytes": effective},
             "cpu_baseline": cpu,
             "parity": (cpu or {}).get("parity"),
             "e2e": {"value": e2e_value, "unit": "Mcells/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,

@@ -868,6 +868,12 @@ int emlab_grid_get_state(const emlab_grid* g, emlab_grid_state* out) {
     return EMLAB_OK;
 }
 
+int emlab_grid_class_bytes(const emlab_grid* g, int* bytes) {
+    if (!g || !bytes) return fail(EMLAB_ERR_INVALID, "null argument");
+    *bytes = g->wide ? 4 : 2;
+    return EMLAB_OK;
+}
+
 static int read_comp(emlab_grid* g, int c, float* host, int stride, int offset) {
     const int nx = g->cfg.nx, ny = g->cfg.ny, nz = g->cfg.nz;
     std::vector<float> tmp((size_t)g->padded);

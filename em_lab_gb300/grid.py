@@ -54,6 +54,7 @@ def load_library() -> C.CDLL:
         "emlab_grid_step": ([P, I], I),
         "emlab_grid_synchronize": ([P, I], I),
         "emlab_grid_get_state": ([P, C.POINTER(abi.GridState)], I),
+        "emlab_grid_class_bytes": ([P, ip], I),
         "emlab_grid_read_fields": ([P, fp, fp], I),
         "emlab_grid_read_components": ([P, fp, fp, fp, fp, fp, fp], I),
         "emlab_grid_write_components": ([P, fp, fp, fp, fp, fp, fp], I),
@@ -335,6 +336,12 @@ class SimulationGrid:
 
     def gpu_memory_bytes(self) -> int:
         return int(self.state().device_bytes)
+
+    def class_bytes(self) -> int:
+        """Bytes of a cell's material class index in the solver pass: 2 or 4."""
+        n = C.c_int()
+        _check(self._lib.emlab_grid_class_bytes(self._h, C.byref(n)))
+        return n.value
 
     def set_kernel(self, kernel: int):
         _check(self._lib.emlab_grid_set_kernel(self._h, int(kernel)))

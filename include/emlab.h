@@ -149,6 +149,9 @@ int emlab_grid_step(emlab_grid* g, int count);
  * EMLAB_ERR_TIMEOUT if a solver kernel gave up a bounded on-device wait since the last call. */
 int emlab_grid_synchronize(emlab_grid* g, int timeout_ms);
 int emlab_grid_get_state(const emlab_grid* g, emlab_grid_state* out);
+/* Bytes of a cell's material class index, which the solver pass reads beside the fields: 2, or 4 where the uploaded
+ * materials make more than 65536 classes. */
+int emlab_grid_class_bytes(const emlab_grid* g, int* bytes);
 /* Read-back of the E and B textures in the reference's RGBA32F layout (E.a = cell sigma,
  * B.a = cell eps_r; src/SimulationGrid.hpp:4-6), 4 floats per cell. Either pointer may be NULL. */
 int emlab_grid_read_fields(emlab_grid* g, float* e_rgba, float* b_rgba);
